@@ -35,7 +35,7 @@
 // max_e |R5 - R7| / |R7| <= rtol or at the depth limit; otherwise it is halved
 // along the dimension with the larger summed fourth difference.
 //
-// k_adaptive_integral then sums mean * solid angle over the pixels inside the
+// k_mean_integral then sums mean * solid angle over the pixels inside the
 // boundary radius (FP64, fixed order), k_correction_sums forms the scales, and
 // k_scale_map64 writes value = mean * solid angle * exposure * correction.
 #include "xts_point.cuh"
@@ -104,36 +104,57 @@ static int upload_gm(cudaStream_t st) {
 // pixel's [-1, 1]^2 parameter square.
 struct QRegion { int sp; float c0, c1, h0, h1; };
 
+// Shared memory: the separation tables, then per warp the row windows of its 32
+// regions ([32][AW] float4 (w7, wd, d0, d1), one float4 of padding per region so that
+// lanes' 16-byte accesses fall in different banks) and the 17 points of the region
+// that the warp evaluates in FP64.
+constexpr int WSTRIDE = AW + 1;
+constexpr int NWARP = AT / 32;
+struct Point64 { double t; int idx; };
 constexpr size_t AO_SQ = 0;
 constexpr size_t AO_COEF = (8 * (ND + 1) + 15) / 16 * 16;
-constexpr size_t AO_WIN = AO_COEF + sizeof(float4) * 2 * ND;  // [4][AW][AT] floats
-constexpr size_t A_SMEM = AO_WIN + sizeof(float) * 4 * AW * AT;
+constexpr size_t AO_WIN = AO_COEF + sizeof(float4) * 2 * ND;
+constexpr size_t AO_P64 = AO_WIN + sizeof(float4) * NWARP * 32 * WSTRIDE;
+constexpr size_t A_SMEM = AO_P64 + sizeof(Point64) * NWARP * 17;
 
-__device__ __forceinline__ float4 f4fma(float a, const float4& y, const float4& c) {
-    return make_float4(fmaf(a, y.x, c.x), fmaf(a, y.y, c.y), fmaf(a, y.z, c.z), fmaf(a, y.w, c.w));
-}
-__device__ __forceinline__ float f4c(const float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
+// One region of a warp's batch, as its lane holds it.
+struct LaneRegion {
+    int sp, s, h, w;  // source * npix + pixel, source, map row and column
+    float c0, c1, h0, h1;
+};
 
-// The region again in FP64, point by point, with the reference design's arithmetic
-// (math/genz_malik.hxx:127-195 as restated by the oracle): the rule points blended
+// What the levels share.
+struct LevelArgs {
+    const double* corners; const SrcInfo* info; const float* lut; const double* upsf;
+    int H, W, E, EP;
+    float rtol;
+    double* mean;
+};
+
+__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// A region again in FP64 by the whole warp, with the reference design's arithmetic
+// (math/genz_malik.hxx:127-195 as restated by the oracle): lane p blends rule point p
 // from the pixel's corner vectors, s = 2 asin(|p - src| / 2), the logsep row and
-// weight, f = (1 - t) U[i - 1] + t U[i], R7 and R5 summed over the points in order,
-// no fused multiply-adds.  Decides the region and, when it is accepted, adds (or,
-// at level 0, stores) area * R7 into mean[e]; otherwise sets *dim.
-__device__ __noinline__ bool gm_region64(const double* __restrict__ corners, int W1, int h, int w, const double* src,
-                                         double c0, double c1, double h0, double h1, bool last,
-                                         const double* __restrict__ U, int E, double rtol, double* mean, bool atomic,
+// weight; then lane = energy: f = (1 - t) U[i - 1] + t U[i], R7 and R5 summed over the
+// points in order, the fourth differences summed over the energies in order, no fused
+// multiply-adds.  Returns true when the region is accepted, after adding (at level 0:
+// storing) area * R7 into its mean; otherwise sets *dim (at level 0 the mean is
+// cleared).  All arguments are warp-uniform.
+__device__ __noinline__ bool gm_region64(const LevelArgs& A, const LaneRegion& R, Point64* pts, bool last, bool level0,
                                          int* dim) {
-    const double* a = corners + 3 * ((size_t)h * W1 + w);            // LL
-    const double* b = corners + 3 * ((size_t)h * W1 + w + 1);        // LR
-    const double* c = corners + 3 * ((size_t)(h + 1) * W1 + w + 1);  // UR
-    const double* d = corners + 3 * ((size_t)(h + 1) * W1 + w);      // UL
-    int ix[17];
-    double tt[17];
-    for (int p = 0; p < 17; ++p) {
-        const double x1 = __dadd_rn(c1, __dmul_rn(c_gm64.off1[p], h1));
-        const double x0 = __dadd_rn(c0, __dmul_rn(c_gm64.off0[p], h0));
-        const double u = x1, v = x0;
+    const int lane = threadIdx.x & 31, W1 = A.W + 1, E = A.E;
+    const double* U = A.upsf + (size_t)R.s * ND * E;
+    double* mean = A.mean + (size_t)R.sp * E;
+    __syncwarp();
+    if (lane < 17) {
+        const double* a = A.corners + 3 * ((size_t)R.h * W1 + R.w);            // LL
+        const double* b = A.corners + 3 * ((size_t)R.h * W1 + R.w + 1);        // LR
+        const double* c = A.corners + 3 * ((size_t)(R.h + 1) * W1 + R.w + 1);  // UR
+        const double* d = A.corners + 3 * ((size_t)(R.h + 1) * W1 + R.w);      // UL
+        const double* src = A.info[R.s].dir;
+        const double u = __dadd_rn(R.c1, __dmul_rn(c_gm64.off1[lane], R.h1));
+        const double v = __dadd_rn(R.c0, __dmul_rn(c_gm64.off0[lane], R.h0));
         const double nn = __dmul_rn(__dsub_rn(1.0, u), __dsub_rn(1.0, v));
         const double pn = __dmul_rn(__dadd_rn(1.0, u), __dsub_rn(1.0, v));
         const double pp = __dmul_rn(__dadd_rn(1.0, u), __dadd_rn(1.0, v));
@@ -149,214 +170,237 @@ __device__ __noinline__ bool gm_region64(const double* __restrict__ corners, int
         const double j = sd < 1e-4 ? 1. : __dadd_rn(1., __dmul_rn(RECIPSTEP, __dadd_rn(LN_1E4, log(sd))));
         int idx = 1 + (int)(unsigned short)j;
         idx = idx > 400 ? 400 : idx;
-        ix[p] = idx;
-        tt[p] = __dmul_rn(REDM1, __dsub_rn(__dmul_rn(__dmul_rn(sd, 1e4), exp(__dmul_rn(SEP_STEP, 2. - idx))), 1.));
+        pts[lane].idx = idx;
+        pts[lane].t = __dmul_rn(REDM1, __dsub_rn(__dmul_rn(__dmul_rn(sd, 1e4), exp(__dmul_rn(SEP_STEP, 2. - idx))), 1.));
     }
-    double rel = 0., dd0 = 0., dd1 = 0.;
-    const double area = __dmul_rn(h0, h1);
-    for (int e = 0; e < E; ++e) {
-        double v7 = 0., v5 = 0., f[9];
-        for (int p = 0; p < 17; ++p) {
-            const double fv = __dadd_rn(__dmul_rn(__dsub_rn(1.0, tt[p]), U[(size_t)(ix[p] - 1) * E + e]),
-                                        __dmul_rn(tt[p], U[(size_t)ix[p] * E + e]));
-            if (p < 9) f[p] = fv;
-            v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], fv));
-            v5 = __dadd_rn(v5, __dmul_rn(c_gm64.w5[p], fv));
-        }
-        const double err = fabs(__dsub_rn(v5, v7));
-        const double r = v7 != 0. ? err / fabs(v7) : (err != 0. ? INFINITY : 0.);
-        rel = r > rel ? r : rel;
-        const double f0 = __dmul_rn(2., f[0]);
-        dd0 = __dadd_rn(dd0, fabs(__dsub_rn(__dsub_rn(__dadd_rn(f[1], f[3]), f0),
-                                            __dmul_rn(1. / 7., __dsub_rn(__dadd_rn(f[5], f[7]), f0)))));
-        dd1 = __dadd_rn(dd1, fabs(__dsub_rn(__dsub_rn(__dadd_rn(f[2], f[4]), f0),
-                                            __dmul_rn(1. / 7., __dsub_rn(__dadd_rn(f[6], f[8]), f0)))));
-    }
-    if (!(rel <= rtol || last)) {
-        *dim = dd0 >= dd1 ? 0 : 1;
-        return false;
-    }
-    for (int e = 0; e < E; ++e) {
-        double v7 = 0.;
-        for (int p = 0; p < 17; ++p) {
-            const double fv = __dadd_rn(__dmul_rn(__dsub_rn(1.0, tt[p]), U[(size_t)(ix[p] - 1) * E + e]),
-                                        __dmul_rn(tt[p], U[(size_t)ix[p] * E + e]));
-            v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], fv));
-        }
-        if (atomic) atomicAdd(mean + e, __dmul_rn(area, v7));
-        else mean[e] = __dmul_rn(area, v7);
-    }
-    return true;
-}
-
-// Evaluates one region.  Returns true when it is accepted, after adding
-// area * R7 into mean[e] (FP64; atomically when `atomic`, else stored: level 0,
-// one region per pixel); otherwise sets *dim.  Y is the source's FP32 mean-PSF
-// table with rows of EP = E rounded up to 4 floats (zeros past E), read four
-// energies at a time, U the source's FP64 table for decisions near the threshold
-// (gm_region64).  The values are added during the acceptance check, so an
-// accepted region (most of them) is evaluated once; a split region's values are
-// taken back out (FP64 atomics; at level 0, cleared).
-__device__ __noinline__ bool gm_region(const PixGeom& g, float c0, float c1, float h0, float h1, bool last,
-                                       const double* sq, const float4* scoef, float* wk, const float* Y,
-                                       const double* U, const double* corners, int W1, int h, int w,
-                                       const double* src, int E, int EP, float rtol, double* mean, bool atomic,
-                                       int* dim) {
-    int ix[17];
-    float tt[17];
-    int rmin = ND, rmax = 0;
-#pragma unroll
-    for (int p = 0; p < 17; ++p) {
-        const double u = c1 + c_gm.off1[p] * h1;  // along w
-        const double v = c0 + c_gm.off0[p] * h0;  // along h
-        const double x = fma(g.Dx, u * v, fma(g.Cx, v, fma(g.Bx, u, g.Ax)));
-        const double y = fma(g.Dy, u * v, fma(g.Cy, v, fma(g.By, u, g.Ay)));
-        const double z = fma(g.Dz, u * v, fma(g.Cz, v, fma(g.Bz, u, g.Az)));
-        ix[p] = point_row(fma(x, x, fma(y, y, z * z)), sq, scoef, &tt[p]);
-        rmin = min(rmin, ix[p] - 1);
-        rmax = max(rmax, ix[p]);
-    }
-    const float area = h0 * h1;  // fraction of the pixel
-    const int nr = rmax - rmin + 1;
-    const bool windowed = nr <= AW;
-    float w7[AW], wd[AW], e0[AW], e1[AW];
-    if (windowed) {  // the four row windows of this region
-#pragma unroll
-        for (int j = 0; j < 4 * AW; ++j) wk[j * AT] = 0.f;
-#pragma unroll
-        for (int p = 0; p < 17; ++p) {
-            const int r = ix[p] - 1 - rmin;
-            const float a = 1.f - tt[p], b = tt[p];
-            wk[(0 * AW + r) * AT] += a * c_gm.w7[p];
-            wk[(0 * AW + r + 1) * AT] += b * c_gm.w7[p];
-            wk[(1 * AW + r) * AT] += a * c_gm.wd[p];
-            wk[(1 * AW + r + 1) * AT] += b * c_gm.wd[p];
-            wk[(2 * AW + r) * AT] += a * c_gm.d0[p];
-            wk[(2 * AW + r + 1) * AT] += b * c_gm.d0[p];
-            wk[(3 * AW + r) * AT] += a * c_gm.d1[p];
-            wk[(3 * AW + r + 1) * AT] += b * c_gm.d1[p];
-        }
-#pragma unroll
-        for (int j = 0; j < AW; ++j) {
-            w7[j] = wk[(0 * AW + j) * AT];
-            wd[j] = wk[(1 * AW + j) * AT];
-            e0[j] = wk[(2 * AW + j) * AT];
-            e1[j] = wk[(3 * AW + j) * AT];
-        }
-    }
-    const float* y0 = Y + (size_t)rmin * EP;
-    const int EQ4 = EP >> 2;
-    // R7, R5 - R7 and the two fourth differences at energies 4qd .. 4qd + 3: from
-    // the windows, or point by point when the rows are too far apart
-    auto rule = [&](int qd, float4& v7, float4& vd, float4& a0, float4& a1) {
-        v7 = vd = a0 = a1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (windowed) {
-#pragma unroll
-            for (int j = 0; j < AW; ++j) {
-                if (j < nr) {
-                    const float4 yv = __ldg((const float4*)(y0 + (size_t)j * EP) + qd);
-                    v7 = f4fma(w7[j], yv, v7);
-                    vd = f4fma(wd[j], yv, vd);
-                    a0 = f4fma(e0[j], yv, a0);
-                    a1 = f4fma(e1[j], yv, a1);
-                }
-            }
-        } else {
-            for (int p = 0; p < 17; ++p) {
-                const float4* yl = (const float4*)(Y + (size_t)(ix[p] - 1) * EP) + qd;
-                const float4 lo = __ldg(yl), hi = __ldg(yl + EQ4);
-                const float4 f = make_float4(fmaf(tt[p], hi.x - lo.x, lo.x), fmaf(tt[p], hi.y - lo.y, lo.y),
-                                             fmaf(tt[p], hi.z - lo.z, lo.z), fmaf(tt[p], hi.w - lo.w, lo.w));
-                v7 = f4fma(c_gm.w7[p], f, v7);
-                vd = f4fma(c_gm.wd[p], f, vd);
-                a0 = f4fma(c_gm.d0[p], f, a0);
-                a1 = f4fma(c_gm.d1[p], f, a1);
-            }
-        }
+    __syncwarp();
+    auto value = [&](int p, int e) {
+        const int i = pts[p].idx;
+        const double t = pts[p].t;
+        return __dadd_rn(__dmul_rn(__dsub_rn(1.0, t), U[(size_t)(i - 1) * E + e]), __dmul_rn(t, U[(size_t)i * E + e]));
     };
-    float rel = 0.f, dd0 = 0.f, dd1 = 0.f, sx7 = 0.f;
+    double rel = 0., dd0 = 0., dd1 = 0.;
     if (!last) {
-        for (int qd = 0; qd < EQ4; ++qd) {
-            float4 v7, vd, a0, a1;
-            rule(qd, v7, vd, a0, a1);
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            double g0 = 0., g1 = 0.;
+            if (e < E) {
+                double v7 = 0., v5 = 0., f[9];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int e = 4 * qd + c;
-                if (e < E) {
-                    const float x7 = f4c(v7, c), xd = f4c(vd, c);
-                    const float r = fabsf(xd) <= rtol * fabsf(x7) ? fabsf(xd) / fmaxf(fabsf(x7), 1e-38f)
-                                                                 : (x7 != 0.f ? fabsf(xd) / fabsf(x7) : 3.4e38f);
-                    rel = fmaxf(rel, r);
-                    dd0 += fabsf(f4c(a0, c));
-                    dd1 += fabsf(f4c(a1, c));
-                    sx7 += fabsf(x7);
-                    // added now, so an accepted region needs no second pass; a split
-                    // region is taken back out below
-                    if (atomic) atomicAdd(mean + e, (double)(area * x7));
-                    else mean[e] = (double)(area * x7);
+                for (int p = 0; p < 17; ++p) {
+                    const double fv = value(p, e);
+                    if (p < 9) f[p] = fv;
+                    v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], fv));
+                    v5 = __dadd_rn(v5, __dmul_rn(c_gm64.w5[p], fv));
                 }
+                const double err = fabs(__dsub_rn(v5, v7));
+                const double r = v7 != 0. ? err / fabs(v7) : (err != 0. ? INFINITY : 0.);
+                rel = r > rel ? r : rel;
+                const double f0 = __dmul_rn(2., f[0]);
+                g0 = fabs(__dsub_rn(__dsub_rn(__dadd_rn(f[1], f[3]), f0),
+                                    __dmul_rn(1. / 7., __dsub_rn(__dadd_rn(f[5], f[7]), f0))));
+                g1 = fabs(__dsub_rn(__dsub_rn(__dadd_rn(f[2], f[4]), f0),
+                                    __dmul_rn(1. / 7., __dsub_rn(__dadd_rn(f[6], f[8]), f0))));
+            }
+            const int n = min(32, E - e0);
+            for (int k = 0; k < n; ++k) {
+                dd0 = __dadd_rn(dd0, shfl_d(g0, k));
+                dd1 = __dadd_rn(dd1, shfl_d(g1, k));
             }
         }
-        // the FP32 estimate's decision, unless it is too close to call
-        const bool near_tol = fabsf(rel - rtol) <= fmaxf(0.05f * rtol, 4e-6f);
-        const bool accept = rel <= rtol;
-        if (accept && !near_tol) return true;
-        // the fourth differences cancel most of the values they are formed from, so
-        // their FP32 error is measured against the values (sx7), not against themselves
-        const bool near_dim = !accept && fabsf(dd0 - dd1) <= 1e-3f * (dd0 + dd1) + 4e-6f * sx7;
-        for (int qd = 0; qd < EQ4; ++qd) {  // take the FP32 values back out
-            float4 v7, vd, a0, a1;
-            rule(qd, v7, vd, a0, a1);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int e = 4 * qd + c;
-                if (e < E) {
-                    if (atomic) atomicAdd(mean + e, -(double)(area * f4c(v7, c)));
-                    else mean[e] = 0.;
-                }
-            }
-        }
-        if (near_tol || near_dim)
-            return gm_region64(corners, W1, h, w, src, c0, c1, h0, h1, false, U, E, (double)rtol, mean, atomic, dim);
-        *dim = dd0 >= dd1 ? 0 : 1;
-        return false;
+        for (int o = 16; o > 0; o >>= 1) rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, o));
     }
-    {  // the depth limit: accepted without a check
-        for (int qd = 0; qd < EQ4; ++qd) {
-            float4 v7, vd, a0, a1;
-            rule(qd, v7, vd, a0, a1);
+    const bool accept = last || rel <= (double)A.rtol;
+    *dim = dd0 >= dd1 ? 0 : 1;
+    const double area = __dmul_rn(R.h0, R.h1);
+    for (int e = lane; e < E; e += 32) {
+        double v = 0.;
+        if (accept) {
+            double v7 = 0.;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int e = 4 * qd + c;
-                if (e < E) {
-                    if (atomic) atomicAdd(mean + e, (double)(area * f4c(v7, c)));
-                    else mean[e] = (double)(area * f4c(v7, c));
-                }
-            }
+            for (int p = 0; p < 17; ++p) v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], value(p, e)));
+            v = __dmul_rn(area, v7);
         }
-        return true;
+        if (level0) mean[e] = v;
+        else if (accept) atomicAdd(mean + e, v);
     }
+    return accept;
 }
 
-// Pushes the two halves of a region (lower half first in the queue), or returns
-// false when the queue is full.
-__device__ __forceinline__ bool push_halves(QRegion* q, int* qcount, int qcap, int sp, float c0, float c1,
-                                            float h0, float h1, int dim) {
-    const int k = atomicAdd(qcount, 2);
-    if (k + 2 > qcap) return false;
-    QRegion a {sp, c0, c1, h0, h1}, b = a;
+// The two halves of a region (lower half first) at q[k], q[k + 1].
+__device__ __forceinline__ void store_halves(QRegion* q, int k, const LaneRegion& R, int dim) {
+    QRegion a{R.sp, R.c0, R.c1, R.h0, R.h1}, b = a;
     if (dim == 0) {
-        a.h0 = b.h0 = 0.5f * h0;
-        a.c0 = c0 - 0.5f * h0;
-        b.c0 = c0 + 0.5f * h0;
+        a.h0 = b.h0 = 0.5f * R.h0;
+        a.c0 = R.c0 - 0.5f * R.h0;
+        b.c0 = R.c0 + 0.5f * R.h0;
     } else {
-        a.h1 = b.h1 = 0.5f * h1;
-        a.c1 = c1 - 0.5f * h1;
-        b.c1 = c1 + 0.5f * h1;
+        a.h1 = b.h1 = 0.5f * R.h1;
+        a.c1 = R.c1 - 0.5f * R.h1;
+        b.c1 = R.c1 + 0.5f * R.h1;
     }
     q[k] = a;
     q[k + 1] = b;
-    return true;
+}
+
+enum { GM_ACCEPT = 0, GM_SPLIT0 = 1, GM_SPLIT1 = 2, GM_FP64 = 3, GM_NONE = 4 };
+
+// The windowed regions of `mask` (lane = region): G lanes per region, lane q of the
+// group the energies q, q + G, ... (table rows and means are read and written in runs
+// of G consecutive values).  Returns each lane's decision for its own region; accepted
+// regions' values are added to (at level 0 stored in) their means, and at level 0 the
+// means of the others are cleared.
+template <int G>
+__device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R, const float4* win, int rmin, int nr,
+                                         unsigned mask, bool last, bool level0) {
+    constexpr int NS = G == 32 ? 8 : 4;  // energies per lane: E <= G * NS
+    const int lane = threadIdx.x & 31, q = lane & (G - 1), E = A.E;
+    int mine = GM_NONE;
+    for (int r0 = 0; r0 < 32; r0 += 32 / G) {
+        if (!((mask >> r0) & ((1u << (32 / G)) - 1))) continue;  // warp-uniform
+        const int rg = r0 + lane / G;
+        const bool on = (mask >> rg) & 1;
+        const int row = __shfl_sync(0xffffffffu, rmin, rg), nrow = __shfl_sync(0xffffffffu, nr, rg);
+        const int n = on ? nrow : 0;
+        const int sp = __shfl_sync(0xffffffffu, R.sp, rg), s = __shfl_sync(0xffffffffu, R.s, rg);
+        const float area = __shfl_sync(0xffffffffu, R.h0, rg) * __shfl_sync(0xffffffffu, R.h1, rg);
+        float v7[NS], vd[NS], a0[NS], a1[NS];
+#pragma unroll
+        for (int c = 0; c < NS; ++c) v7[c] = vd[c] = a0[c] = a1[c] = 0.f;
+        const float* y = A.lut + ((size_t)s * ND + row) * A.EP + q;
+        const float4* wr = win + rg * WSTRIDE;
+        for (int j = 0; j < n; ++j, y += A.EP) {
+            const float4 w = wr[j];
+#pragma unroll
+            for (int c = 0; c < NS; ++c)
+                if (G * c < E) {
+                    const float f = q + G * c < E ? __ldg(y + G * c) : 0.f;
+                    v7[c] = fmaf(w.x, f, v7[c]);
+                    vd[c] = fmaf(w.y, f, vd[c]);
+                    a0[c] = fmaf(w.z, f, a0[c]);
+                    a1[c] = fmaf(w.w, f, a1[c]);
+                }
+        }
+        int code = GM_ACCEPT;
+        if (!last) {
+            float rel = 0.f, dd0 = 0.f, dd1 = 0.f, sx = 0.f;
+#pragma unroll
+            for (int c = 0; c < NS; ++c) {
+                const float x7 = fabsf(v7[c]), xd = fabsf(vd[c]);
+                // 0 / 0 (an all-zero energy, or a lane past E) counts as no error
+                rel = fmaxf(rel, xd == 0.f ? 0.f : (x7 != 0.f ? xd / x7 : 3.4e38f));
+                dd0 += fabsf(a0[c]);
+                dd1 += fabsf(a1[c]);
+                sx += x7;
+            }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+                rel = fmaxf(rel, __shfl_xor_sync(0xffffffffu, rel, o));
+                dd0 += __shfl_xor_sync(0xffffffffu, dd0, o);
+                dd1 += __shfl_xor_sync(0xffffffffu, dd1, o);
+                sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            }
+            const float rtol = A.rtol;
+            const bool accept = rel <= rtol;
+            // the fourth differences cancel most of the values they are formed from, so
+            // their FP32 error is measured against the values (sx), not against themselves
+            const bool near_dim = !accept && fabsf(dd0 - dd1) <= 1e-3f * (dd0 + dd1) + 4e-6f * sx;
+            if (fabsf(rel - rtol) <= fmaxf(0.05f * rtol, 4e-6f) || near_dim) code = GM_FP64;
+            else if (!accept) code = dd0 >= dd1 ? GM_SPLIT0 : GM_SPLIT1;
+        }
+        if (on && (code == GM_ACCEPT || (level0 && code != GM_FP64))) {
+            double* m = A.mean + (size_t)sp * E + q;
+#pragma unroll
+            for (int c = 0; c < NS; ++c)
+                if (q + G * c < E) {
+                    const double v = code == GM_ACCEPT ? (double)(area * v7[c]) : 0.;
+                    if (level0) m[G * c] = v;
+                    else atomicAdd(m + G * c, v);
+                }
+        }
+        const int got = __shfl_sync(0xffffffffu, code, ((lane - r0) & (32 / G - 1)) * G);
+        if (lane >= r0 && lane < r0 + 32 / G && ((mask >> lane) & 1)) mine = got;
+    }
+    return mine;
+}
+
+// One batch of up to 32 regions (lane = region, `on` marks the lanes that hold one).
+template <int G>
+__device__ __forceinline__ void gm_batch(const LevelArgs& A, const LaneRegion& R, bool on, const double* sq,
+                                         const float4* scoef, float4* win, Point64* pts, bool last, bool level0,
+                                         QRegion* qout, int* qcount, int qcap) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int rmin = 0, nr = 0;
+    if (on) {
+        const PixGeom g = pixel_geom(A.corners, A.W + 1, R.h, R.w, A.info[R.s]);
+        int ix[17];
+        float tt[17];
+        int rmax = 0;
+        rmin = ND;
+#pragma unroll
+        for (int p = 0; p < 17; ++p) {
+            const double u = R.c1 + c_gm.off1[p] * R.h1;  // along w
+            const double v = R.c0 + c_gm.off0[p] * R.h0;  // along h
+            const double x = fma(g.Dx, u * v, fma(g.Cx, v, fma(g.Bx, u, g.Ax)));
+            const double y = fma(g.Dy, u * v, fma(g.Cy, v, fma(g.By, u, g.Ay)));
+            const double z = fma(g.Dz, u * v, fma(g.Cz, v, fma(g.Bz, u, g.Az)));
+            ix[p] = point_row(fma(x, x, fma(y, y, z * z)), sq, scoef, &tt[p]);
+            rmin = min(rmin, ix[p] - 1);
+            rmax = max(rmax, ix[p]);
+        }
+        nr = rmax - rmin + 1;
+        if (nr <= AW) {  // the region's row windows
+            float4* wr = win + lane * WSTRIDE;
+            for (int j = 0; j < nr; ++j) wr[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int p = 0; p < 17; ++p) {
+                const float b = tt[p], a = 1.f - b;
+                float4* wj = wr + (ix[p] - 1 - rmin);
+                float4 lo = wj[0], hi = wj[1];
+                lo.x += a * c_gm.w7[p]; lo.y += a * c_gm.wd[p]; lo.z += a * c_gm.d0[p]; lo.w += a * c_gm.d1[p];
+                hi.x += b * c_gm.w7[p]; hi.y += b * c_gm.wd[p]; hi.z += b * c_gm.d0[p]; hi.w += b * c_gm.d1[p];
+                wj[0] = lo;
+                wj[1] = hi;
+            }
+        }
+    }
+    __syncwarp();
+    const unsigned narrow = __ballot_sync(full, on && nr <= AW);
+    int code = gm_decide<G>(A, R, win, rmin, nr, narrow, last, level0);
+    if (on && nr > AW) code = GM_FP64;  // points too far apart for a window (next to the source)
+    // the halves of the split regions: one reservation per warp
+    unsigned split = __ballot_sync(full, code == GM_SPLIT0 || code == GM_SPLIT1);
+    if (split) {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(qcount, 2 * __popc(split));
+        k = __shfl_sync(full, k, 0) + 2 * __popc(split & ((1u << lane) - 1));
+        const bool is = (split >> lane) & 1, fits = is && k + 2 <= qcap;
+        if (fits) store_halves(qout, k, R, code == GM_SPLIT0 ? 0 : 1);
+        const unsigned over = __ballot_sync(full, is && !fits);
+        if (over) gm_decide<G>(A, R, win, rmin, nr, over, true, level0);  // queue full: keep the estimate
+    }
+    unsigned near = __ballot_sync(full, code == GM_FP64);
+    while (near) {
+        const int l = __ffs(near) - 1;
+        near &= near - 1;
+        LaneRegion Q;
+        Q.sp = __shfl_sync(full, R.sp, l); Q.s = __shfl_sync(full, R.s, l);
+        Q.h = __shfl_sync(full, R.h, l); Q.w = __shfl_sync(full, R.w, l);
+        Q.c0 = __shfl_sync(full, R.c0, l); Q.c1 = __shfl_sync(full, R.c1, l);
+        Q.h0 = __shfl_sync(full, R.h0, l); Q.h1 = __shfl_sync(full, R.h1, l);
+        int dim = 0;
+        if (gm_region64(A, Q, pts, last, level0, &dim)) continue;
+        int k = 0;
+        if (lane == 0) k = atomicAdd(qcount, 2);
+        k = __shfl_sync(full, k, 0);
+        if (k + 2 <= qcap) {
+            if (lane == 0) store_halves(qout, k, Q, dim);
+        } else {
+            gm_region64(A, Q, pts, true, level0, &dim);
+        }
+    }
+    __syncwarp();  // the windows are reused by the next batch
 }
 
 __device__ __forceinline__ void load_tables(const SepTab* septab, double* sq, float4* scoef) {
@@ -395,110 +439,55 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, un
 // All levels in one persistent launch (cooperative: every block resident).  Level
 // 0: item k = (source, pixel) k, the whole pixel as one region; level L >= 1: item k
 // = region k of level L - 1's queue.  Levels are separated by grid barriers.
+//
+// A warp takes 32 items: geometry and row windows with one region per lane, then the
+// energies of 32 / G regions at a time with G lanes per region (G = 8 for E <= 32, 16
+// for E <= 64, else 32), so table rows and FP64 means move in runs of consecutive
+// values, and the regions that need FP64 by the whole warp in turn.
+template <int G>
 __global__ void __launch_bounds__(AT, 2)
-k_adaptive_levels(const double* __restrict__ corners, const SrcInfo* __restrict__ info,
-                  const SepTab* __restrict__ septab, const float* __restrict__ lut, const double* __restrict__ upsf,
-                  int S, int H, int W, int E, float rtol, int max_depth, double* __restrict__ mean,
-                  QRegion* __restrict__ q, long long qcap, int* __restrict__ counts, unsigned* __restrict__ bar,
-                  int* __restrict__ status) {
+k_adaptive_levels(LevelArgs A, const SepTab* __restrict__ septab, int S, int max_depth, QRegion* __restrict__ q,
+                  long long qcap, int* __restrict__ counts, unsigned* __restrict__ bar, int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned gen_s;
     double* sq = (double*)(smem + AO_SQ);
     float4* scoef = (float4*)(smem + AO_COEF);
-    float* wk = (float*)(smem + AO_WIN) + threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float4* win = (float4*)(smem + AO_WIN) + warp * 32 * WSTRIDE;
+    Point64* pts = (Point64*)(smem + AO_P64) + warp * 17;
     if (threadIdx.x == 0) gen_s = atomicAdd(&bar[1], 0u);
     load_tables(septab, sq, scoef);
-    const int npix = H * W, W1 = W + 1;
-    const int EP = (E + 3) & ~3;
+    const int npix = A.H * A.W;
     const long long stride = (long long)gridDim.x * AT;
     for (int level = 0; level <= max_depth; ++level) {
-        const bool last = level >= max_depth;
+        const bool last = level >= max_depth, level0 = level == 0;
         QRegion* qout = q + (size_t)(level & 1) * qcap;
-        int* qout_count = counts + level;
-        if (level == 0) {
-            const long long n = (long long)S * npix;
-            for (long long k = (long long)blockIdx.x * AT + threadIdx.x; k < n; k += stride) {
-                const int s = (int)(k / npix), pix = (int)(k - (long long)s * npix);
-                const SrcInfo si = info[s];
-                const int h = pix / W, w = pix - h * W;
-                const PixGeom g = pixel_geom(corners, W1, h, w, si);
-                double* m = mean + (size_t)k * E;
-                int dim = 0;
-                const float* Y = lut + (size_t)s * ND * EP;
-                const double* U = upsf + (size_t)s * ND * E;
-                if (gm_region(g, 0.f, 0.f, 1.f, 1.f, last, sq, scoef, wk, Y, U, corners, W1, h, w, si.dir, E, EP,
-                              rtol, m, false, &dim))
-                    continue;
-                if (!push_halves(qout, qout_count, (int)qcap, (int)k, 0.f, 0.f, 1.f, 1.f, dim))
-                    gm_region(g, 0.f, 0.f, 1.f, 1.f, true, sq, scoef, wk, Y, U, corners, W1, h, w, si.dir, E, EP,
-                              rtol, m, false, &dim);  // queue full: keep the estimate
+        const QRegion* qin = q + (size_t)((level - 1) & 1) * qcap;
+        const long long n = level0 ? (long long)S * npix : min((long long)counts[level - 1], qcap);
+        for (long long k0 = ((long long)blockIdx.x * NWARP + warp) * 32; k0 < n; k0 += stride) {
+            const long long k = k0 + lane;
+            const bool on = k < n;
+            LaneRegion R = {};
+            if (on) {
+                if (level0) {
+                    R.sp = (int)k;
+                    R.h0 = R.h1 = 1.f;
+                } else {
+                    const QRegion r = qin[k];
+                    R.sp = r.sp; R.c0 = r.c0; R.c1 = r.c1; R.h0 = r.h0; R.h1 = r.h1;
+                }
+                R.s = R.sp / npix;
+                const int pix = R.sp - R.s * npix;
+                R.h = pix / A.W;
+                R.w = pix - R.h * A.W;
             }
-        } else {
-            const QRegion* qin = q + (size_t)((level - 1) & 1) * qcap;
-            const long long n = min((long long)counts[level - 1], qcap);
-            for (long long k = (long long)blockIdx.x * AT + threadIdx.x; k < n; k += stride) {
-                const QRegion r = qin[k];
-                const int s = r.sp / npix, pix = r.sp - s * npix;
-                const SrcInfo si = info[s];
-                const int h = pix / W, w = pix - h * W;
-                const PixGeom g = pixel_geom(corners, W1, h, w, si);
-                const float* Y = lut + (size_t)s * ND * EP;
-                const double* U = upsf + (size_t)s * ND * E;
-                double* m = mean + (size_t)r.sp * E;
-                int dim = 0;
-                if (gm_region(g, r.c0, r.c1, r.h0, r.h1, last, sq, scoef, wk, Y, U, corners, W1, h, w, si.dir, E, EP,
-                              rtol, m, true, &dim))
-                    continue;
-                if (!push_halves(qout, qout_count, (int)qcap, r.sp, r.c0, r.c1, r.h0, r.h1, dim))
-                    gm_region(g, r.c0, r.c1, r.h0, r.h1, true, sq, scoef, wk, Y, U, corners, W1, h, w, si.dir, E,
-                              EP, rtol, m, true, &dim);
-            }
+            gm_batch<G>(A, R, on, sq, scoef, win, pts, last, level0, qout, counts + level, (int)qcap);
         }
         if (level == max_depth) break;
         if (!grid_barrier(bar, gridDim.x, &gen_s)) {
             if (threadIdx.x == 0) atomicExch(status, 1);
             return;
         }
-    }
-}
-
-// c7 on the adaptive map: per block (chunk, source) the FP64 sums over pixels
-// inside the boundary radius of mean * solid angle, in a fixed order.
-template <typename T>
-__global__ void __launch_bounds__(AT) k_adaptive_integral(const double* __restrict__ centers,
-                                                          const double* __restrict__ omega,
-                                                          const SrcInfo* __restrict__ info,
-                                                          const T* __restrict__ mean, int H, int W, int E,
-                                                          int nch, double* __restrict__ sums_out) {
-    __shared__ double part[AT];
-    const int s = blockIdx.y, t = threadIdx.x;
-    const SrcInfo si = info[s];
-    const int npix = H * W, W1 = W + 1;
-    double ch2 = 2.0 * sin(0.5 * si.radius_rad);
-    ch2 *= ch2;
-    // thread (g, e): energy e over pixels g, g + G, ... of the block's range
-    const int G = AT / E, g = t / E, e = t - g * E;
-    const int p_lo = (int)((long long)npix * blockIdx.x / nch), p_hi = (int)((long long)npix * (blockIdx.x + 1) / nch);
-    double acc = 0.;
-    if (si.in_fov && t < G * E) {
-        for (int pix = p_lo + g; pix < p_hi; pix += G) {
-            const int h = pix / W, w = pix - h * W;
-            const double* c = centers + 3 * (h * W1 + w);
-            const double x = si.dir[0] - c[0], y = si.dir[1] - c[1], z = si.dir[2] - c[2];
-            const double d2 = x * x + y * y + z * z;
-            bool inside;
-            if (d2 < ch2 * (1.0 - 1e-12)) inside = true;
-            else if (d2 > ch2 * (1.0 + 1e-12)) inside = false;
-            else inside = dir_diff(si.dir, c) <= si.radius_rad;
-            if (inside) acc += (double)mean[((size_t)s * npix + pix) * E + e] * omega[pix];
-        }
-    }
-    part[t] = acc;
-    __syncthreads();
-    for (int ee = t; ee < E; ee += AT) {
-        double v = 0.;
-        for (int gg = 0; gg < G; ++gg) v += part[gg * E + ee];
-        sums_out[((size_t)s * nch + blockIdx.x) * E + ee] = v;
     }
 }
 
@@ -560,9 +549,8 @@ __global__ void k_scale_map(float* __restrict__ out, const double* __restrict__ 
 
 bool srcmap_adaptive_supported(int E) { return E >= 1 && E <= 256; }
 
-int launch_adaptive_map(const double* corners, const double* centers, const double* omega, const SrcInfo* info,
-                        const double* upsf, int S, int H, int W, int E, double rtol, int max_depth, int nch,
-                        double* sums, double* mean64, int* status, cudaStream_t st) {
+int launch_adaptive_map(const double* corners, const SrcInfo* info, const double* upsf, int S, int H, int W, int E,
+                        double rtol, int max_depth, double* mean64, int* status, cudaStream_t st) {
     int rc = upload_gm(st);
     if (rc) return rc;
     const SepTab* tab = nullptr;
@@ -582,12 +570,14 @@ int launch_adaptive_map(const double* corners, const double* centers, const doub
     unsigned* bar = (unsigned*)(counts + 32);
     XTS_LAUNCH("k_lut_scaled", st, k_lut_scaled<<<lut_scaled_grid(S), 256, 0, st>>>(upsf, nullptr, S, E, EP, lut,
                                                                                        nullptr, nullptr));
-    XTS_CUDA(cudaFuncSetAttribute(k_adaptive_levels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A_SMEM));
+    typedef void (*LevelsFn)(LevelArgs, const SepTab*, int, int, QRegion*, long long, int*, unsigned*, int*);
+    const LevelsFn levels = E <= 32 ? k_adaptive_levels<8> : E <= 64 ? k_adaptive_levels<16> : k_adaptive_levels<32>;
+    XTS_CUDA(cudaFuncSetAttribute(levels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A_SMEM));
     XTS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * 64, st));
     int dev = 0, nsm = 148, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adaptive_levels, AT, A_SMEM));
+    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, levels, AT, A_SMEM));
     const unsigned G = (unsigned)(nsm * (per_sm > 0 ? per_sm : 1));
     // one cooperative launch: every block resident, so the grid barriers between levels complete
     cudaLaunchConfig_t cfg = {};
@@ -600,13 +590,11 @@ int launch_adaptive_map(const double* corners, const double* centers, const doub
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const float rtol_f = (float)rtol;
+    const LevelArgs la{corners, info, lut, upsf, H, W, E, EP, (float)rtol, mean64};
     cudaError_t le = cudaSuccess;
-    XTS_LAUNCH("k_adaptive_map", st, le = cudaLaunchKernelEx(&cfg, k_adaptive_levels, corners, info, tab,
-                                                             (const float*)lut, upsf, S, H, W, E, rtol_f, max_depth,
-                                                             mean64, q, cap, counts, bar, status));
+    XTS_LAUNCH("k_adaptive_map", st, le = cudaLaunchKernelEx(&cfg, levels, la, tab, S, max_depth, q, cap, counts, bar,
+                                                             status));
     if (le != cudaSuccess) return cuda_error(le, "cooperative launch of k_adaptive_levels");
-    (void)centers; (void)omega; (void)nch; (void)sums;  // the c7 sums: launch_mean_integral, by the caller
     return XTS_OK;
 }
 
@@ -618,10 +606,11 @@ int launch_adaptive_map(const double* corners, const double* centers, const doub
 // warps' partial sums are added in a fixed order into sums[s][c][e].
 constexpr int MI_WARPS = 8;
 constexpr int MI_EQ = 8;  // energies per lane: E <= 256
+template <typename T>
 __global__ void __launch_bounds__(32 * MI_WARPS) k_mean_integral(const double* __restrict__ centers,
                                                                  const double* __restrict__ omega,
                                                                  const SrcInfo* __restrict__ info,
-                                                                 const float* __restrict__ mean, int H, int W, int E,
+                                                                 const T* __restrict__ mean, int H, int W, int E,
                                                                  int nc, double* __restrict__ sums_out) {
     __shared__ double part[MI_WARPS][AT];
     const int s = blockIdx.y, t = threadIdx.x, lane = t & 31, wp = t >> 5;
@@ -635,7 +624,7 @@ __global__ void __launch_bounds__(32 * MI_WARPS) k_mean_integral(const double* _
 #pragma unroll
     for (int q = 0; q < MI_EQ; ++q) acc[q] = 0.;
     if (si.in_fov) {
-        const float* m = mean + (size_t)s * npix * E;
+        const T* m = mean + (size_t)s * npix * E;
         // 32 pixels per round: each lane tests its own pixel against the boundary, then
         // the warp sums the inside pixels' rows (lane = energy), two rows per step so
         // that two loads are in flight
@@ -661,15 +650,15 @@ __global__ void __launch_bounds__(32 * MI_WARPS) k_mean_integral(const double* _
                 if (l2 >= 0) mask &= mask - 1;
                 const double om1 = __shfl_sync(0xffffffffu, om, l1);
                 const double om2 = __shfl_sync(0xffffffffu, om, l2 < 0 ? l1 : l2);
-                const float* mp1 = m + (size_t)(pix0 + l1) * E;
-                const float* mp2 = m + (size_t)(pix0 + (l2 < 0 ? l1 : l2)) * E;
-                float v1[MI_EQ], v2[MI_EQ];
+                const T* mp1 = m + (size_t)(pix0 + l1) * E;
+                const T* mp2 = m + (size_t)(pix0 + (l2 < 0 ? l1 : l2)) * E;
+                T v1[MI_EQ], v2[MI_EQ];
 #pragma unroll
                 for (int q = 0; q < MI_EQ; ++q) {
                     const int e = lane + 32 * q;
                     const bool on = q < nq && e < E;
-                    v1[q] = on ? mp1[e] : 0.f;
-                    v2[q] = on && l2 >= 0 ? mp2[e] : 0.f;
+                    v1[q] = on ? mp1[e] : (T)0;
+                    v2[q] = on && l2 >= 0 ? mp2[e] : (T)0;
                 }
 #pragma unroll
                 for (int q = 0; q < MI_EQ; ++q) {
@@ -702,7 +691,7 @@ int mean_integral_chunks(int S, int npix) {
 int launch_mean_integral(const double* centers, const double* omega, const SrcInfo* info, const float* mean, int S,
                          int H, int W, int E, int nch, double* sums, cudaStream_t st) {
     if (E < 1 || E > AT) return set_error(XTS_ERR_ARG, "map integral of pixel means: E (%d) above %d", E, AT);
-    XTS_LAUNCH("k_mean_integral", st, k_mean_integral<<<dim3(nch, S), 32 * MI_WARPS, 0, st>>>(
+    XTS_LAUNCH("k_mean_integral", st, k_mean_integral<float><<<dim3(nch, S), 32 * MI_WARPS, 0, st>>>(
                                           centers, omega, info, mean, H, W, E, nch, sums));
     return XTS_OK;
 }
@@ -710,7 +699,7 @@ int launch_mean_integral(const double* centers, const double* omega, const SrcIn
 int launch_mean_integral64(const double* centers, const double* omega, const SrcInfo* info, const double* mean, int S,
                            int H, int W, int E, int nch, double* sums, cudaStream_t st) {
     if (E < 1 || E > AT) return set_error(XTS_ERR_ARG, "map integral of pixel means: E (%d) above %d", E, AT);
-    XTS_LAUNCH("k_adaptive_integral", st, k_adaptive_integral<double><<<dim3(nch, S), AT, 0, st>>>(
+    XTS_LAUNCH("k_mean_integral", st, k_mean_integral<double><<<dim3(nch, S), 32 * MI_WARPS, 0, st>>>(
                                               centers, omega, info, mean, H, W, E, nch, sums));
     return XTS_OK;
 }

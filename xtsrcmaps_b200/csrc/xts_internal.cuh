@@ -199,9 +199,8 @@ int launch_exposure_map_tc(const float* cube, const float* wcube, long long npix
                            const double* back_aeff, const double* ltf, int E, double* out, int* status,
                            cudaStream_t st);
 bool srcmap_adaptive_supported(int E);
-int launch_adaptive_map(const double* corners, const double* centers, const double* omega, const SrcInfo* info,
-                        const double* upsf, int S, int H, int W, int E, double rtol, int max_depth, int nch,
-                        double* sums, double* mean64, int* status, cudaStream_t st);
+int launch_adaptive_map(const double* corners, const SrcInfo* info, const double* upsf, int S, int H, int W, int E,
+                        double rtol, int max_depth, double* mean64, int* status, cudaStream_t st);
 int launch_mean_integral64(const double* centers, const double* omega, const SrcInfo* info, const double* mean, int S,
                            int H, int W, int E, int nch, double* sums, cudaStream_t st);
 int launch_scale_map64(const double* mean, float* out, const double* omega, const double* scale, int S, int npix,

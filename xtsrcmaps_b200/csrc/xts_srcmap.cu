@@ -490,17 +490,17 @@ __global__ void __launch_bounds__(256) k_correction_sums(const double* sums, int
 // The model map with adaptive cubature: pixel means * solid angle, map integral
 // sums, correction, then one scaling pass over the map.
 static int launch_srcmap_adaptive(const SrcmapDev& a, const double* corners, const double* centers,
-                                  const double* omega, const SrcInfo* info, double* scale, int nch,
+                                  const double* omega, const SrcInfo* info, double* scale,
                                   cudaStream_t st) {
     const int H = (int)a.wcs.naxis1, W = (int)a.wcs.naxis2, S = a.S, E = a.E;
-    const int npix = H * W;
+    const int npix = H * W, nch = mean_integral_chunks(S, npix);
     double* sums = (double*)workspace(W_PARTSUM, sizeof(double) * (size_t)S * nch * E + 8);
     double* mean64 = (double*)workspace(W_ADAPT_MEAN, sizeof(double) * (size_t)S * npix * E + 8);
     int* status = (int*)workspace(W_MISC, 64);
     if (!sums || !mean64 || !status) return XTS_ERR_OOM;
     XTS_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
-    int rc = launch_adaptive_map(corners, centers, omega, info, a.upsf, S, H, W, E, a.rtol, a.max_depth, nch,
-                                 sums, mean64, status, st);
+    int rc = launch_adaptive_map(corners, info, a.upsf, S, H, W, E, a.rtol, a.max_depth, mean64,
+                                 status, st);
     if (rc) return rc;
     // c7 from the FP64 means, c9, then the scalings into the FP32 map
     if ((rc = launch_mean_integral64(centers, omega, info, mean64, S, H, W, E, nch, sums, st))) return rc;
@@ -607,7 +607,7 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_adaptive_supported(E))
             return set_error(XTS_ERR_ARG, "adaptive cubature: FP32 maps with E <= 256 only");
-        return launch_srcmap_adaptive(a, corners, centers, omega, info, scale, nch, st);
+        return launch_srcmap_adaptive(a, corners, centers, omega, info, scale, st);
     }
     if (!a.out_f64 && a.kernel == SRCMAP_WINDOWS && srcmap_win_supported(E)) {
         int* status = (int*)workspace(W_MISC, 64);
