@@ -18,9 +18,9 @@
 // as it is.
 //
 // Decisions near the threshold are taken in FP64: when the FP32 estimate of
-// max_e |R5 - R7| / |R7| lies within 5 % of rtol, or the two fourth differences
-// that choose the split dimension are within 0.1 % of each other (or within their
-// FP32 error, 4e-6 of the summed values), the region is
+// max_e |R5 - R7| / |R7| lies within its FP32 error of rtol (4e-6, and 0.1 % of rtol),
+// or the two fourth differences that choose the split dimension within theirs of each
+// other (4e-6 of the summed values), or the points leave the row window, the region is
 // evaluated again point by point in FP64 from the FP64 mean PSF, with the
 // reference design's arithmetic (math/genz_malik.hxx:127-195) and no fused
 // multiply-adds, and that evaluation decides (and gives the value).
@@ -30,8 +30,8 @@
 // exact row, per-row t polynomial).  When they span at most AW consecutive rows,
 // four row windows are formed (the degree-7 value, degree-5 minus degree-7, and
 // the two fourth divided differences that choose the split dimension) and dotted
-// with the source's FP32 mean-PSF rows for every energy; otherwise the points
-// are evaluated one by one.  A region is accepted when
+// with the source's FP32 mean-PSF rows for every energy; otherwise the region is
+// evaluated in FP64.  A region is accepted when
 // max_e |R5 - R7| / |R7| <= rtol or at the depth limit; otherwise it is halved
 // along the dimension with the larger summed fourth difference.
 //
@@ -108,6 +108,8 @@ struct QRegion { int sp; float c0, c1, h0, h1; };
 // regions ([32][AW] float4 (w7, wd, d0, d1), one float4 of padding per region so that
 // lanes' 16-byte accesses fall in different banks) and the 17 points of the region
 // that the warp evaluates in FP64.
+constexpr int ADAPT_BLOCKS = 2;  // per SM
+constexpr int TH = 4, TW = 8;    // pixels of a warp's patch at level 0
 constexpr int WSTRIDE = AW + 1;
 constexpr int NWARP = AT / 32;
 struct Point64 { double t; int idx; };
@@ -179,23 +181,40 @@ __device__ __noinline__ bool gm_region64(const LevelArgs& A, const LaneRegion& R
         const double t = pts[p].t;
         return __dadd_rn(__dmul_rn(__dsub_rn(1.0, t), U[(size_t)(i - 1) * E + e]), __dmul_rn(t, U[(size_t)i * E + e]));
     };
-    double rel = 0., dd0 = 0., dd1 = 0.;
+    auto r7 = [&](int e, double* five) {  // R7 (and R5) at energy e
+        double v7 = 0., v5 = 0.;
+#pragma unroll
+        for (int p = 0; p < 17; ++p) {
+            const double fv = value(p, e);
+            v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], fv));
+            v5 = __dadd_rn(v5, __dmul_rn(c_gm64.w5[p], fv));
+        }
+        *five = v5;
+        return v7;
+    };
+    double rel = 0., first = 0., second = 0.;  // R7 of the lane's first two energies
+    for (int e = lane; e < min(E, last ? 64 : E); e += 32) {
+        double v5;
+        const double v7 = r7(e, &v5);
+        if (e < 32) first = v7;
+        else if (e < 64) second = v7;
+        const double err = fabs(__dsub_rn(v5, v7));
+        const double r = v7 != 0. ? err / fabs(v7) : (err != 0. ? INFINITY : 0.);
+        rel = r > rel ? r : rel;
+    }
     if (!last) {
+        for (int o = 16; o > 0; o >>= 1) rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, o));
+    }
+    const bool accept = last || rel <= (double)A.rtol;
+    if (!accept) {
+        double dd0 = 0., dd1 = 0.;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             double g0 = 0., g1 = 0.;
             if (e < E) {
-                double v7 = 0., v5 = 0., f[9];
+                double f[9];
 #pragma unroll
-                for (int p = 0; p < 17; ++p) {
-                    const double fv = value(p, e);
-                    if (p < 9) f[p] = fv;
-                    v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], fv));
-                    v5 = __dadd_rn(v5, __dmul_rn(c_gm64.w5[p], fv));
-                }
-                const double err = fabs(__dsub_rn(v5, v7));
-                const double r = v7 != 0. ? err / fabs(v7) : (err != 0. ? INFINITY : 0.);
-                rel = r > rel ? r : rel;
+                for (int p = 0; p < 9; ++p) f[p] = value(p, e);
                 const double f0 = __dmul_rn(2., f[0]);
                 g0 = fabs(__dsub_rn(__dsub_rn(__dadd_rn(f[1], f[3]), f0),
                                     __dmul_rn(1. / 7., __dsub_rn(__dadd_rn(f[5], f[7]), f0))));
@@ -208,19 +227,12 @@ __device__ __noinline__ bool gm_region64(const LevelArgs& A, const LaneRegion& R
                 dd1 = __dadd_rn(dd1, shfl_d(g1, k));
             }
         }
-        for (int o = 16; o > 0; o >>= 1) rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, o));
+        *dim = dd0 >= dd1 ? 0 : 1;
     }
-    const bool accept = last || rel <= (double)A.rtol;
-    *dim = dd0 >= dd1 ? 0 : 1;
     const double area = __dmul_rn(R.h0, R.h1);
     for (int e = lane; e < E; e += 32) {
-        double v = 0.;
-        if (accept) {
-            double v7 = 0.;
-#pragma unroll
-            for (int p = 0; p < 17; ++p) v7 = __dadd_rn(v7, __dmul_rn(c_gm64.w7[p], value(p, e)));
-            v = __dmul_rn(area, v7);
-        }
+        double v = 0., v5;
+        if (accept) v = __dmul_rn(area, e < 32 ? first : e < 64 ? second : r7(e, &v5));
         if (level0) mean[e] = v;
         else if (accept) atomicAdd(mean + e, v);
     }
@@ -243,6 +255,29 @@ __device__ __forceinline__ void store_halves(QRegion* q, int k, const LaneRegion
     q[k + 1] = b;
 }
 
+// One region decided in FP64, its halves queued (or its value kept when the queue is full).
+__device__ __noinline__ void gm_fp64(const LevelArgs& A, const LaneRegion& R, Point64* pts, bool last, bool level0,
+                                     QRegion* qout, int* qcount, int qcap) {
+    int dim = 0, k = 0;
+    if (gm_region64(A, R, pts, last, level0, &dim)) return;
+    if ((threadIdx.x & 31) == 0) k = atomicAdd(qcount, 2);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k + 2 > qcap) gm_region64(A, R, pts, true, level0, &dim);
+    else if ((threadIdx.x & 31) == 0) store_halves(qout, k, R, dim);
+}
+
+struct Queue64 { QRegion* q; int* count; int cap; };
+
+__device__ __forceinline__ LaneRegion lane_region(const QRegion& r, int npix, int W) {
+    LaneRegion R;
+    R.sp = r.sp; R.c0 = r.c0; R.c1 = r.c1; R.h0 = r.h0; R.h1 = r.h1;
+    R.s = r.sp / npix;
+    const int pix = r.sp - R.s * npix;
+    R.h = pix / W;
+    R.w = pix - R.h * W;
+    return R;
+}
+
 enum { GM_ACCEPT = 0, GM_SPLIT0 = 1, GM_SPLIT1 = 2, GM_FP64 = 3, GM_NONE = 4 };
 
 // The windowed regions of `mask` (lane = region): G lanes per region, lane q of the
@@ -253,60 +288,85 @@ enum { GM_ACCEPT = 0, GM_SPLIT0 = 1, GM_SPLIT1 = 2, GM_FP64 = 3, GM_NONE = 4 };
 template <int G>
 __device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R, const float4* win, int rmin, int nr,
                                          unsigned mask, bool last, bool level0) {
-    constexpr int NS = G == 32 ? 8 : 4;  // energies per lane: E <= G * NS
+    constexpr int NS = 8;  // energies per lane: E <= G * NS
+    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, q = lane & (G - 1), E = A.E;
     int mine = GM_NONE;
     for (int r0 = 0; r0 < 32; r0 += 32 / G) {
         if (!((mask >> r0) & ((1u << (32 / G)) - 1))) continue;  // warp-uniform
         const int rg = r0 + lane / G;
         const bool on = (mask >> rg) & 1;
-        const int row = __shfl_sync(0xffffffffu, rmin, rg), nrow = __shfl_sync(0xffffffffu, nr, rg);
+        const int row = __shfl_sync(full, rmin, rg), nrow = __shfl_sync(full, nr, rg);
         const int n = on ? nrow : 0;
-        const int sp = __shfl_sync(0xffffffffu, R.sp, rg), s = __shfl_sync(0xffffffffu, R.s, rg);
-        const float area = __shfl_sync(0xffffffffu, R.h0, rg) * __shfl_sync(0xffffffffu, R.h1, rg);
-        float v7[NS], vd[NS], a0[NS], a1[NS];
-#pragma unroll
-        for (int c = 0; c < NS; ++c) v7[c] = vd[c] = a0[c] = a1[c] = 0.f;
-        const float* y = A.lut + ((size_t)s * ND + row) * A.EP + q;
+        const int sp = __shfl_sync(full, R.sp, rg), s = __shfl_sync(full, R.s, rg);
+        const float area = __shfl_sync(full, R.h0, rg) * __shfl_sync(full, R.h1, rg);
+        const float* y0 = A.lut + ((size_t)s * ND + row) * A.EP + q;
         const float4* wr = win + rg * WSTRIDE;
-        for (int j = 0; j < n; ++j, y += A.EP) {
-            const float4 w = wr[j];
+        float v7[NS], vd[NS];
+#pragma unroll
+        for (int c = 0; c < NS; ++c) v7[c] = vd[c] = 0.f;
+        // two rows at a time, so that their loads are in flight together
+        auto dot = [&](const float2* w, float* u, float* v) {
+            const float* y = y0;
+            for (int j = 0; j < n; j += 2, y += 2 * A.EP) {
+                const bool two = j + 1 < n;
+                const float2 wa = w[2 * j], wb = two ? w[2 * j + 2] : make_float2(0.f, 0.f);
+                const float* yb = two ? y + A.EP : y;
+                float fa[NS], fb[NS];
+#pragma unroll
+                for (int c = 0; c < NS; ++c)
+                    if (G * c < E) {  // uniform
+                        const bool in = q + G * c < E;
+                        fa[c] = in ? __ldg(y + G * c) : 0.f;
+                        fb[c] = in ? __ldg(yb + G * c) : 0.f;
+                    }
+#pragma unroll
+                for (int c = 0; c < NS; ++c)
+                    if (G * c < E) {
+                        u[c] = fmaf(wb.x, fb[c], fmaf(wa.x, fa[c], u[c]));
+                        v[c] = fmaf(wb.y, fb[c], fmaf(wa.y, fa[c], v[c]));
+                    }
+            }
+        };
+        dot((const float2*)wr, v7, vd);
+        int code = GM_ACCEPT;
+        if (!last) {
+            float rel = 0.f;
 #pragma unroll
             for (int c = 0; c < NS; ++c)
                 if (G * c < E) {
-                    const float f = q + G * c < E ? __ldg(y + G * c) : 0.f;
-                    v7[c] = fmaf(w.x, f, v7[c]);
-                    vd[c] = fmaf(w.y, f, vd[c]);
-                    a0[c] = fmaf(w.z, f, a0[c]);
-                    a1[c] = fmaf(w.w, f, a1[c]);
+                    const float x7 = fabsf(v7[c]), xd = fabsf(vd[c]);
+                    // 0 / 0 (an all-zero energy, or a lane past E) counts as no error
+                    rel = fmaxf(rel, xd == 0.f ? 0.f : (x7 != 0.f ? __fdividef(xd, x7) : 3.4e38f));
                 }
-        }
-        int code = GM_ACCEPT;
-        if (!last) {
-            float rel = 0.f, dd0 = 0.f, dd1 = 0.f, sx = 0.f;
 #pragma unroll
-            for (int c = 0; c < NS; ++c) {
-                const float x7 = fabsf(v7[c]), xd = fabsf(vd[c]);
-                // 0 / 0 (an all-zero energy, or a lane past E) counts as no error
-                rel = fmaxf(rel, xd == 0.f ? 0.f : (x7 != 0.f ? xd / x7 : 3.4e38f));
-                dd0 += fabsf(a0[c]);
-                dd1 += fabsf(a1[c]);
-                sx += x7;
-            }
+            for (int o = G / 2; o > 0; o >>= 1) rel = fmaxf(rel, __shfl_xor_sync(full, rel, o));
+            const bool accept = rel <= A.rtol;
+            if (fabsf(rel - A.rtol) <= fmaxf(1e-3f * A.rtol, 4e-6f)) code = GM_FP64;
+            if (__any_sync(full, !accept && code != GM_FP64)) {  // the fourth differences of regions to be split
+                float a0[NS], a1[NS];
 #pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) {
-                rel = fmaxf(rel, __shfl_xor_sync(0xffffffffu, rel, o));
-                dd0 += __shfl_xor_sync(0xffffffffu, dd0, o);
-                dd1 += __shfl_xor_sync(0xffffffffu, dd1, o);
-                sx += __shfl_xor_sync(0xffffffffu, sx, o);
+                for (int c = 0; c < NS; ++c) a0[c] = a1[c] = 0.f;
+                if (!accept) dot((const float2*)wr + 1, a0, a1);
+                float dd0 = 0.f, dd1 = 0.f, sx = 0.f;
+#pragma unroll
+                for (int c = 0; c < NS; ++c)
+                    if (G * c < E) {
+                        dd0 += fabsf(a0[c]);
+                        dd1 += fabsf(a1[c]);
+                        sx += fabsf(v7[c]);
+                    }
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) {
+                    dd0 += __shfl_xor_sync(full, dd0, o);
+                    dd1 += __shfl_xor_sync(full, dd1, o);
+                    sx += __shfl_xor_sync(full, sx, o);
+                }
+                // the fourth differences cancel most of the values they are formed from, so
+                // their FP32 error is measured against the values (sx), not against themselves
+                const bool near_dim = fabsf(dd0 - dd1) <= 1e-5f * (dd0 + dd1) + 4e-6f * sx;
+                if (!accept && code != GM_FP64) code = near_dim ? GM_FP64 : dd0 >= dd1 ? GM_SPLIT0 : GM_SPLIT1;
             }
-            const float rtol = A.rtol;
-            const bool accept = rel <= rtol;
-            // the fourth differences cancel most of the values they are formed from, so
-            // their FP32 error is measured against the values (sx), not against themselves
-            const bool near_dim = !accept && fabsf(dd0 - dd1) <= 1e-3f * (dd0 + dd1) + 4e-6f * sx;
-            if (fabsf(rel - rtol) <= fmaxf(0.05f * rtol, 4e-6f) || near_dim) code = GM_FP64;
-            else if (!accept) code = dd0 >= dd1 ? GM_SPLIT0 : GM_SPLIT1;
         }
         if (on && (code == GM_ACCEPT || (level0 && code != GM_FP64))) {
             double* m = A.mean + (size_t)sp * E + q;
@@ -318,7 +378,7 @@ __device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R
                     else atomicAdd(m + G * c, v);
                 }
         }
-        const int got = __shfl_sync(0xffffffffu, code, ((lane - r0) & (32 / G - 1)) * G);
+        const int got = __shfl_sync(full, code, ((lane - r0) & (32 / G - 1)) * G);
         if (lane >= r0 && lane < r0 + 32 / G && ((mask >> lane) & 1)) mine = got;
     }
     return mine;
@@ -328,7 +388,7 @@ __device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R
 template <int G>
 __device__ __forceinline__ void gm_batch(const LevelArgs& A, const LaneRegion& R, bool on, const double* sq,
                                          const float4* scoef, float4* win, Point64* pts, bool last, bool level0,
-                                         QRegion* qout, int* qcount, int qcap) {
+                                         QRegion* qout, int* qcount, int qcap, const Queue64& q64) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int rmin = 0, nr = 0;
@@ -367,37 +427,43 @@ __device__ __forceinline__ void gm_batch(const LevelArgs& A, const LaneRegion& R
     }
     __syncwarp();
     const unsigned narrow = __ballot_sync(full, on && nr <= AW);
-    int code = gm_decide<G>(A, R, win, rmin, nr, narrow, last, level0);
-    if (on && nr > AW) code = GM_FP64;  // points too far apart for a window (next to the source)
-    // the halves of the split regions: one reservation per warp
-    unsigned split = __ballot_sync(full, code == GM_SPLIT0 || code == GM_SPLIT1);
-    if (split) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(qcount, 2 * __popc(split));
-        k = __shfl_sync(full, k, 0) + 2 * __popc(split & ((1u << lane) - 1));
-        const bool is = (split >> lane) & 1, fits = is && k + 2 <= qcap;
-        if (fits) store_halves(qout, k, R, code == GM_SPLIT0 ? 0 : 1);
-        const unsigned over = __ballot_sync(full, is && !fits);
-        if (over) gm_decide<G>(A, R, win, rmin, nr, over, true, level0);  // queue full: keep the estimate
+    int code = GM_NONE;
+    for (unsigned mask = narrow; mask;) {
+        const int c = gm_decide<G>(A, R, win, rmin, nr, mask, last, level0);
+        if ((mask >> lane) & 1) code = c;
+        mask = 0;
+        // the halves of the split regions: one reservation per warp
+        const unsigned split = __ballot_sync(full, code == GM_SPLIT0 || code == GM_SPLIT1);
+        if (split) {
+            int k = 0;
+            if (lane == 0) k = atomicAdd(qcount, 2 * __popc(split));
+            k = __shfl_sync(full, k, 0) + 2 * __popc(split & ((1u << lane) - 1));
+            const bool is = (split >> lane) & 1, fits = is && k + 2 <= qcap;
+            if (fits) store_halves(qout, k, R, code == GM_SPLIT0 ? 0 : 1);
+            mask = __ballot_sync(full, is && !fits);  // queue full: keep their estimates
+            last = true;
+            if (is) code = GM_NONE;
+        }
     }
-    unsigned near = __ballot_sync(full, code == GM_FP64);
-    while (near) {
-        const int l = __ffs(near) - 1;
-        near &= near - 1;
-        LaneRegion Q;
-        Q.sp = __shfl_sync(full, R.sp, l); Q.s = __shfl_sync(full, R.s, l);
-        Q.h = __shfl_sync(full, R.h, l); Q.w = __shfl_sync(full, R.w, l);
-        Q.c0 = __shfl_sync(full, R.c0, l); Q.c1 = __shfl_sync(full, R.c1, l);
-        Q.h0 = __shfl_sync(full, R.h0, l); Q.h1 = __shfl_sync(full, R.h1, l);
-        int dim = 0;
-        if (gm_region64(A, Q, pts, last, level0, &dim)) continue;
+    if (on && nr > AW) code = GM_FP64;  // points too far apart for a window (next to the source)
+    // regions for FP64: queued for the level's second phase, one region per warp there
+    const unsigned near = __ballot_sync(full, code == GM_FP64);
+    if (near) {
         int k = 0;
-        if (lane == 0) k = atomicAdd(qcount, 2);
-        k = __shfl_sync(full, k, 0);
-        if (k + 2 <= qcap) {
-            if (lane == 0) store_halves(qout, k, Q, dim);
-        } else {
-            gm_region64(A, Q, pts, true, level0, &dim);
+        if (lane == 0) k = atomicAdd(q64.count, __popc(near));
+        k = __shfl_sync(full, k, 0) + __popc(near & ((1u << lane) - 1));
+        const bool fits = code == GM_FP64 && k < q64.cap;
+        if (fits) q64.q[k] = QRegion{R.sp, R.c0, R.c1, R.h0, R.h1};
+        unsigned over = __ballot_sync(full, code == GM_FP64 && !fits);
+        while (over) {  // that queue full: here
+            const int l = __ffs(over) - 1;
+            over &= over - 1;
+            LaneRegion Q;
+            Q.sp = __shfl_sync(full, R.sp, l); Q.s = __shfl_sync(full, R.s, l);
+            Q.h = __shfl_sync(full, R.h, l); Q.w = __shfl_sync(full, R.w, l);
+            Q.c0 = __shfl_sync(full, R.c0, l); Q.c1 = __shfl_sync(full, R.c1, l);
+            Q.h0 = __shfl_sync(full, R.h0, l); Q.h1 = __shfl_sync(full, R.h1, l);
+            gm_fp64(A, Q, pts, last, level0, qout, qcount, qcap);
         }
     }
     __syncwarp();  // the windows are reused by the next batch
@@ -441,13 +507,22 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, un
 // = region k of level L - 1's queue.  Levels are separated by grid barriers.
 //
 // A warp takes 32 items: geometry and row windows with one region per lane, then the
-// energies of 32 / G regions at a time with G lanes per region (G = 8 for E <= 32, 16
-// for E <= 64, else 32), so table rows and FP64 means move in runs of consecutive
-// values, and the regions that need FP64 by the whole warp in turn.
+// energies of 32 / G regions at a time with G lanes per region (G = 8 for E <= 64,
+// else 32), so table rows and FP64 means move in runs of consecutive values.  Level 0
+// takes pixels in TH x TW patches, whose points share table rows (1.03 -> 0.69 ms against
+// runs of 32 pixels, L1 misses on the rows).  Regions that need FP64 are queued and
+// follow the level's others, one per warp: inside the batches, whose neighbours tend to
+// need it together, they held the level's end up (2.0 of 4.9 ms, 0.5 now).  50 sources,
+// 200 x 200, 37 energies, rtol 1e-4, depth 6 (4.1 M regions, 0.1 M in FP64): 2.47 ms,
+// 26.1 with one region per thread throughout.  What is left: table rows from L2 below
+// level 0 (a queue's neighbours are of different patches), the levels' last batches, and
+// the FP64 pipe.  Two blocks of 128 registers per SM: 2.52 ms, three of 80: 2.91.
 template <int G>
-__global__ void __launch_bounds__(AT, 2)
+__global__ void __launch_bounds__(AT, ADAPT_BLOCKS)
 k_adaptive_levels(LevelArgs A, const SepTab* __restrict__ septab, int S, int max_depth, QRegion* __restrict__ q,
-                  long long qcap, int* __restrict__ counts, unsigned* __restrict__ bar, int* __restrict__ status) {
+                  long long qcap, int cap64, int* __restrict__ counts, int* __restrict__ work,
+                  int* __restrict__ count64, unsigned* __restrict__ bar,
+                  int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned gen_s;
     double* sq = (double*)(smem + AO_SQ);
@@ -457,32 +532,44 @@ k_adaptive_levels(LevelArgs A, const SepTab* __restrict__ septab, int S, int max
     Point64* pts = (Point64*)(smem + AO_P64) + warp * 17;
     if (threadIdx.x == 0) gen_s = atomicAdd(&bar[1], 0u);
     load_tables(septab, sq, scoef);
-    const int npix = A.H * A.W;
-    const long long stride = (long long)gridDim.x * AT;
+    const int npix = A.H * A.W, pw = (A.W + TW - 1) / TW, per_src = pw * ((A.H + TH - 1) / TH);
     for (int level = 0; level <= max_depth; ++level) {
         const bool last = level >= max_depth, level0 = level == 0;
         QRegion* qout = q + (size_t)(level & 1) * qcap;
         const QRegion* qin = q + (size_t)((level - 1) & 1) * qcap;
-        const long long n = level0 ? (long long)S * npix : min((long long)counts[level - 1], qcap);
-        for (long long k0 = ((long long)blockIdx.x * NWARP + warp) * 32; k0 < n; k0 += stride) {
-            const long long k = k0 + lane;
-            const bool on = k < n;
-            LaneRegion R = {};
-            if (on) {
-                if (level0) {
-                    R.sp = (int)k;
-                    R.h0 = R.h1 = 1.f;
-                } else {
-                    const QRegion r = qin[k];
-                    R.sp = r.sp; R.c0 = r.c0; R.c1 = r.c1; R.h0 = r.h0; R.h1 = r.h1;
-                }
-                R.s = R.sp / npix;
-                const int pix = R.sp - R.s * npix;
-                R.h = pix / A.W;
-                R.w = pix - R.h * A.W;
+        const int n = level0 ? 0 : (int)min((long long)counts[level - 1], qcap);
+        const long long nb = level0 ? (long long)S * per_src : (n + 31) / 32;
+        const Queue64 q64{q + 2 * (size_t)qcap, count64 + level, cap64};
+        // batches from the level's counter, the next one taken ahead: batches next to
+        // sources cost several times the others
+        int nxt = 0;
+        if (lane == 0) nxt = atomicAdd(work + level, 1);
+        for (;;) {
+            const int item = __shfl_sync(0xffffffffu, nxt, 0);
+            if (item >= nb) break;
+            if (lane == 0) nxt = atomicAdd(work + level, 1);
+            QRegion r{0, 0.f, 0.f, 1.f, 1.f};
+            bool on;
+            if (level0) {  // a TH x TW patch of pixels, whose points share table rows
+                const int s = item / per_src, p = item - s * per_src, ph = p / pw;
+                const int h = ph * TH + lane / TW, w = (p - ph * pw) * TW + lane % TW;
+                on = h < A.H && w < A.W;
+                if (on) r.sp = s * npix + h * A.W + w;
+            } else {
+                on = item * 32 + lane < n;
+                if (on) r = qin[item * 32 + lane];
             }
-            gm_batch<G>(A, R, on, sq, scoef, win, pts, last, level0, qout, counts + level, (int)qcap);
+            gm_batch<G>(A, lane_region(r, npix, A.W), on, sq, scoef, win, pts, last, level0, qout, counts + level,
+                        (int)qcap, q64);
         }
+        // the level's regions for FP64, spread over all warps
+        if (!grid_barrier(bar, gridDim.x, &gen_s)) {
+            if (threadIdx.x == 0) atomicExch(status, 1);
+            return;
+        }
+        const int n64 = min(*q64.count, q64.cap);
+        for (int k = blockIdx.x + gridDim.x * warp; k < n64; k += gridDim.x * NWARP)
+            gm_fp64(A, lane_region(q64.q[k], npix, A.W), pts, last, level0, qout, counts + level, (int)qcap);
         if (level == max_depth) break;
         if (!grid_barrier(bar, gridDim.x, &gen_s)) {
             if (threadIdx.x == 0) atomicExch(status, 1);
@@ -560,20 +647,24 @@ int launch_adaptive_map(const double* corners, const SrcInfo* info, const double
     // the mean PSF rows in FP32, [S][401][E]
     const int EP = (E + 3) & ~3;  // table rows padded to whole float4s
     float* lut = (float*)workspace(W_LUT, sizeof(float) * (size_t)S * ND * EP + 16);
-    // two region queues (ping-pong), their counters per level and the grid barrier
+    // two region queues (ping-pong) and one for FP64, their counters per level and the grid barrier
     long long cap = 4LL * S * npix;
     cap = cap < (1 << 20) ? (1 << 20) : cap;
     cap = cap > (1 << 26) ? (1 << 26) : cap;
-    QRegion* q = (QRegion*)workspace(W_SPARSE, sizeof(QRegion) * 2 * (size_t)cap + 16);
-    int* counts = (int*)workspace(W_WMETA, sizeof(int) * 64);
+    const int cap64 = 1 << 20;  // regions of one level decided in FP64 (more are decided where they arise)
+    QRegion* q = (QRegion*)workspace(W_SPARSE, sizeof(QRegion) * (2 * (size_t)cap + cap64) + 16);
+    int* counts = (int*)workspace(W_WMETA, sizeof(int) * 128);
     if (!lut || !q || !counts) return XTS_ERR_OOM;
     unsigned* bar = (unsigned*)(counts + 32);
+    int* work = counts + 40;     // batches taken per level
+    int* count64 = counts + 64;  // regions for FP64 per level
     XTS_LAUNCH("k_lut_scaled", st, k_lut_scaled<<<lut_scaled_grid(S), 256, 0, st>>>(upsf, nullptr, S, E, EP, lut,
                                                                                        nullptr, nullptr));
-    typedef void (*LevelsFn)(LevelArgs, const SepTab*, int, int, QRegion*, long long, int*, unsigned*, int*);
-    const LevelsFn levels = E <= 32 ? k_adaptive_levels<8> : E <= 64 ? k_adaptive_levels<16> : k_adaptive_levels<32>;
+    typedef void (*LevelsFn)(LevelArgs, const SepTab*, int, int, QRegion*, long long, int, int*, int*, int*,
+                             unsigned*, int*);
+    const LevelsFn levels = E <= 64 ? k_adaptive_levels<8> : k_adaptive_levels<32>;
     XTS_CUDA(cudaFuncSetAttribute(levels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A_SMEM));
-    XTS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * 64, st));
+    XTS_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * 128, st));
     int dev = 0, nsm = 148, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -592,8 +683,8 @@ int launch_adaptive_map(const double* corners, const SrcInfo* info, const double
     cfg.numAttrs = 1;
     const LevelArgs la{corners, info, lut, upsf, H, W, E, EP, (float)rtol, mean64};
     cudaError_t le = cudaSuccess;
-    XTS_LAUNCH("k_adaptive_map", st, le = cudaLaunchKernelEx(&cfg, levels, la, tab, S, max_depth, q, cap, counts, bar,
-                                                             status));
+    XTS_LAUNCH("k_adaptive_map", st, le = cudaLaunchKernelEx(&cfg, levels, la, tab, S, max_depth, q, cap, cap64, counts,
+                                                             work, count64, bar, status));
     if (le != cudaSuccess) return cuda_error(le, "cooperative launch of k_adaptive_levels");
     return XTS_OK;
 }
