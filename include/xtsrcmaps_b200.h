@@ -200,7 +200,7 @@ int xts_compute_psf_data(const xts_grid* psf_front, const xts_grid* psf_back,
  * is a DEVICE pointer (no flags argument; XTS_DEVICE_PTRS is implied) and the
  * launches go to `stream` (NULL = the legacy default stream) on the current
  * device, without xts_init.  The King and psf*aeff scratch tables live in one
- * fixed 8 MiB device array that the library holds on every GPU that loads it
+ * fixed device array (8.07 MiB) that the library holds on every GPU that loads it
  * until the process exits: shapes needing more than XTS_NOALLOC_SCRATCH_DOUBLES
  * doubles, 401 * (Mc*Me front + Mc*Me back) rounded up to a multiple of 32, plus
  * C * 401 * E, fail with XTS_ERR_ARG and launch nothing.  All calls share that

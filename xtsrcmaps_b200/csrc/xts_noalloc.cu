@@ -15,7 +15,7 @@
 //     tables, 401 * (Mc*Me front + Mc*Me back), rounded up to a multiple of 32,
 //     then the psf*aeff table, C * 401 * E; larger shapes are rejected with
 //     XTS_ERR_ARG before anything is launched;
-//   * every GPU that loads the library holds the 8 MiB array until the process
+//   * every GPU that loads the library holds the array (8.07 MiB) until the process
 //     exits;
 //   * all calls share the array; each call overwrites every scratch element it
 //     reads, so nothing has to start at zero, but calls that overlap on the GPU
@@ -32,11 +32,14 @@
 
 namespace xts {
 
-int launch_psf_scratch(const PsfDev& a, double* king, double* pa, cudaStream_t st);  // xts_psf.cu
+int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, cudaStream_t st);  // xts_psf.cu
 
 constexpr size_t NOALLOC_SCRATCH_DOUBLES = XTS_NOALLOC_SCRATCH_DOUBLES;
 
-static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_SCRATCH_DOUBLES];
+// beside the NOALLOC_SCRATCH_DOUBLES that the limit counts the array holds the padding of
+// the psf*aeff rows from 401 to 404 doubles, and 3 x 404 doubles of row tables at its end
+constexpr size_t NOALLOC_TABS = NOALLOC_SCRATCH_DOUBLES + NOALLOC_SCRATCH_DOUBLES / 128;
+static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_TABS + 3 * 404];
 
 static double* g_noalloc_ptr[64] = {};
 static std::mutex g_noalloc_mu;
@@ -110,5 +113,5 @@ extern "C" int xts_compute_psf_data_noalloc(const xts_grid* psf_front, const xts
     a.ecb = ecb; a.wecb = wecb; a.S = S;
     a.ltf = front_ltf; a.exposure = exposure;
     a.upsf = upsf; a.partial = partial;
-    return launch_psf_scratch(a, scratch, scratch + pa_off, (cudaStream_t)stream);
+    return launch_psf_scratch(a, scratch, scratch + pa_off, scratch + NOALLOC_TABS, (cudaStream_t)stream);
 }
