@@ -429,8 +429,20 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
 }
 
 // ============================================================================ pass B
-constexpr int BT = 256;  // pixels per tile == threads per block
+// Work unit: a pair of pixels (2i, w), (2i + 1, w) per lane, 32 consecutive pairs of the
+// source's map in (i, w) order per warp and tile.  Per float4 of output and table row an
+// LDS.128 returns 512 bytes to the warp (four cycles of the SM's 128 bytes), whether or
+// not the lanes' rows agree; a pair's two windows overlap (a table row is 3.4 % of the
+// separation wide), so one load of their common rows feeds both pixels: about 3 rows per
+// pair instead of 2 x 2.5.  Sums go quad by quad as packed FMAs straight into the stage,
+// 4, 8 or 16 bytes per store as E allows (an even E at 4 bytes per lane has 2- to 4-way
+// bank conflicts).  Without its stores the pass takes 1.40 ms of 2.34 (400 x 400 x 37 x
+// 500 sources; one pixel per lane at a time: 2.2), so HBM bounds it; where few warps fit
+// beside the table (E = 50: 10) that is what it gains: 40 sources x 800 x 800 x 50 1.33 ->
+// 1.04 ms.
 constexpr int BQ = 13;   // float4 quads of a table row at most: E <= 52
+constexpr int BWMAX = 16;  // warps per block at most
+constexpr int NU = 6;    // common rows of a pair on the fast path
 
 // Table row stride in float4 units: ceil(E/4), made odd.
 static int win_row_quads(int E) {
@@ -438,78 +450,224 @@ static int win_row_quads(int E) {
     return (nq & 1) ? nq : nq + 1;
 }
 
+// Shared memory of a block of nw warps: the source's table, per warp two stages (the
+// pair's upper and lower pixels) of 32 pixels and the alignment pads, an mbarrier.
 struct WinLayout { size_t tab, stage, bar, total; };
-static __host__ __device__ WinLayout win_layout(int E, int EQ) {
+static __host__ __device__ int stage_floats(int E) { return (32 * E + 8 + 3) / 4 * 4; }
+static __host__ __device__ WinLayout win_layout(int E, int EQ, int nw) {
     WinLayout L;
     L.tab = 0;                                            // [ND + RW][EQ] float4 (RW zero guard rows)
-    L.stage = (size_t)(ND + RW) * EQ * 16;                // per warp [32 * E + 8] floats
-    L.bar = (L.stage + sizeof(float) * (size_t)(BT / 32) * (32 * E + 8) + 15) / 16 * 16;
+    L.stage = (size_t)(ND + RW) * EQ * 16;
+    L.bar = L.stage + sizeof(float) * (size_t)nw * 2 * stage_floats(E);
     L.total = L.bar + 16;
     return L;
 }
-
-// One pixel's record as read by pass B: the main record, and for a window of more
-// than REC_ROWS rows its extension.
-struct PixRec { int meta; float4 wa, wb; };
-
-__device__ __forceinline__ PixRec load_rec(const float4* rec, const float4* ext, size_t k, bool valid) {
-    PixRec r;
-    r.meta = 0;
-    r.wa = make_float4(0.f, 0.f, 0.f, 0.f);
-    r.wb = r.wa;
-    if (valid) {
-        const float4 m = __ldg(rec + k);
-        r.meta = __float_as_int(m.w);
-        r.wa = make_float4(m.x, m.y, m.z, 0.f);
-        if (r.meta >= 0 && (r.meta >> 16) > REC_ROWS) {
-            r.wa = __ldg(ext + 2 * k);
-            r.wb = __ldg(ext + 2 * k + 1);
-        }
-    }
-    return r;
+// Warps per block: as many as shared memory holds beside the table, at most BWMAX; 12
+// where the window records come from HBM rather than L2 (more than half of the 126 MB).
+// Reads between the map's writes cost HBM more than their bytes (a bare copy of the pass's
+// traffic at 400 x 400 x 37 x 500: 2.32-2.40 ms with the records, 1.86-1.90 without), and
+// with more warps more so: 2.34 ms with 12, 2.40 with 14, 2.50 with 16, 2.56 with 10; 50
+// sources x 200 x 200 (32 MB of records): 119 us with 12, 100 with 16.
+// Small jobs take as few warps per block as give every SM a block.
+static int win_warps(int E, size_t rec_bytes, long long pairs, int nsm) {
+    int nw = rec_bytes > ((size_t)63 << 20) ? 12 : BWMAX;
+    const long long share = (pairs + 32LL * nsm - 1) / (32LL * nsm);
+    if (share < nw) nw = share < 1 ? 1 : (int)share;
+    while (nw > 0 && win_layout(E, win_row_quads(E), nw).total > 227 * 1024) --nw;
+    return nw;
 }
 
-// Warps run independently: each owns 32 pixels of the tile, a slice of the
-// stage and its own TMA bulk store, so no block barrier is needed except when the
-// block moves on to the next source's table.
-// Pixels of a source in the write pass: the dense map (every source H * W pixels,
-// records from s * npix, output from (s_base + s) * npix) or a cutout window
-// (cut[s].nh * cut[s].nw pixels, records and output from cut[s].offset).
+// A source's pixels in the write pass: the dense map (H x W, records from s * npix,
+// output from (s_base + s) * npix) or a cutout window (records and output from
+// cut[s].offset).
 template <bool CUT>
 struct SrcSpan {
     const xts_cutout* cut;
-    int S, s_base, npix;
-    __device__ __forceinline__ int pixels(int s) const {
-        if (!CUT) return npix;
-        return s < S ? cut[s].nh * cut[s].nw : 0;
+    int S, s_base, H, W, by;  // by: pairs per block and tile
+    __device__ __forceinline__ int rows(int s) const { return !CUT ? H : s < S ? cut[s].nh : 0; }
+    __device__ __forceinline__ int cols(int s) const { return !CUT ? W : s < S ? cut[s].nw : 0; }
+    __device__ __forceinline__ long long rec_base(int s) const {
+        return CUT ? cut[s].offset : (long long)s * ((long long)H * W);
     }
-    __device__ __forceinline__ long long rec_base(int s) const { return CUT ? cut[s].offset : (long long)s * npix; }
     __device__ __forceinline__ long long out_base(int s) const {
-        return CUT ? cut[s].offset : (long long)(s_base + s) * npix;
+        return CUT ? cut[s].offset : (long long)(s_base + s) * ((long long)H * W);
     }
-    __device__ __forceinline__ int tiles(int s) const { return (pixels(s) + BT - 1) / BT; }
+    __device__ __forceinline__ int pairs(int s) const { return (rows(s) + 1) / 2 * cols(s); }
+    __device__ __forceinline__ int tiles(int s) const { return (pairs(s) + by - 1) / by; }
 };
 
+// One lane's place in a source's pairs and the main records of its pixels (hasB: the
+// pair has a lower pixel).
+struct PixPair { int i, col, pix; bool on, hasB; float4 ra, rb; };
+
+template <bool CUT>
+__device__ __forceinline__ void load_pair(PixPair& P, const SrcSpan<CUT>& sp, const float4* win, int s, bool more) {
+    P.ra = P.rb = make_float4(0.f, 0.f, 0.f, 0.f);
+    P.on = P.hasB = false;
+    P.pix = 0;
+    if (more) {
+        const int H = sp.rows(s), W = sp.cols(s);
+        P.on = 2 * P.i < H;
+        P.hasB = 2 * P.i + 1 < H;
+        P.pix = 2 * P.i * W + P.col;
+        const float4* r = win + sp.rec_base(s) + P.pix;
+        if (P.on) P.ra = __ldg(r);
+        if (P.hasB) P.rb = __ldg(r + W);
+    }
+}
+
+__device__ __forceinline__ int rec_rows(const float4& r) { const int m = __float_as_int(r.w); return m < 0 ? 0 : m >> 16; }
+__device__ __forceinline__ int rec_first(const float4& r) { const int m = __float_as_int(r.w); return m < 0 ? 0 : m & 0xffff; }
+
+// A quad of one pixel's values into the stage (dst: the pixel's quad, VW floats aligned),
+// of which the first n count.
+template <int VW>
+__device__ __forceinline__ void store_quad(float* dst, int n, float2 lo, float2 hi) {
+    if (VW == 4) {
+        *(float4*)dst = make_float4(lo.x, lo.y, hi.x, hi.y);
+    } else if (VW == 2) {
+        *(float2*)dst = lo;
+        if (n > 2) *(float2*)(dst + 2) = hi;
+    } else {
+        dst[0] = lo.x;
+        if (n > 1) dst[1] = lo.y;
+        if (n > 2) dst[2] = hi.x;
+        if (n > 3) dst[3] = hi.y;
+    }
+}
+
+// Both pixels' values from their K common rows (first row lo); packed FP32 FMAs.  Rows
+// past a pixel's own window carry weight 0 (the table ends in RW zero rows).
+template <int NQ, int K, int VW>
+__device__ __forceinline__ void pair_values(const float4* tab, int EQ, const float4& ra, const float4& rb, int oa, int ob,
+                                            int lo, bool hasB, float* da, float* db, int E) {
+    const float4* row[K];
+    float2 wa[K], wb[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        row[j] = tab + (lo + j) * EQ;
+        const float a = j == oa ? ra.x : j == oa + 1 ? ra.y : j == oa + 2 ? ra.z : 0.f;
+        const float b = j == ob ? rb.x : j == ob + 1 ? rb.y : j == ob + 2 ? rb.z : 0.f;
+        wa[j] = make_float2(a, a);
+        wb[j] = make_float2(b, b);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        float2 a0 = make_float2(0.f, 0.f), a1 = a0, b0 = a0, b1 = a0;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const float4 y = row[j][q];
+            const float2 y0 = make_float2(y.x, y.y), y1 = make_float2(y.z, y.w);
+            a0 = __ffma2_rn(wa[j], y0, a0);
+            a1 = __ffma2_rn(wa[j], y1, a1);
+            b0 = __ffma2_rn(wb[j], y0, b0);
+            b1 = __ffma2_rn(wb[j], y1, b1);
+        }
+        const int n = q < NQ - 1 ? 4 : E - 4 * (NQ - 1);
+        store_quad<VW>(da + 4 * q, n, a0, a1);
+        if (hasB) store_quad<VW>(db + 4 * q, n, b0, b1);
+    }
+}
+
+template <int NQ, int VW>
+__device__ __forceinline__ void pair_values_k(int kmax, const float4* tab, int EQ, const float4& ra, const float4& rb,
+                                              int oa, int ob, int lo, bool hasB, float* da, float* db, int E) {
+    if (kmax <= 3) pair_values<NQ, 3, VW>(tab, EQ, ra, rb, oa, ob, lo, hasB, da, db, E);
+    else if (kmax <= 4) pair_values<NQ, 4, VW>(tab, EQ, ra, rb, oa, ob, lo, hasB, da, db, E);
+    else pair_values<NQ, NU, VW>(tab, EQ, ra, rb, oa, ob, lo, hasB, da, db, E);
+}
+
+// One pixel's values by itself: a window of any length, a sparse record, or (sparse pool
+// full) point by point from the table with a compensated sum.
+template <int NQ>
+__device__ __noinline__ void pixel_values(const float4* tab, int EQ, int E, const float4& rec, const float4* ext,
+                                          const float2* sparse, const double* corners, const double* omega,
+                                          const SrcInfo* info, const SepTab* septab, int W1, int h, int w, size_t om,
+                                          float* dst) {
+    const int meta = __float_as_int(rec.w);
+    if (meta == META_OVERFLOW) {
+        const SrcInfo si = *info;
+        const PixGeom g = pixel_geom(corners, W1, h, w, si);
+        const float o = omega ? (float)omega[om] : 1.f;
+        const float* Y = (const float*)tab;
+        const int ES = 4 * EQ;
+        for (int e = 0; e < E; ++e) {
+            float acc1 = 0.f, comp = 0.f;
+            for (int p = 0; p < 12; ++p) {
+                float tt;
+                const int idx = point_row(point_q(g, p), septab->q, (const float4*)septab->coef, &tt);
+                const float wgt = (float)c_rule_uv[p][3];
+                const float* yl = Y + (idx - 1) * ES + e;
+                const float term = fmaf((1.f - tt) * wgt, yl[0], tt * wgt * yl[ES]);
+                const float s2 = acc1 + term;
+                comp += fabsf(acc1) >= fabsf(term) ? (acc1 - s2) + term : (term - s2) + acc1;
+                acc1 = s2;
+            }
+            dst[e] = (acc1 + comp) * o;
+        }
+        return;
+    }
+    const int n = meta < 0 ? NSP : meta >> 16, r0 = meta < 0 ? 0 : meta & 0xffff;
+    const float2* se = sparse + (size_t)(meta < 0 ? -1 - meta : 0) * NSP;
+    float4 wx = rec, wy = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (meta >= 0 && n > REC_ROWS) {
+        wx = __ldg(ext);
+        wy = __ldg(ext + 1);
+    }
+    float4 acc[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < n; ++j) {
+        float wj;
+        int row = r0 + j;
+        if (meta < 0) {
+            const float2 e = __ldg(se + j);
+            wj = e.x;
+            row = __float_as_int(e.y);
+        } else {
+            wj = j == 0 ? wx.x : j == 1 ? wx.y : j == 2 ? wx.z : j == 3 ? wx.w
+               : j == 4 ? wy.x : j == 5 ? wy.y : j == 6 ? wy.z : wy.w;
+        }
+        const float4* yr = tab + row * EQ;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const float4 y = yr[q];
+            acc[q].x = fmaf(wj, y.x, acc[q].x);
+            acc[q].y = fmaf(wj, y.y, acc[q].y);
+            acc[q].z = fmaf(wj, y.z, acc[q].z);
+            acc[q].w = fmaf(wj, y.w, acc[q].w);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+        store_quad<1>(dst + 4 * q, q < NQ - 1 ? 4 : E - 4 * (NQ - 1), make_float2(acc[q].x, acc[q].y),
+                      make_float2(acc[q].z, acc[q].w));
+}
+
+// Warps run independently: each owns 32 pairs of the tile, its stages and its own TMA bulk
+// stores, so no block barrier is needed except when the block moves on to the next
+// source's table.  One block per SM.
 template <int NQ, bool CUT>
-__global__ void __launch_bounds__(BT, 2)
+__global__ void __launch_bounds__(32 * BWMAX, 1)
 k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, const float2* __restrict__ sparse,
              const float* __restrict__ lut, const double* __restrict__ corners, const double* __restrict__ omega,
              const SrcInfo* __restrict__ info, const SepTab* __restrict__ septab, const xts_cutout* __restrict__ cut,
              const long long* __restrict__ tile_off,
              int S, int s_base, int H, int W, int E, int EQ, int* status, float* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const WinLayout L = win_layout(E, EQ);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nthr = blockDim.x;
+    const WinLayout L = win_layout(E, EQ, nthr >> 5);
     float4* tab = (float4*)(smem + L.tab);
-    const unsigned bar = smem_u32(smem + L.bar);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    float* stage = (float*)(smem + L.stage) + warp * (32 * E + 8);
+    const unsigned bar = smem_u32(smem + L.bar), full = 0xffffffffu;
+    const int sf = stage_floats(E);
+    float* stage = (float*)(smem + L.stage) + warp * 2 * sf;
     const int W1 = W + 1;
-    const SrcSpan<CUT> sp_{cut, S, s_base, H * W};
-    const long long T = CUT ? tile_off[S] : (long long)S * sp_.tiles(0);
+    const SrcSpan<CUT> sp{cut, S, s_base, H, W, nthr};
+    const long long T = CUT ? tile_off[S] : (long long)S * sp.tiles(0);
     const long long f0 = T * blockIdx.x / gridDim.x, f1 = T * (blockIdx.x + 1) / gridDim.x;
     const unsigned tab_bytes = (unsigned)(ND * EQ * 16);
 
-    for (int k = t; k < RW * EQ; k += BT) tab[ND * EQ + k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = t; k < RW * EQ; k += nthr) tab[ND * EQ + k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t == 0) mbar_init(bar, 1);
     __syncthreads();
 
@@ -527,38 +685,35 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
         while (s < S && tile_off[s + 1] <= f0) ++s;  // skip sources without tiles
         tile = (int)(f0 - tile_off[s]);
     } else {
-        s = (int)(f0 / sp_.tiles(0));
-        tile = (int)(f0 - (long long)s * sp_.tiles(0));
+        s = (int)(f0 / sp.tiles(0));
+        tile = (int)(f0 - (long long)s * sp.tiles(0));
     }
-    int np_s = sp_.pixels(s), nt_s = sp_.tiles(s);
-    const bool any = f0 < f1 && s < S;
-    PixRec rec = load_rec(win, ext, any ? (size_t)(sp_.rec_base(s) + tile * BT + t) : 0, any && tile * BT + t < np_s);
+    // the lane's pair of a tile: (i, col) by one division per source, then by steps of nthr
+    PixPair P;
+    int step_i = 0, step_c = 0;
+    auto place = [&](int src, int tl) {
+        const int Wn = max(sp.cols(src), 1), y = tl * nthr + t;
+        P.i = y / Wn;
+        P.col = y - P.i * Wn;
+        step_i = nthr / Wn;
+        step_c = nthr - step_i * Wn;
+    };
+    place(min(s, S - 1), tile);
+    load_pair(P, sp, win, s, f0 < f1 && s < S && tile * nthr + t < sp.pairs(s));
     for (long long f = f0; f < f1; ++f) {
         int sn = s, tn = tile + 1;  // the next tile
-        while (tn >= sp_.tiles(sn) && sn < S) { tn = 0; ++sn; }
-        int s2 = sn, t2 = tn + 1;   // and the one after
-        while (t2 >= sp_.tiles(s2) && s2 < S) { t2 = 0; ++s2; }
-        const int px0 = tile * BT + warp * 32;  // this warp's first pixel
-        const int npw = min(32, np_s - px0);                                // may be <= 0 in the last tile
-        const long long g0 = (sp_.out_base(s) + px0) * E;                   // first flat output of the whole map
-        const int m = (int)(g0 & 3);                                        // staging residue
-        const int nflat = npw > 0 ? npw * E : 0;
-        const int pix = px0 + lane;
-
-        // the next tile's records, in flight while this tile is computed, and the
-        // one after that on its way into L2
-        PixRec nxt;
-        {
-            const int pn = tn * BT;
-            const bool more = f + 1 < f1 && sn < S;
-            nxt = load_rec(win, ext, more ? (size_t)(sp_.rec_base(sn) + pn + t) : 0,
-                           more && pn + t < sp_.pixels(sn));
-            const int p2 = t2 * BT;
-            if (f + 2 < f1 && s2 < S && p2 + t < sp_.pixels(s2) && (t & 7) == 0) {  // one prefetch per 128-byte line
-                const size_t k2 = (size_t)(sp_.rec_base(s2) + p2 + t);
-                asm volatile("prefetch.global.L2 [%0];" :: "l"(win + k2));
-            }
+        while (tn >= sp.tiles(sn) && sn < S) { tn = 0; ++sn; }
+        // the next tile's records, in flight while this tile is computed
+        const PixPair C = P;
+        const int Ws = sp.cols(s);
+        if (sn == s) {
+            P.i += step_i;
+            P.col += step_c;
+            if (P.col >= Ws) { P.col -= Ws; ++P.i; }
+        } else if (sn < S) {
+            place(sn, tn);
         }
+        load_pair(P, sp, win, sn, f + 1 < f1 && sn < S && tn * nthr + t < sp.pairs(sn));
         if (s != cur) {
             __syncthreads();  // every warp is done with the previous source's table
             if (t == 0) {
@@ -573,144 +728,96 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
                     atomicExch(status, 1);
                     mbar_wait(bar, phase ^ 1);  // bounded: let the copy land before the block exits
                 }
-                if (lane == 0) bulk_wait_all();
+                if ((lane & 7) == 0) bulk_wait_all();
                 return;
             }
         }
-        // entries of this pixel: window rows rbase + j (j < nr), or a sparse record
-        const int meta = rec.meta;
-        const bool valid = lane < npw;
-        const bool sp = valid && meta < 0 && meta != META_OVERFLOW;
-        const bool slow = valid && meta == META_OVERFLOW;
-        const int nent = sp ? NSP : (meta >= 0 ? (meta >> 16) : 0);
-        const int rb = meta >= 0 ? (meta & 0xffff) : 0;
-        const float2* se = sparse + (size_t)(sp ? -1 - meta : 0) * NSP;
-        const int kmax = __reduce_max_sync(0xffffffffu, nent);
-        const float w[RW] = {rec.wa.x, rec.wa.y, rec.wa.z, rec.wa.w, rec.wb.x, rec.wb.y, rec.wb.z, rec.wb.w};
-        float4 acc[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (kmax <= RW) {  // window records only (warp-uniform)
-#pragma unroll
-            for (int j = 0; j < RW; ++j) {
-                if (j < kmax && j < nent) {  // rows past a pixel's own window carry weight 0: lanes
-                    const float4* yr = tab + (rb + j) * EQ;  // past theirs issue no shared loads
-                    const float wj = w[j];
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) {
-                        const float4 y = yr[q];
-                        acc[q].x = fmaf(wj, y.x, acc[q].x);
-                        acc[q].y = fmaf(wj, y.y, acc[q].y);
-                        acc[q].z = fmaf(wj, y.z, acc[q].z);
-                        acc[q].w = fmaf(wj, y.w, acc[q].w);
-                    }
-                }
-            }
-        } else {  // some lanes hold sparse records (pixels next to the source)
-#pragma unroll 1
-            for (int j = 0; j < NSP; ++j) {
-                float wj = 0.f;
-                int row = rb;
-#pragma unroll
-                for (int i = 0; i < RW; ++i)
-                    if (i == j) wj = w[i];
-                if (j < RW) row = rb + j;
-                if (sp) {
-                    const float2 e = __ldg(se + j);
-                    wj = e.x;
-                    row = __float_as_int(e.y);
-                }
-                const float4* yr = tab + row * EQ;
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const float4 y = yr[q];
-                    acc[q].x = fmaf(wj, y.x, acc[q].x);
-                    acc[q].y = fmaf(wj, y.y, acc[q].y);
-                    acc[q].z = fmaf(wj, y.z, acc[q].z);
-                    acc[q].w = fmaf(wj, y.w, acc[q].w);
-                }
-            }
-        }
-        // the stage is reused only now: the previous bulk store's read-out overlapped the sums
-        if (lane == 0) bulk_wait_read();
+        const int nv = __popc(__ballot_sync(full, C.on));  // lanes with pixels (the first nv)
+        // runs of consecutive pixels: lanes [0, n1) end a map row, lanes [n1, nv) begin the
+        // next pair's; a pixel's stage position is its flat output index modulo 4
+        const int n1 = min(Ws - __shfl_sync(full, C.col, 0), nv);
+        const bool narrow = Ws < 32;  // more runs than two: written by plain stores
+        const int pix0 = __shfl_sync(full, C.pix, 0), pix1 = __shfl_sync(full, C.pix, n1 & 31);
+        const unsigned ob = (unsigned)sp.out_base(s), uE = (unsigned)E;  // (residues: 32 bits suffice)
+        auto residue = [&](int pix, int l) { return (int)(((ob + (unsigned)pix - (unsigned)l) * uE) & 3u); };
+        int mA0 = residue(pix0, 0), mB0 = residue(pix0 + Ws, 0);
+        int mA1 = mA0 + ((residue(pix1, n1) - mA0) & 3), mB1 = mB0 + ((residue(pix1 + Ws, n1) - mB0) & 3);
+        if (narrow) mA0 = mA1 = mB0 = mB1 = 0;
+        float* da = stage + (lane < n1 ? mA0 : mA1) + lane * E;
+        float* db = stage + sf + (lane < n1 ? mB0 : mB1) + lane * E;
+
+        // the stages are reused only now: the previous bulk stores' read-out overlapped the loads
+        if ((lane & 7) == 0) bulk_wait_read();
         __syncwarp();
-        float* dst = stage + m + lane * E;
-        if (valid && !slow) {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const int e = 4 * q;
-                dst[e] = acc[q].x;
-                if (q < NQ - 1 || e + 1 < E) dst[e + 1] = acc[q].y;
-                if (q < NQ - 1 || e + 2 < E) dst[e + 2] = acc[q].z;
-                if (q < NQ - 1 || e + 3 < E) dst[e + 3] = acc[q].w;
+        const int na = rec_rows(C.ra), nb = rec_rows(C.rb), fa = rec_first(C.ra), fb = C.hasB ? rec_first(C.rb) : fa;
+        const int lo = min(fa, fb), n = max(fa + na, fb + nb) - lo;
+        const bool own = C.on && (__float_as_int(C.ra.w) < 0 || __float_as_int(C.rb.w) < 0 || na > REC_ROWS ||
+                                  nb > REC_ROWS || n > NU);
+        const int kmax = __reduce_max_sync(full, C.on ? n : 0);
+        if (!__any_sync(full, own)) {
+            if (C.on) {
+                if (!(E & 3)) pair_values_k<NQ, 4>(kmax, tab, EQ, C.ra, C.rb, fa - lo, fb - lo, lo, C.hasB, da, db, E);
+                else if (!(E & 1)) pair_values_k<NQ, 2>(kmax, tab, EQ, C.ra, C.rb, fa - lo, fb - lo, lo, C.hasB, da, db, E);
+                else pair_values_k<NQ, 1>(kmax, tab, EQ, C.ra, C.rb, fa - lo, fb - lo, lo, C.hasB, da, db, E);
             }
-        }
-        if (slow) {  // sparse pool full: point by point from the shared table, compensated sum
-            const SrcInfo si = info[s];
-            int h, wc;
+        } else if (C.on) {
+            int h = 2 * C.i, w = C.col;  // (the lower pixel: h + 1)
+            const size_t k = (size_t)(sp.rec_base(s) + C.pix);
             if (CUT) {
-                const xts_cutout cw = cut[s];
-                h = cw.h0 + pix / cw.nw;
-                wc = cw.w0 + pix % cw.nw;
-            } else {
-                h = pix / W;
-                wc = pix - h * W;
+                h += cut[s].h0;
+                w += cut[s].w0;
             }
-            const PixGeom g = pixel_geom(corners, W1, h, wc, si);
-            const float om = omega ? (float)omega[(size_t)h * W + wc] : 1.f;
-            const float* Y = (const float*)tab;
-            const int ES = 4 * EQ;
-            for (int e = 0; e < E; ++e) {
-                float acc1 = 0.f, comp = 0.f;
-                for (int p = 0; p < 12; ++p) {
-                    float tt;
-                    const int idx = point_row(point_q(g, p), septab->q, (const float4*)septab->coef, &tt);
-                    const float wgt = (float)c_rule_uv[p][3];
-                    const float* yl = Y + (idx - 1) * ES + e;
-                    const float term = fmaf((1.f - tt) * wgt, yl[0], tt * wgt * yl[ES]);
-                    const float s2 = acc1 + term;
-                    comp += fabsf(acc1) >= fabsf(term) ? (acc1 - s2) + term : (term - s2) + acc1;
-                    acc1 = s2;
-                }
-                dst[e] = (acc1 + comp) * om;
-            }
+            for (int b = 0; b < (C.hasB ? 2 : 1); ++b)
+                pixel_values<NQ>(tab, EQ, E, b ? C.rb : C.ra, ext + 2 * (k + (b ? Ws : 0)), sparse, corners, omega,
+                                 info + s, septab, W1, h + b, w, (size_t)(h + b) * W + w, b ? db : da);
         }
         fence_async_shared();
         __syncwarp();
-        // TMA bulk store of the warp's 16-byte aligned body, lanes for the edges
-        if (nflat > 0) {
-            const long long ga = (g0 + 3) & ~3LL, gb = (g0 + nflat) & ~3LL;
-            if (lane == 0 && gb > ga)
-                bulk_store(out + ga, stage + m + (int)(ga - g0), (unsigned)((gb - ga) * 4));
-            if (lane < 8) {
-                const long long g = lane < 4 ? g0 + lane : gb + (lane - 4);
-                const bool head = lane < 4 && g < ga && g < g0 + nflat;
-                const bool tail = lane >= 4 && g >= gb && g >= ga && g < g0 + nflat;
-                if (head || tail) out[g] = stage[m + (int)(g - g0)];
+        const unsigned hb = __ballot_sync(full, C.hasB);
+        if (!narrow) {
+            // eight lanes per run: a TMA bulk store of its 16-byte aligned body, lanes for the edges
+            const int l = lane & 7, lower = (lane >> 3) & 1;
+            const bool second = lane >= 16;
+            const int l0 = second ? n1 : 0, cnt = (second ? nv : n1) - l0;
+            if (cnt > 0 && (!lower || ((hb >> l0) & 1))) {
+                const int m = lower ? (second ? mB1 : mB0) : (second ? mA1 : mA0);
+                const float* src = stage + lower * sf + m + l0 * E;
+                float* dst = out + (sp.out_base(s) + (second ? pix1 : pix0) + lower * Ws) * E;
+                const int nf = cnt * E, head = min((int)((4u - (unsigned)(m + l0 * E)) & 3u), nf);
+                const int body = (nf - head) & ~3;
+                if (l == 0 && body > 0) bulk_store(dst + head, src + head, (unsigned)body * 4u);
+                const int e = l < 4 ? l : head + body + l - 4;
+                if (l < 4 ? e < head : e < nf) dst[e] = src[e];
             }
-        }
-        rec = nxt;
-        if (sn != s) {
-            np_s = sp_.pixels(sn);
-            nt_s = sp_.tiles(sn);
+        } else {
+            for (int l = 0; l < nv; ++l) {
+                const int pix = __shfl_sync(full, C.pix, l);
+                for (int e = lane; e < E; e += 32) {
+                    float* o = out + (sp.out_base(s) + pix) * E + e;
+                    o[0] = stage[l * E + e];
+                    if ((hb >> l) & 1) o[(size_t)Ws * E] = stage[sf + l * E + e];
+                }
+            }
+            __syncwarp();
         }
         s = sn;
         tile = tn;
     }
-    (void)nt_s;
-    if (lane == 0) bulk_wait_all();
+    if ((lane & 7) == 0) bulk_wait_all();
 }
 
 struct WriteArgs {
     const float4* win; const float4* ext; const float2* sparse; const float* lut;
     const double* corners; const double* omega; const SrcInfo* info; const SepTab* tab;
-    const xts_cutout* cut; const long long* tile_off;  // cutouts (cut != NULL): tile_off [S + 1]
+    const xts_cutout* cut; const long long* tile_off;  // cutouts (cut != NULL): tile_off [S + 1] in tiles of pairs
     int S, s_base, H, W, E, EQ;
     int* status; float* out;
 };
 
 template <int NQ>
-static int launch_write_pass(unsigned G, size_t smem, cudaStream_t st, const WriteArgs& a, int* per_sm, bool query) {
+static int launch_write_pass(unsigned G, int warps, size_t smem, cudaStream_t st, const WriteArgs& a, int* per_sm,
+                             bool query) {
+    const int BT = 32 * warps;
     if (query) {
         int pd = 0, pc = 0;
         XTS_CUDA(cudaFuncSetAttribute(k_srcmap_win<NQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -731,7 +838,7 @@ static int launch_write_pass(unsigned G, size_t smem, cudaStream_t st, const Wri
     return XTS_OK;
 }
 
-typedef int (*WritePassFn)(unsigned, size_t, cudaStream_t, const WriteArgs&, int*, bool);
+typedef int (*WritePassFn)(unsigned, int, size_t, cudaStream_t, const WriteArgs&, int*, bool);
 static const WritePassFn k_write_pass[BQ] = {
     launch_write_pass<1>, launch_write_pass<2>, launch_write_pass<3>, launch_write_pass<4>, launch_write_pass<5>,
     launch_write_pass<6>, launch_write_pass<7>, launch_write_pass<8>, launch_write_pass<9>, launch_write_pass<10>,
@@ -739,7 +846,7 @@ static const WritePassFn k_write_pass[BQ] = {
 
 // ============================================================================ host
 bool srcmap_win_supported(int E) {
-    return E >= 1 && E <= 4 * BQ && win_layout(E, win_row_quads(E)).total <= 227 * 1024;
+    return E >= 1 && E <= 4 * BQ && win_warps(E, 0, 1LL << 40, 1) > 0;
 }
 
 // Parts per source group of the dense window pass (n sources of ntile tiles, G
@@ -781,13 +888,17 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     const bool pipe = gs != st;
     const int npix = H * W;
     const int EQ = win_row_quads(E);
-    const WinLayout L = win_layout(E, EQ);
     // sources per chunk: window records of at most ~1 GiB per buffer
     const size_t budget = (size_t)4 << 30;
     int Sc = (int)(budget / win_bytes_per_source(npix));
     if (chunk_sources > 0 && chunk_sources < Sc) Sc = chunk_sources;
     if (g_tuning.chunk_sources > 0 && g_tuning.chunk_sources < Sc) Sc = g_tuning.chunk_sources;
     Sc = Sc < 1 ? 1 : (Sc > S ? S : Sc);
+    int dev = 0, nsm = 148, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int nw = win_warps(E, (size_t)Sc * npix * 16, (long long)Sc * ((H + 1) / 2) * W, nsm);
+    const WinLayout L = win_layout(E, EQ, nw);
     const size_t rec_n = (size_t)Sc * npix + 4, ext_n = (size_t)Sc * npix * 2 + 4;
     const size_t lut_n = (size_t)Sc * ND * EQ * 4 + 4;
     // sparse records for wide pixels: room for 1/8 of the chunk's pixels (at least 64k)
@@ -799,9 +910,6 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     float4* ext0 = (float4*)workspace(W_WMETA, sizeof(float4) * 2 * ext_n);
     float* lut0 = (float*)workspace(W_LUT, sizeof(float) * 2 * lut_n);
     float2* sparse0 = (float2*)workspace(W_SPARSE, sizeof(float2) * 2 * sp_n);
-    int dev = 0, nsm = 148, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     // pass A: one block per work item, items sized for about 16 per block of the
     // resident set (at most window_blocks_per_sm blocks per SM)
     int resident = 0;
@@ -815,7 +923,7 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     double* hist0 = (double*)workspace(W_PARTSUM, sizeof(double) * 2 * hist_n);
     if (!rec0 || !ext0 || !lut0 || !sparse0 || !hist0) return XTS_ERR_OOM;
     const WritePassFn wp = k_write_pass[(E + 3) / 4 - 1];
-    rc = wp(0, L.total, st, WriteArgs{}, &per_sm, true);
+    rc = wp(0, nw, L.total, st, WriteArgs{}, &per_sm, true);
     if (rc) return rc;
     if (per_sm < 1) return set_error(XTS_ERR_ARG, "source-map write pass does not fit on an SM (E=%d)", E);
     cudaEvent_t evA[2], evB[2];  // window pass of a buffer done; write pass of a buffer done
@@ -855,13 +963,13 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
                                    in_fov ? in_fov + s0 : nullptr, st, lut, EQ * 4);
             if (rc) return rc;
         }
-        const long long T = (long long)n * ((npix + BT - 1) / BT);
+        const long long T = (long long)n * (((H + 1) / 2 * W + 32 * nw - 1) / (32 * nw));
         long long G = (long long)nsm * (g_tuning.write_blocks_per_sm > 0 && g_tuning.write_blocks_per_sm < per_sm
                                             ? g_tuning.write_blocks_per_sm : per_sm);
         if (G > T) G = T;
         WriteArgs wa{rec, ext, sparse, lut, corners, means_only ? nullptr : omega, info + s0, tab, nullptr, nullptr,
                      n, s0, H, W, E, EQ, status, out};
-        rc = wp((unsigned)G, L.total, st, wa, nullptr, false);
+        rc = wp((unsigned)G, nw, L.total, st, wa, nullptr, false);
         if (rc) return rc;
         if (on_chunk && (rc = on_chunk(on_chunk_ctx, s0, n, st))) return rc;
         if (pipe) XTS_CUDA(cudaEventRecord(evB[b], st));
@@ -873,8 +981,12 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
 // Items of the cutout work queue: tile_off[s] = the first (source, tile) item of
 // source s (tiles of WT pixels of its window), tile_off[S] = the item count.  One
 // block; the sources in runs of 1024 with a block scan.
-__global__ void __launch_bounds__(1024) k_cut_tiles(const xts_cutout* __restrict__ cut, int S,
-                                                    long long* __restrict__ tile_off) {
+// For the write pass the same of tiles of `by` pixel pairs: pair_off.
+__global__ void __launch_bounds__(1024) k_cut_tiles(const xts_cutout* __restrict__ cut, int S, int by,
+                                                    long long* __restrict__ tile_off,
+                                                    long long* __restrict__ pair_off) {
+    // (two scans, one block each)
+    if (blockIdx.x) tile_off = pair_off;
     __shared__ long long part[32];
     __shared__ long long carry_s;
     const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
@@ -882,7 +994,10 @@ __global__ void __launch_bounds__(1024) k_cut_tiles(const xts_cutout* __restrict
     __syncthreads();
     for (int s0 = 0; s0 < S; s0 += 1024) {
         const int s = s0 + t;
-        const long long n = s < S ? ((long long)cut[s].nh * cut[s].nw + WT - 1) / WT : 0;
+        long long n = 0;
+        if (s < S)
+            n = blockIdx.x ? ((long long)(cut[s].nh + 1) / 2 * cut[s].nw + by - 1) / by
+                           : ((long long)cut[s].nh * cut[s].nw + WT - 1) / WT;
         long long inc = n;
         for (int o = 1; o < 32; o <<= 1) {
             const long long v = __shfl_up_sync(0xffffffffu, inc, o);
@@ -916,7 +1031,11 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     if ((rc = build_septab(st, &tab))) return rc;
     const long long npix = (long long)H * W;
     const int EQ = win_row_quads(E);
-    const WinLayout L = win_layout(E, EQ);
+    int dev = 0, nsm = 148, resident = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int nw = win_warps(E, (size_t)S * npix * 16, (long long)S * npix / 2, nsm);
+    const WinLayout L = win_layout(E, EQ, nw);
     // buffers sized for the largest windows (every window the whole map): nothing here
     // depends on the windows' sizes on the host, so the call needs no synchronisation
     const long long max_items = (long long)S * ((npix + WT - 1) / WT);
@@ -928,9 +1047,11 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     cap = cap < 65536 ? 65536 : cap;
     float2* sparse = (float2*)workspace(W_SPARSE, sizeof(float2) * ((size_t)NSP * cap + 2));
     double* hist = (double*)workspace(W_PARTSUM, sizeof(double) * ((size_t)S * ND + 1));
-    char* items = (char*)workspace(W_CUT_ITEMS, align_up(sizeof(long long) * (S + 1), 256) +
+    char* items = (char*)workspace(W_CUT_ITEMS, 2 * align_up(sizeof(long long) * (S + 1), 256) +
                                                     align_up(sizeof(int) * (size_t)max_items, 256) + 256);
     if (!rec || !ext || !lut || !sparse || !hist || !items) return XTS_ERR_OOM;
+    long long* pair_off = (long long*)items;
+    items += align_up(sizeof(long long) * (S + 1), 256);
     long long* tile_off = (long long*)items;
     int* item_src = (int*)(items + align_up(sizeof(long long) * (S + 1), 256));
     unsigned long long* queue = (unsigned long long*)(items + align_up(sizeof(long long) * (S + 1), 256) +
@@ -939,11 +1060,8 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * (size_t)S * ND, st));
     XTS_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
     XTS_CUDA(cudaMemsetAsync(sparse_count, 0, sizeof(int), st));
-    XTS_LAUNCH("k_cut_tiles", st, k_cut_tiles<<<1, 1024, 0, st>>>(cut, S, tile_off));
+    XTS_LAUNCH("k_cut_tiles", st, k_cut_tiles<<<2, 1024, 0, st>>>(cut, S, 32 * nw, tile_off, pair_off));
     XTS_LAUNCH("k_cut_item_src", st, k_cut_item_src<<<S, 256, 0, st>>>(tile_off, item_src));
-    int dev = 0, nsm = 148, resident = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows_cut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WA_SMEM));
     XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows_cut, WT, WA_SMEM));
     resident = resident < 1 ? 1 : resident;
@@ -956,12 +1074,12 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
                            st, lut, EQ * 4);
     if (rc) return rc;
     const WritePassFn wp = k_write_pass[(E + 3) / 4 - 1];
-    if ((rc = wp(0, L.total, st, WriteArgs{}, &per_sm, true))) return rc;
+    if ((rc = wp(0, nw, L.total, st, WriteArgs{}, &per_sm, true))) return rc;
     if (per_sm < 1) return set_error(XTS_ERR_ARG, "source-map write pass does not fit on an SM (E=%d)", E);
-    WriteArgs wa{rec, ext, sparse, lut, corners, omega, info, tab, cut, tile_off, S, 0, H, W, E, EQ, status, out};
+    WriteArgs wa{rec, ext, sparse, lut, corners, omega, info, tab, cut, pair_off, S, 0, H, W, E, EQ, status, out};
     if (g_tuning.write_blocks_per_sm > 0 && g_tuning.write_blocks_per_sm < per_sm) per_sm = g_tuning.write_blocks_per_sm;
     // pass B: one persistent wave over the same items, split evenly between the blocks
-    return wp((unsigned)(nsm * per_sm), L.total, st, wa, nullptr, false);
+    return wp((unsigned)(nsm * per_sm), nw, L.total, st, wa, nullptr, false);
 }
 
 }  // namespace xts
