@@ -184,6 +184,10 @@ int launch_correction(const double* hist, int nch, const SrcInfo* info, int S, c
                       const double* partial, const double* exposure, int E, double* scale,
                       double* inv_integ, double* correction, double* radius, int* in_fov,
                       cudaStream_t st, float* lut = nullptr, int Epad = 0);  // lut: scaled FP32 table too
+int launch_srcmap_f64(const double* corners, const double* centers, const double* omega, const SrcInfo* info, int S,
+                      int H, int W, int E, const double* upsf, const double* partial, const double* exposure,
+                      double* scale, double* inv_integ, double* correction, double* radius, int* in_fov, double* out,
+                      StreamJoin& geo, cudaStream_t st);
 bool srcmap_win_supported(int E);
 int make_psf_kernel(const xts_wcs& wcs, int Nk, const double* upsf, int E, double* kernel, cudaStream_t st);
 int convolve_map_psf(const double* image, int E, int H, int W, const double* kernel, int K, double* out,

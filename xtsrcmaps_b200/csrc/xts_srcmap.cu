@@ -21,62 +21,17 @@
 //
 // The map is written once: a first pass gives the map integral of every in-FOV
 // source from the pixels whose centre lies within the boundary radius (FP64 row
-// histograms: k_map_integral_hist here for the FP64 path, the window pass of
+// histograms: the row pass of xts_srcmap_f64.cu for the FP64 path, the window pass of
 // xts_srcmap_win.cu for the default FP32 path); k_correction_hist folds them in a
 // fixed order into 1/sum and the containment factor; the write pass then stores
 // value * omega * exposure * factor.  Computing the integral before the write
 // costs less than writing the raw map and reading it back.
 #include <math.h>
 
-#include <type_traits>
-
 #include "xts_geom.cuh"
 #include "xts_internal.cuh"
 
 namespace xts {
-
-// Sommariva & Festa degree-7 12-point rule on [-1,1]^2 (Padova
-// "cub_square_lowcard"), as tabulated in model_map/mm_cubature/cubature.hpp:209-225.
-static const double SQUARE_DEG7[36] = {
-    3.9383136101878902e-01, -3.6699793434042738e-01, 5.2092862230230441e-01,
-    8.0196847620659251e-01, 8.0992592975809186e-01, 2.3740240561379911e-01,
-    -1.8327327664247231e-02, 9.2596092593108370e-01, 2.4166897208389651e-01,
-    3.6699793434042738e-01, 3.9383136101878902e-01, 5.2092862230230441e-01,
-    -8.0992592975809186e-01, 8.0196847620659251e-01, 2.3740240561379911e-01,
-    -9.2596092593108370e-01, -1.8327327664247231e-02, 2.4166897208389651e-01,
-    -3.9383136101878902e-01, 3.6699793434042738e-01, 5.2092862230230441e-01,
-    -8.0196847620659251e-01, -8.0992592975809186e-01, 2.3740240561379911e-01,
-    1.8327327664247231e-02, -9.2596092593108370e-01, 2.4166897208389651e-01,
-    -3.6699793434042738e-01, -3.9383136101878902e-01, 5.2092862230230441e-01,
-    8.0992592975809186e-01, -8.0196847620659251e-01, 2.3740240561379911e-01,
-    9.2596092593108370e-01, 1.8327327664247231e-02, 2.4166897208389651e-01,
-};
-
-constexpr int NPTS = 12;
-// Per point: 0.25*(1-u)(1-v), 0.25*(1+u)(1-v), 0.25*(1+u)(1+v), 0.25*(1-u)(1+v)
-// (corner weights for LL, LR, UR, UL) and 0.25*w.  Scaling by 0.25 is exact, so
-// these reproduce points_weights.hpp:96-107 bit for bit.
-__constant__ double c_blend[NPTS][5];
-
-static int upload_rule(cudaStream_t st) {
-    static int dev_done = -1;
-    int dev = -1;
-    cudaGetDevice(&dev);
-    if (dev_done == dev) return XTS_OK;
-    double b[NPTS][5];
-    for (int p = 0; p < NPTS; ++p) {
-        double u = SQUARE_DEG7[3 * p], v = SQUARE_DEG7[3 * p + 1];
-        b[p][0] = 0.25 * ((1.0 - u) * (1.0 - v));
-        b[p][1] = 0.25 * ((1.0 + u) * (1.0 - v));
-        b[p][2] = 0.25 * ((1.0 + u) * (1.0 + v));
-        b[p][3] = 0.25 * ((1.0 - u) * (1.0 + v));
-        b[p][4] = 0.25 * SQUARE_DEG7[3 * p + 2];
-    }
-    XTS_CUDA(cudaMemcpyToSymbolAsync(c_blend, b, sizeof(b), 0, cudaMemcpyHostToDevice, st));
-    XTS_CUDA(cudaStreamSynchronize(st));
-    dev_done = dev;
-    return XTS_OK;
-}
 
 // ---------------------------------------------------------------- geometry grids
 // corners[i][j] = pix2dir(i + 0.5, j + 0.5), centres[i][j] = pix2dir(i + 1, j + 1),
@@ -218,152 +173,6 @@ __global__ void __launch_bounds__(256) k_boundary_chord(WcsDev w, const double* 
         si.pad = 0;
         info[s] = si;
     }
-}
-
-// ---------------------------------------------------------------- cubature core
-// c2 + c3 for one pixel: the 12 rule points, their LUT columns and the
-// collapsed interpolation weights, in order of first appearance.
-__device__ __forceinline__ int pixel_columns(const double* corners, int W1, int h, int w,
-                                             const double* src, int* keys, double* va, double* vb) {
-    const double* a = corners + 3 * (h * W1 + w);            // LL (h+0.5, w+0.5)
-    const double* b = corners + 3 * (h * W1 + w + 1);        // LR (h+0.5, w+1.5)
-    const double* c = corners + 3 * ((h + 1) * W1 + w + 1);  // UR (h+1.5, w+1.5)
-    const double* d = corners + 3 * ((h + 1) * W1 + w);      // UL (h+1.5, w+0.5)
-    double A[3] = {a[0], a[1], a[2]}, B[3] = {b[0], b[1], b[2]};
-    double Cc[3] = {c[0], c[1], c[2]}, D[3] = {d[0], d[1], d[2]};
-    int n = 0;
-#pragma unroll
-    for (int p = 0; p < NPTS; ++p) {
-        double nn = c_blend[p][0], pn = c_blend[p][1], pp = c_blend[p][2], np = c_blend[p][3];
-        double wt = c_blend[p][4];
-        double x = (nn * A[0] + pn * B[0] + pp * Cc[0] + np * D[0]) - src[0];
-        double y = (nn * A[1] + pn * B[1] + pp * Cc[1] + np * D[1]) - src[1];
-        double z = (nn * A[2] + pn * B[2] + pp * Cc[2] + np * D[2]) - src[2];
-        double s = 2.0 * R2D * asin(0.5 * sqrt(x * x + y * y + z * z));
-        double j = s < 1e-4 ? 1. : 1. + RECIPSTEP * (LN_1E4 + log(s));
-        int idx = 1 + (int)j;
-        idx = idx > 400 ? 400 : (idx < 2 ? 2 : idx);  // the lower clamp only catches non-finite input
-        double t = REDM1 * (s * 1e4 * exp(SEP_STEP * (2. - idx)) - 1.);
-        int k = 0;
-        while (k < n && keys[k] != idx) ++k;
-        if (k == n) { keys[n] = idx; va[n] = 0.; vb[n] = 0.; ++n; }
-        va[k] += (1.0 - t) * wt;
-        vb[k] += t * wt;
-    }
-    return n;
-}
-
-constexpr int TP = 128;  // pixels per tile (flat h*W + w order)
-
-struct PixCols32 { float va[NPTS], vb[NPTS]; short key[NPTS]; int n; };
-struct PixCols64 { double va[NPTS], vb[NPTS]; short key[NPTS]; int n; };
-
-
-// d1 + d2 + c8 + c10: evaluate every pixel of a tile and write the scaled map.
-// Phase 1: one thread per pixel computes its columns (FP64 separations).
-// Phase 2: threads walk the tile's output in flat (pixel, energy) order so
-// global stores are coalesced.
-template <bool F64>
-__global__ void __launch_bounds__(TP) k_srcmap(const double* corners, const double* omega,
-                                               const SrcInfo* info, const float* lut32,
-                                               const double* upsf, const double* scale, int H,
-                                               int W, int E, int Epad, void* outp) {
-    __shared__ typename std::conditional<F64, PixCols64, PixCols32>::type cols[TP];
-    __shared__ double som[TP];
-    int tile = blockIdx.x, s = blockIdx.y;
-    int npix = H * W, W1 = W + 1;
-    int pix0 = tile * TP;
-    int npt = min(TP, npix - pix0);
-    SrcInfo si = info[s];
-    if (threadIdx.x < npt) {
-        int pix = pix0 + threadIdx.x;
-        int h = pix / W, w = pix - h * W;
-        int keys[NPTS]; double va[NPTS], vb[NPTS];
-        int n = pixel_columns(corners, W1, h, w, si.dir, keys, va, vb);
-        for (int k = 0; k < n; ++k) {
-            cols[threadIdx.x].key[k] = (short)keys[k];
-            cols[threadIdx.x].va[k] = va[k];
-            cols[threadIdx.x].vb[k] = vb[k];
-        }
-        cols[threadIdx.x].n = n;
-        som[threadIdx.x] = omega[pix];
-    }
-    __syncthreads();
-    const double* sc = scale + (size_t)s * E;
-    size_t base = ((size_t)s * npix + pix0) * E;
-    int nout = npt * E;
-    if (F64) {
-        const double* U = upsf + (size_t)s * ND * E;
-        double* out = (double*)outp + base;
-        for (int f = threadIdx.x; f < nout; f += blockDim.x) {
-            int p = f / E, e = f - p * E;
-            const PixCols64& c = *(const PixCols64*)&cols[p];
-            double raw = 0.;
-            for (int k = 0; k < c.n; ++k)
-                raw += (c.va[k] * U[(size_t)(c.key[k] - 1) * E + e]) + (c.vb[k] * U[(size_t)c.key[k] * E + e]);
-            out[f] = ((raw * som[p]) * sc[e]);
-        }
-    } else {
-        const float* Y = lut32 + (size_t)s * ND * Epad;
-        float* out = (float*)outp + base;
-        for (int f = threadIdx.x; f < nout; f += blockDim.x) {
-            int p = f / E, e = f - p * E;
-            const PixCols32& c = *(const PixCols32*)&cols[p];
-            // compensated (Neumaier) sum over the pixel's columns
-            float acc = 0.f, comp = 0.f;
-            for (int k = 0; k < c.n; ++k) {
-                float term = fmaf(c.va[k], __ldg(Y + (c.key[k] - 1) * Epad + e), c.vb[k] * __ldg(Y + c.key[k] * Epad + e));
-                float t = acc + term;
-                comp += fabsf(acc) >= fabsf(term) ? (acc - t) + term : (term - t) + acc;
-                acc = t;
-            }
-            out[f] = (float)((double)(acc + comp) * (som[p] * sc[e]));
-        }
-    }
-}
-
-// c7 as a row histogram: sum_pix omega * value(pix, e) = sum_r Hist[r] * uPsf[r][e]
-// with Hist[r] = sum over pixels in the radius of omega * (interpolation weight
-// on row r).  Each block accumulates one chunk of pixels of one in-FOV source
-// into a shared FP64 histogram; k_correction_hist folds the chunks.
-__global__ void __launch_bounds__(256) k_map_integral_hist(const double* corners, const double* centers,
-                                                           const double* omega, const SrcInfo* info,
-                                                           int H, int W, int nch, double* hist_out) {
-    __shared__ double hist[ND];
-    int s = blockIdx.y, ch = blockIdx.x;
-    SrcInfo si = info[s];
-    double* out = hist_out + ((size_t)s * nch + ch) * ND;
-    if (!si.in_fov) {
-        for (int r = threadIdx.x; r < ND; r += blockDim.x) out[r] = 0.;
-        return;
-    }
-    for (int r = threadIdx.x; r < ND; r += blockDim.x) hist[r] = 0.;
-    __syncthreads();
-    // chord^2 of the radius; pixels within a relative 1e-12 of it take the
-    // reference's own test 2 asin(|d|/2) <= radius
-    double ch2 = 2.0 * sin(0.5 * si.radius_rad);
-    ch2 *= ch2;
-    int npix = H * W, W1 = W + 1;
-    for (int pix = ch * blockDim.x + threadIdx.x; pix < npix; pix += nch * blockDim.x) {
-        int h = pix / W, w = pix - h * W;
-        const double* c = centers + 3 * (h * W1 + w);
-        double x = si.dir[0] - c[0], y = si.dir[1] - c[1], z = si.dir[2] - c[2];
-        double d2 = x * x + y * y + z * z;
-        bool inside;
-        if (d2 < ch2 * (1.0 - 1e-12)) inside = true;
-        else if (d2 > ch2 * (1.0 + 1e-12)) inside = false;
-        else inside = dir_diff(si.dir, c) <= si.radius_rad;
-        if (!inside) continue;
-        int keys[NPTS]; double va[NPTS], vb[NPTS];
-        int n = pixel_columns(corners, W1, h, w, si.dir, keys, va, vb);
-        double om = omega[pix];
-        for (int k = 0; k < n; ++k) {
-            atomicAdd(&hist[keys[k] - 1], va[k] * om);
-            atomicAdd(&hist[keys[k]], vb[k] * om);
-        }
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < ND; r += blockDim.x) out[r] = hist[r];
 }
 
 // c9 map_correction_factor (model_map.map_correction_factor.cxx:3-53): the PSF
@@ -555,14 +364,11 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
     // stream before uPsf is read, and on every early return
     StreamJoin geo(a.geo_stream && a.join_ev ? a.geo_stream : st, st, a.join_ev);
     cudaStream_t gs = geo.from;
-    int rc = upload_rule(st);
-    if (rc) return rc;
+    int rc = XTS_OK;
     int H = (int)a.wcs.naxis1, W = (int)a.wcs.naxis2, S = a.S, E = a.E;
     WcsDev w = make_wcs(a.wcs);
     size_t ng = (size_t)(H + 1) * (W + 1);
     int npix = H * W;
-    int ntiles = (npix + TP - 1) / TP;
-    int Epad = (E + 3) & ~3;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -617,21 +423,15 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
                                  a.exposure, scale, a.inv_integ, a.correction, a.radius, a.in_fov, status,
                                  (float*)a.out, a.chunk_sources, a.on_chunk, a.on_chunk_ctx, geo, st);
     }
+    if (a.out_f64)
+        return launch_srcmap_f64(corners, centers, omega, info, S, H, W, E, a.upsf, a.partial, a.exposure, scale,
+                                 a.inv_integ, a.correction, a.radius, a.in_fov, (double*)a.out, geo, st);
     if ((rc = geo.join())) return rc;
-    if (a.out_f64) {  // the reference's own per-point FP64 arithmetic throughout
-        XTS_LAUNCH("k_map_integral_f64", st, k_map_integral_hist<<<dim3(nch, S), 256, 0, st>>>(corners, centers, omega, info, H, W, nch, hist));
-    } else {
-        rc = launch_map_integral_fast(corners, centers, omega, info, S, H, W, nch, hist, st);
-        if (rc) return rc;
-    }
+    rc = launch_map_integral_fast(corners, centers, omega, info, S, H, W, nch, hist, st);
+    if (rc) return rc;
     rc = launch_correction(hist, nch, info, S, a.upsf, a.partial, a.exposure, E, scale, a.inv_integ,
                            a.correction, a.radius, a.in_fov, st);
     if (rc) return rc;
-    if (a.out_f64) {
-        XTS_LAUNCH("k_srcmap_f64", st, k_srcmap<true><<<dim3(ntiles, S), TP, 0, st>>>(corners, omega, info, nullptr, a.upsf, scale,
-                                                                                        H, W, E, Epad, a.out));
-        return XTS_OK;
-    }
     if (a.kernel == SRCMAP_TCGEN05 && E <= 128) {
         int* status = (int*)workspace(W_MISC, 64);
         if (!status) return XTS_ERR_OOM;
