@@ -33,15 +33,34 @@
 namespace xts {
 
 // ============================================================================ pass A
-constexpr int WT = 256;  // pixels per tile == threads per block
-constexpr int NSG = 4;   // sources per group: one pixel's source-independent geometry serves NSG sources
+constexpr int WT = 256;     // pixels per tile == threads per block
+constexpr int NSG_MAX = 8;  // sources per group: one pixel's source-independent geometry serves the group
 
+// A source as the window pass needs it: the boundary test's limits beside its direction.
+struct WinSrc {
+    double dir[3], ch2, radius_rad;  // ch2: squared chord of the boundary radius
+    int in_fov, pad;
+};
+__device__ __forceinline__ WinSrc win_source(const SrcInfo& si) {
+    WinSrc w;
+    w.dir[0] = si.dir[0]; w.dir[1] = si.dir[1]; w.dir[2] = si.dir[2];
+    const double c = 2.0 * sin(0.5 * si.radius_rad);
+    w.ch2 = c * c;
+    w.radius_rad = si.radius_rad;
+    w.in_fov = si.in_fov;
+    w.pad = 0;
+    return w;
+}
+
+// Shared memory of the window pass for nsg sources per group.
 constexpr size_t WA_OFF_BINS = 0;
 constexpr size_t WA_OFF_COEF = sizeof(SepBin) * NSB;
-constexpr size_t WA_OFF_HIST = WA_OFF_COEF + sizeof(float4) * 2 * ND;
-constexpr size_t WA_OFF_WTS = WA_OFF_HIST + (8 * NSG * ND + 15) / 16 * 16;
+constexpr size_t WA_OFF_Q = WA_OFF_COEF + sizeof(float4) * 2 * ND;
+constexpr size_t WA_OFF_D1 = WA_OFF_Q + sizeof(double) * (ND + 1);
+constexpr size_t WA_OFF_WTS = (WA_OFF_D1 + sizeof(float) * ND + 15) / 16 * 16;
 constexpr size_t WA_OFF_SRC = WA_OFF_WTS + sizeof(float) * WT * RW;
-constexpr size_t WA_SMEM = WA_OFF_SRC + sizeof(SrcInfo) * NSG;
+constexpr size_t WA_OFF_HIST = WA_OFF_SRC + sizeof(WinSrc) * NSG_MAX;
+constexpr size_t wa_smem(int nsg) { return WA_OFF_HIST + sizeof(double) * ND * (size_t)nsg; }
 
 constexpr int NSP = 24;  // entries of a sparse record: 12 points x 2 rows
 constexpr int META_OVERFLOW = -0x7fffffff - 1;  // wide pixel without a sparse record
@@ -55,7 +74,9 @@ constexpr float EMSTEP = (float)(REDM1 / (REDM1 + 1.0));  // e^-step: t in row k
 struct PassA {
     const SepBin* sbin;    // shared: row bins
     const float4* scoef;   // shared: per-row records
-    double* hist;          // shared: the block's map-integral rows ([NSG][ND] in the dense pass)
+    const double* sq;      // shared: squared chords of the rows
+    const float* sd1;      // shared: their steps q[k + 1] - q[k]
+    double* hist;          // shared: the block's map-integral rows ([sources of the group][ND])
     float* wts;            // shared: [RW][WT] windows
     float4* rec;
     float4* ext;
@@ -70,6 +91,8 @@ __device__ __forceinline__ PassA pass_a_tables(unsigned char* smem, const SepTab
     PassA A;
     A.sbin = (const SepBin*)(smem + WA_OFF_BINS);
     A.scoef = (const float4*)(smem + WA_OFF_COEF);
+    A.sq = (const double*)(smem + WA_OFF_Q);
+    A.sd1 = (const float*)(smem + WA_OFF_D1);
     A.hist = (double*)(smem + WA_OFF_HIST);
     A.wts = (float*)(smem + WA_OFF_WTS);
     A.rec = rec; A.ext = ext; A.sparse = sparse; A.sparse_cap = sparse_cap; A.sparse_count = sparse_count;
@@ -77,6 +100,13 @@ __device__ __forceinline__ PassA pass_a_tables(unsigned char* smem, const SepTab
     float4* sc = (float4*)(smem + WA_OFF_COEF);
     for (int k = threadIdx.x; k < NSB; k += WT) sb[k] = septab->bins[k];
     for (int k = threadIdx.x; k < 2 * ND; k += WT) sc[k] = ((const float4*)septab->coef)[k];
+    double* sq = (double*)(smem + WA_OFF_Q);
+    float* d1 = (float*)(smem + WA_OFF_D1);
+    for (int k = threadIdx.x; k < ND + 1; k += WT) {
+        const double q = septab->q[k];
+        sq[k] = q;
+        if (k < ND) d1[k] = (float)(septab->q[k + 1] - q);
+    }
     return A;
 }
 
@@ -84,17 +114,22 @@ __device__ __forceinline__ PassA pass_a_tables(unsigned char* smem, const SepTab
 // blend P(u, v) = M + B u + C v + D uv of the corners, so relative to a source s
 // with A = M - s the squared chord is q(u, v) = |A + B u + C v + D uv|^2, whose
 // coefficients split into source-dependent ones (|A|^2, 2 A.B, 2 A.C, 2 A.D) and
-// the rest (|B|^2, |C|^2, 2 B.C, 2 B.D, 2 C.D, |D|^2).  The latter enter each
-// mirror pair's chord offset through eb (even part) and ob (odd part), formed once
-// per pixel for a group of sources.
+// the rest (|B|^2, |C|^2, 2 B.C, 2 B.D, 2 C.D, |D|^2; second-order terms, from the
+// FP32 values of the FP64 differences B, C, D).  The latter enter each mirror pair's
+// chord offset through eb (even part) and ob (odd part), formed once per pixel for a
+// group of sources.  Mirror pairs k and k + 3 have the same weight (the rule's points are
+// three orbits of quarter turns) and go through packed FP32 FMAs together: x holds pair k,
+// y pair k + 3.
 struct PixBase {
     double m[3];      // M, the corners' average (FP64)
-    double c[3];      // pixel centre (boundary-radius test)
     float b2[3], c2[3], d2[3];  // 2B, 2C, 2D
     float bc2;        // 2 B.C
-    float eb[6], ob[6];
+    float2 eb[3], ob[3];
     float om;         // solid angle
+    float off;        // bound on |chord of M - chord of the pixel's centre| per chord: 4.2 |M - centre|
 };
+
+__device__ __forceinline__ float2 pair_c(int k, int j) { return make_float2(c_pair[k][j], c_pair[k + 3][j]); }
 
 __device__ __forceinline__ PixBase pixel_base(const double* __restrict__ corners, const double* __restrict__ centers,
                                               const double* __restrict__ omega, int W1, int h, int w, size_t om_idx) {
@@ -102,30 +137,38 @@ __device__ __forceinline__ PixBase pixel_base(const double* __restrict__ corners
     const double* b = corners + 3 * (h * W1 + w + 1);        // LR
     const double* c = corners + 3 * ((h + 1) * W1 + w + 1);  // UR
     const double* d = corners + 3 * ((h + 1) * W1 + w);      // UL
+    const double* pc = centers + 3 * ((size_t)h * W1 + w);
     PixBase P;
-    double B[3], C[3], D[3];
+    float q4 = 0.f, q5 = 0.f, q6 = 0.f, q7 = 0.f, q8 = 0.f, bc = 0.f, mc = 0.f;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        P.m[i] = 0.25 * ((a[i] + b[i]) + (c[i] + d[i]));
-        B[i] = 0.25 * ((b[i] + c[i]) - (a[i] + d[i]));
-        C[i] = 0.25 * ((c[i] + d[i]) - (a[i] + b[i]));
-        D[i] = 0.25 * ((a[i] + c[i]) - (b[i] + d[i]));
-        P.b2[i] = (float)(2.0 * B[i]);
-        P.c2[i] = (float)(2.0 * C[i]);
-        P.d2[i] = (float)(2.0 * D[i]);
+        const double ac = a[i] + c[i], bd = b[i] + d[i], bad = b[i] - d[i], ca = c[i] - a[i];
+        P.m[i] = 0.25 * (ac + bd);
+        const float B2 = (float)(0.5 * (ca + bad)), C2 = (float)(0.5 * (ca - bad)), D2 = (float)(0.5 * (ac - bd));
+        P.b2[i] = B2;
+        P.c2[i] = C2;
+        P.d2[i] = D2;
+        q4 = fmaf(B2, B2, q4);
+        q5 = fmaf(C2, C2, q5);
+        q6 = fmaf(B2, D2, q6);
+        q7 = fmaf(C2, D2, q7);
+        q8 = fmaf(D2, D2, q8);
+        bc = fmaf(B2, C2, bc);
+        const float x = (float)(P.m[i] - pc[i]);
+        mc = fmaf(x, x, mc);
     }
-    const double* pc = centers + 3 * ((size_t)h * W1 + w);
-    P.c[0] = pc[0]; P.c[1] = pc[1]; P.c[2] = pc[2];
-    const float q4 = (float)fma(B[0], B[0], fma(B[1], B[1], B[2] * B[2]));
-    const float q5 = (float)fma(C[0], C[0], fma(C[1], C[1], C[2] * C[2]));
-    const float q6 = (float)(2.0 * fma(B[0], D[0], fma(B[1], D[1], B[2] * D[2])));
-    const float q7 = (float)(2.0 * fma(C[0], D[0], fma(C[1], D[1], C[2] * D[2])));
-    const float q8 = (float)fma(D[0], D[0], fma(D[1], D[1], D[2] * D[2]));
-    P.bc2 = (float)(2.0 * fma(B[0], C[0], fma(B[1], C[1], B[2] * C[2])));
+    q4 *= 0.25f;  // |B|^2, |C|^2, 2 B.D, 2 C.D, |D|^2 and 2 B.C from the doubled vectors
+    q5 *= 0.25f;
+    q6 *= 0.5f;
+    q7 *= 0.5f;
+    q8 *= 0.25f;
+    P.bc2 = 0.5f * bc;
+    P.off = fmaf(4.2f, sqrtf(mc), 4e-12f);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        P.eb[k] = fmaf(q8, c_pair[k][7], fmaf(q5, c_pair[k][4], q4 * c_pair[k][3]));
-        P.ob[k] = fmaf(q7, c_pair[k][6], q6 * c_pair[k][5]);
+    for (int k = 0; k < 3; ++k) {
+        P.eb[k] = __ffma2_rn(make_float2(q8, q8), pair_c(k, 7),
+                             __ffma2_rn(make_float2(q5, q5), pair_c(k, 4), __fmul2_rn(make_float2(q4, q4), pair_c(k, 3))));
+        P.ob[k] = __ffma2_rn(make_float2(q7, q7), pair_c(k, 6), __fmul2_rn(make_float2(q6, q6), pair_c(k, 5)));
     }
     P.om = omega ? (float)omega[om_idx] : 1.f;  // omega NULL: the pixel means (unit solid angle)
     return P;
@@ -144,41 +187,48 @@ __device__ __forceinline__ int row_lower(double q, const SepBin* bins) {
 // rows to hist (the source's map-integral rows); the rows they touch widen
 // [*rlo, *rhi] when those are given.  (h, w) and W1 locate the pixel's corners for
 // the rare wide pixel, which is redone in FP64 point by point.
-__device__ __forceinline__ void window_source(const PixBase& P, const SrcInfo& si, double ch2,
-                                              const double* __restrict__ corners, int W1, int h, int w,
+__device__ __forceinline__ void window_source(const PixBase& P, const WinSrc& si,
+                                              const double* __restrict__ corners, const double* __restrict__ centers,
+                                              int W1, int h, int w,
                                               size_t kk, const PassA& A, double* hist, int* rlo, int* rhi) {
     const int t = threadIdx.x;
     const double Ax = P.m[0] - si.dir[0], Ay = P.m[1] - si.dir[1], Az = P.m[2] - si.dir[2];
     const double a0 = fma(Ax, Ax, fma(Ay, Ay, Az * Az));  // q at the centre of the blend
     bool inside = false;
     if (si.in_fov) {
-        const double x = si.dir[0] - P.c[0], y = si.dir[1] - P.c[1], z = si.dir[2] - P.c[2];
-        const double d2 = x * x + y * y + z * z;
-        if (d2 < ch2 * (1.0 - 1e-12)) inside = true;
-        else if (d2 > ch2 * (1.0 + 1e-12)) inside = false;
-        else inside = dir_diff(si.dir, P.c) <= si.radius_rad;
+        // |a0 - the centre's squared chord| <= |M - centre| (|A| + chord) <= 4 |M - centre|: the
+        // centre's own chord decides only within that of the boundary's
+        const float gap = (float)(si.ch2 - a0);
+        if (fabsf(gap) > P.off) {
+            inside = gap > 0.f;
+        } else {
+            const double* pc = centers + 3 * ((size_t)h * W1 + w);
+            const double x = si.dir[0] - pc[0], y = si.dir[1] - pc[1], z = si.dir[2] - pc[2];
+            const double d2 = x * x + y * y + z * z;
+            if (d2 < si.ch2 * (1.0 - 1e-12)) inside = true;
+            else if (d2 > si.ch2 * (1.0 + 1e-12)) inside = false;
+            else inside = dir_diff(si.dir, pc) <= si.radius_rad;
+        }
     }
     // q(point) - a0 in FP32: 2 A.B u + 2 A.C v + (2 A.D + 2 B.C) uv + the pixel's part
     const float ax = (float)Ax, ay = (float)Ay, az = (float)Az;
     const float f1 = fmaf(ax, P.b2[0], fmaf(ay, P.b2[1], az * P.b2[2]));
     const float f2 = fmaf(ax, P.c2[0], fmaf(ay, P.c2[1], az * P.c2[2]));
     const float f3 = fmaf(ax, P.d2[0], fmaf(ay, P.d2[1], fmaf(az, P.d2[2], P.bc2)));
-    float dqs[12];
+    float2 dq2[6];  // pairs (k, k + 3): the points themselves, then their mirror images
     float mn = INFINITY, mx = -INFINITY;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const float E = fmaf(f3, c_pair[k][2], P.eb[k]);
-        const float O = fmaf(f2, c_pair[k][1], fmaf(f1, c_pair[k][0], P.ob[k]));
-        dqs[k] = E + O;
-        dqs[k + 6] = E - O;
-        mn = fminf(mn, fminf(dqs[k], dqs[k + 6]));
-        mx = fmaxf(mx, fmaxf(dqs[k], dqs[k + 6]));
+    for (int k = 0; k < 3; ++k) {
+        const float2 E = __ffma2_rn(make_float2(f3, f3), pair_c(k, 2), P.eb[k]);
+        const float2 O = __ffma2_rn(make_float2(f2, f2), pair_c(k, 1),
+                                    __ffma2_rn(make_float2(f1, f1), pair_c(k, 0), P.ob[k]));
+        dq2[k] = __fadd2_rn(E, O);
+        dq2[k + 3] = __ffma2_rn(O, make_float2(-1.f, -1.f), E);
+        mn = fminf(mn, fminf(fminf(dq2[k].x, dq2[k].y), fminf(dq2[k + 3].x, dq2[k + 3].y)));
+        mx = fmaxf(mx, fmaxf(fmaxf(dq2[k].x, dq2[k].y), fmaxf(dq2[k + 3].x, dq2[k + 3].y)));
     }
     const float om = P.om;
-    auto edge = [&](int k) {  // q[k] - a0 in FP32
-        const float4 cw = A.scoef[2 * k + 1];
-        return (float)(__hiloint2double(__float_as_int(cw.w), __float_as_int(cw.z)) - a0);
-    };
+    auto edge = [&](int k) { return (float)(A.sq[k] - a0); };  // q[k] - a0 in FP32
     // Most pixels' points lie in the centre's table row, or in it and one
     // neighbour.  Then one row's polynomial (fitted over two rows) gives every
     // point's t relative to the lower row kl, u = t - 1; a point past the upper
@@ -187,31 +237,37 @@ __device__ __forceinline__ void window_source(const PixBase& P, const SrcInfo& s
     //     s0 = om (S2 - T),  s2 = om e^-step S2,  s1 = om sum(w) - s0 - s2.
     const int kc = row_lower(a0, A.sbin);  // the centre's lower table row
     if (kc >= 2 && kc <= ND - 4) {
-        const float em1 = edge(kc - 1), e0 = edge(kc), e1 = edge(kc + 1), e2 = edge(kc + 2);
-        // rows kc (and kc + 1), or kc - 1 and kc; eb = +inf for one row.  The case is
-        // made opaque to the compiler: specialising the point loop per case would run
-        // up to three copies of it per warp, each with a part of the lanes.
-        const bool up = mn >= e0 && mx < e2, dn = mn >= em1 && mx < e1;
+        // rows kc (and kc + 1), or kc - 1 and kc; eb = +inf for one row.  The outer edges are
+        // bounds from row kc's width (neighbouring widths differ by 6.0 to 7.0 %), so a few
+        // pixels more than need be go on to the general path; the inner ones are exact to
+        // FP32.  The case is made opaque to the compiler: specialising the point loop per case
+        // would run up to three copies of it per warp, each with a part of the lanes.
+        const float w0 = A.sd1[kc], e0 = edge(kc), e1 = e0 + w0;
+        const bool up = mn >= e0 && mx < fmaf(1.06f, w0, e1), dn = mn >= fmaf(-0.934f, w0, e0) && mx < e1;
         int kl = up ? kc : (dn ? kc - 1 : -1);
         float eb = (mn >= e0 && mx < e1) ? INFINITY : (up ? e1 : e0);
-        float eL = up ? e0 : em1;
-        asm volatile("" : "+r"(kl), "+f"(eb), "+f"(eL));
+        asm volatile("" : "+r"(kl), "+f"(eb));
         if (kl >= 0) {  // (warp-divergent: a warp's pixels usually agree)
             const float4 c0 = A.scoef[2 * kl], c1 = A.scoef[2 * kl + 1];
+            const float eL = (float)(__hiloint2double(__float_as_int(c1.w), __float_as_int(c1.z)) - a0);
             // zz = (dl - C)/H and REDM1 dl, dl = q / q_kl - 1 = (dq - eL) / q_kl, as FMAs in dq
             const float kz = c0.x * (1.f / DPOLY_H), z0 = fmaf(-eL, kz, -DPOLY_C / DPOLY_H);
             const float kr = c0.x * (float)REDM1, r0 = -eL * kr;
-            float T = 0.f, S2 = 0.f;
+            const float2 kz2 = make_float2(kz, kz), z02 = make_float2(z0, z0), kr2 = make_float2(kr, kr);
+            const float2 r02 = make_float2(r0, r0), p0 = make_float2(c0.y, c0.y), p1 = make_float2(c0.z, c0.z);
+            const float2 p2 = make_float2(c0.w, c0.w), p3 = make_float2(c1.x, c1.x), p4 = make_float2(c1.y, c1.y);
+            float2 T2 = make_float2(0.f, 0.f), S22 = T2;
 #pragma unroll
-            for (int p = 0; p < 12; ++p) {
-                const float dq = dqs[p];
-                const float zz = fmaf(dq, kz, z0);
-                const float P4 = fmaf(fmaf(fmaf(fmaf(c1.y, zz, c1.x), zz, c0.w), zz, c0.z), zz, c0.y);
-                const float u = fmaf(fmaf(dq, kr, r0), P4, -1.f);
-                const float wp = c_rule_w32[p];
-                T = fmaf(wp, u, T);
-                S2 = fmaf(dq >= eb ? wp : 0.f, u, S2);
+            for (int k = 0; k < 6; ++k) {
+                const float2 dq = dq2[k];
+                const float2 zz = __ffma2_rn(dq, kz2, z02);
+                const float2 P4 = __ffma2_rn(__ffma2_rn(__ffma2_rn(__ffma2_rn(p4, zz, p3), zz, p2), zz, p1), zz, p0);
+                const float2 u = __ffma2_rn(__ffma2_rn(dq, kr2, r02), P4, make_float2(-1.f, -1.f));
+                const float wp = c_rule_w32[k % 3];
+                T2 = __ffma2_rn(make_float2(wp, wp), u, T2);
+                S22 = __ffma2_rn(make_float2(dq.x >= eb ? wp : 0.f, dq.y >= eb ? wp : 0.f), u, S22);
             }
+            const float T = T2.x + T2.y, S2 = S22.x + S22.y;
             const float s0 = om * (S2 - T), s2 = om * (EMSTEP * S2);
             const float s1 = fmaf(om, c_rule_wsum, -s0) - s2;
             const bool two = eb != INFINITY;
@@ -228,6 +284,14 @@ __device__ __forceinline__ void window_source(const PixBase& P, const SrcInfo& s
             A.rec[kk] = make_float4(s0, s1, s2, __int_as_float(kl | (nent << 16)));
             return;
         }
+    }
+    float dqs[12];  // the rule's points in order: pair k at k, its mirror image at k + 6
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        dqs[k] = dq2[k].x;
+        dqs[k + 3] = dq2[k].y;
+        dqs[k + 6] = dq2[k + 3].x;
+        dqs[k + 9] = dq2[k + 3].y;
     }
     // General path: the window of RW rows around the centre's row, the row edges
     // as FP32 offsets from a0.
@@ -296,7 +360,9 @@ __device__ __forceinline__ void window_source(const PixBase& P, const SrcInfo& s
     } else {
         // a wide pixel (next to the source): its 12 points again with FP64 chords
         // from the corners, for its sparse record and its map-integral rows alike
-        const PixQ g = pixel_q(pixel_geom(corners, W1, h, w, si));
+        SrcInfo sd;
+        sd.dir[0] = si.dir[0]; sd.dir[1] = si.dir[1]; sd.dir[2] = si.dir[2];
+        const PixQ g = pixel_q(pixel_geom(corners, W1, h, w, sd));
         int meta = META_OVERFLOW;
         const int slot = atomicAdd(A.sparse_count, 1);
         float2* sr = slot < A.sparse_cap ? A.sparse + (size_t)slot * NSP : nullptr;
@@ -323,12 +389,7 @@ __device__ __forceinline__ void window_source(const PixBase& P, const SrcInfo& s
     }
 }
 
-__device__ __forceinline__ double boundary_chord2(const SrcInfo& si) {
-    const double c = 2.0 * sin(0.5 * si.radius_rad);
-    return c * c;
-}
-
-// The dense map: block b takes item b = (g, p), part p of the P parts of group g (NSG
+// The dense map: block b takes item b = (g, p), part p of the P parts of group g (nsg
 // sources; tiles [p nt / P, (p + 1) nt / P) of WT pixels), forms each pixel's
 // source-independent geometry once and the windows of the group's sources from it,
 // and adds the item's non-zero rows to hist_out[s] (cleared before the launch) with
@@ -338,20 +399,20 @@ __device__ __forceinline__ double boundary_chord2(const SrcInfo& si) {
 __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restrict__ corners, const double* __restrict__ centers,
                                                       const double* __restrict__ omega, const SrcInfo* __restrict__ info,
                                                       const SepTab* __restrict__ septab, int S, int H, int W,
-                                                      int P,
+                                                      int P, int nsg,
                                                       double* __restrict__ hist_out, float4* __restrict__ rec,
                                                       float4* __restrict__ ext, float2* __restrict__ sparse,
                                                       int sparse_cap, int* __restrict__ sparse_count) {
     extern __shared__ __align__(16) unsigned char smem[];
     const PassA A = pass_a_tables(smem, septab, rec, ext, sparse, sparse_cap, sparse_count);
-    SrcInfo* ssrc = (SrcInfo*)(smem + WA_OFF_SRC);
+    WinSrc* ssrc = (WinSrc*)(smem + WA_OFF_SRC);
     const int t = threadIdx.x;
     const int npix = H * W, W1 = W + 1;
     const int nt = (npix + WT - 1) / WT;
     const int item = blockIdx.x;
-    const int g = item / P, p = item - g * P, s0 = g * NSG, ns = min(NSG, S - s0);
-    if (t < ns) ssrc[t] = info[s0 + t];
-    for (int r = t; r < NSG * ND; r += WT) A.hist[r] = 0.;
+    const int g = item / P, p = item - g * P, s0 = g * nsg, ns = min(nsg, S - s0);
+    if (t < ns) ssrc[t] = win_source(info[s0 + t]);
+    for (int r = t; r < ns * ND; r += WT) A.hist[r] = 0.;
     __syncthreads();
     const int ta = (int)((long long)p * nt / P), tb = (int)((long long)(p + 1) * nt / P);
     for (int tile = ta; tile < tb; ++tile) {
@@ -360,9 +421,8 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restric
         const int h = pix / W, w = pix - h * W;
         const PixBase Q = pixel_base(corners, centers, omega, W1, h, w, (size_t)pix);
         for (int j = 0; j < ns; ++j) {
-            const SrcInfo& si = ssrc[j];
-            window_source(Q, si, boundary_chord2(si), corners, W1, h, w, (size_t)(s0 + j) * npix + pix, A,
-                          A.hist + j * ND, nullptr, nullptr);
+            window_source(Q, ssrc[j], corners, centers, W1, h, w, (size_t)(s0 + j) * npix + pix, A, A.hist + j * ND,
+                          nullptr, nullptr);
         }
     }
     __syncthreads();
@@ -372,9 +432,9 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restric
     }
 }
 
-// Cutouts: one persistent launch over a work queue of (source, tile) items, tile
-// = WT consecutive pixels of the source's window (row-major, nw wide).  A block
-// takes the next item from the queue (one atomic), builds its pixels' records
+// Cutouts: one persistent launch over a work queue of (source, run) items, run = `run`
+// consecutive pixels of the source's window (row-major, nw wide; a multiple of WT).  A
+// block takes the next item from the queue (one atomic), builds its pixels' records
 // and the item's map-integral rows in shared memory, and adds the rows it touched
 // to hist_out[s] with FP64 atomics.  item_src[i] is the source of item i, tile_off[s]
 // its first item and tile_off[S] the number of items.
@@ -386,7 +446,7 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
                                                           const int* __restrict__ item_src,
                                                           const long long* __restrict__ tile_off,
                                                           unsigned long long* __restrict__ queue,
-                                                          const SepTab* __restrict__ septab, int S, int W,
+                                                          const SepTab* __restrict__ septab, int S, int W, int run,
                                                           double* __restrict__ hist_out, float4* __restrict__ rec,
                                                           float4* __restrict__ ext, float2* __restrict__ sparse,
                                                           int sparse_cap, int* __restrict__ sparse_count) {
@@ -394,29 +454,30 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
     __shared__ long long item_s;
     __shared__ int rmin_s, rmax_s;
     const PassA A = pass_a_tables(smem, septab, rec, ext, sparse, sparse_cap, sparse_count);
+    WinSrc* ssrc = (WinSrc*)(smem + WA_OFF_SRC);
     const int t = threadIdx.x, W1 = W + 1;
     for (int r = t; r < ND; r += WT) A.hist[r] = 0.;
     const long long n_items = tile_off[S];
     for (;;) {
         if (t == 0) {
-            item_s = (long long)atomicAdd(queue, 1ull);
+            const long long it = (long long)atomicAdd(queue, 1ull);
+            item_s = it;
             rmin_s = ND;
             rmax_s = -1;
+            if (it < n_items) ssrc[0] = win_source(info[item_src[it]]);
         }
         __syncthreads();  // also orders the previous item's flush before this item's adds
         const long long item = item_s;
         if (item >= n_items) break;
         const int s = item_src[item];
         const xts_cutout cw = cut[s];
-        const SrcInfo si = info[s];
-        const double ch2 = boundary_chord2(si);
-        const long long npix = (long long)cw.nh * cw.nw;
-        const long long pix = (item - tile_off[s]) * WT + t;
-        if (pix < npix) {
-            const int i = (int)(pix / cw.nw), j = (int)(pix - (long long)i * cw.nw);
+        const long long npix = (long long)cw.nh * cw.nw, p0 = (item - tile_off[s]) * run;
+        const long long p1 = min(npix, p0 + run);
+        for (long long pix = p0 + t; pix < p1; pix += WT) {
+            const int i = (int)((unsigned)pix / (unsigned)cw.nw), j = (int)(pix - (long long)i * cw.nw);
             const int h = cw.h0 + i, w = cw.w0 + j;
             const PixBase P = pixel_base(corners, centers, omega, W1, h, w, (size_t)h * W + w);
-            window_source(P, si, ch2, corners, W1, h, w, (size_t)(cw.offset + pix), A, A.hist, &rmin_s, &rmax_s);
+            window_source(P, ssrc[0], corners, centers, W1, h, w, (size_t)(cw.offset + pix), A, A.hist, &rmin_s, &rmax_s);
         }
         __syncthreads();
         for (int r = rmin_s + t; r <= rmax_s; r += WT) {
@@ -849,11 +910,19 @@ bool srcmap_win_supported(int E) {
     return E >= 1 && E <= 4 * BQ && win_warps(E, 0, 1LL << 40, 1) > 0;
 }
 
-// Parts per source group of the dense window pass (n sources of ntile tiles, G
-// blocks): about 16 queue items per block (c2: 1.66 ms at 8, 1.57 at 16, 1.63 at 32),
-// at most one part per tile.
-static int window_parts(int n, int ntile, int G) {
-    const long long ng = (n + NSG - 1) / NSG;
+// Sources per group of the dense window pass: a pixel's own geometry (a third of the work
+// of one source) is formed once per group, while there are items (group, tile) for every
+// resident block twice over.
+static int window_group(int n, int ntile, int G) {
+    int nsg = NSG_MAX;
+    while (nsg > 1 && (long long)((n + nsg - 1) / nsg) * ntile < 2LL * G) nsg >>= 1;
+    return nsg;
+}
+// Parts per source group (n sources of ntile tiles, G blocks): about 16 queue items per
+// block (with 4 sources per group, c2: 1.66 ms at 8, 1.57 at 16, 1.63 at 32), at most one
+// part per tile.
+static int window_parts(int n, int nsg, int ntile, int G) {
+    const long long ng = (n + nsg - 1) / nsg;
     long long P = (16LL * G + ng - 1) / ng;
     if (P > ntile) P = ntile;
     return P < 1 ? 1 : (int)P;
@@ -913,12 +982,13 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     // pass A: one block per work item, items sized for about 16 per block of the
     // resident set (at most window_blocks_per_sm blocks per SM)
     int resident = 0;
-    XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WA_SMEM));
-    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows, WT, WA_SMEM));
+    XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wa_smem(NSG_MAX)));
+    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows, WT, wa_smem(NSG_MAX)));
     resident = resident < 1 ? 1 : resident;
     if (g_tuning.window_blocks_per_sm > 0 && g_tuning.window_blocks_per_sm < resident)
         resident = g_tuning.window_blocks_per_sm;
-    const int nparts = window_parts(Sc, (npix + WT - 1) / WT, resident * nsm);
+    const int ntile = (npix + WT - 1) / WT, nsg = window_group(Sc, ntile, resident * nsm);
+    const int nparts = window_parts(Sc, nsg, ntile, resident * nsm);
     const size_t hist_n = (size_t)Sc * ND + 1;
     double* hist0 = (double*)workspace(W_PARTSUM, sizeof(double) * 2 * hist_n);
     if (!rec0 || !ext0 || !lut0 || !sparse0 || !hist0) return XTS_ERR_OOM;
@@ -941,13 +1011,12 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
         // the window pass is geometry only: it runs on the geometry stream, once
         // the write pass that last read its buffers is done
         if (pipe && k >= 2) XTS_CUDA(cudaStreamWaitEvent(gs, evB[b], 0));
-        const int n_items = (n + NSG - 1) / NSG * nparts;  // one block per item
+        const int n_items = (n + nsg - 1) / nsg * nparts;  // one block per item
         XTS_CUDA(cudaMemsetAsync(sparse_count, 0, sizeof(int), gs));
         XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * (size_t)n * ND, gs));
-        XTS_LAUNCH("k_pixel_windows", gs, k_pixel_windows<<<n_items, WT, WA_SMEM, gs>>>(
+        XTS_LAUNCH("k_pixel_windows", gs, k_pixel_windows<<<n_items, WT, wa_smem(nsg), gs>>>(
                                               corners, centers, means_only ? nullptr : omega, info + s0, tab, n, H, W,
-                                              nparts,
-                                              hist, rec, ext, sparse, (int)cap,
+                                              nparts, nsg, hist, rec, ext, sparse, (int)cap,
                                               sparse_count));
         if (pipe) {
             XTS_CUDA(cudaEventRecord(evA[b], gs));
@@ -979,10 +1048,10 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
 
 // ============================================================================ cutouts
 // Items of the cutout work queue: tile_off[s] = the first (source, tile) item of
-// source s (tiles of WT pixels of its window), tile_off[S] = the item count.  One
+// source s (runs of `run` pixels of its window), tile_off[S] = the item count.  One
 // block; the sources in runs of 1024 with a block scan.
 // For the write pass the same of tiles of `by` pixel pairs: pair_off.
-__global__ void __launch_bounds__(1024) k_cut_tiles(const xts_cutout* __restrict__ cut, int S, int by,
+__global__ void __launch_bounds__(1024) k_cut_tiles(const xts_cutout* __restrict__ cut, int S, int by, int run,
                                                     long long* __restrict__ tile_off,
                                                     long long* __restrict__ pair_off) {
     // (two scans, one block each)
@@ -997,7 +1066,7 @@ __global__ void __launch_bounds__(1024) k_cut_tiles(const xts_cutout* __restrict
         long long n = 0;
         if (s < S)
             n = blockIdx.x ? ((long long)(cut[s].nh + 1) / 2 * cut[s].nw + by - 1) / by
-                           : ((long long)cut[s].nh * cut[s].nw + WT - 1) / WT;
+                           : ((long long)cut[s].nh * cut[s].nw + run - 1) / run;
         long long inc = n;
         for (int o = 1; o < 32; o <<= 1) {
             const long long v = __shfl_up_sync(0xffffffffu, inc, o);
@@ -1039,6 +1108,9 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     // buffers sized for the largest windows (every window the whole map): nothing here
     // depends on the windows' sizes on the host, so the call needs no synchronisation
     const long long max_items = (long long)S * ((npix + WT - 1) / WT);
+    // pixels per item: eight tiles where there are plenty (an item's queue access, barriers and
+    // flush of its rows are then shared by eight pixels per thread), one in small jobs
+    const int run = max_items >= 16384 ? 8 * WT : max_items >= 4096 ? 2 * WT : WT;
     const size_t rec_n = (size_t)S * npix + 4;
     float4* rec = (float4*)workspace(W_WIN, sizeof(float4) * rec_n);
     float4* ext = (float4*)workspace(W_WMETA, sizeof(float4) * 2 * rec_n);
@@ -1060,15 +1132,15 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * (size_t)S * ND, st));
     XTS_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
     XTS_CUDA(cudaMemsetAsync(sparse_count, 0, sizeof(int), st));
-    XTS_LAUNCH("k_cut_tiles", st, k_cut_tiles<<<2, 1024, 0, st>>>(cut, S, 32 * nw, tile_off, pair_off));
+    XTS_LAUNCH("k_cut_tiles", st, k_cut_tiles<<<2, 1024, 0, st>>>(cut, S, 32 * nw, run, tile_off, pair_off));
     XTS_LAUNCH("k_cut_item_src", st, k_cut_item_src<<<S, 256, 0, st>>>(tile_off, item_src));
-    XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows_cut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WA_SMEM));
-    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows_cut, WT, WA_SMEM));
+    XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows_cut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wa_smem(1)));
+    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows_cut, WT, wa_smem(1)));
     resident = resident < 1 ? 1 : resident;
     if (g_tuning.queue_blocks_per_sm > 0 && g_tuning.queue_blocks_per_sm < resident) resident = g_tuning.queue_blocks_per_sm;
     // pass A: one persistent wave pulling (source, tile) items from the queue
-    XTS_LAUNCH("k_pixel_windows", st, k_pixel_windows_cut<<<(unsigned)(resident * nsm), WT, WA_SMEM, st>>>(
-                                          corners, centers, omega, info, cut, item_src, tile_off, queue, tab, S, W,
+    XTS_LAUNCH("k_pixel_windows", st, k_pixel_windows_cut<<<(unsigned)(resident * nsm), WT, wa_smem(1), st>>>(
+                                          corners, centers, omega, info, cut, item_src, tile_off, queue, tab, S, W, run,
                                           hist, rec, ext, sparse, (int)cap, sparse_count));
     rc = launch_correction(hist, 1, info, S, upsf, partial, exposure, E, scale, inv_integ, correction, radius, in_fov,
                            st, lut, EQ * 4);
