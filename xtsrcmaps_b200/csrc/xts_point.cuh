@@ -39,12 +39,15 @@ constexpr int SB_BITS = 5;
 constexpr int NSB = (1025 - SB_EXP0 + 1) << SB_BITS;
 
 // Separation tables shared by every launch (see build_septab).
-struct SepTab {
-    double q[ND + 1];      // squared chord of S[k] (k = 0..400), q[401] = +inf guard
+// The window pass copies the whole of it into shared memory at once.
+struct alignas(16) SepTab {
+    SepBin bins[NSB];
     float coef[ND][8];     // row k (= idx - 1): {1/q[k], c0..c4 of P_k(z), q[k] as two words},
                            // z = (d - DPOLY_C)/DPOLY_H
-    SepBin bins[NSB];
+    double q[ND + 1];      // squared chord of S[k] (k = 0..400), q[401] = +inf guard
+    float d1[ND];          // q[k + 1] - q[k]
 };
+static_assert(sizeof(SepTab) % 16 == 0, "one bulk copy");
 // centre and half-width of the fitted d range, [-0.002, 0.146]: two table rows (the
 // ratio q[k + 2] / q[k] - 1 is at most 0.1445), so one row's polynomial also gives
 // t for the points of the next row (t error below 1e-8 over the range)
@@ -71,6 +74,7 @@ static int build_septab(cudaStream_t st, const SepTab** out) {
         h.q[k] = (double)(ch * ch);
     }
     h.q[ND] = INFINITY;
+    for (int k = 0; k < ND; ++k) h.d1[k] = (float)(h.q[k + 1] - h.q[k]);
     for (int k = 0; k < ND; ++k) {
         for (int j = 0; j < 8; ++j) h.coef[k][j] = 0.f;
         if (k == 0) continue;

@@ -53,12 +53,9 @@ __device__ __forceinline__ WinSrc win_source(const SrcInfo& si) {
 }
 
 // Shared memory of the window pass for nsg sources per group.
-constexpr size_t WA_OFF_BINS = 0;
-constexpr size_t WA_OFF_COEF = sizeof(SepBin) * NSB;
-constexpr size_t WA_OFF_Q = WA_OFF_COEF + sizeof(float4) * 2 * ND;
-constexpr size_t WA_OFF_D1 = WA_OFF_Q + sizeof(double) * (ND + 1);
-constexpr size_t WA_OFF_WTS = (WA_OFF_D1 + sizeof(float) * ND + 15) / 16 * 16;
-constexpr size_t WA_OFF_SRC = WA_OFF_WTS + sizeof(float) * WT * RW;
+constexpr size_t WA_OFF_WTS = sizeof(SepTab);  // (the tables first)
+constexpr size_t WA_OFF_BAR = WA_OFF_WTS + sizeof(float) * WT * RW;
+constexpr size_t WA_OFF_SRC = WA_OFF_BAR + 16;
 constexpr size_t WA_OFF_HIST = WA_OFF_SRC + sizeof(WinSrc) * NSG_MAX;
 constexpr size_t wa_smem(int nsg) { return WA_OFF_HIST + sizeof(double) * ND * (size_t)nsg; }
 
@@ -85,29 +82,36 @@ struct PassA {
     int* sparse_count;
 };
 
-// Shared tables of pass A, loaded by every block (the histogram is zeroed by the caller).
+// Shared tables of pass A: one bulk copy per block, in flight while the caller clears the
+// histogram and prepares its sources; tables_ready() (by every thread, after a block
+// barrier) waits for it.
 __device__ __forceinline__ PassA pass_a_tables(unsigned char* smem, const SepTab* septab, float4* rec, float4* ext,
                                                float2* sparse, int sparse_cap, int* sparse_count) {
     PassA A;
-    A.sbin = (const SepBin*)(smem + WA_OFF_BINS);
-    A.scoef = (const float4*)(smem + WA_OFF_COEF);
-    A.sq = (const double*)(smem + WA_OFF_Q);
-    A.sd1 = (const float*)(smem + WA_OFF_D1);
+    const SepTab* tab = (const SepTab*)smem;
+    A.sbin = tab->bins;
+    A.scoef = (const float4*)tab->coef;
+    A.sq = tab->q;
+    A.sd1 = tab->d1;
     A.hist = (double*)(smem + WA_OFF_HIST);
     A.wts = (float*)(smem + WA_OFF_WTS);
     A.rec = rec; A.ext = ext; A.sparse = sparse; A.sparse_cap = sparse_cap; A.sparse_count = sparse_count;
-    SepBin* sb = (SepBin*)(smem + WA_OFF_BINS);
-    float4* sc = (float4*)(smem + WA_OFF_COEF);
-    for (int k = threadIdx.x; k < NSB; k += WT) sb[k] = septab->bins[k];
-    for (int k = threadIdx.x; k < 2 * ND; k += WT) sc[k] = ((const float4*)septab->coef)[k];
-    double* sq = (double*)(smem + WA_OFF_Q);
-    float* d1 = (float*)(smem + WA_OFF_D1);
-    for (int k = threadIdx.x; k < ND + 1; k += WT) {
-        const double q = septab->q[k];
-        sq[k] = q;
-        if (k < ND) d1[k] = (float)(septab->q[k + 1] - q);
+    if (threadIdx.x == 0) {
+        const unsigned bar = smem_u32(smem + WA_OFF_BAR);
+        mbar_init(bar, 1);
+        bulk_load(smem, septab, (unsigned)sizeof(SepTab), bar);
     }
     return A;
+}
+// False (in every thread) when the bounded wait ran out: the block sets *status and returns.
+__device__ __forceinline__ bool tables_ready(unsigned char* smem, int* status) {
+    const bool ok = mbar_wait(smem_u32(smem + WA_OFF_BAR), 0);
+    if (__syncthreads_and(ok)) return true;
+    if (threadIdx.x == 0) {
+        atomicExch(status, 1);
+        mbar_wait(smem_u32(smem + WA_OFF_BAR), 0);  // bounded: let the copy land before the block exits
+    }
+    return false;
 }
 
 // Source-independent geometry of one pixel: its rule points are the bilinear
@@ -389,6 +393,13 @@ __device__ __forceinline__ void window_source(const PixBase& P, const WinSrc& si
     }
 }
 
+// This lane's pixel of the warp's next run of 32 from pixel p0 on.
+__device__ __forceinline__ int next_run(int* counter, int p0) {
+    int c = 0;
+    if ((threadIdx.x & 31) == 0) c = atomicAdd(counter, 32);
+    return p0 + __shfl_sync(0xffffffffu, c, 0) + (threadIdx.x & 31);
+}
+
 // The dense map: block b takes item b = (g, p), part p of the P parts of group g (nsg
 // sources; tiles [p nt / P, (p + 1) nt / P) of WT pixels), forms each pixel's
 // source-independent geometry once and the windows of the group's sources from it,
@@ -402,11 +413,14 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restric
                                                       int P, int nsg,
                                                       double* __restrict__ hist_out, float4* __restrict__ rec,
                                                       float4* __restrict__ ext, float2* __restrict__ sparse,
-                                                      int sparse_cap, int* __restrict__ sparse_count) {
+                                                      int sparse_cap, int* __restrict__ sparse_count,
+                                                      int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const PassA A = pass_a_tables(smem, septab, rec, ext, sparse, sparse_cap, sparse_count);
+    __shared__ int next_s;
     WinSrc* ssrc = (WinSrc*)(smem + WA_OFF_SRC);
     const int t = threadIdx.x;
+    if (t == 0) next_s = 0;
     const int npix = H * W, W1 = W + 1;
     const int nt = (npix + WT - 1) / WT;
     const int item = blockIdx.x;
@@ -414,10 +428,12 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restric
     if (t < ns) ssrc[t] = win_source(info[s0 + t]);
     for (int r = t; r < ns * ND; r += WT) A.hist[r] = 0.;
     __syncthreads();
-    const int ta = (int)((long long)p * nt / P), tb = (int)((long long)(p + 1) * nt / P);
-    for (int tile = ta; tile < tb; ++tile) {
-        const int pix = tile * WT + t;
-        if (pix >= npix) continue;
+    if (!tables_ready(smem, status)) return;
+    // warps take runs of 32 pixels from the item as they finish the last one: pixels next to
+    // a source or at a row's edge cost several times the others
+    const int pa = (int)((long long)p * nt / P) * WT, pb = min((int)((long long)(p + 1) * nt / P) * WT, npix);
+    for (int pix = next_run(&next_s, pa); pix - (t & 31) < pb; pix = next_run(&next_s, pa)) {
+        if (pix >= pb) continue;
         const int h = pix / W, w = pix - h * W;
         const PixBase Q = pixel_base(corners, centers, omega, W1, h, w, (size_t)pix);
         for (int j = 0; j < ns; ++j) {
@@ -449,14 +465,17 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
                                                           const SepTab* __restrict__ septab, int S, int W, int run,
                                                           double* __restrict__ hist_out, float4* __restrict__ rec,
                                                           float4* __restrict__ ext, float2* __restrict__ sparse,
-                                                          int sparse_cap, int* __restrict__ sparse_count) {
+                                                          int sparse_cap, int* __restrict__ sparse_count,
+                                                          int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ long long item_s;
-    __shared__ int rmin_s, rmax_s;
+    __shared__ int rmin_s, rmax_s, next_s;
     const PassA A = pass_a_tables(smem, septab, rec, ext, sparse, sparse_cap, sparse_count);
     WinSrc* ssrc = (WinSrc*)(smem + WA_OFF_SRC);
     const int t = threadIdx.x, W1 = W + 1;
     for (int r = t; r < ND; r += WT) A.hist[r] = 0.;
+    __syncthreads();
+    if (!tables_ready(smem, status)) return;
     const long long n_items = tile_off[S];
     for (;;) {
         if (t == 0) {
@@ -464,6 +483,7 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
             item_s = it;
             rmin_s = ND;
             rmax_s = -1;
+            next_s = 0;
             if (it < n_items) ssrc[0] = win_source(info[item_src[it]]);
         }
         __syncthreads();  // also orders the previous item's flush before this item's adds
@@ -471,10 +491,10 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
         if (item >= n_items) break;
         const int s = item_src[item];
         const xts_cutout cw = cut[s];
-        const long long npix = (long long)cw.nh * cw.nw, p0 = (item - tile_off[s]) * run;
-        const long long p1 = min(npix, p0 + run);
-        for (long long pix = p0 + t; pix < p1; pix += WT) {
-            const int i = (int)((unsigned)pix / (unsigned)cw.nw), j = (int)(pix - (long long)i * cw.nw);
+        const int npix = cw.nh * cw.nw, p0 = (int)((item - tile_off[s]) * run), p1 = min(npix, p0 + run);  // (<= 2^30)
+        for (int pix = next_run(&next_s, p0); pix - (t & 31) < p1; pix = next_run(&next_s, p0)) {
+            if (pix >= p1) continue;
+            const int i = pix / cw.nw, j = pix - i * cw.nw;
             const int h = cw.h0 + i, w = cw.w0 + j;
             const PixBase P = pixel_base(corners, centers, omega, W1, h, w, (size_t)h * W + w);
             window_source(P, ssrc[0], corners, centers, W1, h, w, (size_t)(cw.offset + pix), A, A.hist, &rmin_s, &rmax_s);
@@ -918,12 +938,13 @@ static int window_group(int n, int ntile, int G) {
     while (nsg > 1 && (long long)((n + nsg - 1) / nsg) * ntile < 2LL * G) nsg >>= 1;
     return nsg;
 }
-// Parts per source group (n sources of ntile tiles, G blocks): about 16 queue items per
-// block (with 4 sources per group, c2: 1.66 ms at 8, 1.57 at 16, 1.63 at 32), at most one
-// part per tile.
+constexpr int ITEMS = 8;  // work items per resident block
+// Parts per source group (n sources of ntile tiles, G blocks): about ITEMS items per
+// resident block (500 sources x 400 x 400: 1.52 ms at 4, 1.34 at 8, 1.35 at 16; 40 x 800 x
+// 800: 383 us at 8, 397 at 16), at most one part per tile.
 static int window_parts(int n, int nsg, int ntile, int G) {
     const long long ng = (n + nsg - 1) / nsg;
-    long long P = (16LL * G + ng - 1) / ng;
+    long long P = ((long long)ITEMS * G + ng - 1) / ng;
     if (P > ntile) P = ntile;
     return P < 1 ? 1 : (int)P;
 }
@@ -1017,7 +1038,7 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
         XTS_LAUNCH("k_pixel_windows", gs, k_pixel_windows<<<n_items, WT, wa_smem(nsg), gs>>>(
                                               corners, centers, means_only ? nullptr : omega, info + s0, tab, n, H, W,
                                               nparts, nsg, hist, rec, ext, sparse, (int)cap,
-                                              sparse_count));
+                                              sparse_count, status));
         if (pipe) {
             XTS_CUDA(cudaEventRecord(evA[b], gs));
             XTS_CUDA(cudaStreamWaitEvent(st, evA[b], 0));
@@ -1141,7 +1162,7 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     // pass A: one persistent wave pulling (source, tile) items from the queue
     XTS_LAUNCH("k_pixel_windows", st, k_pixel_windows_cut<<<(unsigned)(resident * nsm), WT, wa_smem(1), st>>>(
                                           corners, centers, omega, info, cut, item_src, tile_off, queue, tab, S, W, run,
-                                          hist, rec, ext, sparse, (int)cap, sparse_count));
+                                          hist, rec, ext, sparse, (int)cap, sparse_count, status));
     rc = launch_correction(hist, 1, info, S, upsf, partial, exposure, E, scale, inv_integ, correction, radius, in_fov,
                            st, lut, EQ * 4);
     if (rc) return rc;
