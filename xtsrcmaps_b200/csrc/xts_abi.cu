@@ -902,14 +902,20 @@ static int fused_maps(const xts_expcube* cube, const xts_expcube* wcube, const d
     // exposure and mean PSF on the library's highest-priority stream: the window pass
     // (one short block per work item, on the geometry stream) fills the GPU, and these
     // kernels' blocks are then scheduled ahead of its pending ones as slots free up
+    // (a job whose window pass leaves SMs free has no use for the priority: on the caller's
+    // stream, without the two events' 5 us on the host)
     if (rc == XTS_OK) {
-        cudaStream_t ps = g_ctx.prio_stream;
-        XTS_CUDA(cudaEventRecord(g_ctx.pfork_ev, sg.st));
-        XTS_CUDA(cudaStreamWaitEvent(ps, g_ctx.pfork_ev, 0));
-        rc = launch_exposure(ea, ps);
-        if (rc == XTS_OK) rc = launch_psf(pa, ps);
-        XTS_CUDA(cudaEventRecord(g_ctx.pjoin_ev, ps));
-        XTS_CUDA(cudaStreamWaitEvent(sg.st, g_ctx.pjoin_ev, 0));
+        const bool prio = (long long)S * (long long)npix > (1 << 20);
+        cudaStream_t ps = prio ? g_ctx.prio_stream : sg.st;
+        if (prio) {
+            XTS_CUDA(cudaEventRecord(g_ctx.pfork_ev, sg.st));
+            XTS_CUDA(cudaStreamWaitEvent(ps, g_ctx.pfork_ev, 0));
+        }
+        rc = launch_psf(pa, ps, &ea);
+        if (prio) {
+            XTS_CUDA(cudaEventRecord(g_ctx.pjoin_ev, ps));
+            XTS_CUDA(cudaStreamWaitEvent(sg.st, g_ctx.pjoin_ev, 0));
+        }
     }
     if (rc != XTS_OK) {
         if (fork) StreamJoin{g_ctx.geo_stream, sg.st, g_ctx.join_ev}.join();

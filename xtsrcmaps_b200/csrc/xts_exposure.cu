@@ -1,69 +1,17 @@
-// xts_exposure.cu -- step (a) of the point-source path (exposure) and the two
-// IRF set-up routines that feed it (livetime-efficiency factors, King PSF
-// normalisation).
+// xts_exposure.cu -- the sources' livetime pixels and the two IRF set-up routines
+// that feed step (a) (livetime-efficiency factors, King PSF normalisation); step
+// (a) itself is in xts_tables.cuh and xts_tables.cu.
 //
-//   a1 exp_costhetas        exposure/exposure.cxx:29-40
-//   a2 src_cosbins (gather) exposure/exposure.cxx:42-63 + healpix/healpix.cxx:181-229
-//   a3 aeff_value           irf/irf.aeff_value.cxx:11-55, math/bilerp.cxx:6-27
+//   a2 source pixels        exposure/exposure.cxx:42-63 + healpix/healpix.cxx:181-229
 //   a4 LTF                  irf/irf.cxx:70-109
-//   a5 exposure contraction exposure/exposure.cxx:159-263, exposure/exposure.contract.cpp:13-42
 //   b1 normalize_rpsf       irf/irf.normalize_rpsf.cpp:11-61, irf/irf.hxx:22-77
 #include <math.h>
 
 #include "xts_geom.cuh"
 #include "xts_internal.cuh"
+#include "xts_tables.cuh"
 
 namespace xts {
-
-// math/bilerp.cxx:6-27: upper_bound index, weight and complement.  The
-// reference asserts the value lies inside the grid; the index is clamped to the
-// last interval here instead of reading past the end.
-__device__ inline void lerp_pars(const double* g, int n, double v, bool has_lb, double lb,
-                                 double* wgt, double* cmpl, int* idx) {
-    if (has_lb && v < lb) { *wgt = 0.; *cmpl = 0.; *idx = 1; return; }
-    int lo = 0, hi = n;  // first i with g[i] > v
-    while (lo < hi) { int m = (lo + hi) >> 1; if (v < g[m]) hi = m; else lo = m + 1; }
-    int i = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
-    double t = (v - g[i - 1]) / (g[i] - g[i - 1]);
-    *wgt = t; *cmpl = 1. - t; *idx = i;
-}
-
-// a1 + a3: cos-theta bin centres and the front/back effective-area tables [C, E].
-__global__ void k_exposure_tables(int C, double cosmin, int thetabin, const double* logEs, int E,
-                                  xts_grid af, xts_grid ab, double* costh, double* front,
-                                  double* back) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= C * E) return;
-    int c = i / E, e = i - c * E;
-    double f = ((double)c + 0.5) / C;
-    f = thetabin ? f * f : f;
-    double ct = 1. - f * (1. - cosmin);
-    if (e == 0) costh[c] = ct;
-    const xts_grid* gs[2] = {&af, &ab};
-    double* outs[2] = {front, back};
-    for (int k = 0; k < 2; ++k) {
-        const xts_grid& g = *gs[k];
-        double cw, cc, ew, ec; int ci, ei;
-        lerp_pars(g.cosths, g.n_cos, ct, true, g.min_cos_theta, &cw, &cc, &ci);
-        lerp_pars(g.logEs, g.n_e, logEs[e], false, 0., &ew, &ec, &ei);
-        int Me = g.n_e;
-        const double* P = g.params;
-        double xx = cc * ec * P[(ci - 1) * Me + (ei - 1)];
-        double xy = cc * ew * P[(ci - 1) * Me + ei];
-        double yx = cw * ec * P[ci * Me + (ei - 1)];
-        double yy = cw * ew * P[ci * Me + ei];
-        outs[k][i] = 1e4 * (xx + xy + yx + yy);
-    }
-}
-
-// The NESTED pixel of each source (exposure/exposure.cxx:42-63), -1 when the
-// position is not finite.
-__device__ __forceinline__ long long src_pixel(const double* src_sph, int s, long long nside) {
-    const double theta = HALFPI - src_sph[2 * s + 1] * D2R;
-    const double phi = D2R * src_sph[2 * s];
-    const long long pix = ang2pix_nest(theta, phi, nside);
-    return pix < 0 || pix >= 12 * nside * nside ? -1 : pix;
-}
 
 __global__ void k_src_pixels(const double* src_sph, int S, long long nside, long long* pix) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -74,64 +22,6 @@ int launch_src_pixels(const double* src_sph, int S, long long nside, long long* 
     if (S > 0)
         XTS_LAUNCH("k_src_pixels", st, k_src_pixels<<<(S + 127) / 128, 128, 0, st>>>(src_sph, S, nside, pix));
     return XTS_OK;
-}
-
-// a2: livetime rows of each source's NESTED pixel, float -> double [S, C].  With
-// `gathered` the cubes hold only those rows already, [S][C] in source order.
-__global__ void k_src_cosbins(const double* src_sph, int S, const float* cube, const float* wcube,
-                              long long nside, int C, int gathered, double* ecb, double* wecb) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S * C) return;
-    int s = i / C, c = i - s * C;
-    const long long pix = gathered ? s : src_pixel(src_sph, s, nside);
-    if (pix < 0) {  // non-finite source position
-        ecb[i] = wecb[i] = __longlong_as_double(0x7ff8000000000000ll);
-        return;
-    }
-    ecb[i] = (double)cube[pix * C + c];
-    wecb[i] = (double)wcube[pix * C + c];
-}
-
-// a5 on FP64 cores: E[s,e] = ((X.Af L0 + X.Ab L0) + W.Af L1) + W.Ab L1.
-__global__ void k_exposure_f64(const double* ecb, const double* wecb, int S, int C,
-                               const double* af, const double* ab, const double* ltf, int E,
-                               double* out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S * E) return;
-    int s = i / E, e = i - s * E;
-    double ef = 0, wf = 0, eb = 0, wb = 0;
-#pragma unroll 8
-    for (int c = 0; c < C; ++c) {  // unrolled: eight rows of loads in flight, sums still in c order
-        double x = ecb[s * C + c], w = wecb[s * C + c];
-        double a = af[c * E + e], b = ab[c * E + e];
-        ef = fma(x, a, ef); wf = fma(w, a, wf);
-        eb = fma(x, b, eb); wb = fma(w, b, wb);
-    }
-    double l0 = ltf[e], l1 = ltf[E + e];
-    out[i] = ((ef * l0 + eb * l0) + wf * l1) + wb * l1;
-}
-
-int launch_exposure_contract(const double* ecb, const double* wecb, int S, int C, const double* af,
-                             const double* ab, const double* ltf, int E, double* out,
-                             cudaStream_t st) {
-    int n = S * E;
-    if (n == 0) return XTS_OK;
-    XTS_LAUNCH("k_exposure_f64", st, k_exposure_f64<<<(n + 127) / 128, 128, 0, st>>>(ecb, wecb, S, C, af, ab, ltf, E, out));
-    return XTS_OK;
-}
-
-int launch_exposure(const ExposureDev& a, cudaStream_t st) {
-    int n = a.C * a.E;
-    XTS_LAUNCH("k_exposure_tables", st, k_exposure_tables<<<(n + 127) / 128, 128, 0, st>>>(a.C, a.cosmin, a.thetabin, a.logEs, a.E,
-                                                      a.af, a.ab, a.exp_costhetas, a.front_aeff,
-                                                      a.back_aeff));
-    n = a.S * a.C;
-    if (n > 0) {
-        XTS_LAUNCH("k_src_cosbins", st, k_src_cosbins<<<(n + 127) / 128, 128, 0, st>>>(a.src_sph, a.S, a.cube, a.wcube, a.nside,
-                                                      a.C, a.gathered ? 1 : 0, a.ecb, a.wecb));
-    }
-    return launch_exposure_contract(a.ecb, a.wecb, a.S, a.C, a.front_aeff, a.back_aeff, a.ltf, a.E,
-                                    a.exposure, st);
 }
 
 // a4: piecewise-linear efficiency in log E.  Row 1 from p0, row 0 from p1, and

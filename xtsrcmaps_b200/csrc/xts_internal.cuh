@@ -116,7 +116,11 @@ struct PsfDev {
     const double* ltf; const double* exposure;
     double* upsf; double* partial;
 };
-int launch_psf(const PsfDev& a, cudaStream_t st);
+// the mean PSF; with e, e's exposure too (a.exposure its output), their tables sharing launches
+int launch_psf(const PsfDev& a, cudaStream_t st, const ExposureDev* e = nullptr);
+int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, cudaStream_t st,
+                       const ExposureDev* e = nullptr);
+int launch_psf_tables(const ExposureDev* e, const PsfDev& p, double* king, double* pa, double* rows, cudaStream_t st);
 
 struct SrcmapDev {
     xts_wcs wcs;

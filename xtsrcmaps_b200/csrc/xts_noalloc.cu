@@ -32,8 +32,6 @@
 
 namespace xts {
 
-int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, cudaStream_t st);  // xts_psf.cu
-
 constexpr size_t NOALLOC_SCRATCH_DOUBLES = XTS_NOALLOC_SCRATCH_DOUBLES;
 
 // beside the NOALLOC_SCRATCH_DOUBLES that the limit counts the array holds the padding of

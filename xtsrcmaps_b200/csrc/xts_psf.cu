@@ -15,77 +15,9 @@
 #include <math.h>
 
 #include "xts_internal.cuh"
+#include "xts_tables.cuh"
 
 namespace xts {
-
-__device__ __forceinline__ double sep_deg(int d) {  // psf/psf.hxx:24-31
-    const double xstep = log(70. / 1e-4) / (400 - 1.);
-    return d == 0 ? 0.0 : 1e-4 * exp((d - 1) * xstep);
-}
-
-__device__ inline double king_f2(double u, double g) {
-    if (g == 1) g = 1.001;
-    return (1. - 1. / g) * pow(1. + u / g, -g);
-}
-
-// b3: K[side][c][e][d] = evaluate_king(sep[d] rad, 1, params[c,e,:]) (irf/irf.hxx:22-45);
-// the separation is the fastest axis of this table and of psf*aeff, so that the
-// contraction below reads runs of rows of one energy.
-__global__ void k_king(xts_grid pf, xts_grid pb, double* kf, double* kb) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int side = blockIdx.y;
-    const xts_grid& g = side ? pb : pf;
-    int McMe = g.n_cos * g.n_e;
-    if (i >= ND * McMe) return;
-    int ce = i / ND, d = i - ce * ND;
-    const double* p = g.params + (size_t)ce * 6;
-    double sep = sep_deg(d) * D2R;
-    double ncore = p[0], ntail = p[1], score = p[2], stail = p[3];
-    double rc = sep / score, uc = rc * rc / 2.;
-    double rt = sep / stail, ut = rt * rt / 2.;
-    (side ? kb : kf)[i] = ncore * king_f2(uc, p[4]) + ntail * ncore * king_f2(ut, p[5]);
-}
-
-__device__ inline void lerp_pars2(const double* g, int n, double v, double* wgt, double* cmpl,
-                                  int* idx) {
-    int lo = 0, hi = n;
-    while (lo < hi) { int m = (lo + hi) >> 1; if (v < g[m]) hi = m; else lo = m + 1; }
-    int i = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
-    double t = (v - g[i - 1]) / (g[i] - g[i - 1]);
-    *wgt = t; *cmpl = 1. - t; *idx = i;
-}
-
-// b4 + the aeff product of b5, both sides summed: PA[c][e][d], rows padded to NDP.
-// One block per (e, c), whose bilinear weights four threads look up.
-constexpr int NDP = (ND + 3) / 4 * 4;
-
-__global__ void k_psf_aeff(xts_grid pf, xts_grid pb, const double* kf, const double* kb,
-                           const double* costh, int C, const double* logEs, int E,
-                           const double* af, const double* ab, double* pa) {
-    __shared__ double wgt[4], cmpl[4];  // side 0 energy, cos-theta, side 1 energy, cos-theta
-    __shared__ int idx[4];
-    const int e = blockIdx.x, c = blockIdx.y;
-    if (threadIdx.x < 4) {
-        const int k = threadIdx.x;
-        const xts_grid& g = k >> 1 ? pb : pf;
-        if (k & 1) lerp_pars2(g.cosths, g.n_cos, costh[c], &wgt[k], &cmpl[k], &idx[k]);
-        else lerp_pars2(g.logEs, g.n_e, logEs[e], &wgt[k], &cmpl[k], &idx[k]);
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < ND; d += blockDim.x) {
-        double v = 0.;
-        for (int side = 0; side < 2; ++side) {
-            const xts_grid& g = side ? pb : pf;
-            const double ew = wgt[2 * side], ec = cmpl[2 * side], cw = wgt[2 * side + 1], cc = cmpl[2 * side + 1];
-            const int ei = idx[2 * side], ci = idx[2 * side + 1], Me = g.n_e;
-            const double* K = (side ? kb : kf) + d;
-            const size_t r0 = (size_t)((ci - 1) * Me + ei - 1) * ND, r1 = (size_t)(ci * Me + ei - 1) * ND;
-            double b = cc * ec * K[r0] + cc * ew * K[r0 + ND] + cw * ec * K[r1] + cw * ew * K[r1 + ND];
-            v += b * (side ? ab : af)[c * E + e];
-        }
-        pa[((size_t)c * E + e) * NDP + d] = v;
-    }
-}
 
 // b5, b6 and b7 in one kernel: a block forms the mean PSF of TS sources at TE energies
 // over all 401 rows in shared memory, integrates it and writes uPsf and the partial
@@ -154,19 +86,6 @@ __device__ __forceinline__ double scan_run(const double* y, const double* st, co
         }
     }
     return run;
-}
-
-// Row tables of the integral, [NDP] each: 2 pi sin(theta), half the widths of the bins that
-// end there, and the row's weight in the integral over all bins.
-__global__ void k_psf_rows(double* tab) {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= NDP) return;
-    const double th = D2R * sep_deg(d);
-    tab[d] = d < ND ? TWOPI * sin(th) : 0.;
-    const double below = d > 0 && d < ND ? 0.5 * (th - D2R * sep_deg(d - 1)) : 0.;
-    const double above = d + 1 < ND ? 0.5 * (D2R * sep_deg(d + 1) - th) : 0.;
-    tab[NDP + d] = below;
-    tab[2 * NDP + d] = tab[d] * (below + above);
 }
 
 template <int TS, int TE>
@@ -330,16 +249,12 @@ static int launch_psf_mean(const PsfDev& a, const double* pa, const double* tab,
 // The launches with caller-provided scratch: king holds both sides' King tables
 // (401 * (Mc * Me front + Mc * Me back) doubles), pa the summed psf * aeff table
 // (C * E * 404 doubles, 16-byte aligned), tab 3 * 404 doubles.  Nothing here allocates.
-int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, cudaStream_t st) {
+// With e, its exposure (the one that a.exposure points to) is formed beside the tables.
+int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, cudaStream_t st, const ExposureDev* e) {
     if (a.C > PSF_MAX_C) return set_error(XTS_ERR_ARG, "compute_psf_data: C=%d exceeds %d", a.C, PSF_MAX_C);
     if (a.E > PSF_MAX_E) return set_error(XTS_ERR_ARG, "compute_psf_data: E=%d exceeds %d", a.E, PSF_MAX_E);
-    const size_t kf_n = (size_t)ND * a.pf.n_cos * a.pf.n_e, kb_n = (size_t)ND * a.pb.n_cos * a.pb.n_e;
-    const int mx = (int)(kf_n > kb_n ? kf_n : kb_n);
-    XTS_LAUNCH("k_king", st, k_king<<<dim3((mx + 127) / 128, 2), 128, 0, st>>>(a.pf, a.pb, king, king + kf_n));
-    XTS_LAUNCH("k_psf_aeff", st, k_psf_aeff<<<dim3(a.E, a.C), 128, 0, st>>>(a.pf, a.pb, king, king + kf_n, a.costh, a.C,
-                                                                            a.logEs, a.E, a.af, a.ab, pa));
-    if (a.S == 0) return XTS_OK;
-    XTS_LAUNCH("k_psf_rows", st, k_psf_rows<<<(NDP + 127) / 128, 128, 0, st>>>(tab));
+    const int rc = launch_psf_tables(e, a, king, pa, tab, st);
+    if (rc || a.S == 0) return rc;
     // 8 sources x 4 energies (most products per load of psf*aeff) where that fills the GPU
     // with two blocks per SM; 4 x 4 while most SMs get a block (50 sources x 37 energies: 130
     // blocks); below, one energy per block (7 x 21: 42 blocks instead of 12)
@@ -349,12 +264,12 @@ int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, c
     return launch_psf_mean<4, 1>(a, pa, tab, st);
 }
 
-int launch_psf(const PsfDev& a, cudaStream_t st) {
+int launch_psf(const PsfDev& a, cudaStream_t st, const ExposureDev* e) {
     double* king = (double*)workspace(W_KING, sizeof(double) * ND * ((size_t)a.pf.n_cos * a.pf.n_e +
                                                                      (size_t)a.pb.n_cos * a.pb.n_e));
     double* pa = (double*)workspace(W_PSFTAB, sizeof(double) * ((size_t)a.C * a.E + 4) * NDP);
     if (!king || !pa) return XTS_ERR_OOM;
-    return launch_psf_scratch(a, king, pa + 4 * NDP, pa, st);
+    return launch_psf_scratch(a, king, pa + 4 * NDP, pa, st, e);
 }
 
 }  // namespace xts

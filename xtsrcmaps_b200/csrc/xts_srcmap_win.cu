@@ -28,6 +28,8 @@
 // staged and written by one TMA bulk store per tile, so the pass streams the
 // window records in and the map out; the next tile's records are loaded while
 // the current one is computed.
+#include <vector>
+
 #include "xts_point.cuh"
 
 namespace xts {
@@ -887,6 +889,26 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
     if ((lane & 7) == 0) bulk_wait_all();
 }
 
+// Resident blocks per SM of a kernel at a launch shape, asked of the driver once per kernel,
+// shape and device (the answer does not change); the kernel's shared-memory limit is raised
+// to the largest shape asked for.  Calls are serialised by the library's lock.
+template <typename F>
+static int resident_blocks(F* kernel, int threads, size_t smem, int dev, int* out) {
+    struct Known { const void* k; int threads, dev, blocks; size_t smem; };
+    static std::vector<Known> known;
+    size_t limit = 0;
+    for (const Known& n : known) {
+        if (n.k != (const void*)kernel || n.dev != dev) continue;
+        if (n.threads == threads && n.smem == smem) { *out = n.blocks; return XTS_OK; }
+        if (n.smem > limit) limit = n.smem;
+    }
+    if (smem > limit)
+        XTS_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, (const void*)kernel, threads, smem));
+    known.push_back(Known{(const void*)kernel, threads, dev, *out, smem});
+    return XTS_OK;
+}
+
 struct WriteArgs {
     const float4* win; const float4* ext; const float2* sparse; const float* lut;
     const double* corners; const double* omega; const SrcInfo* info; const SepTab* tab;
@@ -900,11 +922,10 @@ static int launch_write_pass(unsigned G, int warps, size_t smem, cudaStream_t st
                              bool query) {
     const int BT = 32 * warps;
     if (query) {
-        int pd = 0, pc = 0;
-        XTS_CUDA(cudaFuncSetAttribute(k_srcmap_win<NQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        XTS_CUDA(cudaFuncSetAttribute(k_srcmap_win<NQ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pd, k_srcmap_win<NQ, false>, BT, smem));
-        XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pc, k_srcmap_win<NQ, true>, BT, smem));
+        int pd = 0, pc = 0, dev = 0, rc;
+        cudaGetDevice(&dev);
+        if ((rc = resident_blocks(k_srcmap_win<NQ, false>, BT, smem, dev, &pd))) return rc;
+        if ((rc = resident_blocks(k_srcmap_win<NQ, true>, BT, smem, dev, &pc))) return rc;
         *per_sm = pd < pc ? pd : pc;
         return XTS_OK;
     }
@@ -1003,14 +1024,13 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     // pass A: one block per work item, items sized for about 16 per block of the
     // resident set (at most window_blocks_per_sm blocks per SM)
     int resident = 0;
-    XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wa_smem(NSG_MAX)));
-    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows, WT, wa_smem(NSG_MAX)));
+    if ((rc = resident_blocks(k_pixel_windows, WT, wa_smem(NSG_MAX), dev, &resident))) return rc;
     resident = resident < 1 ? 1 : resident;
     if (g_tuning.window_blocks_per_sm > 0 && g_tuning.window_blocks_per_sm < resident)
         resident = g_tuning.window_blocks_per_sm;
     const int ntile = (npix + WT - 1) / WT, nsg = window_group(Sc, ntile, resident * nsm);
     const int nparts = window_parts(Sc, nsg, ntile, resident * nsm);
-    const size_t hist_n = (size_t)Sc * ND + 1;
+    const size_t hist_n = (size_t)Sc * ND + 1;  // the last double: the sparse records' count
     double* hist0 = (double*)workspace(W_PARTSUM, sizeof(double) * 2 * hist_n);
     if (!rec0 || !ext0 || !lut0 || !sparse0 || !hist0) return XTS_ERR_OOM;
     const WritePassFn wp = k_write_pass[(E + 3) / 4 - 1];
@@ -1028,18 +1048,19 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
         float* lut = lut0 + b * lut_n;
         float2* sparse = sparse0 + b * sp_n;
         double* hist = hist0 + b * hist_n;
-        int* sparse_count = status + 1 + b;
+        int* sparse_count = (int*)(hist + (size_t)n * ND);
         // the window pass is geometry only: it runs on the geometry stream, once
         // the write pass that last read its buffers is done
         if (pipe && k >= 2) XTS_CUDA(cudaStreamWaitEvent(gs, evB[b], 0));
         const int n_items = (n + nsg - 1) / nsg * nparts;  // one block per item
-        XTS_CUDA(cudaMemsetAsync(sparse_count, 0, sizeof(int), gs));
-        XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * (size_t)n * ND, gs));
+        XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * ((size_t)n * ND + 1), gs));
         XTS_LAUNCH("k_pixel_windows", gs, k_pixel_windows<<<n_items, WT, wa_smem(nsg), gs>>>(
                                               corners, centers, means_only ? nullptr : omega, info + s0, tab, n, H, W,
                                               nparts, nsg, hist, rec, ext, sparse, (int)cap,
                                               sparse_count, status));
-        if (pipe) {
+        if (Sc >= S) {  // one chunk: nothing else follows on the geometry stream
+            if ((rc = geo.join())) return rc;
+        } else if (pipe) {
             XTS_CUDA(cudaEventRecord(evA[b], gs));
             XTS_CUDA(cudaStreamWaitEvent(st, evA[b], 0));
         }
@@ -1062,7 +1083,7 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
         rc = wp((unsigned)G, nw, L.total, st, wa, nullptr, false);
         if (rc) return rc;
         if (on_chunk && (rc = on_chunk(on_chunk_ctx, s0, n, st))) return rc;
-        if (pipe) XTS_CUDA(cudaEventRecord(evB[b], st));
+        if (pipe && Sc < S) XTS_CUDA(cudaEventRecord(evB[b], st));
     }
     return geo.join();
 }
@@ -1149,14 +1170,12 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     int* item_src = (int*)(items + align_up(sizeof(long long) * (S + 1), 256));
     unsigned long long* queue = (unsigned long long*)(items + align_up(sizeof(long long) * (S + 1), 256) +
                                                       align_up(sizeof(int) * (size_t)max_items, 256));
-    int* sparse_count = status + 1;
-    XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * (size_t)S * ND, st));
+    int* sparse_count = (int*)(hist + (size_t)S * ND);
+    XTS_CUDA(cudaMemsetAsync(hist, 0, sizeof(double) * ((size_t)S * ND + 1), st));
     XTS_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
-    XTS_CUDA(cudaMemsetAsync(sparse_count, 0, sizeof(int), st));
     XTS_LAUNCH("k_cut_tiles", st, k_cut_tiles<<<2, 1024, 0, st>>>(cut, S, 32 * nw, run, tile_off, pair_off));
     XTS_LAUNCH("k_cut_item_src", st, k_cut_item_src<<<S, 256, 0, st>>>(tile_off, item_src));
-    XTS_CUDA(cudaFuncSetAttribute(k_pixel_windows_cut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wa_smem(1)));
-    XTS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_pixel_windows_cut, WT, wa_smem(1)));
+    if ((rc = resident_blocks(k_pixel_windows_cut, WT, wa_smem(1), dev, &resident))) return rc;
     resident = resident < 1 ? 1 : resident;
     if (g_tuning.queue_blocks_per_sm > 0 && g_tuning.queue_blocks_per_sm < resident) resident = g_tuning.queue_blocks_per_sm;
     // pass A: one persistent wave pulling (source, tile) items from the queue
