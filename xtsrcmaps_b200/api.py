@@ -120,10 +120,11 @@ class _Call:
     def inp(self, x, kind="f64"):
         if self.device:
             t = self.torch
-            dt = {"f64": t.float64, "f32": t.float32, "i32": t.int32}[kind]
+            dt = t.float64 if kind == "f64" else t.float32 if kind == "f32" else t.int32
             if not _is_cuda(x):
                 x = t.as_tensor(np.asarray(x), device=self.dev)
-            x = x.to(dt).contiguous()
+            if x.dtype is not dt or not x.is_contiguous():
+                x = x.to(dt).contiguous()
             self.keep.append(x)
             return C.c_void_p(x.data_ptr()), x
         a = np.ascontiguousarray(np.asarray(x), dtype=self._NP[kind])
@@ -148,7 +149,7 @@ class _Call:
         cp, c = self.inp(g.cosths)
         ep, e = self.inp(g.logEs)
         pp, p = self.inp(params)
-        return L.XtsGrid(cp, len(c), ep, len(e), pp, n_par, float(g.min_cos_theta))
+        return L.XtsGrid(cp, c.shape[0], ep, e.shape[0], pp, n_par, float(g.min_cos_theta))
 
 
 def _device_of(*xs) -> Optional[Any]:

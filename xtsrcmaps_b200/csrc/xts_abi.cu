@@ -45,6 +45,8 @@ struct Ctx {
     cudaEvent_t chunk_ev[N_CHUNK_EV] = {};
     void* buf[N_SLOTS] = {};
     size_t cap[N_SLOTS] = {};
+    char* pin = nullptr;    // page-locked copy of a host-mode call's small inputs
+    bool pin_busy = false;  // its last copy to the device has not been waited for
 };
 static Ctx g_ctx;
 
@@ -129,6 +131,9 @@ static void release_all() {
         g_ctx.buf[i] = nullptr;
         g_ctx.cap[i] = 0;
     }
+    if (g_ctx.pin) cudaFreeHost(g_ctx.pin);
+    g_ctx.pin = nullptr;
+    g_ctx.pin_busy = false;
 }
 
 // Kernel timing -------------------------------------------------------------
@@ -186,15 +191,53 @@ struct Stager {
     Pending pend[8];
     int npend = 0;
 
+    static constexpr size_t ARENA = 2 << 20, ARENA_MAX = 256 << 10;  // whole; largest input in it
+    size_t arena = 0, copied = 0;  // bytes of the arena in use; of these, on their way
+    bool sent = false;
+    ~Stager() {
+        if (sent) g_ctx.pin_busy = true;  // not waited for (an error on the way)
+    }
+    Stager(bool d, cudaStream_t s) : dev(d), st(s) {}
+
+    // Small host inputs are gathered in page-locked memory and go to the device in one copy
+    // (ready()): a copy of its own from pageable memory costs each of them about 5 us.
     template <typename T>
     const T* in(const T* p, size_t n) {
         if (rc || dev || !p || n == 0) return p;
+        const size_t bytes = n * sizeof(T);
+        if (bytes <= ARENA_MAX && arena + bytes <= ARENA) {
+            char* d = (char*)workspace(S_ARENA, ARENA);
+            if (!d) { rc = XTS_ERR_OOM; return nullptr; }
+            if (!g_ctx.pin) {
+                cudaError_t e = cudaHostAlloc((void**)&g_ctx.pin, ARENA, cudaHostAllocDefault);
+                if (e != cudaSuccess) { g_ctx.pin = nullptr; rc = cuda_error(e, "cudaHostAlloc"); return nullptr; }
+            }
+            if (g_ctx.pin_busy) {  // an earlier call returned an error with its copy in flight
+                cudaDeviceSynchronize();
+                g_ctx.pin_busy = false;
+            }
+            const size_t at = arena;
+            memcpy(g_ctx.pin + at, p, bytes);
+            arena = align_up(at + bytes, 256);
+            return (const T*)(d + at);
+        }
         if (next_in > S_IN17) { rc = set_error(XTS_ERR_ARG, "too many staged inputs"); return nullptr; }
-        void* d = workspace(next_in++, n * sizeof(T));
+        void* d = workspace(next_in++, bytes);
         if (!d) { rc = XTS_ERR_OOM; return nullptr; }
-        cudaError_t e = cudaMemcpyAsync(d, p, n * sizeof(T), cudaMemcpyHostToDevice, st);
+        cudaError_t e = cudaMemcpyAsync(d, p, bytes, cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) { rc = cuda_error(e, "cudaMemcpyAsync H2D"); return nullptr; }
         return (const T*)d;
+    }
+    // Starts the copy of the inputs gathered so far; called before the launches that read
+    // them.  Returns rc.
+    int ready() {
+        if (rc || arena <= copied) return rc;
+        cudaError_t e = cudaMemcpyAsync((char*)workspace(S_ARENA, ARENA) + copied, g_ctx.pin + copied, arena - copied,
+                                        cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) return rc = cuda_error(e, "cudaMemcpyAsync H2D");
+        copied = arena;
+        sent = true;
+        return XTS_OK;
     }
     template <typename T>
     T* out(T* p, size_t n) {
@@ -233,6 +276,7 @@ struct Stager {
             if (e != cudaSuccess) return cuda_error(e, "cudaMemcpyAsync D2H");
         }
         XTS_CUDA(cudaStreamSynchronize(st));
+        sent = false;
         return XTS_OK;
     }
 };
@@ -292,7 +336,7 @@ static int run_srcmap(Stager& sg, SrcmapDev& a, void* model_map, size_t npix, bo
         a.on_chunk = chunk_done;
         a.on_chunk_ctx = &cc;
     }
-    int rc = sg.rc ? sg.rc : launch_srcmap(a, sg.st);
+    int rc = sg.ready() ? sg.rc : launch_srcmap(a, sg.st);
     if (cc.host && rc == XTS_OK) {
         if (cc.n == 0) rc = chunk_done(&cc, 0, S, sg.st);  // path without chunk hooks: one chunk
         if (rc == XTS_OK) rc = cc.issue(sg.st);
@@ -339,6 +383,7 @@ static void stage_cubes(Stager& sg, const xts_expcube* cube, const xts_expcube* 
     long long* pix_d = (long long*)workspace(W_SRCPIX, sizeof(long long) * (size_t)S);
     if (!pix_d) { sg.rc = XTS_ERR_OOM; return; }
     std::vector<long long> pix((size_t)S);
+    if (sg.ready()) return;
     int rc = launch_src_pixels(src_d, S, cube->nside, pix_d, sg.st);
     if (rc) { sg.rc = rc; return; }
     cudaError_t e = cudaMemcpyAsync(pix.data(), pix_d, sizeof(long long) * (size_t)S, cudaMemcpyDeviceToHost, sg.st);
@@ -460,7 +505,7 @@ int xts_livetime_efficiency_factors(const double* logEs, int E, const float* p0,
     const float* d_p0 = sg.in(p0, 6);
     const float* d_p1 = sg.in(p1, 6);
     double* d_out = sg.out(ltf, (size_t)2 * E);
-    int rc = sg.rc ? sg.rc : launch_ltf(d_loge, E, d_p0, d_p1, d_out, sg.st);
+    int rc = sg.ready() ? sg.rc : launch_ltf(d_loge, E, d_p0, d_p1, d_out, sg.st);
     return sg.finish(rc);
 }
 
@@ -474,7 +519,7 @@ int xts_normalize_rpsf(double* params, int Mc, int Me, const double* grid_logEs,
     double* d_par = const_cast<double*>(sg.in((const double*)params, n));
     const double* d_glog = sg.in(grid_logEs, (size_t)Me);
     if (!sg.dev && !sg.rc) sg.pend[sg.npend++] = {params, d_par, n * sizeof(double)};
-    int rc = sg.rc ? sg.rc
+    int rc = sg.ready() ? sg.rc
                    : launch_normalize_rpsf(d_par, Mc, Me, d_glog, scale0, scale1, scale_index, sg.st);
     return sg.finish(rc);
 }
@@ -509,7 +554,7 @@ int xts_compute_exposure(const xts_expcube* cube, const xts_expcube* wcube, cons
     a.ecb = out->src_exposure_cosbins ? sg.out(out->src_exposure_cosbins, (size_t)S * C) : sg.scratch<double>((size_t)S * C);
     a.wecb = out->src_weighted_exposure_cosbins ? sg.out(out->src_weighted_exposure_cosbins, (size_t)S * C) : sg.scratch<double>((size_t)S * C);
     a.exposure = out->exposure ? sg.out(out->exposure, (size_t)S * E) : sg.scratch<double>((size_t)S * E);
-    int rc = sg.rc ? sg.rc : launch_exposure(a, sg.st);
+    int rc = sg.ready() ? sg.rc : launch_exposure(a, sg.st);
     return sg.finish(rc);
 }
 
@@ -526,7 +571,7 @@ int xts_exposure_contract(const double* ecb, const double* wecb, int S, int C, c
     const double* d_ab = sg.in(ab, (size_t)C * E);
     const double* d_ltf = sg.in(ltf, (size_t)2 * E);
     double* d_out = sg.out(exposure, (size_t)S * E);
-    int rc = sg.rc ? sg.rc
+    int rc = sg.ready() ? sg.rc
                    : launch_exposure_contract(d_ecb, d_wecb, S, C, d_af, d_ab, d_ltf, E, d_out,
                                               sg.st);
     return sg.finish(rc);
@@ -558,7 +603,7 @@ int xts_compute_psf_data(const xts_grid* psf_front, const xts_grid* psf_back,
     a.exposure = sg.in(exposure, (size_t)S * E);
     a.upsf = sg.out(upsf, (size_t)S * ND * E);
     a.partial = sg.out(partial, (size_t)S * ND * E);
-    int rc = sg.rc ? sg.rc : launch_psf(a, sg.st);
+    int rc = sg.ready() ? sg.rc : launch_psf(a, sg.st);
     return sg.finish(rc);
 }
 
@@ -596,7 +641,7 @@ int xts_point_src_model_map_wcs(const xts_wcs* wcs, const double* src_sph, int S
     a.kernel = srcmap_kernel(flags);
     // the map geometry and the window passes on the geometry stream (forked here,
     // after the inputs are staged), so the chunks of the window path pipeline
-    if (sg.rc == XTS_OK && S > 0) {
+    if (sg.ready() == XTS_OK && S > 0) {
         XTS_CUDA(cudaEventRecord(g_ctx.fork_ev, sg.st));
         XTS_CUDA(cudaStreamWaitEvent(g_ctx.geo_stream, g_ctx.fork_ev, 0));
         a.geo_stream = g_ctx.geo_stream;
@@ -636,7 +681,7 @@ int xts_exposure_map(const xts_expcube* cube, const xts_expcube* wcube, const do
     ea.ecb = ea.wecb = ea.exposure = nullptr;
     double* out = sg.out(exposure_map, (size_t)npix * E);
     int* status = (int*)workspace(W_MISC, 64);
-    int rc = sg.rc ? sg.rc : (status ? XTS_OK : XTS_ERR_OOM);
+    int rc = sg.ready() ? sg.rc : (status ? XTS_OK : XTS_ERR_OOM);
     if (rc == XTS_OK) {
         cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), sg.st);
         if (e != cudaSuccess) rc = cuda_error(e, "cudaMemsetAsync");
@@ -845,7 +890,7 @@ static int fused_maps(const xts_expcube* cube, const xts_expcube* wcube, const d
     // stream from here on, beside the livetime-cube upload, the exposure and the
     // mean PSF, and joins the launching stream before the correction factors.
     const double* src_d = sg.in(src_sph, (size_t)2 * S);
-    const bool fork = sg.rc == XTS_OK && S > 0;
+    const bool fork = sg.ready() == XTS_OK && S > 0;
     if (fork) {
         XTS_CUDA(cudaEventRecord(g_ctx.fork_ev, sg.st));
         XTS_CUDA(cudaStreamWaitEvent(g_ctx.geo_stream, g_ctx.fork_ev, 0));
@@ -898,7 +943,7 @@ static int fused_maps(const xts_expcube* cube, const xts_expcube* wcube, const d
         if (stats) memset(stats, 0, sizeof(*stats));
     }
     if (fork) { ma.geo_stream = g_ctx.geo_stream; ma.join_ev = g_ctx.join_ev; }
-    int rc = sg.rc;
+    int rc = sg.ready();
     // exposure and mean PSF on the library's highest-priority stream: the window pass
     // (one short block per work item, on the geometry stream) fills the GPU, and these
     // kernels' blocks are then scheduled ahead of its pending ones as slots free up
@@ -963,7 +1008,7 @@ int xts_make_psf_kernel(const xts_wcs* kernel_wcs, int Nk, const double* upsf, i
     Stager sg{(flags & XTS_DEVICE_PTRS) != 0, stream ? (cudaStream_t)stream : g_ctx.stream};
     const double* u = sg.in(upsf, (size_t)ND * E);
     double* k = sg.out(kernel, (size_t)E * Nk * Nk);
-    int rc = sg.rc ? sg.rc : make_psf_kernel(*kernel_wcs, Nk, u, E, k, sg.st);
+    int rc = sg.ready() ? sg.rc : make_psf_kernel(*kernel_wcs, Nk, u, E, k, sg.st);
     return sg.finish(rc);
 }
 
@@ -979,7 +1024,7 @@ int xts_convolve_map_psf(const double* image, int E, int H, int W, const double*
     const double* im = sg.in(image, (size_t)E * H * W);
     const double* ke = sg.in(kernel, (size_t)E * K * K);
     double* o = sg.out(out, (size_t)E * PH * PW);
-    int rc = sg.rc ? sg.rc : convolve_map_psf(im, E, H, W, ke, K, o, sg.st);
+    int rc = sg.ready() ? sg.rc : convolve_map_psf(im, E, H, W, ke, K, o, sg.st);
     return sg.finish(rc);
 }
 
@@ -1076,7 +1121,7 @@ int xts_point_src_model_map_cutouts(const xts_wcs* wcs, const double* src_sph, i
     a.correction = info ? sg.out(info->correction, (size_t)S * E) : nullptr;
     a.radius = info ? sg.out(info->psf_radius, (size_t)S) : nullptr;
     a.in_fov = info ? sg.out(info->in_fov, (size_t)S) : nullptr;
-    int rc = sg.rc ? sg.rc : (S > 0 ? launch_srcmap(a, sg.st) : XTS_OK);
+    int rc = sg.ready() ? sg.rc : (S > 0 ? launch_srcmap(a, sg.st) : XTS_OK);
     rc = sg.finish(rc);
     if (rc == XTS_OK && !dev && S > 0) rc = srcmap_status(sg.st);
     return rc;
@@ -1112,7 +1157,7 @@ int xts_crop_allsky(const float* allsky, int E0, long NY, long NX, const long ra
     Stager sg{(flags & XTS_DEVICE_PTRS) != 0, stream ? (cudaStream_t)stream : g_ctx.stream};
     const float* sky = sg.in(allsky, (size_t)E0 * NY * NX);
     float* o = sg.out(out, (size_t)E0 * ny * nx);
-    int rc = sg.rc ? sg.rc : crop_allsky(sky, E0, NY, NX, range, o, sg.st);
+    int rc = sg.ready() ? sg.rc : crop_allsky(sky, E0, NY, NX, range, o, sg.st);
     return sg.finish(rc);
 }
 
@@ -1125,7 +1170,7 @@ int xts_trilerp_ehw(const float* src, int E0, int H0, int W0, float* dst, int E1
     Stager sg{(flags & XTS_DEVICE_PTRS) != 0, stream ? (cudaStream_t)stream : g_ctx.stream};
     const float* sp = sg.in(src, (size_t)E0 * H0 * W0);
     float* dp = sg.out(dst, (size_t)E1 * H1 * W1);
-    int rc = sg.rc ? sg.rc : trilerp_ehw(sp, E0, H0, W0, dp, E1, H1, W1, sg.st);
+    int rc = sg.ready() ? sg.rc : trilerp_ehw(sp, E0, H0, W0, dp, E1, H1, W1, sg.st);
     return sg.finish(rc);
 }
 
@@ -1161,7 +1206,7 @@ int xts_scale_model_map(const xts_wcs* wcs, const double* src_sph, int S, const 
     a.radius = info ? sg.out(info->psf_radius, (size_t)S) : nullptr;
     a.in_fov = info ? sg.out(info->in_fov, (size_t)S) : nullptr;
     a.means_given = true;
-    int rc = sg.rc ? sg.rc : launch_srcmap(a, sg.st);
+    int rc = sg.ready() ? sg.rc : launch_srcmap(a, sg.st);
     return sg.finish(rc);
 }
 

@@ -61,7 +61,7 @@ void prof_mark(const char* name, cudaStream_t st, bool begin);
 enum Slot {
     // staged inputs / outputs (host-pointer mode)
     S_IN0, S_IN1, S_IN2, S_IN3, S_IN4, S_IN5, S_IN6, S_IN7, S_IN8, S_IN9, S_IN10, S_IN11,
-    S_IN12, S_IN13, S_IN14, S_IN15, S_IN16, S_IN17,
+    S_IN12, S_IN13, S_IN14, S_IN15, S_IN16, S_IN17, S_ARENA,
     S_OUT0, S_OUT1, S_OUT2, S_OUT3, S_OUT4, S_OUT5, S_OUT6, S_OUT7, S_OUT8, S_OUT9, S_OUT10,
     S_OUT11, S_OUT12, S_OUT13, S_OUT14, S_OUT15,
     // internal scratch
