@@ -19,14 +19,13 @@
 //     training it
 //     also writes the pre-activations z1..z3 and the activations h1, h2,
 //     transposed ([128][n], coalesced across the threads of a warp).
-//   * k_gemm_bf16: C = A B^T for the backward pass (dW = dZ^T H, dH = dZ W), with
-//     either operand given transposed (gathered into the swizzled layout by the
-//     loading threads), a two-stage shared-memory ring and split-K whose partial
-//     tiles are summed in a fixed order (k_sum_splits), so training is
-//     reproducible.
-//   * k_mlp_bwd_elem: dZ = dH * gelu'(Z) per layer in the [unit][row] layout, with
-//     the bias (and output-layer and first-layer weight) gradients reduced per
-//     block into partials that k_bwd_reduce sums in a fixed order.
+//   * k_mlp_backward: dZ of all three layers per tile of 128 rows, dH on the tensor
+//     cores and never outside tensor memory, the bias, output-layer and first-layer
+//     weight gradients as per-block partials.
+//   * k_gemm_bf16: C = A B^T (the hidden weights' gradients dZ^T H), with either operand
+//     given transposed (gathered into the swizzled layout by the loading threads), a
+//     two-stage shared-memory ring and split-K into partial tiles.
+//   * k_mlp_grad_sum: all partials summed in a fixed order, so training is reproducible.
 //   * k_mlp_adam: the update of the FP32 master parameters and the BF16 copies.
 //
 // Every mbarrier wait is bounded (WAIT_LIMIT polls); a timeout sets the status
@@ -597,7 +596,9 @@ __device__ __forceinline__ void load_chunk(unsigned char* dst, const __nv_bfloat
 
 __global__ void __launch_bounds__(MT, 1)
 k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat16* __restrict__ B, int b_trans,
-            int M, int K, int cps, float* __restrict__ C, int c_trans, int atomic, int* __restrict__ status) {
+            int M, int K, int cps, float* __restrict__ C, int c_trans, int atomic, int* __restrict__ status,
+            const __nv_bfloat16* __restrict__ A2, const __nv_bfloat16* __restrict__ B2) {
+    if (blockIdx.z) { A = A2; B = B2; }  // a second product of the same shape in the same launch
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int t = threadIdx.x, warp = t >> 5;
@@ -658,7 +659,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat1
         for (int c0 = 0; c0 < MH; c0 += 16) {
             float v[16];
             tmem_ld16(trow + (unsigned)c0, v);
-            float* Cs = atomic ? C + (size_t)blockIdx.y * M * MH : C;  // split-K: this split's partial tile
+            float* Cs = atomic ? C + (size_t)(blockIdx.z * gridDim.y + blockIdx.y) * M * MH : C;  // split-K: this split's partial tile
 #pragma unroll
             for (int j = 0; j < 16; ++j)
                 *(c_trans ? Cs + (size_t)(c0 + j) * M + m : Cs + (size_t)m * MH + c0 + j) = v[j];
@@ -675,84 +676,236 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat1
 }
 
 // ====================================================================== backward
-// Per layer, in the [unit][row] layout: dz = dh * gelu'(z) (head: dh = dy * w4).
-// Block (row range, unit j): bias gradient, and for the head the output-layer
-// weight, for layer 1 the first-layer weights, reduced per block.
-enum { BW_HEAD = 0, BW_HIDDEN = 1, BW_FIRST = 2 };
-constexpr int BW_ROWS = 1024;  // rows per block (256 threads x 4)
+// One kernel from the saved pre-activations to dz3, dz2 and the gradients' column sums.
+// Per tile of 128 rows (thread = row and half of the units, as in the forward kernel):
+//   dz3 = dy w4 gelu'(z3), into the A operand and, [unit][row], to memory;
+//   dh2 = dz3 W3 on the tensor cores; dz2 = dh2 gelu'(z2), the same two places;
+//   dh1 = dz2 W2; dz1 = dh1 gelu'(z1).
+// Neither dh leaves tensor memory.  The sums over rows (biases, output and first-layer
+// weights) are taken 32 units at a time: 31 shuffles leave unit l's sum over the warp's
+// rows in lane l.  Each block adds its tiles' sums in order and writes them once;
+// k_mlp_grad_sum adds the blocks' in a fixed order, so trainings repeat bit for bit.
+// 37,888 rows: one launch of 48 us in place of three element-wise kernels, two GEMMs
+// with a transposing gather and three reductions (27 + 28 + 9 us each, one
+// after another).
+enum { BQ_B3 = 0, BQ_W4 = 1, BQ_B2 = 2, BQ_B1 = 3, BQ_W1 = 4, BQ_LOSS = 9, BQ_B4 = 10, BQ_N = 11 };
+struct BwdLayout {
+    static constexpr size_t w3t = 0, w2t = 2 * ATOM, act = 4 * ATOM;  // W3^T, W2^T, the A operand
+    static constexpr size_t w4 = 6 * ATOM;
+    static constexpr size_t red = w4 + 4 * MH;      // [6][4 row warps][MH]
+    static constexpr size_t sred = red + 4 * 6 * 4 * MH;  // [4][2]: loss, dy
+    static constexpr size_t bars = sred + 4 * 8;
+    static constexpr size_t total = bars + 64;
+};
+constexpr size_t BWD_SMEM = BwdLayout::total + 1024;
 
-__global__ void __launch_bounds__(256) k_mlp_bwd_elem(int mode, const float* __restrict__ params, MlpNorm nm,
-                                                      const float* __restrict__ zT, const float* __restrict__ dhT,
-                                                      const float* __restrict__ yn, const float* __restrict__ Y,
-                                                      const float* __restrict__ X, long long n,
-                                                      __nv_bfloat16* __restrict__ dzT,
-                                                      float* __restrict__ part) {
-    __shared__ float red[8][8];
-    const int j = blockIdx.y, t = threadIdx.x, lane = t & 31, wp = t >> 5;
-    const float w4 = __bfloat162float(__float2bfloat16_rn(params[XTS_MLP_W4 + j]));
-    const float inv_n = 1.f / (float)n;
-    // accumulators: 0 bias, 1 w4 (head) / dy (head, unit 0), 2 loss, 3..7 first-layer weights
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const long long r0 = (long long)blockIdx.x * BW_ROWS;
-    for (int i = 0; i < BW_ROWS / 256; ++i) {
-        const long long r = r0 + t + 256 * i;
-        if (r >= n) break;
-        const size_t k = (size_t)j * n + r;
-        const float z = zT[k];
-        float dh;
-        if (mode == BW_HEAD) {
-            const float tgt = (Y[r] - nm.out_mu) / nm.out_sd;
-            const float d = yn[r] - tgt;
-            const float dy = 2.f * d * inv_n;
-            dh = dy * w4;
-            acc[1] = fmaf(dy, gelu(z), acc[1]);
-            if (j == 0) { acc[2] = fmaf(d, d, acc[2]); acc[3] += dy; }
-        } else {
-            dh = dhT[k];
-        }
-        const float dz = dh * gelu_grad(z);
-        acc[0] += dz;
-        if (mode == BW_FIRST) {
+// v[i] of every lane -> the sum over the lanes of v[lane].
+__device__ __forceinline__ float lane_sums(float* v) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-            for (int q = 0; q < MI; ++q) acc[3 + q] = fmaf(dz, (X[r * MI + q] - nm.mu[q]) / nm.sd[q], acc[3 + q]);
-        } else {
-            dzT[k] = __float2bfloat16_rn(dz);
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
     }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        float v = acc[q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[wp][q] = v;
-    }
-    __syncthreads();
-    if (t < 8) {
-        float v = 0.f;
-        for (int w = 0; w < 8; ++w) v += red[w][t];
-        part[((size_t)blockIdx.x * MH + j) * 8 + t] = v;
-    }
+    return v[0];
 }
 
-// The per-block partials of k_mlp_bwd_elem summed over the row blocks in order and
-// added to the gradient (and the loss); one thread per (unit, quantity).
-__global__ void k_bwd_reduce(int mode, const float* __restrict__ part, int nbx, float inv_n,
-                             float* __restrict__ grads, float* __restrict__ loss) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= MH * 8) return;
-    const int j = i >> 3, q = i & 7;
-    float v = 0.f;
-    for (int b = 0; b < nbx; ++b) v += part[((size_t)b * MH + j) * 8 + q];
-    if (mode == BW_HEAD) {
-        if (q == 0) grads[XTS_MLP_B3 + j] += v;
-        if (q == 1) grads[XTS_MLP_W4 + j] += v;
-        if (j == 0 && q == 2 && loss) *loss += v * inv_n;
-        if (j == 0 && q == 3) grads[XTS_MLP_B4] += v;
-    } else if (mode == BW_HIDDEN) {
-        if (q == 0) grads[XTS_MLP_B2 + j] += v;
-    } else {
-        if (q == 0) grads[XTS_MLP_B1 + j] += v;
-        if (q >= 3 && q < 3 + MI) grads[XTS_MLP_W1 + j * MI + (q - 3)] += v;
+__global__ void __launch_bounds__(FT, 2)
+k_mlp_backward(const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf, MlpNorm nm,
+               const float* __restrict__ X, const float* __restrict__ Y, long long n, FwdSaves sv,
+               __nv_bfloat16* __restrict__ dz3, __nv_bfloat16* __restrict__ dz2, float* __restrict__ part,
+               int* __restrict__ status) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, r = t & (MT - 1), hf = t >> 7, cb = 64 * hf, rw = warp & 3;
+    float* w4 = (float*)(smem + BwdLayout::w4);
+    float* red = (float*)(smem + BwdLayout::red);
+    float* sred = (float*)(smem + BwdLayout::sred);
+    unsigned long long* bars = (unsigned long long*)(smem + BwdLayout::bars);
+    unsigned* tmem_slot = (unsigned*)(smem + BwdLayout::bars + 32);
+    const unsigned bar = smem_u32(&bars[0]);
+    unsigned char* act = smem + BwdLayout::act;
+    // W^T operands: row = in, K = out; a warp stores 32 consecutive outs of one in
+    for (int idx = t; idx < 2 * MH * (MH / 8); idx += FT) {
+        const int l = idx / (MH * (MH / 8)), rem = idx - l * (MH * (MH / 8));
+        const int j = rem & (MH - 1), ch = rem >> 7;
+        const uint4 v = *reinterpret_cast<const uint4*>(wbf + (size_t)l * MH * MH + j * MH + ch * 8);
+        const unsigned short* e = reinterpret_cast<const unsigned short*>(&v);
+        unsigned char* dst = smem + (l ? BwdLayout::w3t : BwdLayout::w2t);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) *reinterpret_cast<unsigned short*>(dst + sw_off(ch * 8 + q, j)) = e[q];
     }
+    for (int k = t; k < MH; k += FT) w4[k] = __bfloat162float(__float2bfloat16_rn(params[XTS_MLP_W4 + k]));
+    if (t == 0) mbar_init(bar, 1);
+    if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 128);
+    fence_async_shared();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+    const unsigned trow = tmem + ((unsigned)(rw * 32) << 16) + (unsigned)cb;
+    const float inv_n = 1.f / (float)n;
+    float total[BQ_N];  // thread t < MH: unit t's sums over the block's tiles (loss, b4: thread 0)
+#pragma unroll
+    for (int q = 0; q < BQ_N; ++q) total[q] = 0.f;
+    auto add_red = [&](int slot, int q) {
+        if (t < MH) {
+            const float* v = red + (size_t)slot * 4 * MH + t;
+            total[q] += ((v[0] + v[MH]) + v[2 * MH]) + v[3 * MH];
+        }
+    };
+    unsigned ph = 0;
+    bool ok = true;
+    for (long long tile = blockIdx.x; tile < n / MT && ok; tile += gridDim.x) {
+        const long long row = tile * MT + r;
+        const float d = sv.yn[row] - (Y[row] - nm.out_mu) / nm.out_sd, dy = 2.f * d * inv_n;
+        if (!hf) {
+            float a = d * d, b = dy;
+            for (int o = 16; o > 0; o >>= 1) {
+                a += __shfl_xor_sync(0xffffffffu, a, o);
+                b += __shfl_xor_sync(0xffffffffu, b, o);
+            }
+            if (lane == 0) { sred[2 * rw] = a; sred[2 * rw + 1] = b; }
+        }
+        float xs[MI];
+#pragma unroll
+        for (int q = 0; q < MI; ++q) xs[q] = (X[row * MI + q] - nm.mu[q]) / nm.sd[q];
+        for (int stage = 0; stage < 3 && ok; ++stage) {  // dz3, dz2, dz1
+            const float* z = stage == 0 ? sv.z3 : stage == 1 ? sv.z2 : sv.z1;
+            __nv_bfloat16* dzT = stage == 0 ? dz3 : dz2;
+#pragma unroll 1
+            for (int g = 0; g < 2; ++g) {
+                const int c0 = cb + 32 * g;
+                float dz[32], aux[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) aux[j] = z[(size_t)(c0 + j) * n + row];
+                if (stage > 0) {
+                    tmem_ld16(trow + (unsigned)(32 * g), dz);
+                    tmem_ld16(trow + (unsigned)(32 * g + 16), dz + 16);
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const float dh = stage == 0 ? dy * w4[c0 + j] : dz[j];
+                    dz[j] = dh * gelu_grad(aux[j]);
+                }
+                if (stage < 2) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float* u = dz + 8 * q;
+                        const uint4 pk = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]),
+                                                    pack_bf16(u[6], u[7]));
+                        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&pk);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) dzT[(size_t)(c0 + 8 * q + j) * n + row] = hb[j];
+                        *reinterpret_cast<uint4*>(act + sw_off(r, c0 + 8 * q)) = pk;
+                    }
+                }
+                float* rd = red + rw * MH + c0 + lane;  // slot k at rd[k * 4 * MH]
+                if (stage == 0) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) aux[j] = dy * gelu(aux[j]);
+                    rd[1 * 4 * MH] = lane_sums(aux);
+                    rd[0] = lane_sums(dz);
+                } else if (stage == 1) {
+                    rd[2 * 4 * MH] = lane_sums(dz);
+                } else {
+#pragma unroll 1
+                    for (int q = 0; q < MI; ++q) {
+                        const float x = q == 0 ? xs[0] : q == 1 ? xs[1] : q == 2 ? xs[2] : q == 3 ? xs[3] : xs[4];
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) aux[j] = dz[j] * x;
+                        rd[(1 + q) * 4 * MH] = lane_sums(aux);
+                    }
+                    rd[0] = lane_sums(dz);
+                }
+            }
+            fence_async_shared();
+            tc_fence_before();
+            __syncthreads();
+            if (stage == 0) {
+                add_red(0, BQ_B3);
+                add_red(1, BQ_W4);
+                if (t == 0) {
+                    total[BQ_LOSS] += ((sred[0] + sred[2]) + sred[4]) + sred[6];
+                    total[BQ_B4] += ((sred[1] + sred[3]) + sred[5]) + sred[7];
+                }
+            } else if (stage == 1) {
+                add_red(2, BQ_B2);
+            } else {
+                add_red(0, BQ_B1);
+#pragma unroll
+                for (int q = 0; q < MI; ++q) add_red(1 + q, BQ_W1 + q);
+                __syncthreads();  // the sums are read before the next tile writes its own
+                break;
+            }
+            if (t == 0) {
+                tc_fence_after();
+                mma_chain(tmem, smem_u32(act), smem_u32(smem + (stage == 0 ? BwdLayout::w3t : BwdLayout::w2t)), MH / 16,
+                          false);
+                mma_commit(bar);
+            }
+            const bool got = mbar_wait(bar, ph);
+            if (!__syncthreads_and(got)) { ok = false; break; }  // ph stays: the exit path waits on it
+            ph ^= 1;
+            tc_fence_after();
+        }
+    }
+    if (!ok && t == 0) {
+        atomicExch(status, 1);
+        mbar_wait(bar, ph);  // bounded: let an issued MMA land
+    }
+    if (t < MH)
+#pragma unroll
+        for (int q = 0; q < BQ_N; ++q)
+            if (q < BQ_LOSS || t == 0) part[((size_t)q * MH + t) * gridDim.x + blockIdx.x] = total[q];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) tmem_free(tmem, 128);
+}
+
+// The gradients from their parts, added to grads (and the loss): blocks 0 .. 127 the
+// hidden weights' split-K tiles (wpart [2][nsplit][MH * MH]: W3, W2), summed in order;
+// further blocks one warp per (quantity, unit) of k_mlp_backward's nb blocks.
+__global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, int nb,
+                                                      const float* __restrict__ wpart, int nsplit, float inv_n,
+                                                      float* __restrict__ grads, float* __restrict__ loss) {
+    const int wb = 2 * MH * MH / 256;
+    if ((int)blockIdx.x < wb) {
+        const int i = blockIdx.x * 256 + threadIdx.x, l = i / (MH * MH), e = i - l * (MH * MH);
+        const float* w = wpart + (size_t)l * nsplit * MH * MH + e;
+        float v = 0.f;
+        int k = 0;
+        for (; k + 16 <= nsplit; k += 16) {  // sixteen loads in flight, summed in order
+            float u[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) u[j] = w[(size_t)(k + j) * MH * MH];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v += u[j];
+        }
+        for (; k < nsplit; ++k) v += w[(size_t)k * MH * MH];
+        grads[(l ? XTS_MLP_W2 : XTS_MLP_W3) + e] += v;
+        return;
+    }
+    const int i = ((int)blockIdx.x - wb) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int q = i / MH, j = i - q * MH;
+    if (q >= BQ_N || (q >= BQ_LOSS && j > 0)) return;
+    const float* p = part + (size_t)i * nb;
+    float v = 0.f;
+    for (int b = lane; b < nb; b += 32) v += p[b];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane) return;
+    if (q == BQ_LOSS) {
+        if (loss) *loss += v * inv_n;
+        return;
+    }
+    const int at = q == BQ_B3 ? XTS_MLP_B3 + j : q == BQ_W4 ? XTS_MLP_W4 + j : q == BQ_B2 ? XTS_MLP_B2 + j
+                 : q == BQ_B1 ? XTS_MLP_B1 + j : q == BQ_B4 ? XTS_MLP_B4 : XTS_MLP_W1 + j * MI + (q - BQ_W1);
+    grads[at] += v;
 }
 
 // C[i] += sum over the splits s (in order) of part[s][i]
@@ -822,7 +975,7 @@ int launch_gemm_bf16(const void* A, int a_trans, const void* B, int b_trans, int
     }
     XTS_LAUNCH("k_gemm_bf16", st, k_gemm_bf16<<<dim3(mt, nsplit), MT, GEMM_SMEM, st>>>(
                                       (const __nv_bfloat16*)A, a_trans, (const __nv_bfloat16*)B, b_trans, M, K, cps,
-                                      dst, c_trans, accumulate, status));
+                                      dst, c_trans, accumulate, status, nullptr, nullptr));
     if (accumulate)
         XTS_LAUNCH("k_sum_splits", st, k_sum_splits<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(dst, nsplit, nc, C));
     return XTS_OK;
@@ -879,40 +1032,31 @@ static int mlp_backprop(const xts_mlp* net, const float* X, const float* Y, long
     const size_t hn = (size_t)MH * n;
     float* z = (float*)workspace(W_MLP_Z, sizeof(float) * 3 * hn);
     __nv_bfloat16* h = (__nv_bfloat16*)workspace(W_MLP_H, sizeof(__nv_bfloat16) * 2 * hn);
-    __nv_bfloat16* dz = (__nv_bfloat16*)workspace(W_MLP_DZ, sizeof(__nv_bfloat16) * hn);
-    float* dh = (float*)workspace(W_MLP_DH, sizeof(float) * hn);
+    __nv_bfloat16* dz = (__nv_bfloat16*)workspace(W_MLP_DZ, sizeof(__nv_bfloat16) * 2 * hn);
     float* yn = (float*)workspace(W_MLP_Y, sizeof(float) * n);
-    if (!z || !h || !dz || !dh || !yn) return XTS_ERR_OOM;
+    if (!z || !h || !dz || !yn) return XTS_ERR_OOM;
     FwdSaves sv{z, z + hn, z + 2 * hn, h, h + hn, yn};
     int rc = forward(net, X, n, nullptr, nullptr, sv, status, st);
     if (rc) return rc;
-    const MlpNorm nm = mlp_norm(net);
-    const int nbx = (int)((n + BW_ROWS - 1) / BW_ROWS);
-    const dim3 eg((unsigned)nbx, MH);
-    const float inv_n = 1.f / (float)n;
-    float* part = (float*)workspace(W_MLP_PART2, sizeof(float) * (size_t)nbx * MH * 8);
-    if (!part) return XTS_ERR_OOM;
-    const __nv_bfloat16* w2 = (const __nv_bfloat16*)net->wbf16;
-    const __nv_bfloat16* w3 = w2 + MH * MH;
-    // head: dz3 = dy w4 gelu'(z3); dW3 = dz3^T h2; dh2 = dz3 W3
-    XTS_LAUNCH("k_mlp_bwd", st, k_mlp_bwd_elem<<<eg, 256, 0, st>>>(BW_HEAD, net->params, nm, sv.z3, nullptr, yn, Y,
-                                                                     X, n, dz, part));
-    XTS_LAUNCH("k_bwd_reduce", st, k_bwd_reduce<<<(MH * 8 + 255) / 256, 256, 0, st>>>(BW_HEAD, part, nbx, inv_n,
-                                                                                      grads, loss));
-    if ((rc = launch_gemm_bf16(dz, 0, sv.h2, 0, MH, (int)n, grads + XTS_MLP_W3, 0, 1, status, st))) return rc;
-    if ((rc = launch_gemm_bf16(dz, 1, w3, 1, (int)n, MH, dh, 1, 0, status, st))) return rc;
-    // layer 2: dz2 = dh2 gelu'(z2); dW2 = dz2^T h1; dh1 = dz2 W2
-    XTS_LAUNCH("k_mlp_bwd", st, k_mlp_bwd_elem<<<eg, 256, 0, st>>>(BW_HIDDEN, net->params, nm, sv.z2, dh, yn, Y, X,
-                                                                     n, dz, part));
-    XTS_LAUNCH("k_bwd_reduce", st, k_bwd_reduce<<<(MH * 8 + 255) / 256, 256, 0, st>>>(BW_HIDDEN, part, nbx, inv_n,
-                                                                                      grads, loss));
-    if ((rc = launch_gemm_bf16(dz, 0, sv.h1, 0, MH, (int)n, grads + XTS_MLP_W2, 0, 1, status, st))) return rc;
-    if ((rc = launch_gemm_bf16(dz, 1, w2, 1, (int)n, MH, dh, 1, 0, status, st))) return rc;
-    // layer 1: dz1 = dh1 gelu'(z1); dW1 = dz1^T x
-    XTS_LAUNCH("k_mlp_bwd", st, k_mlp_bwd_elem<<<eg, 256, 0, st>>>(BW_FIRST, net->params, nm, sv.z1, dh, yn, Y, X,
-                                                                     n, dz, part));
-    XTS_LAUNCH("k_bwd_reduce", st, k_bwd_reduce<<<(MH * 8 + 255) / 256, 256, 0, st>>>(BW_FIRST, part, nbx, inv_n,
-                                                                                      grads, loss));
+    const long long ntiles = n / MT;
+    const int nb = (int)(ntiles < 2 * sm_count() ? ntiles : 2 * sm_count());
+    float* part = (float*)workspace(W_MLP_PART2, sizeof(float) * (size_t)BQ_N * MH * nb);
+    // the hidden weights' gradients dz3^T h2 and dz2^T h1 contract over the rows: their K
+    // chunks of 64 rows in splits, two blocks per SM together
+    const int nkc = (int)(n / 64);
+    const int want = sm_count() < nkc ? sm_count() : nkc, cps = (nkc + want - 1) / want, nsplit = (nkc + cps - 1) / cps;
+    float* wpart = (float*)workspace(W_MLP_PART, sizeof(float) * 2 * (size_t)nsplit * MH * MH);
+    if (!part || !wpart) return XTS_ERR_OOM;
+    XTS_CUDA(cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BWD_SMEM));
+    XTS_CUDA(cudaFuncSetAttribute(k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
+    XTS_LAUNCH("k_mlp_backward", st, k_mlp_backward<<<nb, FT, BWD_SMEM, st>>>(
+                                         net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, Y, n, sv, dz,
+                                         dz + hn, part, status));
+    XTS_LAUNCH("k_gemm_bf16", st, k_gemm_bf16<<<dim3(1, nsplit, 2), MT, GEMM_SMEM, st>>>(
+                                      dz, 0, sv.h2, 0, MH, (int)n, cps, wpart, 0, 1, status, dz + hn, sv.h1));
+    const int blocks = 2 * MH * MH / 256 + (BQ_N * MH + 7) / 8;
+    XTS_LAUNCH("k_mlp_grad_sum", st, k_mlp_grad_sum<<<blocks, 256, 0, st>>>(part, nb, wpart, nsplit, 1.f / (float)n,
+                                                                            grads, loss));
     return XTS_OK;
 }
 
