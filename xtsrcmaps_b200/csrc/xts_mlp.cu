@@ -15,17 +15,14 @@
 //     threads).  Layer 1 (K = 5) is one K = 16 MMA over the features split into
 //     three BF16 terms; the GELUs run on CUDA cores; each hidden layer's BF16
 //     activations are written by their row's threads straight into the swizzled
-//     A operand of the next MMA; the output layer is a per-row dot product.  For
-//     training it
-//     also writes the pre-activations z1..z3 and the activations h1, h2,
-//     transposed ([128][n], coalesced across the threads of a warp).
-//   * k_mlp_backward: dZ of all three layers per tile of 128 rows, dH on the tensor
-//     cores and never outside tensor memory, the bias, output-layer and first-layer
-//     weight gradients as per-block partials.
-//   * k_gemm_bf16: C = A B^T (the hidden weights' gradients dZ^T H), with either operand
-//     given transposed (gathered into the swizzled layout by the loading threads), a
-//     two-stage shared-memory ring and split-K into partial tiles.
-//   * k_mlp_grad_sum: all partials summed in a fixed order, so training is reproducible.
+//     A operand of the next MMA; the output layer is a per-row dot product.
+//   * k_mlp_gradient: forward and backward pass of a training batch in one kernel, the
+//     hidden weights' gradients accumulated in tensor memory.
+//   * k_gemm_bf16: C = A B^T, with either operand given transposed (gathered into the
+//     swizzled layout by the loading threads), a two-stage shared-memory ring and
+//     split-K whose partial tiles are summed in a fixed order (k_sum_splits).
+//   * k_mlp_grad_sum: k_mlp_gradient's partials summed in a fixed order, so training is
+//     reproducible.
 //   * k_mlp_adam: the update of the FP32 master parameters and the BF16 copies.
 //
 // Every mbarrier wait is bounded (WAIT_LIMIT polls); a timeout sets the status
@@ -141,7 +138,7 @@ __device__ __forceinline__ void fill_w1_operand(unsigned char* dst, const float*
         *reinterpret_cast<__nv_bfloat16*>(dst + ns_off(j, k)) = w;
     }
 }
-__device__ __forceinline__ void store_x_split(unsigned char* act, int r, const float* x) {
+__device__ __forceinline__ void split_x(const float* x, uint4* q) {
     unsigned short e[16];
 #pragma unroll
     for (int k = 0; k < MI; ++k) {
@@ -154,13 +151,22 @@ __device__ __forceinline__ void store_x_split(unsigned char* act, int r, const f
         e[2 * MI + k] = __bfloat16_as_ushort(lo);
     }
     e[15] = 0;
-    uint4 q[2];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         reinterpret_cast<unsigned*>(q)[i] = (unsigned)e[2 * i] | ((unsigned)e[2 * i + 1] << 16);
     }
+}
+__device__ __forceinline__ void store_x_split(unsigned char* act, int r, const float* x) {
+    uint4 q[2];
+    split_x(x, q);
     *reinterpret_cast<uint4*>(act + sw_off(r, 0)) = q[0];
     *reinterpret_cast<uint4*>(act + sw_off(r, 8)) = q[1];
+}
+__device__ __forceinline__ void store_x_split_ns(unsigned char* op, int r, const float* x) {
+    uint4 q[2];
+    split_x(x, q);
+    *reinterpret_cast<uint4*>(op + ns_off(r, 0)) = q[0];
+    *reinterpret_cast<uint4*>(op + ns_off(r, 8)) = q[1];
 }
 // the layer-1 MMA: A = K columns 0..15 of the swizzled activation operand, B = W1
 __device__ __forceinline__ void mma_layer1(unsigned tmem, unsigned a, unsigned w1op) {
@@ -230,23 +236,14 @@ struct FwdLayout {
 };
 constexpr size_t FWD_SMEM = FwdLayout::total + 1024;
 
-struct FwdSaves {  // training only; all NULL for inference
-    float* z1; float* z2; float* z3;  // [128][n]
-    __nv_bfloat16* h1; __nv_bfloat16* h2;  // [128][n]
-    float* yn;  // [n] standardised output
-};
-
 // Thread t works on row r = t & 127 of the tile and hidden columns [64 hf, 64 hf + 64),
 // hf = t >> 7: warp w reads tensor-memory lanes 32 (w & 3).. and, in the A operand,
 // writes the [128][64] atom hf of its rows.  All three layers run on the tensor cores
 // (layer 1 as one K = 16 MMA over the split features); the GELUs on CUDA cores.
-// SAVE: training (pre-activations, activations and the standardised output saved;
-// y unused); else inference (y only).
-template <bool SAVE>
 __global__ void __launch_bounds__(FT, 2)
 k_mlp_forward(const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf, MlpNorm nm,
               const float* __restrict__ X, long long n, const unsigned long long* __restrict__ n_dev,
-              long long ldx, float* __restrict__ y, FwdSaves sv, int* __restrict__ status) {
+              long long ldx, float* __restrict__ y, int* __restrict__ status) {
     if (n_dev) n = min(n, (long long)*n_dev);  // rows counted on the device (at most n)
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -320,8 +317,6 @@ k_mlp_forward(const float* __restrict__ params, const __nv_bfloat16* __restrict_
             ph ^= 1;
             tc_fence_after();
             const float* bias = layer == 1 ? b1 : layer == 2 ? b2 : b3;
-            float* zs = SAVE ? (layer == 1 ? sv.z1 : layer == 2 ? sv.z2 : sv.z3) : nullptr;
-            __nv_bfloat16* hs = SAVE ? (layer == 1 ? sv.h1 : sv.h2) : nullptr;
             for (int c0 = 0; c0 < 64; c0 += 16) {
                 float v[16], bv[16];
                 tmem_ld16(trow + (unsigned)c0, v);
@@ -334,10 +329,6 @@ k_mlp_forward(const float* __restrict__ params, const __nv_bfloat16* __restrict_
 #pragma unroll
                 for (int j = 0; j < 16; j += 2) {
                     const float2 z = __fadd2_rn(make_float2(v[j], v[j + 1]), make_float2(bv[j], bv[j + 1]));
-                    if (SAVE && live) {
-                        zs[(size_t)(cc + j) * n + row] = z.x;
-                        zs[(size_t)(cc + j + 1) * n + row] = z.y;
-                    }
                     const float2 g2 = gelu2(z);
                     v[j] = g2.x;
                     v[j + 1] = g2.y;
@@ -348,11 +339,6 @@ k_mlp_forward(const float* __restrict__ params, const __nv_bfloat16* __restrict_
                         const float* u = v + 8 * q;
                         uint4 pk = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]),
                                               pack_bf16(u[6], u[7]));
-                        if (SAVE && live) {
-                            const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&pk);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) hs[(size_t)(cc + 8 * q + j) * n + row] = hb[j];
-                        }
                         *reinterpret_cast<uint4*>(smem + FwdLayout::act + sw_off(r, cc + 8 * q)) = pk;
                     }
                 } else {
@@ -371,8 +357,7 @@ k_mlp_forward(const float* __restrict__ params, const __nv_bfloat16* __restrict_
         __syncthreads();
         if (!hf && live) {
             const float yn = (yacc + ypart[r]) + b4[0];
-            if (SAVE) sv.yn[row] = yn;
-            else y[row] = fmaf(yn, nm.out_sd, nm.out_mu);
+            y[row] = fmaf(yn, nm.out_sd, nm.out_mu);
         }
     }
     if (!ok && t == 0) {
@@ -386,7 +371,7 @@ k_mlp_forward(const float* __restrict__ params, const __nv_bfloat16* __restrict_
 }
 
 // ====================================================================== inference
-// k_mlp_infer: the same forward arithmetic as k_mlp_forward<false>, with four tiles in
+// k_mlp_infer: the same forward arithmetic as k_mlp_forward, with four tiles in
 // flight per SM.  One block per SM of four warpgroups; warpgroup g owns tile slot g
 // (its BF16 activation operand and accumulator columns [128 g, 128 g + 128) of tensor
 // memory) and runs its own tiles, thread = row, all 128 columns per thread; the three
@@ -596,9 +581,7 @@ __device__ __forceinline__ void load_chunk(unsigned char* dst, const __nv_bfloat
 
 __global__ void __launch_bounds__(MT, 1)
 k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat16* __restrict__ B, int b_trans,
-            int M, int K, int cps, float* __restrict__ C, int c_trans, int atomic, int* __restrict__ status,
-            const __nv_bfloat16* __restrict__ A2, const __nv_bfloat16* __restrict__ B2) {
-    if (blockIdx.z) { A = A2; B = B2; }  // a second product of the same shape in the same launch
+            int M, int K, int cps, float* __restrict__ C, int c_trans, int atomic, int* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int t = threadIdx.x, warp = t >> 5;
@@ -659,7 +642,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat1
         for (int c0 = 0; c0 < MH; c0 += 16) {
             float v[16];
             tmem_ld16(trow + (unsigned)c0, v);
-            float* Cs = atomic ? C + (size_t)(blockIdx.z * gridDim.y + blockIdx.y) * M * MH : C;  // split-K: this split's partial tile
+            float* Cs = atomic ? C + (size_t)blockIdx.y * M * MH : C;  // split-K: this split's partial tile
 #pragma unroll
             for (int j = 0; j < 16; ++j)
                 *(c_trans ? Cs + (size_t)(c0 + j) * M + m : Cs + (size_t)m * MH + c0 + j) = v[j];
@@ -675,224 +658,386 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat1
     if (warp == 0) tmem_free(tmem, 128);
 }
 
-// ====================================================================== backward
-// One kernel from the saved pre-activations to dz3, dz2 and the gradients' column sums.
-// Per tile of 128 rows (thread = row and half of the units, as in the forward kernel):
-//   dz3 = dy w4 gelu'(z3), into the A operand and, [unit][row], to memory;
-//   dh2 = dz3 W3 on the tensor cores; dz2 = dh2 gelu'(z2), the same two places;
-//   dh1 = dz2 W2; dz1 = dh1 gelu'(z1).
-// Neither dh leaves tensor memory.  The sums over rows (biases, output and first-layer
-// weights) are taken 32 units at a time: 31 shuffles leave unit l's sum over the warp's
-// rows in lane l.  Each block adds its tiles' sums in order and writes them once;
+// ====================================================================== training
+// One kernel from the batch to all partial sums of the gradient.  A block takes tiles of
+// 128 rows; thread = row r and 32 of the 128 units (four warpgroups).  Per tile:
+//   z1 = W1 x -> accumulator A, h1 to shared memory;  z2 = W2 h1 -> B, h2;  z3 = W3 h2 -> A;
+//   dz3 = dy w4 gelu'(z3), to shared memory as BF16;  dh2 = dz3 W3 -> A,  dW3 += dz3^T h2;
+//   dz2 = dh2 gelu'(z2);  dh1 = dz2 W2 -> B,  dW2 += dz2^T h1,  z1 once more -> A;
+//   dz1 = dh1 gelu'(z1).
+// No pre-activation, activation or dh leaves the SM: A, B, dW3 and dW2 fill the 512
+// columns of tensor memory, the two weight gradients staying there over the block's tiles.
+// Each operand is stored once: W, dz and h are read as K-major in the one product and,
+// with the transpose bits of the instruction, along the other axis in the next.  A weight
+// product is waited for only before its operands are written again.  Sums over rows
+// (biases, W1, w4): each warp turns 32 rows x 16 units through its own shared memory and a
+// lane adds eight rows of a pair of units (a shuffle butterfly took four instructions per
+// value and sum, this takes one and a half).  Each block writes its sums once;
 // k_mlp_grad_sum adds the blocks' in a fixed order, so trainings repeat bit for bit.
-// 37,888 rows: one launch of 48 us in place of three element-wise kernels, two GEMMs
-// with a transposing gather and three reductions (27 + 28 + 9 us each, one
-// after another).
+// 37,888 rows (two tiles per block): @GRAD@
 enum { BQ_B3 = 0, BQ_W4 = 1, BQ_B2 = 2, BQ_B1 = 3, BQ_W1 = 4, BQ_LOSS = 9, BQ_B4 = 10, BQ_N = 11 };
-struct BwdLayout {
-    static constexpr size_t w3t = 0, w2t = 2 * ATOM, act = 4 * ATOM;  // W3^T, W2^T, the A operand
-    static constexpr size_t w4 = 6 * ATOM;
-    static constexpr size_t red = w4 + 4 * MH;      // [6][4 row warps][MH]
-    static constexpr size_t sred = red + 4 * 6 * 4 * MH;  // [4][2]: loss, dy
+constexpr int GT = 4 * MT;  // threads
+struct GradLayout {
+    static constexpr size_t w2 = 0, w3 = 2 * ATOM, h1 = 4 * ATOM, h2 = 6 * ATOM, dz = 8 * ATOM;
+    static constexpr size_t w1 = 10 * ATOM, xop = w1 + W1OP;     // layer 1's operands, no swizzle
+    static constexpr size_t turn = xop + W1OP;                   // [16 warps][32 rows][8] pairs
+    static constexpr size_t xs = turn + 16 * 32 * 8 * 8;         // [MT][8]: x, then y's parts 1..3
+    static constexpr size_t tot = xs + MT * 8 * 4;               // [9][4 row warps][MH]
+    static constexpr size_t f32 = tot + 9 * 4 * MH * 4;          // b1, b2, b3, w4, y's part 0 [MT], b4 (+3)
+    static constexpr size_t sred = f32 + 4 * (5 * MH + 4);       // [4][2]: loss, dy
     static constexpr size_t bars = sred + 4 * 8;
     static constexpr size_t total = bars + 64;
 };
-constexpr size_t BWD_SMEM = BwdLayout::total + 1024;
+constexpr size_t GRAD_SMEM = GradLayout::total + 1024;
+static_assert(GRAD_SMEM <= 232448, "shared memory of one block");
 
-// v[i] of every lane -> the sum over the lanes of v[lane].
-__device__ __forceinline__ float lane_sums(float* v) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int i = 0; i < o; ++i) {
-            const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
+// An operand of [128][64] atoms read along its other axis (M or N = the atom's 64
+// contiguous elements, K = its rows): 128-byte swizzle, next 64 elements ATOM bytes on
+// (leading offset), next 8 rows 1024 bytes on (stride offset); 16 rows per MMA step.
+static __device__ __forceinline__ unsigned long long m_desc_mn(unsigned addr) {
+    return (unsigned long long)((addr >> 4) & 0x3FFF) | ((unsigned long long)(ATOM >> 4) << 16) | (64ull << 32) |
+           (1ull << 46) | (2ull << 61);
+}
+constexpr unsigned A_MN = 1u << 15, B_MN = 1u << 16;
+
+// D = A B over K = 128; A K-major (adv 0) or along its other axis, B along its other axis
+template <bool AT>
+__device__ __forceinline__ void mma_chain_t(unsigned tmem, unsigned a, unsigned b, bool acc0) {
+    for (int ks = 0; ks < 8; ++ks) {
+        const unsigned long long da = AT ? m_desc_mn(a + (unsigned)(ks * 2048))
+                                         : m_desc(a + (unsigned)((ks >> 2) * ATOM + (ks & 3) * 32));
+        const unsigned long long db = m_desc_mn(b + (unsigned)(ks * 2048));
+        const unsigned acc = (acc0 || ks > 0) ? 1u : 0u;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+                     :: "r"(tmem), "l"(da), "l"(db), "r"(M_IDESC | B_MN | (AT ? A_MN : 0u)), "r"(acc), "r"(0u));
     }
-    return v[0];
 }
 
-__global__ void __launch_bounds__(FT, 2)
-k_mlp_backward(const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf, MlpNorm nm,
-               const float* __restrict__ X, const float* __restrict__ Y, long long n, FwdSaves sv,
-               __nv_bfloat16* __restrict__ dz3, __nv_bfloat16* __restrict__ dz2, float* __restrict__ part,
-               int* __restrict__ status) {
+__device__ __forceinline__ void store_bf16x16(unsigned char* op, int r, int c, const float* u) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+        *reinterpret_cast<uint4*>(op + sw_off(r, c + 8 * q)) =
+            make_uint4(pack_bf16(u[8 * q], u[8 * q + 1]), pack_bf16(u[8 * q + 2], u[8 * q + 3]),
+                       pack_bf16(u[8 * q + 4], u[8 * q + 5]), pack_bf16(u[8 * q + 6], u[8 * q + 7]));
+}
+
+// Sums over the warp's 32 rows (lane = row) of 16 units, added to tot[unit], and with XW
+// the five sums weighted by the rows' features, to tot[(1 + q) * 4 * MH + unit].  Pair p of
+// row r at word pair 8 r + (p ^ (r / 2 & 7)): writes (a row per lane) and reads (eight pairs
+// of four rows) each touch all banks once per half warp.  The lane that adds to a slot of
+// tot is always the same.
+template <bool XW>
+__device__ __forceinline__ void row_sums(float2* turn, const float* v, const float* xs, float* tot) {
+    const int lane = threadIdx.x & 31, pair = lane & 7, rg = lane >> 3;
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 8; ++p) turn[lane * 8 + (p ^ ((lane >> 1) & 7))] = make_float2(v[2 * p], v[2 * p + 1]);
+    __syncwarp();
+    constexpr int NS = XW ? 1 + MI : 1;
+    float2 s[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) s[k] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = rg + 4 * i;
+        const float2 u = turn[row * 8 + (pair ^ ((row >> 1) & 7))];
+        s[0] = __fadd2_rn(s[0], u);
+        if (XW) {
+            const float4 x = *reinterpret_cast<const float4*>(xs + row * 8);
+            const float x4 = xs[row * 8 + 4];
+            s[1 % NS] = __ffma2_rn(u, make_float2(x.x, x.x), s[1 % NS]);
+            s[2 % NS] = __ffma2_rn(u, make_float2(x.y, x.y), s[2 % NS]);
+            s[3 % NS] = __ffma2_rn(u, make_float2(x.z, x.z), s[3 % NS]);
+            s[4 % NS] = __ffma2_rn(u, make_float2(x.w, x.w), s[4 % NS]);
+            s[5 % NS] = __ffma2_rn(u, make_float2(x4, x4), s[5 % NS]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+#pragma unroll
+        for (int o = 8; o <= 16; o <<= 1) {
+            s[k].x += __shfl_xor_sync(0xffffffffu, s[k].x, o);
+            s[k].y += __shfl_xor_sync(0xffffffffu, s[k].y, o);
+        }
+        if (rg == 0) {
+            float2* d = reinterpret_cast<float2*>(tot + k * 4 * MH + 2 * pair);
+            *d = __fadd2_rn(*d, s[k]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(GT, 1)
+k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf, MlpNorm nm,
+               const float* __restrict__ X, const float* __restrict__ Y, long long n, float* __restrict__ part,
+               float* __restrict__ wpart, int* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, r = t & (MT - 1), hf = t >> 7, cb = 64 * hf, rw = warp & 3;
-    float* w4 = (float*)(smem + BwdLayout::w4);
-    float* red = (float*)(smem + BwdLayout::red);
-    float* sred = (float*)(smem + BwdLayout::sred);
-    unsigned long long* bars = (unsigned long long*)(smem + BwdLayout::bars);
-    unsigned* tmem_slot = (unsigned*)(smem + BwdLayout::bars + 32);
-    const unsigned bar = smem_u32(&bars[0]);
-    unsigned char* act = smem + BwdLayout::act;
-    // W^T operands: row = in, K = out; a warp stores 32 consecutive outs of one in
-    for (int idx = t; idx < 2 * MH * (MH / 8); idx += FT) {
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, r = t & (MT - 1), qd = t >> 7, cb = 32 * qd, rw = warp & 3;
+    unsigned char* h1 = smem + GradLayout::h1;
+    unsigned char* h2 = smem + GradLayout::h2;
+    unsigned char* dz = smem + GradLayout::dz;
+    unsigned char* xop = smem + GradLayout::xop;
+    float2* turn = (float2*)(smem + GradLayout::turn) + warp * 256;
+    float* xs = (float*)(smem + GradLayout::xs);
+    float* tot = (float*)(smem + GradLayout::tot);
+    float* b1 = (float*)(smem + GradLayout::f32);
+    float* b2 = b1 + MH;
+    float* b3 = b2 + MH;
+    float* w4 = b3 + MH;
+    float* y0 = w4 + MH;
+    float* b4 = y0 + MT;
+    float* sred = (float*)(smem + GradLayout::sred);
+    unsigned long long* bars = (unsigned long long*)(smem + GradLayout::bars);
+    unsigned* tmem_slot = (unsigned*)(smem + GradLayout::bars + 32);
+    const unsigned bar = smem_u32(&bars[0]), wbar = smem_u32(&bars[1]);
+    const unsigned s_w1 = smem_u32(smem + GradLayout::w1), s_w2 = smem_u32(smem + GradLayout::w2);
+    const unsigned s_w3 = smem_u32(smem + GradLayout::w3), s_x = smem_u32(xop);
+    const unsigned s_h1 = smem_u32(h1), s_h2 = smem_u32(h2), s_dz = smem_u32(dz);
+
+    for (int idx = t; idx < 2 * MH * (MH / 8); idx += GT) {
         const int l = idx / (MH * (MH / 8)), rem = idx - l * (MH * (MH / 8));
-        const int j = rem & (MH - 1), ch = rem >> 7;
-        const uint4 v = *reinterpret_cast<const uint4*>(wbf + (size_t)l * MH * MH + j * MH + ch * 8);
-        const unsigned short* e = reinterpret_cast<const unsigned short*>(&v);
-        unsigned char* dst = smem + (l ? BwdLayout::w3t : BwdLayout::w2t);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) *reinterpret_cast<unsigned short*>(dst + sw_off(ch * 8 + q, j)) = e[q];
+        const int row = rem >> 4, ch = rem & 15;
+        const uint4 v = *reinterpret_cast<const uint4*>(wbf + (size_t)l * MH * MH + row * MH + ch * 8);
+        *reinterpret_cast<uint4*>(smem + (l ? GradLayout::w3 : GradLayout::w2) + sw_off(row, ch * 8)) = v;
     }
-    for (int k = t; k < MH; k += FT) w4[k] = __bfloat162float(__float2bfloat16_rn(params[XTS_MLP_W4 + k]));
-    if (t == 0) mbar_init(bar, 1);
-    if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 128);
+    fill_w1_operand(smem + GradLayout::w1, params, t, GT);
+    for (int k = t; k < 9 * 4 * MH; k += GT) tot[k] = 0.f;
+    if (t < MH) {
+        b1[t] = params[XTS_MLP_B1 + t];
+        b2[t] = params[XTS_MLP_B2 + t];
+        b3[t] = params[XTS_MLP_B3 + t];
+        w4[t] = __bfloat162float(__float2bfloat16_rn(params[XTS_MLP_W4 + t]));
+    }
+    if (t == 0) {
+        b4[0] = params[XTS_MLP_B4];
+        mbar_init(bar, 1);
+        mbar_init(wbar, 1);
+    }
+    if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 512);
     fence_async_shared();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = *tmem_slot;
-    const unsigned trow = tmem + ((unsigned)(rw * 32) << 16) + (unsigned)cb;
+    const unsigned tm = *tmem_slot, t_a = tm, t_b = tm + 128, t_w3 = tm + 256, t_w2 = tm + 384;
+    const unsigned lane0 = (unsigned)(rw * 32) << 16;
     const float inv_n = 1.f / (float)n;
-    float total[BQ_N];  // thread t < MH: unit t's sums over the block's tiles (loss, b4: thread 0)
+    float sum_d2 = 0.f, sum_dy = 0.f;
+    unsigned ph = 0, wph = 0;
+    bool ok = true, got = true, wpend = false;  // wpend: a weight product not yet waited for
+    // operands in shared memory and the accumulators' last readers, then the MMAs of issue
+    auto mma_phase = [&](auto issue) {
+        fence_async_shared();
+        tc_fence_before();
+        __syncthreads();
+        if (t == 0) {
+            tc_fence_after();
+            issue();
+        }
+        const bool g = mbar_wait(bar, ph);
+        if (!__syncthreads_and(g && got)) return false;  // ph stays: the exit path waits on it
+        ph ^= 1;
+        tc_fence_after();
+        return true;
+    };
+    // each thread sees the weight product complete; a timeout ends the next mma_phase
+    auto weights_done = [&]() {
+        if (wpend && mbar_wait(wbar, wph)) {
+            wph ^= 1;
+            wpend = false;
+        }
+        got = got && !wpend;
+        __syncwarp();
+    };
+    auto layer1 = [&](unsigned d) {  // as mma_layer1, the A operand without swizzle
+        const unsigned long long da = m_desc_ns(s_x), db = m_desc_ns(s_w1);
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+                     :: "r"(d), "l"(da), "l"(db), "r"(M_IDESC), "r"(0u), "r"(0u));
+    };
+    // 16 pre-activations of this thread's row: accumulator plus bias
+    auto load_z = [&](unsigned acc, const float* bias, int c, float* z) {
+        tmem_ld16(acc + lane0 + (unsigned)c, z);
 #pragma unroll
-    for (int q = 0; q < BQ_N; ++q) total[q] = 0.f;
-    auto add_red = [&](int slot, int q) {
-        if (t < MH) {
-            const float* v = red + (size_t)slot * 4 * MH + t;
-            total[q] += ((v[0] + v[MH]) + v[2 * MH]) + v[3 * MH];
+        for (int q = 0; q < 4; ++q) {
+            const float4 b = reinterpret_cast<const float4*>(bias + c)[q];
+            z[4 * q] += b.x; z[4 * q + 1] += b.y; z[4 * q + 2] += b.z; z[4 * q + 3] += b.w;
         }
     };
-    unsigned ph = 0;
-    bool ok = true;
-    for (long long tile = blockIdx.x; tile < n / MT && ok; tile += gridDim.x) {
+    auto act16 = [&](float* z) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+            const float2 g = gelu2(make_float2(z[j], z[j + 1]));
+            z[j] = g.x;
+            z[j + 1] = g.y;
+        }
+    };
+    const long long ntiles = n / MT;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const long long row = tile * MT + r;
-        const float d = sv.yn[row] - (Y[row] - nm.out_mu) / nm.out_sd, dy = 2.f * d * inv_n;
-        if (!hf) {
-            float a = d * d, b = dy;
-            for (int o = 16; o > 0; o >>= 1) {
-                a += __shfl_xor_sync(0xffffffffu, a, o);
-                b += __shfl_xor_sync(0xffffffffu, b, o);
-            }
-            if (lane == 0) { sred[2 * rw] = a; sred[2 * rw + 1] = b; }
+        if (qd == 0) {
+            float x[MI];
+#pragma unroll
+            for (int k = 0; k < MI; ++k) xs[r * 8 + k] = x[k] = (X[row * MI + k] - nm.mu[k]) / nm.sd[k];
+            store_x_split_ns(xop, r, x);
         }
-        float xs[MI];
-#pragma unroll
-        for (int q = 0; q < MI; ++q) xs[q] = (X[row * MI + q] - nm.mu[q]) / nm.sd[q];
-        for (int stage = 0; stage < 3 && ok; ++stage) {  // dz3, dz2, dz1
-            const float* z = stage == 0 ? sv.z3 : stage == 1 ? sv.z2 : sv.z1;
-            __nv_bfloat16* dzT = stage == 0 ? dz3 : dz2;
+        const float target = (Y[row] - nm.out_mu) / nm.out_sd;
+        if (!(ok = mma_phase([&] { layer1(t_a); mma_commit(bar); }))) break;
+        weights_done();  // the previous tile's dW2 has read h1 and dz
+        float v[16], u[16];
 #pragma unroll 1
-            for (int g = 0; g < 2; ++g) {
-                const int c0 = cb + 32 * g;
-                float dz[32], aux[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) aux[j] = z[(size_t)(c0 + j) * n + row];
-                if (stage > 0) {
-                    tmem_ld16(trow + (unsigned)(32 * g), dz);
-                    tmem_ld16(trow + (unsigned)(32 * g + 16), dz + 16);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const float dh = stage == 0 ? dy * w4[c0 + j] : dz[j];
-                    dz[j] = dh * gelu_grad(aux[j]);
-                }
-                if (stage < 2) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float* u = dz + 8 * q;
-                        const uint4 pk = make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]),
-                                                    pack_bf16(u[6], u[7]));
-                        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&pk);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) dzT[(size_t)(c0 + 8 * q + j) * n + row] = hb[j];
-                        *reinterpret_cast<uint4*>(act + sw_off(r, c0 + 8 * q)) = pk;
-                    }
-                }
-                float* rd = red + rw * MH + c0 + lane;  // slot k at rd[k * 4 * MH]
-                if (stage == 0) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) aux[j] = dy * gelu(aux[j]);
-                    rd[1 * 4 * MH] = lane_sums(aux);
-                    rd[0] = lane_sums(dz);
-                } else if (stage == 1) {
-                    rd[2 * 4 * MH] = lane_sums(dz);
-                } else {
-#pragma unroll 1
-                    for (int q = 0; q < MI; ++q) {
-                        const float x = q == 0 ? xs[0] : q == 1 ? xs[1] : q == 2 ? xs[2] : q == 3 ? xs[3] : xs[4];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) aux[j] = dz[j] * x;
-                        rd[(1 + q) * 4 * MH] = lane_sums(aux);
-                    }
-                    rd[0] = lane_sums(dz);
-                }
-            }
-            fence_async_shared();
-            tc_fence_before();
-            __syncthreads();
-            if (stage == 0) {
-                add_red(0, BQ_B3);
-                add_red(1, BQ_W4);
-                if (t == 0) {
-                    total[BQ_LOSS] += ((sred[0] + sred[2]) + sred[4]) + sred[6];
-                    total[BQ_B4] += ((sred[1] + sred[3]) + sred[5]) + sred[7];
-                }
-            } else if (stage == 1) {
-                add_red(2, BQ_B2);
-            } else {
-                add_red(0, BQ_B1);
-#pragma unroll
-                for (int q = 0; q < MI; ++q) add_red(1 + q, BQ_W1 + q);
-                __syncthreads();  // the sums are read before the next tile writes its own
-                break;
-            }
-            if (t == 0) {
-                tc_fence_after();
-                mma_chain(tmem, smem_u32(act), smem_u32(smem + (stage == 0 ? BwdLayout::w3t : BwdLayout::w2t)), MH / 16,
-                          false);
-                mma_commit(bar);
-            }
-            const bool got = mbar_wait(bar, ph);
-            if (!__syncthreads_and(got)) { ok = false; break; }  // ph stays: the exit path waits on it
-            ph ^= 1;
-            tc_fence_after();
+        for (int c = cb; c < cb + 32; c += 16) {
+            load_z(t_a, b1, c, v);
+            act16(v);
+            store_bf16x16(h1, r, c, v);
         }
+        if (!(ok = mma_phase([&] { mma_chain(t_b, s_h1, s_w2, 8, false); mma_commit(bar); }))) break;
+#pragma unroll 1
+        for (int c = cb; c < cb + 32; c += 16) {
+            load_z(t_b, b2, c, v);
+            act16(v);
+            store_bf16x16(h2, r, c, v);
+        }
+        if (!(ok = mma_phase([&] { mma_chain(t_a, s_h2, s_w3, 8, false); mma_commit(bar); }))) break;
+        float yp = 0.f;
+#pragma unroll 1
+        for (int c = cb; c < cb + 32; c += 16) {
+            load_z(t_a, b3, c, v);
+            act16(v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) yp = fmaf(v[j], w4[c + j], yp);
+        }
+        *(qd ? xs + r * 8 + MI - 1 + qd : y0 + r) = yp;
+        __syncthreads();
+        const float yn = ((y0[r] + xs[r * 8 + MI]) + (xs[r * 8 + MI + 1] + xs[r * 8 + MI + 2])) + b4[0];
+        const float d = yn - target, dy = 2.f * d * inv_n;
+        if (qd == 0) {
+            sum_d2 = fmaf(d, d, sum_d2);
+            sum_dy += dy;
+        }
+#pragma unroll 1
+        for (int c = cb; c < cb + 32; c += 16) {
+            load_z(t_a, b3, c, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                u[j] = dy * gelu(v[j]);
+                v[j] = dy * w4[c + j] * gelu_grad(v[j]);
+            }
+            store_bf16x16(dz, r, c, v);
+            row_sums<false>(turn, v, nullptr, tot + (BQ_B3 * 4 + rw) * MH + c);
+            row_sums<false>(turn, u, nullptr, tot + (BQ_W4 * 4 + rw) * MH + c);
+        }
+        const bool first = tile == blockIdx.x;
+        if (!(ok = mma_phase([&] {
+                  mma_chain_t<false>(t_a, s_dz, s_w3, false);
+                  mma_commit(bar);
+                  mma_chain_t<true>(t_w3, s_dz, s_h2, !first);
+                  mma_commit(wbar);
+              })))
+            break;
+        wpend = true;
+#pragma unroll 1
+        for (int c = cb; c < cb + 32; c += 16) {
+            load_z(t_b, b2, c, v);
+            tmem_ld16(t_a + lane0 + (unsigned)c, u);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = u[j] * gelu_grad(v[j]);
+            row_sums<false>(turn, v, nullptr, tot + (BQ_B2 * 4 + rw) * MH + c);
+            weights_done();  // dW3 has read dz
+            store_bf16x16(dz, r, c, v);
+        }
+        if (!(ok = mma_phase([&] {
+                  mma_chain_t<false>(t_b, s_dz, s_w2, false);
+                  layer1(t_a);
+                  mma_commit(bar);
+                  mma_chain_t<true>(t_w2, s_dz, s_h1, !first);
+                  mma_commit(wbar);
+              })))
+            break;
+        wpend = true;
+#pragma unroll 1
+        for (int c = cb; c < cb + 32; c += 16) {
+            load_z(t_a, b1, c, v);
+            tmem_ld16(t_b + lane0 + (unsigned)c, u);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = u[j] * gelu_grad(v[j]);
+            row_sums<true>(turn, v, xs + rw * 32 * 8, tot + (BQ_B1 * 4 + rw) * MH + c);
+        }
+        __syncthreads();  // xs is read before the next tile's is written
     }
-    if (!ok && t == 0) {
+    if (ok) {
+        weights_done();
+        ok = __syncthreads_and(got);
+    }
+    if (ok) {
+        tc_fence_after();
+        const int l = qd >> 1, hc = 64 * (qd & 1);
+        float* dst = wpart + (((size_t)l * gridDim.x + blockIdx.x) * MH + r) * MH + hc;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 16) {
+            float w[16];
+            tmem_ld16((l ? t_w2 : t_w3) + lane0 + (unsigned)(hc + c), w);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                reinterpret_cast<float4*>(dst + c)[q] = make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            sum_d2 += __shfl_xor_sync(0xffffffffu, sum_d2, o);
+            sum_dy += __shfl_xor_sync(0xffffffffu, sum_dy, o);
+        }
+        if (qd == 0 && lane == 0) { sred[2 * rw] = sum_d2; sred[2 * rw + 1] = sum_dy; }
+    } else if (t == 0) {
         atomicExch(status, 1);
-        mbar_wait(bar, ph);  // bounded: let an issued MMA land
+        mbar_wait(bar, ph);  // bounded: let issued MMAs land
+        if (wpend) mbar_wait(wbar, wph);
     }
-    if (t < MH)
-#pragma unroll
-        for (int q = 0; q < BQ_N; ++q)
-            if (q < BQ_LOSS || t == 0) part[((size_t)q * MH + t) * gridDim.x + blockIdx.x] = total[q];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_free(tmem, 128);
+    if (ok) {
+        for (int k = t; k < 9 * MH; k += GT) {
+            const float* a = tot + (size_t)(k / MH) * 4 * MH + k % MH;
+            part[(size_t)k * gridDim.x + blockIdx.x] = ((a[0] + a[MH]) + a[2 * MH]) + a[3 * MH];
+        }
+        if (t < 2)
+            part[(size_t)(BQ_LOSS + t) * MH * gridDim.x + blockIdx.x] =
+                ((sred[t] + sred[2 + t]) + sred[4 + t]) + sred[6 + t];
+    }
+    if (warp == 0) tmem_free(tm, 512);
 }
 
-// The gradients from their parts, added to grads (and the loss): blocks 0 .. 127 the
-// hidden weights' split-K tiles (wpart [2][nsplit][MH * MH]: W3, W2), summed in order;
-// further blocks one warp per (quantity, unit) of k_mlp_backward's nb blocks.
-__global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, int nb,
-                                                      const float* __restrict__ wpart, int nsplit, float inv_n,
-                                                      float* __restrict__ grads, float* __restrict__ loss) {
-    const int wb = 2 * MH * MH / 256;
-    if ((int)blockIdx.x < wb) {
-        const int i = blockIdx.x * 256 + threadIdx.x, l = i / (MH * MH), e = i - l * (MH * MH);
-        const float* w = wpart + (size_t)l * nsplit * MH * MH + e;
-        float v = 0.f;
-        int k = 0;
-        for (; k + 16 <= nsplit; k += 16) {  // sixteen loads in flight, summed in order
-            float u[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) u[j] = w[(size_t)(k + j) * MH * MH];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v += u[j];
+// The gradients from their parts, written to (add 0) or added to grads; the loss likewise.
+// Blocks 0 .. 255: 128 elements each of the hidden weights' tiles (wpart
+// [2][nb][MH * MH]: W3, W2), warp w the tiles k = w mod 8, the warps' sums in order;
+// further blocks: one warp per (quantity, unit) of k_mlp_gradient's nb blocks.
+constexpr int GS_WB = 2 * MH * MH / 128;
+__global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, const float* __restrict__ wpart,
+                                                      int nb, float inv_n, int add, float* __restrict__ grads,
+                                                      float* __restrict__ loss) {
+    __shared__ float4 red[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if ((int)blockIdx.x < GS_WB) {
+        const int l = blockIdx.x / (GS_WB / 2), e0 = (blockIdx.x - l * (GS_WB / 2)) * 128;
+        const float* w = wpart + (size_t)l * nb * MH * MH + e0 + 4 * lane;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int k = warp; k < nb; k += 8) {
+            const float4 u = *reinterpret_cast<const float4*>(w + (size_t)k * MH * MH);
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
         }
-        for (; k < nsplit; ++k) v += w[(size_t)k * MH * MH];
-        grads[(l ? XTS_MLP_W2 : XTS_MLP_W3) + e] += v;
+        red[warp][lane] = v;
+        __syncthreads();
+        if (threadIdx.x < 128) {
+            const float* f = reinterpret_cast<const float*>(red) + threadIdx.x;
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s += f[128 * k];
+            float* g = grads + (l ? XTS_MLP_W2 : XTS_MLP_W3) + e0 + threadIdx.x;
+            *g = add ? *g + s : s;
+        }
         return;
     }
-    const int i = ((int)blockIdx.x - wb) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int q = i / MH, j = i - q * MH;
+    const int i = ((int)blockIdx.x - GS_WB) * 8 + warp, q = i / MH, j = i - q * MH;
     if (q >= BQ_N || (q >= BQ_LOSS && j > 0)) return;
     const float* p = part + (size_t)i * nb;
     float v = 0.f;
@@ -900,12 +1045,12 @@ __global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ 
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane) return;
     if (q == BQ_LOSS) {
-        if (loss) *loss += v * inv_n;
+        if (loss) *loss = add ? *loss + v * inv_n : v * inv_n;
         return;
     }
     const int at = q == BQ_B3 ? XTS_MLP_B3 + j : q == BQ_W4 ? XTS_MLP_W4 + j : q == BQ_B2 ? XTS_MLP_B2 + j
                  : q == BQ_B1 ? XTS_MLP_B1 + j : q == BQ_B4 ? XTS_MLP_B4 : XTS_MLP_W1 + j * MI + (q - BQ_W1);
-    grads[at] += v;
+    grads[at] = add ? grads[at] + v : v;
 }
 
 // C[i] += sum over the splits s (in order) of part[s][i]
@@ -975,7 +1120,7 @@ int launch_gemm_bf16(const void* A, int a_trans, const void* B, int b_trans, int
     }
     XTS_LAUNCH("k_gemm_bf16", st, k_gemm_bf16<<<dim3(mt, nsplit), MT, GEMM_SMEM, st>>>(
                                       (const __nv_bfloat16*)A, a_trans, (const __nv_bfloat16*)B, b_trans, M, K, cps,
-                                      dst, c_trans, accumulate, status, nullptr, nullptr));
+                                      dst, c_trans, accumulate, status));
     if (accumulate)
         XTS_LAUNCH("k_sum_splits", st, k_sum_splits<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(dst, nsplit, nc, C));
     return XTS_OK;
@@ -983,21 +1128,14 @@ int launch_gemm_bf16(const void* A, int a_trans, const void* B, int b_trans, int
 
 // X: row-major [n][5] (ldx 0) or feature-major [5][ldx] (ldx >= n)
 static int forward(const xts_mlp* net, const float* X, long long n, const unsigned long long* n_dev, float* y,
-                   FwdSaves sv, int* status, cudaStream_t st, long long ldx = 0) {
+                   int* status, cudaStream_t st, long long ldx = 0) {
     // per call: the attribute belongs to the current device's context
-    XTS_CUDA(cudaFuncSetAttribute(k_mlp_forward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FWD_SMEM));
-    XTS_CUDA(cudaFuncSetAttribute(k_mlp_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FWD_SMEM));
-    const bool save = sv.z1 != nullptr;
-    if (save && !(sv.z2 && sv.z3 && sv.h1 && sv.h2 && sv.yn)) return set_error(XTS_ERR_ARG, "mlp forward: saves");
-    if (!save && !y) return set_error(XTS_ERR_ARG, "mlp forward: output");
+    XTS_CUDA(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FWD_SMEM));
+    if (!y) return set_error(XTS_ERR_ARG, "mlp forward: output");
     const long long ntiles = (n + MT - 1) / MT;
     const int bps = g_tuning.mlp_blocks_per_sm > 0 ? g_tuning.mlp_blocks_per_sm : 2;  // blocks per SM (two fit)
     const long long g = ntiles < bps * sm_count() ? ntiles : bps * sm_count();
-    if (save) {
-        XTS_LAUNCH("k_mlp_forward", st, k_mlp_forward<true><<<(unsigned)g, FT, FWD_SMEM, st>>>(
-                                            net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, n, n_dev,
-                                            ldx, y, sv, status));
-    } else if (g_tuning.mlp_blocks_per_sm == 0) {
+    if (g_tuning.mlp_blocks_per_sm == 0) {
         // inference: four tiles in flight per SM, one block per SM
         XTS_CUDA(cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INF_SMEM));
         const long long gi = (ntiles + IG - 1) / IG < sm_count() ? (ntiles + IG - 1) / IG : sm_count();
@@ -1005,66 +1143,46 @@ static int forward(const xts_mlp* net, const float* X, long long n, const unsign
                                             net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, n, n_dev,
                                             ldx, y, status));
     } else {
-        XTS_LAUNCH("k_mlp_forward", st, k_mlp_forward<false><<<(unsigned)g, FT, FWD_SMEM, st>>>(
+        XTS_LAUNCH("k_mlp_forward", st, k_mlp_forward<<<(unsigned)g, FT, FWD_SMEM, st>>>(
                                             net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, n, n_dev,
-                                            ldx, y, sv, status));
+                                            ldx, y, status));
     }
     return XTS_OK;
 }
 
 int launch_mlp_forward(const xts_mlp* net, const float* X, long long n, float* y, int* status, cudaStream_t st) {
     if (n <= 0) return XTS_OK;
-    return forward(net, X, n, nullptr, y, FwdSaves{}, status, st);
+    return forward(net, X, n, nullptr, y, status, st);
 }
 
 int launch_mlp_forward_dev(const xts_mlp* net, const float* X, const unsigned long long* n_dev, long long n_max,
                            float* y, int* status, cudaStream_t st, long long ldx) {
     if (n_max <= 0) return XTS_OK;
     if (ldx && ldx < n_max) return set_error(XTS_ERR_ARG, "mlp forward: feature stride below the row count");
-    return forward(net, X, n_max, n_dev, y, FwdSaves{}, status, st, ldx);
+    return forward(net, X, n_max, n_dev, y, status, st, ldx);
 }
 
-// forward with saves, then the gradient accumulated into grads (zero on entry)
-static int mlp_backprop(const xts_mlp* net, const float* X, const float* Y, long long n, float* grads,
+// the gradient written (add 0) or added to grads, the loss likewise
+static int mlp_backprop(const xts_mlp* net, const float* X, const float* Y, long long n, int add, float* grads,
                         float* loss, int* status, cudaStream_t st) {
     if (n <= 0 || n % MT) return set_error(XTS_ERR_ARG, "surrogate training: n (%lld) must be a positive multiple of 128", n);
     if (n > (1ll << 24)) return set_error(XTS_ERR_ARG, "surrogate training: n (%lld) above 2^24 rows per batch", n);
-    const size_t hn = (size_t)MH * n;
-    float* z = (float*)workspace(W_MLP_Z, sizeof(float) * 3 * hn);
-    __nv_bfloat16* h = (__nv_bfloat16*)workspace(W_MLP_H, sizeof(__nv_bfloat16) * 2 * hn);
-    __nv_bfloat16* dz = (__nv_bfloat16*)workspace(W_MLP_DZ, sizeof(__nv_bfloat16) * 2 * hn);
-    float* yn = (float*)workspace(W_MLP_Y, sizeof(float) * n);
-    if (!z || !h || !dz || !yn) return XTS_ERR_OOM;
-    FwdSaves sv{z, z + hn, z + 2 * hn, h, h + hn, yn};
-    int rc = forward(net, X, n, nullptr, nullptr, sv, status, st);
-    if (rc) return rc;
-    const long long ntiles = n / MT;
-    const int nb = (int)(ntiles < 2 * sm_count() ? ntiles : 2 * sm_count());
+    const int nb = (int)(n / MT < sm_count() ? n / MT : sm_count());
     float* part = (float*)workspace(W_MLP_PART2, sizeof(float) * (size_t)BQ_N * MH * nb);
-    // the hidden weights' gradients dz3^T h2 and dz2^T h1 contract over the rows: their K
-    // chunks of 64 rows in splits, two blocks per SM together
-    const int nkc = (int)(n / 64);
-    const int want = sm_count() < nkc ? sm_count() : nkc, cps = (nkc + want - 1) / want, nsplit = (nkc + cps - 1) / cps;
-    float* wpart = (float*)workspace(W_MLP_PART, sizeof(float) * 2 * (size_t)nsplit * MH * MH);
+    float* wpart = (float*)workspace(W_MLP_PART, sizeof(float) * 2 * (size_t)nb * MH * MH);
     if (!part || !wpart) return XTS_ERR_OOM;
-    XTS_CUDA(cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BWD_SMEM));
-    XTS_CUDA(cudaFuncSetAttribute(k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
-    XTS_LAUNCH("k_mlp_backward", st, k_mlp_backward<<<nb, FT, BWD_SMEM, st>>>(
-                                         net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, Y, n, sv, dz,
-                                         dz + hn, part, status));
-    XTS_LAUNCH("k_gemm_bf16", st, k_gemm_bf16<<<dim3(1, nsplit, 2), MT, GEMM_SMEM, st>>>(
-                                      dz, 0, sv.h2, 0, MH, (int)n, cps, wpart, 0, 1, status, dz + hn, sv.h1));
-    const int blocks = 2 * MH * MH / 256 + (BQ_N * MH + 7) / 8;
-    XTS_LAUNCH("k_mlp_grad_sum", st, k_mlp_grad_sum<<<blocks, 256, 0, st>>>(part, nb, wpart, nsplit, 1.f / (float)n,
-                                                                            grads, loss));
+    XTS_CUDA(cudaFuncSetAttribute(k_mlp_gradient, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GRAD_SMEM));
+    XTS_LAUNCH("k_mlp_gradient", st, k_mlp_gradient<<<nb, GT, GRAD_SMEM, st>>>(
+                                         net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, Y, n, part,
+                                         wpart, status));
+    XTS_LAUNCH("k_mlp_grad_sum", st, k_mlp_grad_sum<<<GS_WB + (BQ_N * MH + 7) / 8, 256, 0, st>>>(
+                                         part, wpart, nb, 1.f / (float)n, add, grads, loss));
     return XTS_OK;
 }
 
 int launch_mlp_grads(const xts_mlp* net, const float* X, const float* Y, long long n, float* grads, float* loss,
                      int* status, cudaStream_t st) {
-    XTS_CUDA(cudaMemsetAsync(grads, 0, sizeof(float) * XTS_MLP_NPARAM, st));
-    if (loss) XTS_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), st));
-    int rc = mlp_backprop(net, X, Y, n, grads, loss, status, st);
+    int rc = mlp_backprop(net, X, Y, n, 0, grads, loss, status, st);
     if (rc) return rc;
     return mlp_status(status, st);
 }
@@ -1072,7 +1190,7 @@ int launch_mlp_grads(const xts_mlp* net, const float* X, const float* Y, long lo
 int launch_mlp_train_step(const xts_mlp* net, const float* X, const float* Y, long long n, float* grads,
                           float* m, float* v, int step, float lr, float* loss, int* status, cudaStream_t st) {
     if (step < 1) return set_error(XTS_ERR_ARG, "surrogate training: step must be >= 1");
-    int rc = mlp_backprop(net, X, Y, n, grads, loss, status, st);
+    int rc = mlp_backprop(net, X, Y, n, 1, grads, loss, status, st);
     if (rc) return rc;
     const float c1 = (float)(1.0 / (1.0 - pow(0.9, step))), c2 = (float)(1.0 / (1.0 - pow(0.999, step)));
     XTS_LAUNCH("k_mlp_adam", st, k_mlp_adam<<<(XTS_MLP_NPARAM + 255) / 256, 256, 0, st>>>(
