@@ -674,7 +674,10 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int a_trans, const __nv_bfloat1
 // lane adds eight rows of a pair of units (a shuffle butterfly took four instructions per
 // value and sum, this takes one and a half).  Each block writes its sums once;
 // k_mlp_grad_sum adds the blocks' in a fixed order, so trainings repeat bit for bit.
-// 37,888 rows (two tiles per block): @GRAD@
+// 37,888 rows (two tiles per block): 43 us and 9 us for the sums, where a forward, a
+// backward and a weight-product kernel that pass z, h and dz through memory took 37, 48 and
+// 42 us.  A further tile per block takes 12.5 us, about half of it issuing (the GELUs, their
+// derivatives and the sums), the rest the five waits for products that need the whole tile.
 enum { BQ_B3 = 0, BQ_W4 = 1, BQ_B2 = 2, BQ_B1 = 3, BQ_W1 = 4, BQ_LOSS = 9, BQ_B4 = 10, BQ_N = 11 };
 constexpr int GT = 4 * MT;  // threads
 struct GradLayout {
@@ -825,22 +828,31 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
     float sum_d2 = 0.f, sum_dy = 0.f;
     unsigned ph = 0, wph = 0;
     bool ok = true, got = true, wpend = false;  // wpend: a weight product not yet waited for
-    // operands in shared memory and the accumulators' last readers, then the MMAs of issue
-    auto mma_phase = [&](auto issue) {
+    // mma_issue: operands in shared memory and the accumulators' last readers, then the
+    // MMAs of issue; mma_wait: their end.  Work between the two overlaps them.  A wait that
+    // timed out in any thread ends the loop at the next mma_issue.
+    bool pend = false;
+    auto mma_issue = [&](auto issue) {
         fence_async_shared();
         tc_fence_before();
-        __syncthreads();
+        if (!__syncthreads_and(got)) return false;
         if (t == 0) {
             tc_fence_after();
             issue();
         }
-        const bool g = mbar_wait(bar, ph);
-        if (!__syncthreads_and(g && got)) return false;  // ph stays: the exit path waits on it
-        ph ^= 1;
-        tc_fence_after();
+        pend = true;
         return true;
     };
-    // each thread sees the weight product complete; a timeout ends the next mma_phase
+    auto mma_wait = [&]() {
+        if (mbar_wait(bar, ph)) {
+            ph ^= 1;
+            pend = false;
+        }
+        got = got && !pend;
+        __syncwarp();
+        tc_fence_after();
+    };
+    // each thread sees the weight product complete; a timeout ends the loop
     auto weights_done = [&]() {
         if (wpend && mbar_wait(wbar, wph)) {
             wph ^= 1;
@@ -864,6 +876,24 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
             z[4 * q] += b.x; z[4 * q + 1] += b.y; z[4 * q + 2] += b.z; z[4 * q + 3] += b.w;
         }
     };
+    // the same and 16 values of dh, one wait for both
+    auto load_z_dh = [&](unsigned acc, const float* bias, unsigned dacc, int c, float* z, float* dh) {
+        unsigned ra[16], rb[16];
+        tmem_ld16_issue(acc + lane0 + (unsigned)c, ra);
+        tmem_ld16_issue(dacc + lane0 + (unsigned)c, rb);
+        tmem_ld_done(ra);
+        tmem_ld_done(rb);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 b = reinterpret_cast<const float4*>(bias + c)[q];
+            z[4 * q] = __uint_as_float(ra[4 * q]) + b.x;
+            z[4 * q + 1] = __uint_as_float(ra[4 * q + 1]) + b.y;
+            z[4 * q + 2] = __uint_as_float(ra[4 * q + 2]) + b.z;
+            z[4 * q + 3] = __uint_as_float(ra[4 * q + 3]) + b.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) dh[j] = __uint_as_float(rb[j]);
+    };
     auto act16 = [&](float* z) {
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
@@ -873,32 +903,43 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
         }
     };
     const long long ntiles = n / MT;
+    float xn[MI], tn;  // the next tile's features and target of this row
+    auto load_row = [&](long long tile) {
+        const long long row = (tile < ntiles ? tile : (long long)blockIdx.x) * MT + r;
+        if (qd == 0)
+#pragma unroll
+            for (int k = 0; k < MI; ++k) xn[k] = X[row * MI + k];
+        tn = Y[row];
+    };
+    load_row(blockIdx.x);
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long row = tile * MT + r;
         if (qd == 0) {
             float x[MI];
 #pragma unroll
-            for (int k = 0; k < MI; ++k) xs[r * 8 + k] = x[k] = (X[row * MI + k] - nm.mu[k]) / nm.sd[k];
+            for (int k = 0; k < MI; ++k) xs[r * 8 + k] = x[k] = (xn[k] - nm.mu[k]) / nm.sd[k];
             store_x_split_ns(xop, r, x);
         }
-        const float target = (Y[row] - nm.out_mu) / nm.out_sd;
-        if (!(ok = mma_phase([&] { layer1(t_a); mma_commit(bar); }))) break;
+        const float target = (tn - nm.out_mu) / nm.out_sd;
+        if (!(ok = mma_issue([&] { layer1(t_a); mma_commit(bar); }))) break;
+        mma_wait();
         weights_done();  // the previous tile's dW2 has read h1 and dz
-        float v[16], u[16];
+        float v[32], u[32];
 #pragma unroll 1
         for (int c = cb; c < cb + 32; c += 16) {
             load_z(t_a, b1, c, v);
             act16(v);
             store_bf16x16(h1, r, c, v);
         }
-        if (!(ok = mma_phase([&] { mma_chain(t_b, s_h1, s_w2, 8, false); mma_commit(bar); }))) break;
+        if (!(ok = mma_issue([&] { mma_chain(t_b, s_h1, s_w2, 8, false); mma_commit(bar); }))) break;
+        mma_wait();
 #pragma unroll 1
         for (int c = cb; c < cb + 32; c += 16) {
             load_z(t_b, b2, c, v);
             act16(v);
             store_bf16x16(h2, r, c, v);
         }
-        if (!(ok = mma_phase([&] { mma_chain(t_a, s_h2, s_w3, 8, false); mma_commit(bar); }))) break;
+        if (!(ok = mma_issue([&] { mma_chain(t_a, s_h2, s_w3, 8, false); mma_commit(bar); }))) break;
+        mma_wait();
         float yp = 0.f;
 #pragma unroll 1
         for (int c = cb; c < cb + 32; c += 16) {
@@ -915,20 +956,18 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
             sum_d2 = fmaf(d, d, sum_d2);
             sum_dy += dy;
         }
-#pragma unroll 1
-        for (int c = cb; c < cb + 32; c += 16) {
-            load_z(t_a, b3, c, v);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+        for (int g = 0; g < 32; g += 16) {
+            load_z(t_a, b3, cb + g, v + g);
+#pragma unroll
+            for (int j = g; j < g + 16; ++j) {
                 u[j] = dy * gelu(v[j]);
-                v[j] = dy * w4[c + j] * gelu_grad(v[j]);
+                v[j] = dy * w4[cb + j] * gelu_grad(v[j]);
             }
-            store_bf16x16(dz, r, c, v);
-            row_sums<false>(turn, v, nullptr, tot + (BQ_B3 * 4 + rw) * MH + c);
-            row_sums<false>(turn, u, nullptr, tot + (BQ_W4 * 4 + rw) * MH + c);
+            store_bf16x16(dz, r, cb + g, v + g);
         }
         const bool first = tile == blockIdx.x;
-        if (!(ok = mma_phase([&] {
+        if (!(ok = mma_issue([&] {
                   mma_chain_t<false>(t_a, s_dz, s_w3, false);
                   mma_commit(bar);
                   mma_chain_t<true>(t_w3, s_dz, s_h2, !first);
@@ -936,17 +975,22 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
               })))
             break;
         wpend = true;
-#pragma unroll 1
-        for (int c = cb; c < cb + 32; c += 16) {
-            load_z(t_b, b2, c, v);
-            tmem_ld16(t_a + lane0 + (unsigned)c, u);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = u[j] * gelu_grad(v[j]);
-            row_sums<false>(turn, v, nullptr, tot + (BQ_B2 * 4 + rw) * MH + c);
-            weights_done();  // dW3 has read dz
-            store_bf16x16(dz, r, c, v);
+        for (int g = 0; g < 32; g += 16) {
+            row_sums<false>(turn, v + g, nullptr, tot + (BQ_B3 * 4 + rw) * MH + cb + g);
+            row_sums<false>(turn, u + g, nullptr, tot + (BQ_W4 * 4 + rw) * MH + cb + g);
         }
-        if (!(ok = mma_phase([&] {
+        mma_wait();
+#pragma unroll
+        for (int g = 0; g < 32; g += 16) {
+            load_z_dh(t_b, b2, t_a, cb + g, v + g, u);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[g + j] = u[j] * gelu_grad(v[g + j]);
+        }
+        weights_done();  // dW3 has read dz
+        store_bf16x16(dz, r, cb, v);
+        store_bf16x16(dz, r, cb + 16, v + 16);
+        if (!(ok = mma_issue([&] {
                   mma_chain_t<false>(t_b, s_dz, s_w2, false);
                   layer1(t_a);
                   mma_commit(bar);
@@ -955,10 +999,14 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
               })))
             break;
         wpend = true;
+#pragma unroll
+        for (int g = 0; g < 32; g += 16)
+            row_sums<false>(turn, v + g, nullptr, tot + (BQ_B2 * 4 + rw) * MH + cb + g);
+        load_row(tile + gridDim.x);
+        mma_wait();
 #pragma unroll 1
         for (int c = cb; c < cb + 32; c += 16) {
-            load_z(t_a, b1, c, v);
-            tmem_ld16(t_b + lane0 + (unsigned)c, u);
+            load_z_dh(t_a, b1, t_b, c, v, u);
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = u[j] * gelu_grad(v[j]);
             row_sums<true>(turn, v, xs + rw * 32 * 8, tot + (BQ_B1 * 4 + rw) * MH + c);
@@ -972,14 +1020,14 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
     if (ok) {
         tc_fence_after();
         const int l = qd >> 1, hc = 64 * (qd & 1);
-        float* dst = wpart + (((size_t)l * gridDim.x + blockIdx.x) * MH + r) * MH + hc;
+        float4* dst = reinterpret_cast<float4*>(wpart) + ((size_t)l * gridDim.x + blockIdx.x) * (MH * MH / 4) + r;
 #pragma unroll 1
         for (int c = 0; c < 64; c += 16) {
             float w[16];
             tmem_ld16((l ? t_w2 : t_w3) + lane0 + (unsigned)(hc + c), w);
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                reinterpret_cast<float4*>(dst + c)[q] = make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+                dst[((hc + c) / 4 + q) * MH] = make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
         }
         for (int o = 16; o > 0; o >>= 1) {
             sum_d2 += __shfl_xor_sync(0xffffffffu, sum_d2, o);
@@ -988,7 +1036,7 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
         if (qd == 0 && lane == 0) { sred[2 * rw] = sum_d2; sred[2 * rw + 1] = sum_dy; }
     } else if (t == 0) {
         atomicExch(status, 1);
-        mbar_wait(bar, ph);  // bounded: let issued MMAs land
+        if (pend) mbar_wait(bar, ph);  // bounded: let issued MMAs land
         if (wpend) mbar_wait(wbar, wph);
     }
     tc_fence_before();
@@ -1008,7 +1056,7 @@ k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict
 
 // The gradients from their parts, written to (add 0) or added to grads; the loss likewise.
 // Blocks 0 .. 255: 128 elements each of the hidden weights' tiles (wpart
-// [2][nb][MH * MH]: W3, W2), warp w the tiles k = w mod 8, the warps' sums in order;
+// [2][nb][column / 4][row][4]: W3, W2), warp w the tiles k = w mod 8, the warps' sums in order;
 // further blocks: one warp per (quantity, unit) of k_mlp_gradient's nb blocks.
 constexpr int GS_WB = 2 * MH * MH / 128;
 __global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, const float* __restrict__ wpart,
@@ -1032,7 +1080,8 @@ __global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ 
             float s = 0.f;
 #pragma unroll
             for (int k = 0; k < 8; ++k) s += f[128 * k];
-            float* g = grads + (l ? XTS_MLP_W2 : XTS_MLP_W3) + e0 + threadIdx.x;
+            const int e = (e0 + (int)threadIdx.x) >> 2, col = (e / MH) * 4 + (threadIdx.x & 3), row = e & (MH - 1);
+            float* g = grads + (l ? XTS_MLP_W2 : XTS_MLP_W3) + row * MH + col;
             *g = add ? *g + s : s;
         }
         return;
