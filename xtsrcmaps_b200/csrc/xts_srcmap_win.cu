@@ -58,8 +58,16 @@ __device__ __forceinline__ WinSrc win_source(const SrcInfo& si) {
 constexpr size_t WA_OFF_WTS = sizeof(SepTab);  // (the tables first)
 constexpr size_t WA_OFF_BAR = WA_OFF_WTS + sizeof(float) * WT * RW;
 constexpr size_t WA_OFF_SRC = WA_OFF_BAR + 16;
-constexpr size_t WA_OFF_HIST = WA_OFF_SRC + sizeof(WinSrc) * NSG_MAX;
+// Wide pixels put off: map pixel, source of the group | inside << 8, omega's bits, sparse
+// record (-1: none).  The dense pass keeps an item's (what does not fit is found again by its
+// records, wide_left), the cutouts' pass a warp's of a run.
+constexpr int WIDE_CAP = 128;
+constexpr size_t WA_OFF_WIDE = WA_OFF_SRC + sizeof(WinSrc) * NSG_MAX;
+constexpr size_t WA_OFF_HIST = WA_OFF_WIDE + sizeof(int4) * WIDE_CAP;
+static_assert(WA_OFF_WIDE % 16 == 0 && WA_OFF_HIST % 16 == 0, "alignment");
 constexpr size_t wa_smem(int nsg) { return WA_OFF_HIST + sizeof(double) * ND * (size_t)nsg; }
+constexpr size_t WA_OFF_WARP = (wa_smem(1) + 15) / 16 * 16;  // the cutouts' pass: [WT] wide pixels, 32 per warp
+constexpr size_t WA_CUT_SMEM = WA_OFF_WARP + sizeof(int4) * WT;
 
 constexpr int NSP = 24;  // entries of a sparse record: 12 points x 2 rows
 constexpr int META_OVERFLOW = -0x7fffffff - 1;  // wide pixel without a sparse record
@@ -82,6 +90,7 @@ struct PassA {
     float2* sparse;
     int sparse_cap;
     int* sparse_count;
+    int4* wide;            // shared: wide pixels [WIDE_CAP]
 };
 
 // Shared tables of pass A: one bulk copy per block, in flight while the caller clears the
@@ -98,6 +107,7 @@ __device__ __forceinline__ PassA pass_a_tables(unsigned char* smem, const SepTab
     A.hist = (double*)(smem + WA_OFF_HIST);
     A.wts = (float*)(smem + WA_OFF_WTS);
     A.rec = rec; A.ext = ext; A.sparse = sparse; A.sparse_cap = sparse_cap; A.sparse_count = sparse_count;
+    A.wide = (int4*)(smem + WA_OFF_WIDE);
     if (threadIdx.x == 0) {
         const unsigned bar = smem_u32(smem + WA_OFF_BAR);
         mbar_init(bar, 1);
@@ -188,15 +198,96 @@ __device__ __forceinline__ int row_lower(double q, const SepBin* bins) {
     return sb.k0 + (q >= sb.thr);
 }
 
+// Point p of a wide pixel (next to the source) with FP64 chords from the corners, for its
+// sparse record and its map-integral rows alike.
+__device__ __forceinline__ void wide_point(const int4& e, int p, const SepBin* sbin, const float4* scoef,
+                                           float2* sparse, const double* __restrict__ corners, int W1, double dx,
+                                           double dy, double dz, double* hist, int* rlo, int* rhi) {
+    const int h = e.x / (W1 - 1);
+    SrcInfo sd;
+    sd.dir[0] = dx; sd.dir[1] = dy; sd.dir[2] = dz;
+    const PixQ g = pixel_q(pixel_geom(corners, W1, h, e.x - h * (W1 - 1), sd));
+    float tt;
+    const int idx = point_row_bin(point_q2(g, p), sbin, scoef, &tt);
+    const float wo = c_rule_w32[p] * __int_as_float(e.z);
+    const float wa = (1.f - tt) * wo, wb = tt * wo;
+    if (e.w >= 0) {
+        float2* sr = sparse + (size_t)e.w * NSP;
+        sr[2 * p] = make_float2(wa, __int_as_float(idx - 1));
+        sr[2 * p + 1] = make_float2(wb, __int_as_float(idx));
+    }
+    if (e.y >> 8) {
+        atomicAdd(&hist[idx - 1], (double)wa);
+        atomicAdd(&hist[idx], (double)wb);
+        if (rlo) {
+            atomicMin(rlo, idx - 1);
+            atomicMax(rhi, idx);
+        }
+    }
+}
+// Wide pixels a thread per (point, pixel), neighbouring lanes on different pixels (their
+// rows differ, so the histogram's atomics rarely meet).  The pixel's own lane did its
+// twelve points one after another before, a run next to a source having a few such lanes.
+// The dense pass takes an item's together at its end (50 sources x 200 x 200: 105 -> 82 us,
+// 500 x 400 x 400: 1.24 -> 1.22 ms; a warp's at once, source by source: 93 us and 1.35 ms);
+// the cutouts' pass, whose items are small and all next to a source, a warp's at once
+// (1.00 -> 0.93 ms; at the item's end 1.02).
+__device__ __forceinline__ void wide_of_warp(bool wide, const int4& e, const PassA& A,
+                                             const double* __restrict__ corners, int W1, const WinSrc& si,
+                                             int4* list, int* rlo, int* rhi) {
+    const unsigned mask = __ballot_sync(0xffffffffu, wide);
+    if (!mask) return;
+    const int lane = threadIdx.x & 31, n = __popc(mask);
+    if (wide) list[__popc(mask & ((1u << lane) - 1))] = e;
+    __syncwarp();
+    for (int k = lane; k < 12 * n; k += 32) {
+        const int p = k / n;
+        wide_point(list[k - p * n], p, A.sbin, A.scoef, A.sparse, corners, W1, si.dir[0], si.dir[1], si.dir[2], A.hist, rlo,
+                   rhi);
+    }
+    __syncwarp();
+}
+__device__ __forceinline__ void wide_of_item(int n, const PassA& A, const double* __restrict__ corners, int W1,
+                                             const WinSrc* src) {
+    for (int k = threadIdx.x; k < 12 * n; k += WT) {
+        const int p = k / n;
+        const int4 e = A.wide[k - p * n];
+        const int j = e.y & 0xff;
+        wide_point(e, p, A.sbin, A.scoef, A.sparse, corners, W1, src[j].dir[0], src[j].dir[1], src[j].dir[2],
+                   A.hist + j * ND, nullptr, nullptr);
+    }
+}
+
+// The item's wide pixels that found the list full: marked by z = 1 in their records (omega
+// and the inside test in x and y).  Kept out of the pass's common path and its registers:
+// called there the pass takes 1.28 ms (500 x 400 x 400), inlined there 1.35, inlined here 1.27.
+__device__ __noinline__ void wide_left(const PassA A, const double* __restrict__ corners, int W1,
+                                          const WinSrc* src, int ns, int s0, int npix, int pa, int pb) {
+    for (int j = 0; j < ns; ++j)
+        for (int pix = pa + threadIdx.x; pix < pb; pix += WT) {
+            float4* rec = A.rec + (size_t)(s0 + j) * npix + pix;
+            const float4 r = *rec;
+            const int meta = __float_as_int(r.w);
+            if (meta >= 0 || r.z == 0.f) continue;
+            const int4 e = make_int4(pix, r.y != 0.f ? 256 : 0, __float_as_int(r.x), meta == META_OVERFLOW ? -1 : -1 - meta);
+            for (int p = 0; p < 12; ++p)
+                wide_point(e, p, A.sbin, A.scoef, A.sparse, corners, W1, src[j].dir[0], src[j].dir[1], src[j].dir[2],
+                           A.hist + j * ND, nullptr, nullptr);
+            *rec = make_float4(0.f, 0.f, 0.f, r.w);
+        }
+}
+
 // One (source, pixel): the pixel's window for source si, record index kk.  Pixels
 // whose centre lies within the boundary radius (squared chord ch2) add their window
 // rows to hist (the source's map-integral rows); the rows they touch widen
 // [*rlo, *rhi] when those are given.  (h, w) and W1 locate the pixel's corners for
-// the rare wide pixel, which is redone in FP64 point by point.
-__device__ __forceinline__ void window_source(const PixBase& P, const WinSrc& si,
+// the rare wide pixel: on the item's list (CUT: returned with true).
+template <bool CUT>
+__device__ __forceinline__ bool window_source(const PixBase& P, const WinSrc& si,
                                               const double* __restrict__ corners, const double* __restrict__ centers,
                                               int W1, int h, int w,
-                                              size_t kk, const PassA& A, double* hist, int* rlo, int* rhi) {
+                                              size_t kk, const PassA& A, double* hist, int* rlo, int* rhi, int j,
+                                              int* nwide, int4* entry) {
     const int t = threadIdx.x;
     const double Ax = P.m[0] - si.dir[0], Ay = P.m[1] - si.dir[1], Az = P.m[2] - si.dir[2];
     const double a0 = fma(Ax, Ax, fma(Ay, Ay, Az * Az));  // q at the centre of the blend
@@ -288,7 +379,7 @@ __device__ __forceinline__ void window_source(const PixBase& P, const WinSrc& si
                 }
             }
             A.rec[kk] = make_float4(s0, s1, s2, __int_as_float(kl | (nent << 16)));
-            return;
+            return false;
         }
     }
     float dqs[12];  // the rule's points in order: pair k at k, its mirror image at k + 6
@@ -364,35 +455,21 @@ __device__ __forceinline__ void window_source(const PixBase& P, const WinSrc& si
             A.ext[2 * kk + 1] = make_float4(f[4], f[5], f[6], f[7]);
         }
     } else {
-        // a wide pixel (next to the source): its 12 points again with FP64 chords
-        // from the corners, for its sparse record and its map-integral rows alike
-        SrcInfo sd;
-        sd.dir[0] = si.dir[0]; sd.dir[1] = si.dir[1]; sd.dir[2] = si.dir[2];
-        const PixQ g = pixel_q(pixel_geom(corners, W1, h, w, sd));
-        int meta = META_OVERFLOW;
-        const int slot = atomicAdd(A.sparse_count, 1);
-        float2* sr = slot < A.sparse_cap ? A.sparse + (size_t)slot * NSP : nullptr;
-        for (int p = 0; p < 12; ++p) {
-            float tt;
-            const int idx = point_row_bin(point_q2(g, p), A.sbin, A.scoef, &tt);
-            const float wo = c_rule_w32[p] * om;
-            const float wa = (1.f - tt) * wo, wb = tt * wo;
-            if (sr) {
-                sr[2 * p] = make_float2(wa, __int_as_float(idx - 1));
-                sr[2 * p + 1] = make_float2(wb, __int_as_float(idx));
-            }
-            if (inside) {
-                atomicAdd(&hist[idx - 1], (double)wa);
-                atomicAdd(&hist[idx], (double)wb);
-                if (rlo) {
-                    atomicMin(rlo, idx - 1);
-                    atomicMax(rhi, idx);
-                }
-            }
+        int slot = atomicAdd(A.sparse_count, 1);
+        if (slot >= A.sparse_cap) slot = -1;
+        const float meta = __int_as_float(slot >= 0 ? -1 - slot : META_OVERFLOW);
+        const int4 e = make_int4(h * (W1 - 1) + w, j | (inside ? 256 : 0), __float_as_int(om), slot);
+        if (CUT) {
+            A.rec[kk] = make_float4(0.f, 0.f, 0.f, meta);
+            *entry = e;
+            return true;
         }
-        if (sr) meta = -1 - slot;
-        A.rec[kk] = make_float4(0.f, 0.f, 0.f, __int_as_float(meta));
+        const int at = atomicAdd(nwide, 1);
+        const float full = at >= WIDE_CAP ? 1.f : 0.f;
+        if (at < WIDE_CAP) A.wide[at] = e;
+        A.rec[kk] = make_float4(full * om, inside ? full : 0.f, full, meta);
     }
+    return false;
 }
 
 // This lane's pixel of the warp's next run of 32 from pixel p0 on.
@@ -418,11 +495,11 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restric
                                                       int sparse_cap, int* __restrict__ sparse_count,
                                                       int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int next_s, nwide_s;
     const PassA A = pass_a_tables(smem, septab, rec, ext, sparse, sparse_cap, sparse_count);
-    __shared__ int next_s;
     WinSrc* ssrc = (WinSrc*)(smem + WA_OFF_SRC);
     const int t = threadIdx.x;
-    if (t == 0) next_s = 0;
+    if (t == 0) next_s = nwide_s = 0;
     const int npix = H * W, W1 = W + 1;
     const int nt = (npix + WT - 1) / WT;
     const int item = blockIdx.x;
@@ -439,10 +516,13 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restric
         const int h = pix / W, w = pix - h * W;
         const PixBase Q = pixel_base(corners, centers, omega, W1, h, w, (size_t)pix);
         for (int j = 0; j < ns; ++j) {
-            window_source(Q, ssrc[j], corners, centers, W1, h, w, (size_t)(s0 + j) * npix + pix, A, A.hist + j * ND,
-                          nullptr, nullptr);
+            window_source<false>(Q, ssrc[j], corners, centers, W1, h, w, (size_t)(s0 + j) * npix + pix, A,
+                                 A.hist + j * ND, nullptr, nullptr, j, &nwide_s, nullptr);
         }
     }
+    __syncthreads();
+    wide_of_item(min(nwide_s, WIDE_CAP), A, corners, W1, ssrc);
+    if (nwide_s > WIDE_CAP) wide_left(A, corners, W1, ssrc, ns, s0, npix, pa, pb);
     __syncthreads();
     for (int r = t; r < ns * ND; r += WT) {
         const double v = A.hist[r];
@@ -495,11 +575,16 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
         const xts_cutout cw = cut[s];
         const int npix = cw.nh * cw.nw, p0 = (int)((item - tile_off[s]) * run), p1 = min(npix, p0 + run);  // (<= 2^30)
         for (int pix = next_run(&next_s, p0); pix - (t & 31) < p1; pix = next_run(&next_s, p0)) {
-            if (pix >= p1) continue;
-            const int i = pix / cw.nw, j = pix - i * cw.nw;
-            const int h = cw.h0 + i, w = cw.w0 + j;
-            const PixBase P = pixel_base(corners, centers, omega, W1, h, w, (size_t)h * W + w);
-            window_source(P, ssrc[0], corners, centers, W1, h, w, (size_t)(cw.offset + pix), A, A.hist, &rmin_s, &rmax_s);
+            int4 e;
+            bool wide = false;
+            if (pix < p1) {
+                const int i = pix / cw.nw, j = pix - i * cw.nw;
+                const int h = cw.h0 + i, w = cw.w0 + j;
+                const PixBase P = pixel_base(corners, centers, omega, W1, h, w, (size_t)h * W + w);
+                wide = window_source<true>(P, ssrc[0], corners, centers, W1, h, w, (size_t)(cw.offset + pix), A, A.hist,
+                                           &rmin_s, &rmax_s, 0, nullptr, &e);
+            }
+            wide_of_warp(wide, e, A, corners, W1, ssrc[0], (int4*)(smem + WA_OFF_WARP) + (t & ~31), &rmin_s, &rmax_s);
         }
         __syncthreads();
         for (int r = rmin_s + t; r <= rmax_s; r += WT) {
@@ -1175,11 +1260,11 @@ int launch_srcmap_win_cut(const double* corners, const double* centers, const do
     XTS_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
     XTS_LAUNCH("k_cut_tiles", st, k_cut_tiles<<<2, 1024, 0, st>>>(cut, S, 32 * nw, run, tile_off, pair_off));
     XTS_LAUNCH("k_cut_item_src", st, k_cut_item_src<<<S, 256, 0, st>>>(tile_off, item_src));
-    if ((rc = resident_blocks(k_pixel_windows_cut, WT, wa_smem(1), dev, &resident))) return rc;
+    if ((rc = resident_blocks(k_pixel_windows_cut, WT, WA_CUT_SMEM, dev, &resident))) return rc;
     resident = resident < 1 ? 1 : resident;
     if (g_tuning.queue_blocks_per_sm > 0 && g_tuning.queue_blocks_per_sm < resident) resident = g_tuning.queue_blocks_per_sm;
     // pass A: one persistent wave pulling (source, tile) items from the queue
-    XTS_LAUNCH("k_pixel_windows", st, k_pixel_windows_cut<<<(unsigned)(resident * nsm), WT, wa_smem(1), st>>>(
+    XTS_LAUNCH("k_pixel_windows", st, k_pixel_windows_cut<<<(unsigned)(resident * nsm), WT, WA_CUT_SMEM, st>>>(
                                           corners, centers, omega, info, cut, item_src, tile_off, queue, tab, S, W, run,
                                           hist, rec, ext, sparse, (int)cap, sparse_count, status));
     rc = launch_correction(hist, 1, info, S, upsf, partial, exposure, E, scale, inv_integ, correction, radius, in_fov,
