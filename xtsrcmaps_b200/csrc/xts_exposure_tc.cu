@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(X_THREADS, 1)
 k_exposure_map_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_bhi, const __grid_constant__ CUtensorMap tm_blo,
                   int npix, int C, int E, int groups, double* __restrict__ out, int* __restrict__ status) {
+    after_previous();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     unsigned long long* bars = (unsigned long long*)(smem + X_BARS);
@@ -252,6 +253,8 @@ k_exposure_map_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 // and the padding columns of each half, are zero.
 __global__ void k_exposure_b(const double* af, const double* ab, const double* ltf, int C, int E, int N,
                              float* bhi, float* blo) {
+    after_previous();
+    let_next_start();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N * 2 * XKP) return;
     const int e = k / (2 * XKP), kk = k - e * (2 * XKP);
@@ -312,8 +315,8 @@ int launch_exposure_map_tc(const float* cube, const float* wcube, long long npix
     float* bhi = b;
     float* blo = b + (size_t)N * 2 * XKP;
     const int nb = N * 2 * XKP;
-    XTS_LAUNCH("k_exposure_b", st, k_exposure_b<<<(nb + 255) / 256, 256, 0, st>>>(front_aeff, back_aeff, ltf, C, E, N,
-                                                                                  bhi, blo));
+    XTS_LAUNCH("k_exposure_b", st, launch_next(k_exposure_b, (nb + 255) / 256, 256, 0, st, front_aeff, back_aeff, ltf,
+                                               C, E, N, bhi, blo));
     CUtensorMap mx, mw, mbh, mbl;
     int rc;
     if ((rc = x_map(&mx, cube, npix, C, XM))) return rc;
@@ -328,8 +331,8 @@ int launch_exposure_map_tc(const float* cube, const float* wcube, long long npix
     const int groups = (E + XN - 1) / XN;  // at most 4, fewer than SMs
     const long long items = (npix + XM - 1) / XM * groups;
     const int G = (int)(items < nsm ? items : nsm);
-    XTS_LAUNCH("k_exposure_map_tc", st, k_exposure_map_tc<<<G, X_THREADS, smem, st>>>(mx, mw, mbh, mbl, (int)npix, C, E,
-                                                                                       groups, out, status));
+    XTS_LAUNCH("k_exposure_map_tc", st, launch_next(k_exposure_map_tc, G, X_THREADS, smem, st, mx, mw, mbh, mbl, (int)npix,
+                                                    C, E, groups, out, status));
     return XTS_OK;
 }
 

@@ -57,6 +57,32 @@ void prof_mark(const char* name, cudaStream_t st, bool begin);
         XTS_CHECK_LAUNCH(name);                                \
     } while (0)
 
+// Launch of a kernel whose blocks may be set up while the previous kernel of the stream
+// still runs (programmatic dependent launch): they wait in after_previous() for its end.
+// A previous kernel that calls let_next_start() allows it from the start of its last
+// blocks on, else from their exits.  Any other work between the two (a copy, an event) makes
+// it an ordinary launch.  A link of a chain of short kernels costs 1 to 2 us less: a call with 7
+// sources 72.2 -> 68.5 us, 50 sources x 200 x 200 214 -> 207, in doubles 323 -> 311, an all-sky
+// exposure map 185 -> 181.
+#ifdef __CUDACC__
+template <typename... P, typename... A>
+inline void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // a failure stays for the check after the launch
+}
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // Grow-only device workspace, one buffer per slot ------------------------------
 enum Slot {
     // staged inputs / outputs (host-pointer mode)

@@ -774,6 +774,7 @@ __global__ void __launch_bounds__(GT, 1)
 k_mlp_gradient(const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf, MlpNorm nm,
                const float* __restrict__ X, const float* __restrict__ Y, long long n, float* __restrict__ part,
                float* __restrict__ wpart, int* __restrict__ status) {
+    let_next_start();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, r = t & (MT - 1), qd = t >> 7, cb = 32 * qd, rw = warp & 3;
@@ -1062,6 +1063,7 @@ constexpr int GS_WB = 2 * MH * MH / 128;
 __global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, const float* __restrict__ wpart,
                                                       int nb, float inv_n, int add, float* __restrict__ grads,
                                                       float* __restrict__ loss) {
+    after_previous();
     __shared__ float4 red[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if ((int)blockIdx.x < GS_WB) {
@@ -1224,8 +1226,9 @@ static int mlp_backprop(const xts_mlp* net, const float* X, const float* Y, long
     XTS_LAUNCH("k_mlp_gradient", st, k_mlp_gradient<<<nb, GT, GRAD_SMEM, st>>>(
                                          net->params, (const __nv_bfloat16*)net->wbf16, mlp_norm(net), X, Y, n, part,
                                          wpart, status));
-    XTS_LAUNCH("k_mlp_grad_sum", st, k_mlp_grad_sum<<<GS_WB + (BQ_N * MH + 7) / 8, 256, 0, st>>>(
-                                         part, wpart, nb, 1.f / (float)n, add, grads, loss));
+    XTS_LAUNCH("k_mlp_grad_sum", st, launch_next(
+                                         k_mlp_grad_sum, GS_WB + (BQ_N * MH + 7) / 8, 256, 0, st, part, wpart, nb,
+                                         1.f / (float)n, add, grads, loss));
     return XTS_OK;
 }
 

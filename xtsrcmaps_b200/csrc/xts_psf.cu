@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(PM_THREADS, 2) k_psf_mean(const double* __rest
                                                            const double* __restrict__ ltf,
                                                            const double* __restrict__ expo, double* __restrict__ upsf,
                                                            double* __restrict__ partial) {
+    after_previous();
     extern __shared__ __align__(16) double psh[];
     constexpr int NW = PM_THREADS / 32;
     static_assert(NW % TE == 0 && (TS == 8 || TS == 4), "warps per energy, fragment rows");
@@ -241,8 +242,9 @@ static int launch_psf_mean(const PsfDev& a, const double* pa, const double* tab,
     if (smem > 48 * 1024)
         XTS_CUDA(cudaFuncSetAttribute(k_psf_mean<TS, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 g((a.E + TE - 1) / TE, (a.S + TS - 1) / TS);
-    XTS_LAUNCH("k_psf_mean", st, k_psf_mean<TS, TE><<<g, PM_THREADS, smem, st>>>(
-                                     pa, tab, a.C, a.E, a.ecb, a.wecb, a.S, a.ltf, a.exposure, a.upsf, a.partial));
+    XTS_LAUNCH("k_psf_mean", st, launch_next(
+                                     k_psf_mean<TS, TE>, g, PM_THREADS, smem, st, pa, tab, a.C, a.E, a.ecb, a.wecb, a.S,
+                                     a.ltf, a.exposure, a.upsf, a.partial));
     return XTS_OK;
 }
 

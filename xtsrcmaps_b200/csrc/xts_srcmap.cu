@@ -55,6 +55,7 @@ constexpr int GEO_THREADS = (GT + 1) * (GT + 1) + GT * GT;  // 145 tasks, one pe
 
 __global__ void __launch_bounds__(GEO_THREADS) k_map_geometry(WcsDev w, int H, int W, double* corners,
                                                              double* centers, double* omega) {
+    let_next_start();
     __shared__ double cen[(GT + 1) * (GT + 1)][3];
     const int i0 = blockIdx.y * GT, j0 = blockIdx.x * GT, W1 = W + 1, t = threadIdx.x;
     double v[3];
@@ -119,6 +120,7 @@ __device__ __forceinline__ double block_reduce(double x, double* red, Op op) {
 __global__ void __launch_bounds__(256) k_boundary_chord(WcsDev w, const double* src_sph, int Hf, int Wf,
                                                         const double* corners, SrcInfo* info,
                                                         const xts_cutout* cut) {
+    after_previous();
     __shared__ double red[32];
     const int s = blockIdx.x, W1 = Wf + 1;
     int h0 = 0, w0 = 0, H = Hf, W = Wf;
@@ -209,6 +211,7 @@ __global__ void __launch_bounds__(256) k_correction_hist(const double* hist_in, 
                                                          const double* expo, int E, double* scale,
                                                          double* inv_out, double* fac_out,
                                                          double* rad_out, int* fov_out, float* lut, int Epad) {
+    let_next_start();
     __shared__ double hsum[ND];
     __shared__ double ssc[8];
     int s = blockIdx.x;
@@ -385,7 +388,7 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
     const dim3 gg((unsigned)((W + GT) / GT), (unsigned)((H + GT) / GT));  // tiles over the (H+1) x (W+1) grid
     XTS_LAUNCH("k_map_geometry", gs, k_map_geometry<<<gg, GEO_THREADS, 0, gs>>>(w, H, W, corners, centers, omega));
     if (S == 0) return XTS_OK;
-    XTS_LAUNCH("k_boundary", gs, k_boundary_chord<<<S, 256, 0, gs>>>(w, a.src_sph, H, W, corners, info, a.cut));
+    XTS_LAUNCH("k_boundary", gs, launch_next(k_boundary_chord, S, 256, 0, gs, w, a.src_sph, H, W, corners, info, a.cut));
     if (a.cut) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_win_supported(E))

@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(256) k_write_rows64(const double* __restrict__
                                                       const double* __restrict__ upsf,
                                                       const double* __restrict__ scale, int H, int W, int E,
                                                       unsigned magic, double* __restrict__ out) {
+    after_previous();
     __shared__ Rec64 sr[B64];
     __shared__ double2 wide[8][12];  // per warp the points of a wide pixel: t, row
     const int s = blockIdx.y, npix = H * W, pix0 = blockIdx.x * B64, np = min(B64, npix - pix0);
@@ -355,7 +356,7 @@ int launch_srcmap_f64(const double* corners, const double* centers, const double
                                inv_integ ? inv_integ + oE : nullptr, correction ? correction + oE : nullptr,
                                radius ? radius + s0 : nullptr, in_fov ? in_fov + s0 : nullptr, st);
         if (rc) return rc;
-        XTS_LAUNCH("k_srcmap_f64", st, k_write_rows64<<<dim3((npix + B64 - 1) / B64, n), 256, 0, st>>>(
+        XTS_LAUNCH("k_srcmap_f64", st, launch_next(k_write_rows64, dim3((npix + B64 - 1) / B64, n), 256, 0, st,
                                            corners, omega, info + s0, tab, t64, rec, ext, upsf + oE * ND, scale + oE, H, W,
                                            E, magic, out + (size_t)s0 * npix * E));
     }

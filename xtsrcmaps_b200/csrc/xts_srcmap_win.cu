@@ -822,6 +822,7 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
              const SrcInfo* __restrict__ info, const SepTab* __restrict__ septab, const xts_cutout* __restrict__ cut,
              const long long* __restrict__ tile_off,
              int S, int s_base, int H, int W, int E, int EQ, int* status, float* __restrict__ out) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nthr = blockDim.x;
     const WinLayout L = win_layout(E, EQ, nthr >> 5);
@@ -1015,13 +1016,13 @@ static int launch_write_pass(unsigned G, int warps, size_t smem, cudaStream_t st
         return XTS_OK;
     }
     if (a.cut)
-        XTS_LAUNCH("k_srcmap", st, k_srcmap_win<NQ, true><<<G, BT, smem, st>>>(
-                                       a.win, a.ext, a.sparse, a.lut, a.corners, a.omega, a.info, a.tab, a.cut,
-                                       a.tile_off, a.S, a.s_base, a.H, a.W, a.E, a.EQ, a.status, a.out));
+        XTS_LAUNCH("k_srcmap", st, launch_next(
+                                       k_srcmap_win<NQ, true>, G, BT, smem, st, a.win, a.ext, a.sparse, a.lut,
+                                       a.corners, a.omega, a.info, a.tab, a.cut, a.tile_off, a.S, a.s_base, a.H, a.W, a.E, a.EQ, a.status, a.out));
     else
-        XTS_LAUNCH("k_srcmap", st, k_srcmap_win<NQ, false><<<G, BT, smem, st>>>(
-                                       a.win, a.ext, a.sparse, a.lut, a.corners, a.omega, a.info, a.tab, nullptr,
-                                       nullptr, a.S, a.s_base, a.H, a.W, a.E, a.EQ, a.status, a.out));
+        XTS_LAUNCH("k_srcmap", st, launch_next(
+                                       k_srcmap_win<NQ, false>, G, BT, smem, st, a.win, a.ext, a.sparse, a.lut,
+                                       a.corners, a.omega, a.info, a.tab, nullptr, nullptr, a.S, a.s_base, a.H, a.W, a.E, a.EQ, a.status, a.out));
     return XTS_OK;
 }
 

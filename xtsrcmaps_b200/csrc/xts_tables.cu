@@ -20,6 +20,7 @@ struct TablesArgs {
 
 __global__ void __launch_bounds__(TB) k_tables(const __grid_constant__ TablesArgs A) {
     const int b = blockIdx.x, t = threadIdx.x;
+    let_next_start();
     if (b < A.end[0])
         exposure_table(b * TB + t, A.e.C, A.e.cosmin, A.e.thetabin, A.e.logEs, A.e.E, A.e.af, A.e.ab, A.e.exp_costhetas,
                        A.e.front_aeff, A.e.back_aeff);
@@ -42,6 +43,8 @@ struct ContractArgs {
 
 __global__ void __launch_bounds__(TB) k_exposure_psf(const __grid_constant__ ContractArgs A) {
     const int b = blockIdx.x;
+    after_previous();
+    let_next_start();
     if (b < A.nb) exposure_value(b * TB + threadIdx.x, A.ecb, A.wecb, A.S, A.C, A.af, A.ab, A.ltf, A.E, A.exposure);
     else
         psf_aeff_block((b - A.nb) % A.E, (b - A.nb) / A.E, A.pf, A.pb, A.kf, A.kb, A.costh, A.C, A.logEs, A.E, A.af, A.ab,
@@ -93,7 +96,7 @@ int launch_exposure_contract(const double* ecb, const double* wecb, int S, int C
     if ((long long)S * E == 0) return XTS_OK;
     ContractArgs A = {};
     exposure_args(A, ecb, wecb, S, C, af, ab, ltf, E, out);
-    XTS_LAUNCH("k_exposure_f64", st, k_exposure_psf<<<A.nb, TB, 0, st>>>(A));
+    XTS_LAUNCH("k_exposure_f64", st, launch_next(k_exposure_psf, A.nb, TB, 0, st, A));
     return XTS_OK;
 }
 
@@ -110,7 +113,7 @@ int launch_psf_tables(const ExposureDev* e, const PsfDev& p, double* king, doubl
     ContractArgs A = {};
     psf_args(A, p, king, pa);
     if (e) exposure_args(A, e->ecb, e->wecb, e->S, e->C, e->front_aeff, e->back_aeff, e->ltf, e->E, e->exposure);
-    XTS_LAUNCH("k_exposure_psf", st, k_exposure_psf<<<A.nb + p.E * p.C, TB, 0, st>>>(A));
+    XTS_LAUNCH("k_exposure_psf", st, launch_next(k_exposure_psf, A.nb + p.E * p.C, TB, 0, st, A));
     return XTS_OK;
 }
 
