@@ -11,6 +11,10 @@ GOLDEN = os.path.join(ROOT, "tests", "golden")
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200, sm_100a)")
+    # a reference folder without its sources counts as an absent one
+    ref = os.environ.get("XTS_REFERENCE", "/root/reference")
+    if not os.path.exists(os.path.join(ref, "xtsrcmaps", "main.cxx")):
+        os.environ["XTS_REFERENCE"] = os.path.join(ref, "absent")
 
 
 @pytest.fixture(scope="session")
