@@ -12,7 +12,8 @@
 // every (source, pixel)'s whole-pixel region and writes accepted pixels' means;
 // an unaccepted region pushes its two halves onto a device-side queue; after a
 // grid-wide barrier (bounded waits) the next level takes the previous level's
-// queue, one region per thread, and accepted regions add area * R7 into their
+// queue.  A warp takes 32 regions, forms their windows a region per lane and their
+// energies eight lanes (or all) to a region; accepted regions add area * R7 into their
 // pixel's FP64 mean with FP64 atomics (order-free to within a few FP64 ulps).
 // The queue has a fixed capacity; a region whose halves do not fit is accepted
 // as it is.
@@ -23,7 +24,8 @@
 // other (4e-6 of the summed values), or the points leave the row window, the region is
 // evaluated again point by point in FP64 from the FP64 mean PSF, with the
 // reference design's arithmetic (math/genz_malik.hxx:127-195) and no fused
-// multiply-adds, and that evaluation decides (and gives the value).
+// multiply-adds, and that evaluation decides (and gives the value).  These regions are
+// queued per level and taken one per warp.
 //
 // A region's 17 points give LUT rows and interpolation weights exactly as the
 // 12-point rule's do (xts_point.cuh: FP64 chord of the corner-vector blend,

@@ -8,24 +8,25 @@
 // dot product with uPsf is the map integral of c7 (model_map.map_integral.cxx:4-48):
 //     sum_pix omega * value(pix, e) = sum_r Hist[r] * uPsf[r][e].
 // The rule points' squared chords are FP32 offsets from the pixel centre's FP64
-// squared chord (the biquadratic form of xts_point.cuh), compared with the
-// window's row edges, also as FP32 offsets from the centre: one FP64 table
-// search per pixel, none per point.  The histogram takes each window row of a
+// squared chord (the biquadratic form of xts_point.cuh), six mirror pairs as packed
+// FP32 operations: one FP64 table search per pixel, none per point.  A work item is a
+// group of up to eight sources and a part of the map; a pixel's own geometry is formed
+// once for the group.  The histogram takes each window row of a
 // pixel inside the radius by one FP64 shared-memory atomic add.  Every pixel's
 // window is written once as a 16-byte record (3 FP32 weights and the first row /
 // row count), with the 8 weights of a window longer than 3 rows in a 32-byte
 // extension.  Pixels whose points leave the 8-row window (those next to the
-// source) are "wide": they get a sparse record of their 24 (row, weight) pairs
-// from a shared pool instead, or, if the pool is full, are evaluated point by
-// point in pass B.
+// source) are "wide": their points are redone in FP64, a thread per point, into a
+// sparse record of their 24 (row, weight) pairs from a shared pool, or, if the pool
+// is full, again point by point in pass B.
 //
 // Pass B, k_srcmap_win (the write pass, d1 + d2 + c8 + c10): the source's scaled
 // table Y' = uPsf * exposure * correction (FP32, [401][EQ] float4, EQ odd so
 // different rows fall in different shared-memory bank groups) is brought into
-// shared memory by one TMA bulk copy; each thread reads its pixel's window
-// record and forms value[e] = sum_j W[j] * Y'[row_j][e] for all energies in
-// registers (rows rbase + j, or the 24 rows of a sparse record).  Values are
-// staged and written by one TMA bulk store per tile, so the pass streams the
+// shared memory by one TMA bulk copy; each thread reads the window records of two
+// pixels of neighbouring rows and forms value[e] = sum_j W[j] * Y'[row_j][e] of both from
+// one load of each table row (rows rbase + j, or the 24 rows of a sparse record).  Values
+// are staged and written by TMA bulk stores, so the pass streams the
 // window records in and the map out; the next tile's records are loaded while
 // the current one is computed.
 #include <vector>
@@ -483,7 +484,7 @@ __device__ __forceinline__ int next_run(int* counter, int p0) {
 // sources; tiles [p nt / P, (p + 1) nt / P) of WT pixels), forms each pixel's
 // source-independent geometry once and the windows of the group's sources from it,
 // and adds the item's non-zero rows to hist_out[s] (cleared before the launch) with
-// FP64 atomics.  Items are small (about 16 per resident block), so blocks retire
+// FP64 atomics.  Items are small (about 8 per resident block), so blocks retire
 // steadily: the hardware balances them, and kernels of a higher-priority stream
 // (exposure and PSF beside this pass) get their slots as they free up.
 __global__ void __launch_bounds__(WT, 3) k_pixel_windows(const double* __restrict__ corners, const double* __restrict__ centers,
@@ -1107,7 +1108,7 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     float4* ext0 = (float4*)workspace(W_WMETA, sizeof(float4) * 2 * ext_n);
     float* lut0 = (float*)workspace(W_LUT, sizeof(float) * 2 * lut_n);
     float2* sparse0 = (float2*)workspace(W_SPARSE, sizeof(float2) * 2 * sp_n);
-    // pass A: one block per work item, items sized for about 16 per block of the
+    // pass A: one block per work item, items sized for about 8 per block of the
     // resident set (at most window_blocks_per_sm blocks per SM)
     int resident = 0;
     if ((rc = resident_blocks(k_pixel_windows, WT, wa_smem(NSG_MAX), dev, &resident))) return rc;
