@@ -31,3 +31,26 @@ def test_maps_f64(H, W, E, pix, sep):
     m, info = A.point_src_model_map_wcs(wcs, src, ex, u, part, out_dtype="float64")
     assert max_rel(m, ref["map"]) < 1e-10
     assert max_rel(info.inv_map_integral, ref["inv_integ"]) < 1e-10
+
+
+_FIRST_CALL = """
+import sys
+sys.path[:0] = [%r, %r]
+import numpy as np
+from test_write_pass_gpu import _tables
+A, wcs, src, ex, u, p = _tables(6, 3, 61, 83, 0.2)
+m, _ = A.point_src_model_map_wcs(wcs, src, ex, u, p, out_dtype="float64")
+assert np.isfinite(m).all()
+"""
+
+
+@pytest.mark.gpu
+def test_first_map_of_a_process():
+    """FP64 host maps before any other map of the process: the status word that the host reads
+    after the call is this call's, not what the memory held."""
+    import os
+    import subprocess
+    import sys
+
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.run([sys.executable, "-c", _FIRST_CALL % (os.path.dirname(here), here)], check=True, timeout=300)

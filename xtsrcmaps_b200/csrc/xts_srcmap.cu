@@ -370,6 +370,12 @@ int finish_mean_map(const SrcmapDev& a, const double* centers, const double* ome
     return finish_mean_map_range(a, 0, a.S, centers, omega, info, scale, st);
 }
 
+// (map_status clears the word for the call that is about to be launched: a path without
+// bounded waits, too, since the host reads the word after every call)
+static int* map_status(cudaStream_t st) {
+    int* status = (int*)workspace(W_MISC, 64);
+    return status && cudaMemsetAsync(status, 0, sizeof(int), st) == cudaSuccess ? status : nullptr;
+}
 int srcmap_status(cudaStream_t st) {
     int* status = (int*)workspace(W_MISC, 64);
     if (!status) return XTS_ERR_OOM;
@@ -414,9 +420,8 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_win_supported(E))
             return set_error(XTS_ERR_ARG, "cutout maps: FP32 maps with E <= %d only", 52);
-        int* status = (int*)workspace(W_MISC, 64);
+        int* status = map_status(st);
         if (!status) return XTS_ERR_OOM;
-        XTS_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
         return launch_srcmap_win_cut(corners, centers, omega, info, a.cut, S, H, W, E, a.upsf, a.partial,
                                      a.exposure, scale, a.inv_integ, a.correction, a.radius, a.in_fov, status,
                                      (float*)a.out, st);
@@ -425,12 +430,14 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_adaptive_supported(E))
             return set_error(XTS_ERR_ARG, "scale_model_map: FP32 maps with E <= 256 only");
+        if (!map_status(st)) return XTS_ERR_OOM;
         return finish_mean_map(a, centers, omega, info, scale, nch, st);
     }
     if (a.surrogate) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_adaptive_supported(E))
             return set_error(XTS_ERR_ARG, "surrogate map: FP32 maps with E <= 256 only");
+        if (!map_status(st)) return XTS_ERR_OOM;
         return launch_srcmap_surrogate(a, corners, centers, omega, info, scale, nch, st);
     }
     if (a.adaptive) {
@@ -440,13 +447,14 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
         return launch_srcmap_adaptive(a, corners, centers, omega, info, scale, st);
     }
     if (!a.out_f64 && a.kernel == SRCMAP_WINDOWS && srcmap_win_supported(E)) {
-        int* status = (int*)workspace(W_MISC, 64);
+        int* status = map_status(st);
         if (!status) return XTS_ERR_OOM;
-        XTS_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
         return launch_srcmap_win(corners, centers, omega, info, S, H, W, E, a.upsf, a.partial,
                                  a.exposure, scale, a.inv_integ, a.correction, a.radius, a.in_fov, status,
                                  (float*)a.out, a.chunk_sources, a.on_chunk, a.on_chunk_ctx, geo, st);
     }
+    int* status = map_status(st);
+    if (!status) return XTS_ERR_OOM;
     if (a.out_f64)
         return launch_srcmap_f64(corners, centers, omega, info, S, H, W, E, a.upsf, a.partial, a.exposure, scale,
                                  a.inv_integ, a.correction, a.radius, a.in_fov, (double*)a.out, geo, st);
@@ -457,9 +465,6 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
                            a.correction, a.radius, a.in_fov, st);
     if (rc) return rc;
     if (a.kernel == SRCMAP_TCGEN05 && E <= 128) {
-        int* status = (int*)workspace(W_MISC, 64);
-        if (!status) return XTS_ERR_OOM;
-        XTS_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
         rc = launch_srcmap_tc(corners, omega, info, a.upsf, scale, S, H, W, E, (float*)a.out, status, st);
         if (rc) return rc;
         return XTS_OK;

@@ -574,9 +574,8 @@ int launch_srcmap_surrogate(const SrcmapDev& a, const double* corners, const dou
     // the rule's pixel means for every value (the window and write passes of the plain
     // path over the unscaled table); the network's values replace them below
     if (srcmap_win_supported(E)) {
-        int* wstatus = (int*)workspace(W_MISC, 64);
+        int* wstatus = (int*)workspace(W_MISC, 64);  // (cleared for this call)
         if (!wstatus) return XTS_ERR_OOM;
-        XTS_CUDA(cudaMemsetAsync(wstatus, 0, sizeof(int), st));
         StreamJoin same(st, st, nullptr);
         rc = launch_srcmap_win(corners, centers, omega, info, S, H, W, E, a.upsf, a.partial, a.exposure, nullptr,
                                nullptr, nullptr, nullptr, nullptr, wstatus, mean, 0, nullptr, nullptr, same, st, true);
