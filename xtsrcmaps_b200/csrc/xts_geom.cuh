@@ -44,6 +44,17 @@ XTS_HD inline void sph2dir(double ra, double dec, double* v) {
     v[0] = cr * cd; v[1] = sr * cd; v[2] = sd;
 }
 
+// native sphere -> (ra, dec) from the sines and cosines of theta and of phi - phi_p
+XTS_HD inline void native2sph(const WcsDev& w, double st, double ct, double cdp, double sdp, double* ra, double* dec) {
+    double xr = st * w.cos_dp - ct * w.sin_dp * cdp;
+    double yr = -ct * sdp;
+    double a = w.alpha_p + atan2(yr, xr) * R2D;
+    double dd = asin(clamp1(st * w.sin_dp + ct * w.cos_dp * cdp)) * R2D;
+    while (a < 0.) a += 360.;
+    while (a >= 360.) a -= 360.;
+    *ra = a; *dec = dd;
+}
+
 // sky_geom.hxx:237-250 (wcsp2s): 1-based pixel -> (ra, dec) degrees, ra in [0, 360)
 XTS_HD inline void pix2sph(const WcsDev& w, double p1, double p2, double* ra, double* dec) {
     double dp1 = p1 - w.crpix1, dp2 = p2 - w.crpix2, x, y;
@@ -63,14 +74,7 @@ XTS_HD inline void pix2sph(const WcsDev& w, double p1, double p2, double* ra, do
     }
     double st = sin(theta * D2R), ct = cos(theta * D2R);
     double dphi = (phi - w.phi_p) * D2R;
-    double cdp = cos(dphi), sdp = sin(dphi);
-    double xr = st * w.cos_dp - ct * w.sin_dp * cdp;
-    double yr = -ct * sdp;
-    double a = w.alpha_p + atan2(yr, xr) * R2D;
-    double dd = asin(clamp1(st * w.sin_dp + ct * w.cos_dp * cdp)) * R2D;
-    while (a < 0.) a += 360.;
-    while (a >= 360.) a -= 360.;
-    *ra = a; *dec = dd;
+    native2sph(w, st, ct, cos(dphi), sin(dphi), ra, dec);
 }
 
 // sky_geom.hxx:179-206 (wcss2p): (ra, dec) -> 1-based pixel
@@ -100,6 +104,11 @@ XTS_HD inline void sph2pix(const WcsDev& w, double ra, double dec, double* p1, d
     }
     *p1 = w.crpix1 + dp1; *p2 = w.crpix2 + dp2;
 }
+
+// A plate carree map without rotation: theta depends on the row only, phi on the column.
+XTS_HD inline bool separable(const WcsDev& w) { return w.proj == 0 && !w.rotated; }
+XTS_HD inline double native_theta(const WcsDev& w, double p2) { return w.cdelt2 * (p2 - w.crpix2); }
+XTS_HD inline double native_dphi(const WcsDev& w, double p1) { return (w.cdelt1 * (p1 - w.crpix1) - w.phi_p) * D2R; }
 
 XTS_HD inline void pix2dir(const WcsDev& w, double p1, double p2, double* v) {
     double ra, dec;
