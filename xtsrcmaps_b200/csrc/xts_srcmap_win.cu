@@ -632,14 +632,16 @@ static __host__ __device__ WinLayout win_layout(int E, int EQ, int nw) {
     return L;
 }
 // Warps per block: as many as shared memory holds beside the table, at most BWMAX; 12
-// where the window records come from HBM rather than L2 (more than half of the 126 MB).
+// above 32 energies where the window records come from HBM (more than twice the 126 MB L2).
 // Reads between the map's writes cost HBM more than their bytes (a bare copy of the pass's
 // traffic at 400 x 400 x 37 x 500: 2.32-2.40 ms with the records, 1.86-1.90 without), and
-// with more warps more so: 2.34 ms with 12, 2.40 with 14, 2.50 with 16, 2.56 with 10; 50
-// sources x 200 x 200 (32 MB of records): 119 us with 12, 100 with 16.
+// with more warps more so: 2.34 ms with 12, 2.40 with 14, 2.50 with 16, 2.56 with 10.  Fewer
+// energies leave the pass short of loads in flight instead: 500 x 400 x 400 x 20 1.72 ms with
+// 12, 1.45 with 16; x 28 (300 sources) 1.23 and 1.13; x 36 1.39 and 1.44.  37 energies:
+// 35 sources 234 and 205 us, 100 (256 MB of records) 520 and 522, 125 628 and 645.
 // Small jobs take as few warps per block as give every SM a block.
 static int win_warps(int E, size_t rec_bytes, long long pairs, int nsm) {
-    int nw = rec_bytes > ((size_t)63 << 20) ? 12 : BWMAX;
+    int nw = rec_bytes > ((size_t)256 << 20) && E > 32 ? 12 : BWMAX;
     const long long share = (pairs + 32LL * nsm - 1) / (32LL * nsm);
     if (share < nw) nw = share < 1 ? 1 : (int)share;
     while (nw > 0 && win_layout(E, win_row_quads(E), nw).total > 227 * 1024) --nw;
