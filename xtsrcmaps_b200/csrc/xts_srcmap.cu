@@ -79,8 +79,9 @@ constexpr int GEO_THREADS = (GT + 1) * (GT + 1) + GT * GT;  // 145 tasks, one pe
 constexpr int GR = 2 * GT + 1;                           // rows (columns) of points: centres, then corners
 
 __global__ void __launch_bounds__(GEO_THREADS) k_map_geometry(WcsDev w, int H, int W, double* corners,
-                                                             double* centers, double* omega) {
+                                                             double* centers, double* omega, int* status) {
     let_next_start();
+    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *status = 0;  // (see launch_srcmap)
     __shared__ double cen[(GT + 1) * (GT + 1)][3];
     __shared__ double row[GR][2], col[GR][2];  // sin, cos of theta; of phi - phi_p
     const int i0 = blockIdx.y * GT, j0 = blockIdx.x * GT, W1 = W + 1, t = threadIdx.x;
@@ -343,14 +344,12 @@ __global__ void __launch_bounds__(256) k_correction_sums(const double* sums, int
 // sums, correction, then one scaling pass over the map.
 static int launch_srcmap_adaptive(const SrcmapDev& a, const double* corners, const double* centers,
                                   const double* omega, const SrcInfo* info, double* scale,
-                                  cudaStream_t st) {
+                                  int* status, cudaStream_t st) {
     const int H = (int)a.wcs.naxis1, W = (int)a.wcs.naxis2, S = a.S, E = a.E;
     const int npix = H * W, nch = mean_integral_chunks(S, npix);
     double* sums = (double*)workspace(W_PARTSUM, sizeof(double) * (size_t)S * nch * E + 8);
     double* mean64 = (double*)workspace(W_ADAPT_MEAN, sizeof(double) * (size_t)S * npix * E + 8);
-    int* status = (int*)workspace(W_MISC, 64);
-    if (!sums || !mean64 || !status) return XTS_ERR_OOM;
-    XTS_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
+    if (!sums || !mean64) return XTS_ERR_OOM;
     int rc = launch_adaptive_map(corners, info, a.upsf, S, H, W, E, a.rtol, a.max_depth, mean64,
                                  status, st);
     if (rc) return rc;
@@ -389,12 +388,6 @@ int finish_mean_map(const SrcmapDev& a, const double* centers, const double* ome
     return finish_mean_map_range(a, 0, a.S, centers, omega, info, scale, st);
 }
 
-// (map_status clears the word for the call that is about to be launched: a path without
-// bounded waits, too, since the host reads the word after every call)
-static int* map_status(cudaStream_t st) {
-    int* status = (int*)workspace(W_MISC, 64);
-    return status && cudaMemsetAsync(status, 0, sizeof(int), st) == cudaSuccess ? status : nullptr;
-}
 int srcmap_status(cudaStream_t st) {
     int* status = (int*)workspace(W_MISC, 64);
     if (!status) return XTS_ERR_OOM;
@@ -430,17 +423,20 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
     SrcInfo* info = (SrcInfo*)workspace(W_SRCINFO, sizeof(SrcInfo) * (S > 0 ? S : 1));
     double* hist = (double*)workspace(W_PARTSUM, sizeof(double) * (size_t)S * nch * ND + 8);
     double* scale = (double*)workspace(W_SCALE, sizeof(double) * (size_t)S * E + 8);
-    if (!corners || !centers || !omega || !info || !hist || !scale) return XTS_ERR_OOM;
+    // the status word of this call's bounded waits, which the host reads after every call: the
+    // geometry kernel clears it, ahead of every kernel that may set it on whichever stream (a
+    // clear on the launching stream ran beside the window pass, or after it)
+    int* status = (int*)workspace(W_MISC, 64);
+    if (!corners || !centers || !omega || !info || !hist || !scale || !status) return XTS_ERR_OOM;
     const dim3 gg((unsigned)((W + GT) / GT), (unsigned)((H + GT) / GT));  // tiles over the (H+1) x (W+1) grid
-    XTS_LAUNCH("k_map_geometry", gs, k_map_geometry<<<gg, GEO_THREADS, 0, gs>>>(w, H, W, corners, centers, omega));
+    XTS_LAUNCH("k_map_geometry", gs, k_map_geometry<<<gg, GEO_THREADS, 0, gs>>>(w, H, W, corners, centers, omega,
+                                                                                status));
     if (S == 0) return XTS_OK;
     XTS_LAUNCH("k_boundary", gs, launch_next(k_boundary_chord, S, 256, 0, gs, w, a.src_sph, H, W, corners, info, a.cut));
     if (a.cut) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_win_supported(E))
             return set_error(XTS_ERR_ARG, "cutout maps: FP32 maps with E <= %d only", 52);
-        int* status = map_status(st);
-        if (!status) return XTS_ERR_OOM;
         return launch_srcmap_win_cut(corners, centers, omega, info, a.cut, S, H, W, E, a.upsf, a.partial,
                                      a.exposure, scale, a.inv_integ, a.correction, a.radius, a.in_fov, status,
                                      (float*)a.out, st);
@@ -449,31 +445,25 @@ int launch_srcmap(const SrcmapDev& a, cudaStream_t st) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_adaptive_supported(E))
             return set_error(XTS_ERR_ARG, "scale_model_map: FP32 maps with E <= 256 only");
-        if (!map_status(st)) return XTS_ERR_OOM;
         return finish_mean_map(a, centers, omega, info, scale, nch, st);
     }
     if (a.surrogate) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_adaptive_supported(E))
             return set_error(XTS_ERR_ARG, "surrogate map: FP32 maps with E <= 256 only");
-        if (!map_status(st)) return XTS_ERR_OOM;
         return launch_srcmap_surrogate(a, corners, centers, omega, info, scale, nch, st);
     }
     if (a.adaptive) {
         if ((rc = geo.join())) return rc;
         if (a.out_f64 || !srcmap_adaptive_supported(E))
             return set_error(XTS_ERR_ARG, "adaptive cubature: FP32 maps with E <= 256 only");
-        return launch_srcmap_adaptive(a, corners, centers, omega, info, scale, st);
+        return launch_srcmap_adaptive(a, corners, centers, omega, info, scale, status, st);
     }
     if (!a.out_f64 && a.kernel == SRCMAP_WINDOWS && srcmap_win_supported(E)) {
-        int* status = map_status(st);
-        if (!status) return XTS_ERR_OOM;
         return launch_srcmap_win(corners, centers, omega, info, S, H, W, E, a.upsf, a.partial,
                                  a.exposure, scale, a.inv_integ, a.correction, a.radius, a.in_fov, status,
                                  (float*)a.out, a.chunk_sources, a.on_chunk, a.on_chunk_ctx, geo, st);
     }
-    int* status = map_status(st);
-    if (!status) return XTS_ERR_OOM;
     if (a.out_f64)
         return launch_srcmap_f64(corners, centers, omega, info, S, H, W, E, a.upsf, a.partial, a.exposure, scale,
                                  a.inv_integ, a.correction, a.radius, a.in_fov, (double*)a.out, geo, st);
