@@ -101,7 +101,7 @@ __device__ __forceinline__ int row_of(double q, const SepTab* __restrict__ tab) 
     int b = (__double2hiint(q) >> (20 - SB_BITS)) - (SB_EXP0 << SB_BITS);
     b = min(max(b, 0), NSB - 1);
     const int4 v = __ldg((const int4*)&tab->bins[b]);  // k0, -, thr
-    return v.x + (q >= __hiloint2double(v.w, v.z));
+    return min(v.x + (q >= __hiloint2double(v.w, v.z)), ND - 2);  // (q = +inf is past the last row's end)
 }
 
 __device__ __forceinline__ double poly64(const double* c, double z) {
@@ -182,7 +182,9 @@ __global__ void __launch_bounds__(256, 2) k_pixel_rows64(const double* __restric
         R.row = k;
         R.n = 0;
         R.w0 = R.w1 = R.w2 = 0.;
-        if (mn >= qk && mx < top) {  // (a NaN fails)
+        // (mx >= mn fails where every q is NaN, as for a source without a finite position: fmin and
+        // fmax skip NaN and leave mn = +inf, mx = -inf)
+        if (mx >= mn && mn >= qk && mx < top) {
             double c[P64];
             row_poly(t64, k, c);
             double T = 0., S2 = 0.;
@@ -204,7 +206,7 @@ __global__ void __launch_bounds__(256, 2) k_pixel_rows64(const double* __restric
             }
         } else {
             const int k1 = row_of(mx, tab), t = threadIdx.x;
-            const int n = mn >= qk && mx < t64->q[ND - 1] ? k1 - k + 2 : 0;
+            const int n = mx >= mn && mn >= qk && mx < t64->q[ND - 1] ? k1 - k + 2 : 0;
             const bool windowed = n >= 4 && n <= NW64;  // (fewer rows: above)
             if (windowed)
                 for (int j = 0; j < n; ++j) win[j][t] = 0.;
