@@ -7,11 +7,12 @@
 // (degree 11 over two rows, fitted in long double: below 1e-16 in t) gives every point's t,
 // a point past the upper edge has t' = (t - 1) e^-step in the next row (an identity of
 // the reference's formula), and three row weights times the solid angle are the pixel's
-// 32-byte record.  Points over up to NW64 rows are evaluated one by one into a window of
-// row weights (the record's extension).  Pixels with more rows than that (next to the
-// source) or beyond the table's range (the reference's own formula) are "wide": their
-// points are evaluated here for the map integral and again by the write pass.  The row weights of pixels inside the
-// boundary radius enter the block's row histogram (c7, as in xts_srcmap_win.cu).
+// 32-byte record.  Points over up to NW64 rows, and those beyond the table's ends (the
+// reference's own formula), are evaluated one by one into a window of row weights: the
+// record again up to three rows, else its extension.  Pixels with more rows than NW64 (next
+// to the source) are "wide": their points are evaluated here for the map integral and again
+// by the write pass.  The row weights of pixels inside the boundary radius enter the block's
+// row histogram (c7, as in xts_srcmap_win.cu).
 //
 // Pass B, k_write_rows64: value = (sum of row weight * uPsf row) * scale in flat
 // (pixel, energy) order, so stores and table reads are coalesced.
@@ -206,8 +207,10 @@ __global__ void __launch_bounds__(256, 2) k_pixel_rows64(const double* __restric
             }
         } else {
             const int k1 = row_of(mx, tab), t = threadIdx.x;
-            const int n = mx >= mn && mn >= qk && mx < t64->q[ND - 1] ? k1 - k + 2 : 0;
-            const bool windowed = n >= 4 && n <= NW64;  // (fewer rows: above)
+            const int n = mx >= mn ? k1 - k + 2 : 0;
+            // (2 or 3 rows: points beyond the table's ends.  As wide pixels, evaluated again for every
+            // energy, they took all-sky maps of 1 degree, 20 sources x 37 energies, 1654 us; 448 so)
+            const bool windowed = n > 0 && n <= NW64;
             if (windowed)
                 for (int j = 0; j < n; ++j) win[j][t] = 0.;
             if (windowed || inside)
@@ -228,9 +231,17 @@ __global__ void __launch_bounds__(256, 2) k_pixel_rows64(const double* __restric
                 double* x = ext + ((size_t)s * npix + pix) * NW64;
                 for (int j = 0; j < n; ++j) {
                     const double v = win[j][t];
-                    x[j] = v;
+                    if (n > 3) x[j] = v;
                     if (inside) atomicAdd(&hist[k + j], v);
                 }
+                if (n <= 3) {
+                    R.w0 = win[0][t];
+                    R.w1 = win[1][t];
+                    if (n == 3) R.w2 = win[2][t];
+                }
+            } else if (n == 0) {  // no finite point: NaN from any two rows
+                R.n = 2;
+                R.w0 = R.w1 = __longlong_as_double(0x7ff8000000000000ll);
             }
         }
         double2* o = (double2*)(rec + (size_t)s * npix + pix);
