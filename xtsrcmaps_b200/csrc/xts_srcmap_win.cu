@@ -708,7 +708,8 @@ __device__ __forceinline__ void store_quad(float* dst, int n, float2 lo, float2 
 }
 
 // Both pixels' values from their K common rows (first row lo); packed FP32 FMAs.  Rows
-// past a pixel's own window carry weight 0 (the table ends in RW zero rows).
+// past a pixel's own window carry weight 0 (the table ends in RW zero rows), which adds
+// nothing only where the table is finite: the caller sees to that.
 template <int NQ, int K, int VW>
 __device__ __forceinline__ void pair_values(const float4* tab, int EQ, const float4& ra, const float4& rb, int oa, int ob,
                                             int lo, bool hasB, float* da, float* db, int E) {
@@ -844,6 +845,7 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
     __syncthreads();
 
     int cur = -1;
+    bool finite = true;  // the source's whole table: else each pixel's values by its own rows
     unsigned phase = 0;
     // (source, tile) of f, advanced by counting: no 64-bit division per tile
     int s, tile;
@@ -903,6 +905,14 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
                 if ((lane & 7) == 0) bulk_wait_all();
                 return;
             }
+            // (rolled: unrolled it cost the cutouts 1.3 %, so nothing measurable)
+            float z = 0.f;  // 0, or NaN
+#pragma unroll 1
+            for (int k = t; k < ND * EQ; k += nthr) {
+                const float4 y = tab[k];
+                z = fmaf(y.x, 0.f, fmaf(y.y, 0.f, fmaf(y.z, 0.f, fmaf(y.w, 0.f, z))));
+            }
+            finite = __syncthreads_and(z == 0.f);
         }
         const int nv = __popc(__ballot_sync(full, C.on));  // lanes with pixels (the first nv)
         // runs of consecutive pixels: lanes [0, n1) end a map row, lanes [n1, nv) begin the
@@ -923,8 +933,8 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
         __syncwarp();
         const int na = rec_rows(C.ra), nb = rec_rows(C.rb), fa = rec_first(C.ra), fb = C.hasB ? rec_first(C.rb) : fa;
         const int lo = min(fa, fb), n = max(fa + na, fb + nb) - lo;
-        const bool own = C.on && (__float_as_int(C.ra.w) < 0 || __float_as_int(C.rb.w) < 0 || na > REC_ROWS ||
-                                  nb > REC_ROWS || n > NU);
+        const bool own = C.on && (!finite || __float_as_int(C.ra.w) < 0 || __float_as_int(C.rb.w) < 0 ||
+                                  na > REC_ROWS || nb > REC_ROWS || n > NU);
         const int kmax = __reduce_max_sync(full, C.on ? n : 0);
         if (!__any_sync(full, own)) {
             if (C.on) {
