@@ -313,14 +313,14 @@ __device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R
             for (int j = 0; j < n; j += 2, y += 2 * A.EP) {
                 const bool two = j + 1 < n;
                 const float2 wa = w[2 * j], wb = two ? w[2 * j + 2] : make_float2(0.f, 0.f);
-                const float* yb = two ? y + A.EP : y;
+                const float* yb = y + A.EP;  // (past the last row: not read, as 0 x inf is no 0)
                 float fa[NS], fb[NS];
 #pragma unroll
                 for (int c = 0; c < NS; ++c)
                     if (G * c < E) {  // uniform
                         const bool in = q + G * c < E;
                         fa[c] = in ? __ldg(y + G * c) : 0.f;
-                        fb[c] = in ? __ldg(yb + G * c) : 0.f;
+                        fb[c] = in && two ? __ldg(yb + G * c) : 0.f;
                     }
 #pragma unroll
                 for (int c = 0; c < NS; ++c)
