@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(PM_THREADS, 2) k_psf_mean(const double* __rest
                 const double2 h = __ldg((const double2*)(tab + 2 * NDP + d));
                 const double2 u = make_double2(acc[0][0] * g0 + w[0] * g1, acc[0][1] * g0 + w[1] * g1);
                 *(double2*)(tile + q * NDP + d) = u;
-                if (d < ND) sum = fma(h.x, u.x, sum);  // (rows from 401 on are padding: 0 times an
-                if (d + 1 < ND) sum = fma(h.y, u.y, sum);  // infinite 1 / exposure is no 0)
+                sum = fma(h.x, u.x, sum);
+                if (d + 1 < ND) sum = fma(h.y, u.y, sum);  // (rows from 401 on are padding, zeros)
             }
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);

@@ -142,9 +142,11 @@ static __device__ __forceinline__ void psf_aeff_block(int e, int c, const xts_gr
         else lerp_pars(g.logEs, g.n_e, logEs[e], false, 0., &wgt[k], &cmpl[k], &idx[k]);
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < NDP; d += blockDim.x) {
-        double v = 0.;  // (the padding rows' value)
-        for (int side = 0; side < (d < ND ? 2 : 0); ++side) {
+    // the padding rows enter the totals with weight 0
+    if (threadIdx.x < NDP - ND) pa[((size_t)c * E + e) * NDP + ND + threadIdx.x] = 0.;
+    for (int d = threadIdx.x; d < ND; d += blockDim.x) {
+        double v = 0.;
+        for (int side = 0; side < 2; ++side) {
             const xts_grid& g = side ? pb : pf;
             const double ew = wgt[2 * side], ec = cmpl[2 * side], cw = wgt[2 * side + 1], cc = cmpl[2 * side + 1];
             const int ei = idx[2 * side], ci = idx[2 * side + 1], Me = g.n_e;
