@@ -131,10 +131,9 @@ __device__ __forceinline__ bool tables_ready(unsigned char* smem, int* status) {
 // blend P(u, v) = M + B u + C v + D uv of the corners, so relative to a source s
 // with A = M - s the squared chord is q(u, v) = |A + B u + C v + D uv|^2, whose
 // coefficients split into source-dependent ones (|A|^2, 2 A.B, 2 A.C, 2 A.D) and
-// the rest (|B|^2, |C|^2, 2 B.C, 2 B.D, 2 C.D, |D|^2; second-order terms, from the
-// FP32 values of the FP64 differences B, C, D).  The latter enter each mirror pair's
-// chord offset through eb (even part) and ob (odd part), formed once per pixel for a
-// group of sources.  Mirror pairs k and k + 3 have the same weight (the rule's points are
+// the rest (|B|^2, |C|^2, 2 B.C, 2 B.D, 2 C.D, |D|^2; FP64 products rounded once).  The
+// latter enter each mirror pair's chord offset through eb (even part) and ob (odd part),
+// formed once per pixel for a group of sources.  Mirror pairs k and k + 3 have the same weight (the rule's points are
 // three orbits of quarter turns) and go through packed FP32 FMAs together: x holds pair k,
 // y pair k + 3.
 struct PixBase {
@@ -156,30 +155,29 @@ __device__ __forceinline__ PixBase pixel_base(const double* __restrict__ corners
     const double* d = corners + 3 * ((h + 1) * W1 + w);      // UL
     const double* pc = centers + 3 * ((size_t)h * W1 + w);
     PixBase P;
-    float q4 = 0.f, q5 = 0.f, q6 = 0.f, q7 = 0.f, q8 = 0.f, bc = 0.f, mc = 0.f;
+    double bb = 0., cc = 0., bd2 = 0., cd2 = 0., dd = 0., bc = 0.;
+    float mc = 0.f;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const double ac = a[i] + c[i], bd = b[i] + d[i], bad = b[i] - d[i], ca = c[i] - a[i];
         P.m[i] = 0.25 * (ac + bd);
-        const float B2 = (float)(0.5 * (ca + bad)), C2 = (float)(0.5 * (ca - bad)), D2 = (float)(0.5 * (ac - bd));
-        P.b2[i] = B2;
-        P.c2[i] = C2;
-        P.d2[i] = D2;
-        q4 = fmaf(B2, B2, q4);
-        q5 = fmaf(C2, C2, q5);
-        q6 = fmaf(B2, D2, q6);
-        q7 = fmaf(C2, D2, q7);
-        q8 = fmaf(D2, D2, q8);
-        bc = fmaf(B2, C2, bc);
+        const double B2 = 0.5 * (ca + bad), C2 = 0.5 * (ca - bad), D2 = 0.5 * (ac - bd);
+        P.b2[i] = (float)B2;
+        P.c2[i] = (float)C2;
+        P.d2[i] = (float)D2;
+        bb = fma(B2, B2, bb);
+        cc = fma(C2, C2, cc);
+        bd2 = fma(B2, D2, bd2);
+        cd2 = fma(C2, D2, cd2);
+        dd = fma(D2, D2, dd);
+        bc = fma(B2, C2, bc);
         const float x = (float)(P.m[i] - pc[i]);
         mc = fmaf(x, x, mc);
     }
-    q4 *= 0.25f;  // |B|^2, |C|^2, 2 B.D, 2 C.D, |D|^2 and 2 B.C from the doubled vectors
-    q5 *= 0.25f;
-    q6 *= 0.5f;
-    q7 *= 0.5f;
-    q8 *= 0.25f;
-    P.bc2 = 0.5f * bc;
+    // |B|^2, |C|^2, 2 B.D, 2 C.D, |D|^2 and 2 B.C from the doubled vectors
+    const float q4 = 0.25f * (float)bb, q5 = 0.25f * (float)cc, q6 = 0.5f * (float)bd2, q7 = 0.5f * (float)cd2;
+    const float q8 = 0.25f * (float)dd;
+    P.bc2 = 0.5f * (float)bc;
     P.off = fmaf(4.2f, sqrtf(mc), 4e-12f);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
