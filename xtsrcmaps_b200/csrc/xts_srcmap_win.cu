@@ -334,12 +334,13 @@ __device__ __forceinline__ bool window_source(const PixBase& P, const WinSrc& si
     const int kc = row_lower(a0, A.sbin);  // the centre's lower table row
     if (kc >= 2 && kc <= ND - 4) {
         // rows kc (and kc + 1), or kc - 1 and kc; eb = +inf for one row.  The outer edges are
-        // bounds from row kc's width (neighbouring widths differ by 6.0 to 7.0 %), so a few
-        // pixels more than need be go on to the general path; the inner ones are exact to
-        // FP32.  The case is made opaque to the compiler: specialising the point loop per case
-        // would run up to three copies of it per warp, each with a part of the lanes.
-        const float w0 = A.sd1[kc], e0 = edge(kc), e1 = e0 + w0;
-        const bool up = mn >= e0 && mx < fmaf(1.06f, w0, e1), dn = mn >= fmaf(-0.934f, w0, e0) && mx < e1;
+        // bounds from row kc's width: a row is 5.27 (the widest) to 6.98 % wider than the one
+        // below it, so a few pixels more than need be go on to the general path.  The inner
+        // edges are FP64 differences, rounded.  The case is made opaque to the compiler:
+        // specialising the point loop per case would run up to three copies of it per warp,
+        // each with a part of the lanes.
+        const float w0 = A.sd1[kc], e0 = edge(kc), e1 = edge(kc + 1);
+        const bool up = mn >= e0 && mx < fmaf(1.05f, w0, e1), dn = mn >= fmaf(-0.934f, w0, e0) && mx < e1;
         int kl = up ? kc : (dn ? kc - 1 : -1);
         float eb = (mn >= e0 && mx < e1) ? INFINITY : (up ? e1 : e0);
         asm volatile("" : "+r"(kl), "+f"(eb));
