@@ -19,9 +19,9 @@
 // as it is.
 //
 // Decisions near the threshold are taken in FP64: when the FP32 estimate of
-// max_e |R5 - R7| / |R7| lies within its FP32 error of rtol (4e-6, and 0.1 % of rtol),
-// or the two fourth differences that choose the split dimension within theirs of each
-// other (4e-6 of the summed values), or the points leave the row window, the region is
+// max_e |R5 - R7| / |R7| lies within 5 % of rtol (and within its FP32 error, 4e-6), or the
+// two fourth differences that choose the split dimension are within 0.1 % of each other (and
+// their FP32 error, 4e-6 of the summed values), or the points leave the row window, the region is
 // evaluated again point by point in FP64 from the FP64 mean PSF, with the
 // reference design's arithmetic (math/genz_malik.hxx:127-195) and no fused
 // multiply-adds, and that evaluation decides (and gives the value).  These regions are
@@ -344,7 +344,7 @@ __device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R
 #pragma unroll
             for (int o = G / 2; o > 0; o >>= 1) rel = fmaxf(rel, __shfl_xor_sync(full, rel, o));
             const bool accept = rel <= A.rtol;
-            if (fabsf(rel - A.rtol) <= fmaxf(1e-3f * A.rtol, 4e-6f)) code = GM_FP64;
+            if (fabsf(rel - A.rtol) <= fmaxf(0.05f * A.rtol, 4e-6f)) code = GM_FP64;
             if (__any_sync(full, !accept && code != GM_FP64)) {  // the fourth differences of regions to be split
                 float a0[NS], a1[NS];
 #pragma unroll
@@ -366,7 +366,7 @@ __device__ __forceinline__ int gm_decide(const LevelArgs& A, const LaneRegion& R
                 }
                 // the fourth differences cancel most of the values they are formed from, so
                 // their FP32 error is measured against the values (sx), not against themselves
-                const bool near_dim = fabsf(dd0 - dd1) <= 1e-5f * (dd0 + dd1) + 4e-6f * sx;
+                const bool near_dim = fabsf(dd0 - dd1) <= 1e-3f * (dd0 + dd1) + 4e-6f * sx;
                 if (!accept && code != GM_FP64) code = near_dim ? GM_FP64 : dd0 >= dd1 ? GM_SPLIT0 : GM_SPLIT1;
             }
         }
