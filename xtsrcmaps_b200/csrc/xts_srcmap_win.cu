@@ -815,10 +815,36 @@ __device__ __noinline__ void pixel_values(const float4* tab, int EQ, int E, cons
                       make_float2(acc[q].z, acc[q].w));
 }
 
+// A warp's 32 pairs in a map of fewer than 32 columns, five runs of consecutive pixels one
+// after the other over both stages (whose pads hold the residues): the first pairs' upper and
+// lower pixels (n1 each), both rows of the whole rows of pairs (pixels pixm .. pixl - 1), the
+// last pairs' upper and lower pixels (rem each, from pixl).  Written pixel by pixel with plain
+// stores, 300 x 400 x 31 x 37 values took 585 us, so 434; 20 columns 457 and 363.
+struct NarrowRuns { int at[5], pixm, pixl, rem; };
+__device__ __forceinline__ NarrowRuns narrow_runs(int pix0, int n1, int nv, int W, unsigned ob, int E) {
+    NarrowRuns r;
+    auto after = [&](int at, int pix) {
+        return at + ((int)((ob + (unsigned)pix) * (unsigned)E - (unsigned)at) & 3);
+    };
+    const int nf = (nv - n1) / W;
+    r.rem = nv - n1 - nf * W;
+    r.pixm = (pix0 / (2 * W) + 1) * 2 * W;
+    r.pixl = r.pixm + 2 * nf * W;
+    r.at[0] = after(0, pix0);
+    r.at[1] = after(r.at[0] + n1 * E, pix0 + W);
+    r.at[2] = after(r.at[1] + n1 * E, r.pixm);
+    r.at[3] = after(r.at[2] + 2 * nf * W * E, r.pixl);
+    r.at[4] = after(r.at[3] + r.rem * E, r.pixl + W);
+    return r;
+}
+
 // Warps run independently: each owns 32 pairs of the tile, its stages and its own TMA bulk
 // stores, so no block barrier is needed except when the block moves on to the next
 // source's table.  One block per SM.
-template <int NQ, bool CUT>
+// NARROW: a dense map of fewer than 32 columns (the cutouts' windows, wide and narrow ones, go
+// through the form without it; one form for both had cost the wide maps and the cutouts up to
+// 5 % in registers and code).
+template <int NQ, bool CUT, bool NARROW>
 __global__ void __launch_bounds__(32 * BWMAX, 1)
 k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, const float2* __restrict__ sparse,
              const float* __restrict__ lut, const double* __restrict__ corners, const double* __restrict__ omega,
@@ -917,7 +943,7 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
         // runs of consecutive pixels: lanes [0, n1) end a map row, lanes [n1, nv) begin the
         // next pair's; a pixel's stage position is its flat output index modulo 4
         const int n1 = min(Ws - __shfl_sync(full, C.col, 0), nv);
-        const bool narrow = Ws < 32;  // more runs than two: written by plain stores
+        const bool narrow = CUT && Ws < 32;  // more runs than two: written by plain stores
         const int pix0 = __shfl_sync(full, C.pix, 0), pix1 = __shfl_sync(full, C.pix, n1 & 31);
         const unsigned ob = (unsigned)sp.out_base(s), uE = (unsigned)E;  // (residues: 32 bits suffice)
         auto residue = [&](int pix, int l) { return (int)(((ob + (unsigned)pix - (unsigned)l) * uE) & 3u); };
@@ -926,6 +952,21 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
         if (narrow) mA0 = mA1 = mB0 = mB1 = 0;
         float* da = stage + (lane < n1 ? mA0 : mA1) + lane * E;
         float* db = stage + sf + (lane < n1 ? mB0 : mB1) + lane * E;
+        NarrowRuns nr;
+        if (NARROW) {
+            nr = narrow_runs(pix0, n1, nv, Ws, ob, E);
+            const int l = lane - (nv - nr.rem);  // of the last pairs
+            if (l >= 0) {
+                da = stage + nr.at[3] + l * E;
+                db = stage + nr.at[4] + l * E;
+            } else if (lane >= n1) {
+                da = stage + nr.at[2] + (C.pix - nr.pixm) * E;
+                db = da + Ws * E;
+            } else {
+                da = stage + nr.at[0] + lane * E;
+                db = stage + nr.at[1] + lane * E;
+            }
+        }
 
         // the stages are reused only now: the previous bulk stores' read-out overlapped the loads
         if ((lane & 7) == 0) bulk_wait_read();
@@ -955,7 +996,25 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
         fence_async_shared();
         __syncwarp();
         const unsigned hb = __ballot_sync(full, C.hasB);
-        if (!narrow) {
+        if (NARROW) {  // as below, a run after the other
+            const int l = lane & 7, lower = (lane >> 3) & 1;
+            const bool second = lane >= 16;
+            const int l0 = second ? nv - nr.rem : 0, cnt = second ? nr.rem : n1;
+            const bool on = cnt > 0 && (!lower || ((hb >> l0) & 1));
+#pragma unroll 1
+            for (int k = 0; k < (nr.pixl > nr.pixm ? 2 : 1); ++k) {  // (a map of odd height has no last lower row)
+                const int pix = k ? nr.pixm : (second ? nr.pixl : pix0) + lower * Ws;
+                const int n = k ? (lane < 8 ? min(nr.pixl, H * W) - nr.pixm : 0) : on ? cnt : 0;
+                const int at = k ? nr.at[2] : second ? (lower ? nr.at[4] : nr.at[3]) : lower ? nr.at[1] : nr.at[0];
+                if (n <= 0) continue;
+                const float* src = stage + at;
+                float* dst = out + (sp.out_base(s) + pix) * E;
+                const int nf = n * E, head = min((int)((4u - (unsigned)at) & 3u), nf), body = (nf - head) & ~3;
+                if (l == 0 && body > 0) bulk_store(dst + head, src + head, (unsigned)body * 4u);
+                const int e = l < 4 ? l : head + body + l - 4;
+                if (l < 4 ? e < head : e < nf) dst[e] = src[e];
+            }
+        } else if (!narrow) {
             // eight lanes per run: a TMA bulk store of its 16-byte aligned body, lanes for the edges
             const int l = lane & 7, lower = (lane >> 3) & 1;
             const bool second = lane >= 16;
@@ -1020,20 +1079,22 @@ static int launch_write_pass(unsigned G, int warps, size_t smem, cudaStream_t st
                              bool query) {
     const int BT = 32 * warps;
     if (query) {
-        int pd = 0, pc = 0, dev = 0, rc;
+        int pd = 0, pn = 0, pc = 0, dev = 0, rc;
         cudaGetDevice(&dev);
-        if ((rc = resident_blocks(k_srcmap_win<NQ, false>, BT, smem, dev, &pd))) return rc;
-        if ((rc = resident_blocks(k_srcmap_win<NQ, true>, BT, smem, dev, &pc))) return rc;
+        if ((rc = resident_blocks(k_srcmap_win<NQ, false, false>, BT, smem, dev, &pd))) return rc;
+        if ((rc = resident_blocks(k_srcmap_win<NQ, false, true>, BT, smem, dev, &pn))) return rc;
+        if ((rc = resident_blocks(k_srcmap_win<NQ, true, false>, BT, smem, dev, &pc))) return rc;
         *per_sm = pd < pc ? pd : pc;
+        if (pn < *per_sm) *per_sm = pn;
         return XTS_OK;
     }
     if (a.cut)
         XTS_LAUNCH("k_srcmap", st, launch_next(
-                                       k_srcmap_win<NQ, true>, G, BT, smem, st, a.win, a.ext, a.sparse, a.lut,
+                                       k_srcmap_win<NQ, true, false>, G, BT, smem, st, a.win, a.ext, a.sparse, a.lut,
                                        a.corners, a.omega, a.info, a.tab, a.cut, a.tile_off, a.S, a.s_base, a.H, a.W, a.E, a.EQ, a.status, a.out));
     else
         XTS_LAUNCH("k_srcmap", st, launch_next(
-                                       k_srcmap_win<NQ, false>, G, BT, smem, st, a.win, a.ext, a.sparse, a.lut,
+                                       a.W < 32 ? k_srcmap_win<NQ, false, true> : k_srcmap_win<NQ, false, false>, G, BT, smem, st, a.win, a.ext, a.sparse, a.lut,
                                        a.corners, a.omega, a.info, a.tab, nullptr, nullptr, a.S, a.s_base, a.H, a.W, a.E, a.EQ, a.status, a.out));
     return XTS_OK;
 }
