@@ -1170,7 +1170,8 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     const bool pipe = gs != st;
     const int npix = H * W;
     const int EQ = win_row_quads(E);
-    // sources per chunk: window records of at most ~1 GiB per buffer
+    // sources per chunk: window records and their extensions of at most 4 GiB; two sets of
+    // buffers where there is more than one chunk
     const size_t budget = (size_t)4 << 30;
     int Sc = (int)(budget / win_bytes_per_source(npix));
     if (chunk_sources > 0 && chunk_sources < Sc) Sc = chunk_sources;
@@ -1187,11 +1188,11 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     long long cap = (long long)Sc * npix / 8;
     cap = cap < 65536 ? 65536 : cap;
     cap = cap > (long long)Sc * npix ? (long long)Sc * npix : cap;
-    const size_t sp_n = (size_t)NSP * cap + 2;
-    float4* rec0 = (float4*)workspace(W_WIN, sizeof(float4) * 2 * rec_n);
-    float4* ext0 = (float4*)workspace(W_WMETA, sizeof(float4) * 2 * ext_n);
-    float* lut0 = (float*)workspace(W_LUT, sizeof(float) * 2 * lut_n);
-    float2* sparse0 = (float2*)workspace(W_SPARSE, sizeof(float2) * 2 * sp_n);
+    const size_t sp_n = (size_t)NSP * cap + 2, nset = Sc < S ? 2 : 1;
+    float4* rec0 = (float4*)workspace(W_WIN, sizeof(float4) * nset * rec_n);
+    float4* ext0 = (float4*)workspace(W_WMETA, sizeof(float4) * nset * ext_n);
+    float* lut0 = (float*)workspace(W_LUT, sizeof(float) * nset * lut_n);
+    float2* sparse0 = (float2*)workspace(W_SPARSE, sizeof(float2) * nset * sp_n);
     // pass A: one block per work item, items sized for about 8 per block of the
     // resident set (at most window_blocks_per_sm blocks per SM)
     int resident = 0;
@@ -1202,7 +1203,7 @@ int launch_srcmap_win(const double* corners, const double* centers, const double
     const int ntile = (npix + WT - 1) / WT, nsg = window_group(Sc, ntile, resident * nsm);
     const int nparts = window_parts(Sc, nsg, ntile, resident * nsm);
     const size_t hist_n = (size_t)Sc * ND + 1;  // the last double: the sparse records' count
-    double* hist0 = (double*)workspace(W_PARTSUM, sizeof(double) * 2 * hist_n);
+    double* hist0 = (double*)workspace(W_PARTSUM, sizeof(double) * nset * hist_n);
     if (!rec0 || !ext0 || !lut0 || !sparse0 || !hist0) return XTS_ERR_OOM;
     const WritePassFn wp = k_write_pass[(E + 3) / 4 - 1];
     rc = wp(0, nw, L.total, st, WriteArgs{}, &per_sm, true);
