@@ -99,16 +99,19 @@ void pipe_events(cudaEvent_t a[2], cudaEvent_t b[2]) {
     }
 }
 
+void workspace_free(int slot) {
+    if (!g_ctx.buf[slot]) return;
+    cudaStreamSynchronize(g_ctx.stream);
+    cudaDeviceSynchronize();
+    cudaFree(g_ctx.buf[slot]);
+    g_ctx.buf[slot] = nullptr;
+    g_ctx.cap[slot] = 0;
+}
+
 void* workspace(int slot, size_t bytes) {
     bytes = align_up(bytes ? bytes : 1, 256);
     if (g_ctx.cap[slot] >= bytes) return g_ctx.buf[slot];
-    if (g_ctx.buf[slot]) {
-        cudaStreamSynchronize(g_ctx.stream);
-        cudaDeviceSynchronize();
-        cudaFree(g_ctx.buf[slot]);
-        g_ctx.buf[slot] = nullptr;
-        g_ctx.cap[slot] = 0;
-    }
+    workspace_free(slot);
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) {

@@ -98,6 +98,7 @@ enum Slot {
     N_SLOTS
 };
 void* workspace(int slot, size_t bytes);  // nullptr + error set on OOM
+void workspace_free(int slot);            // gives the slot's buffer back, after all work on the device
 cudaStream_t default_stream();
 int ensure_device();
 

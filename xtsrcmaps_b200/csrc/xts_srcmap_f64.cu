@@ -346,14 +346,23 @@ int launch_srcmap_f64(const double* corners, const double* centers, const double
     const Tab64* t64 = nullptr;
     if ((rc = build_septab(st, &tab)) || (rc = build_tab64(st, &t64))) return rc;
     const int npix = H * W;
-    // sources per chunk: records of at most 1 GiB (extensions 2 GiB)
+    // sources per chunk: records of at most 1 GiB (extensions 2 GiB), fewer where the GPU's
+    // memory does not hold those, so that a map that fills it needs room for one source's
     long long Sc = ((long long)1 << 30) / ((long long)npix * (long long)sizeof(Rec64));
     Sc = Sc < 1 ? 1 : (Sc > S ? S : Sc);
-    const int nch = rows64_chunks((int)Sc, npix);
-    Rec64* rec = (Rec64*)workspace(W_WIN, sizeof(Rec64) * (size_t)Sc * npix);
-    double* hist = (double*)workspace(W_PARTSUM, sizeof(double) * (size_t)Sc * nch * ND);
-    double* ext = (double*)workspace(W_WMETA, sizeof(double) * NW64 * (size_t)Sc * npix);
-    if (!rec || !hist || !ext) return XTS_ERR_OOM;
+    int nch;
+    Rec64* rec;
+    double *hist, *ext;
+    for (;; Sc = (Sc + 1) / 2) {
+        nch = rows64_chunks((int)Sc, npix);
+        rec = (Rec64*)workspace(W_WIN, sizeof(Rec64) * (size_t)Sc * npix);
+        ext = (double*)workspace(W_WMETA, sizeof(double) * NW64 * (size_t)Sc * npix);
+        hist = (double*)workspace(W_PARTSUM, sizeof(double) * (size_t)Sc * nch * ND);
+        if (rec && ext && hist) break;
+        if (Sc == 1) return XTS_ERR_OOM;
+        workspace_free(W_WIN);
+        workspace_free(W_WMETA);
+    }
     // f E < 2^32 for every flat index f < B64 E of a tile
     const unsigned magic = E > 1 && (unsigned long long)B64 * E * E < (1ull << 32) ? 0xffffffffu / (unsigned)E + 1u : 0u;
     for (int s0 = 0; s0 < S; s0 += (int)Sc) {
