@@ -258,11 +258,14 @@ int launch_psf_scratch(const PsfDev& a, double* king, double* pa, double* tab, c
     const int rc = launch_psf_tables(e, a, king, pa, tab, st);
     if (rc || a.S == 0) return rc;
     // 8 sources x 4 energies (most products per load of psf*aeff) where that fills the GPU
-    // with two blocks per SM; 4 x 4 while most SMs get a block (50 sources x 37 energies: 130
-    // blocks); below, one energy per block (7 x 21: 42 blocks instead of 12)
+    // with two blocks per SM; 4 x 4 while two of three SMs get a block (50 sources x 37
+    // energies: 130 blocks); below, one energy per block (7 x 21: 42 blocks instead of 12)
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const long long e4 = (a.E + 3) / 4;
-    if (e4 * ((a.S + 7) / 8) >= 296) return launch_psf_mean<8, 4>(a, pa, tab, st);
-    if (e4 * ((a.S + 3) / 4) >= 100) return launch_psf_mean<4, 4>(a, pa, tab, st);
+    if (e4 * ((a.S + 7) / 8) >= 2 * nsm) return launch_psf_mean<8, 4>(a, pa, tab, st);
+    if (3 * e4 * ((a.S + 3) / 4) >= 2 * nsm) return launch_psf_mean<4, 4>(a, pa, tab, st);
     return launch_psf_mean<4, 1>(a, pa, tab, st);
 }
 

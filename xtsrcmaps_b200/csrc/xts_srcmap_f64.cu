@@ -328,10 +328,10 @@ __global__ void __launch_bounds__(256) k_write_rows64(const double* __restrict__
     }
 }
 
-// Chunks per source of the histogram: about four blocks per resident one, at least 4
-// pixels per thread.
-static int rows64_chunks(int S, int npix) {
-    int n = (4 * 296 + S - 1) / S;
+// Chunks per source of the histogram: about four blocks per resident one (two per SM), at
+// least 4 pixels per thread.
+static int rows64_chunks(int S, int npix, int nsm) {
+    int n = (8 * nsm + S - 1) / S;
     const int mx = (npix + 1023) / 1024;
     return n < 1 ? 1 : (n > mx ? mx : n);
 }
@@ -346,6 +346,9 @@ int launch_srcmap_f64(const double* corners, const double* centers, const double
     const Tab64* t64 = nullptr;
     if ((rc = build_septab(st, &tab)) || (rc = build_tab64(st, &t64))) return rc;
     const int npix = H * W;
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     // sources per chunk: records of at most 1 GiB (extensions 2 GiB), fewer where the GPU's
     // memory does not hold those, so that a map that fills it needs room for one source's
     long long Sc = ((long long)1 << 30) / ((long long)npix * (long long)sizeof(Rec64));
@@ -354,7 +357,7 @@ int launch_srcmap_f64(const double* corners, const double* centers, const double
     Rec64* rec;
     double *hist, *ext;
     for (;; Sc = (Sc + 1) / 2) {
-        nch = rows64_chunks((int)Sc, npix);
+        nch = rows64_chunks((int)Sc, npix, nsm);
         rec = (Rec64*)workspace(W_WIN, sizeof(Rec64) * (size_t)Sc * npix);
         ext = (double*)workspace(W_WMETA, sizeof(double) * NW64 * (size_t)Sc * npix);
         hist = (double*)workspace(W_PARTSUM, sizeof(double) * (size_t)Sc * nch * ND);
