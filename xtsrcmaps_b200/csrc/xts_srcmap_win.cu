@@ -604,7 +604,10 @@ __global__ void __launch_bounds__(WT, 3) k_pixel_windows_cut(const double* __res
 // separation wide), so one load of their common rows feeds both pixels: about 3 rows per
 // pair instead of 2 x 2.5.  Sums go quad by quad as packed FMAs straight into the stage,
 // 4, 8 or 16 bytes per store as E allows (an even E at 4 bytes per lane has 2- to 4-way
-// bank conflicts).  Without its stores the pass takes 1.40 ms of 2.34 (400 x 400 x 37 x
+// bank conflicts; those of the 16-byte stores, whose lanes are E floats apart, stay: 8-way
+// for 32 energies, 4-way for 16 and 48, 2-way for 8, 24 and 40, none for 4 times an odd
+// number: a call of 50 sources x 200 x 200 takes 375 us with 32 energies, 287 with 40, 387
+// with 48 and 325 with 52).  Without its stores the pass takes 1.40 ms of 2.34 (400 x 400 x 37 x
 // 500 sources; one pixel per lane at a time: 2.2), so HBM bounds it; where few warps fit
 // beside the table (E = 50: 10) that is what it gains: 40 sources x 800 x 800 x 50 1.33 ->
 // 1.04 ms.
@@ -800,25 +803,34 @@ __device__ __noinline__ void pixel_values(const float4* tab, int EQ, int E, cons
     float4 acc[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j = 0; j < n; ++j) {
-        float wj;
-        int row = r0 + j;
-        if (meta < 0) {
-            const float2 e = __ldg(se + j);
-            wj = e.x;
-            row = __float_as_int(e.y);
-        } else {
-            wj = j == 0 ? wx.x : j == 1 ? wx.y : j == 2 ? wx.z : j == 3 ? wx.w
-               : j == 4 ? wy.x : j == 5 ? wy.y : j == 6 ? wy.z : wy.w;
-        }
-        const float4* yr = tab + row * EQ;
+    // Four entries' loads in flight (one at a time, as the compiler chose for 45 to 48 energies
+    // once the function grew: 1 source x 224 x 224 x 45 27.7 us, 22.0 before, 19.9 so).  The
+    // warps next to a source, whose pixels are all of this kind, are the last of a small job.
+    for (int j = 0; j < n; j += 4) {
+        float2 e[4];  // weight, row
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const float4 y = yr[q];
-            acc[q].x = fmaf(wj, y.x, acc[q].x);
-            acc[q].y = fmaf(wj, y.y, acc[q].y);
-            acc[q].z = fmaf(wj, y.z, acc[q].z);
-            acc[q].w = fmaf(wj, y.w, acc[q].w);
+        for (int i = 0; i < 4; ++i) {
+            if (meta < 0) {
+                e[i] = __ldg(se + j + i);  // (NSP is a multiple of four)
+            } else {
+                const float lo4 = i == 0 ? wx.x : i == 1 ? wx.y : i == 2 ? wx.z : wx.w;
+                const float hi4 = i == 0 ? wy.x : i == 1 ? wy.y : i == 2 ? wy.z : wy.w;
+                e[i] = make_float2(j ? hi4 : lo4, __int_as_float(r0 + j + i));  // (n <= 8)
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (j + i >= n) break;
+            const float wj = e[i].x;
+            const float4* yr = tab + __float_as_int(e[i].y) * EQ;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const float4 y = yr[q];
+                acc[q].x = fmaf(wj, y.x, acc[q].x);
+                acc[q].y = fmaf(wj, y.y, acc[q].y);
+                acc[q].z = fmaf(wj, y.z, acc[q].z);
+                acc[q].w = fmaf(wj, y.w, acc[q].w);
+            }
         }
     }
 #pragma unroll
@@ -942,14 +954,15 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
                 if ((lane & 7) == 0) bulk_wait_all();
                 return;
             }
-            // (rolled: unrolled it cost the cutouts 1.3 %, so nothing measurable)
-            float z = 0.f;  // 0, or NaN
-#pragma unroll 1
+            // (one float4 at a time cost jobs of a few sources 1 to 2 us)
+            float2 z0 = make_float2(0.f, 0.f), z1 = z0;  // 0, or NaN
+#pragma unroll 4
             for (int k = t; k < ND * EQ; k += nthr) {
                 const float4 y = tab[k];
-                z = fmaf(y.x, 0.f, fmaf(y.y, 0.f, fmaf(y.z, 0.f, fmaf(y.w, 0.f, z))));
+                z0 = __ffma2_rn(make_float2(y.x, y.y), make_float2(0.f, 0.f), z0);
+                z1 = __ffma2_rn(make_float2(y.z, y.w), make_float2(0.f, 0.f), z1);
             }
-            finite = __syncthreads_and(z == 0.f);
+            finite = __syncthreads_and((z0.x + z0.y) + (z1.x + z1.y) == 0.f);
         }
         const int nv = __popc(__ballot_sync(full, C.on));  // lanes with pixels (the first nv)
         // runs of consecutive pixels: lanes [0, n1) end a map row, lanes [n1, nv) begin the
