@@ -751,48 +751,49 @@ __device__ __forceinline__ void pair_values_k(int kmax, const float4* tab, int E
     else pair_values<NQ, NU, VW>(tab, EQ, ra, rb, oa, ob, lo, hasB, da, db, E);
 }
 
-// One pixel's values by itself: a window of any length, a sparse record, or (sparse pool
-// full) point by point from the table with a compensated sum.
-template <int NQ>
-__device__ __noinline__ void pixel_values(const float4* tab, int EQ, int E, const float4& rec, const float4* ext,
-                                          const float2* sparse, const double* corners, const double* omega,
-                                          const SrcInfo* info, const SepTab* septab, int W1, int h, int w, size_t om,
-                                          float* dst) {
-    const int meta = __float_as_int(rec.w);
-    if (meta == META_OVERFLOW) {
-        const SrcInfo si = *info;
-        const PixGeom g = pixel_geom(corners, W1, h, w, si);
-        const float o = omega ? (float)omega[om] : 1.f;
-        const float* Y = (const float*)tab;
-        const int ES = 4 * EQ;
-        // the points' rows and weights once for all energies (formed again for each, an all-sky
-        // map of 1 degree, 50 sources x 360 x 180 x 37, most of its pixels past the table's end
-        // and beyond the pool, took 15.5 ms; so 1.7)
-        int at[12];
-        float wa[12], wb[12];
+// A wide pixel's values where the sparse pool was full: point by point from the table with a
+// compensated sum.
+__device__ __forceinline__ void point_values(const float4* tab, int EQ, int E, const double* corners,
+                                             const double* omega, const SrcInfo* info, const SepTab* septab, int W1,
+                                             int h, int w, size_t om, float* dst) {
+    const SrcInfo si = *info;
+    const PixGeom g = pixel_geom(corners, W1, h, w, si);
+    const float o = omega ? (float)omega[om] : 1.f;
+    const float* Y = (const float*)tab;
+    const int ES = 4 * EQ;
+    // the points' rows and weights once for all energies (formed again for each, an all-sky
+    // map of 1 degree, 50 sources x 360 x 180 x 37, most of its pixels past the table's end
+    // and beyond the pool, took 15.5 ms; so 1.7)
+    int at[12];
+    float wa[12], wb[12];
+#pragma unroll
+    for (int p = 0; p < 12; ++p) {
+        float tt;
+        at[p] = (point_row(point_q(g, p), septab->q, (const float4*)septab->coef, &tt) - 1) * ES;
+        const float wgt = (float)c_rule_uv[p][3];
+        wa[p] = (1.f - tt) * wgt;
+        wb[p] = tt * wgt;
+    }
+#pragma unroll 1
+    for (int e = 0; e < E; ++e) {
+        float acc1 = 0.f, comp = 0.f;
 #pragma unroll
         for (int p = 0; p < 12; ++p) {
-            float tt;
-            at[p] = (point_row(point_q(g, p), septab->q, (const float4*)septab->coef, &tt) - 1) * ES;
-            const float wgt = (float)c_rule_uv[p][3];
-            wa[p] = (1.f - tt) * wgt;
-            wb[p] = tt * wgt;
+            const float* yl = Y + at[p] + e;
+            const float term = fmaf(wa[p], yl[0], wb[p] * yl[ES]);
+            const float s2 = acc1 + term;
+            comp += fabsf(acc1) >= fabsf(term) ? (acc1 - s2) + term : (term - s2) + acc1;
+            acc1 = s2;
         }
-#pragma unroll 1
-        for (int e = 0; e < E; ++e) {
-            float acc1 = 0.f, comp = 0.f;
-#pragma unroll
-            for (int p = 0; p < 12; ++p) {
-                const float* yl = Y + at[p] + e;
-                const float term = fmaf(wa[p], yl[0], wb[p] * yl[ES]);
-                const float s2 = acc1 + term;
-                comp += fabsf(acc1) >= fabsf(term) ? (acc1 - s2) + term : (term - s2) + acc1;
-                acc1 = s2;
-            }
-            dst[e] = (acc1 + comp) * o;
-        }
-        return;
+        dst[e] = (acc1 + comp) * o;
     }
+}
+
+// One pixel's values by itself: a window of any length or a sparse record.
+template <int NQ>
+__device__ __forceinline__ void record_values(const float4* tab, int EQ, int E, const float4& rec, const float4* ext,
+                                              const float2* sparse, float* dst) {
+    const int meta = __float_as_int(rec.w);
     const int n = meta < 0 ? NSP : meta >> 16, r0 = meta < 0 ? 0 : meta & 0xffff;
     const float2* se = sparse + (size_t)(meta < 0 ? -1 - meta : 0) * NSP;
     float4 wx = rec, wy = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -837,6 +838,30 @@ __device__ __noinline__ void pixel_values(const float4* tab, int EQ, int E, cons
     for (int q = 0; q < NQ; ++q)
         store_quad<1>(dst + 4 * q, q < NQ - 1 ? 4 : E - 4 * (NQ - 1), make_float2(acc[q].x, acc[q].y),
                       make_float2(acc[q].z, acc[q].w));
+}
+
+// Both for the kernel's rare pixels, in one function, or (dense maps up to 24 energies) one
+// each: with the one, those kernels spilled 28 to 36 bytes of registers in their common path
+// (28 sources x 757 x 757 x 15 energies: 326 us, 295 with two; 22 energies, 14 sources: 207 and
+// 181), while the cutouts' kernel (37 energies, 500: 1,250 us, 1,300 with two) and the dense one
+// of more energies (5 x 125 x 125 x 47: 22.0 and 24.0) lose by two.
+template <int NQ>
+__device__ __noinline__ void record_values_call(const float4* tab, int EQ, int E, const float4& rec, const float4* ext,
+                                                const float2* sparse, float* dst) {
+    record_values<NQ>(tab, EQ, E, rec, ext, sparse, dst);
+}
+__device__ __noinline__ void point_values_call(const float4* tab, int EQ, int E, const double* corners,
+                                               const double* omega, const SrcInfo* info, const SepTab* septab, int W1,
+                                               int h, int w, size_t om, float* dst) {
+    point_values(tab, EQ, E, corners, omega, info, septab, W1, h, w, om, dst);
+}
+template <int NQ>
+__device__ __noinline__ void pixel_values(const float4* tab, int EQ, int E, const float4& rec, const float4* ext,
+                                          const float2* sparse, const double* corners, const double* omega,
+                                          const SrcInfo* info, const SepTab* septab, int W1, int h, int w, size_t om,
+                                          float* dst) {
+    if (__float_as_int(rec.w) == META_OVERFLOW) point_values(tab, EQ, E, corners, omega, info, septab, W1, h, w, om, dst);
+    else record_values<NQ>(tab, EQ, E, rec, ext, sparse, dst);
 }
 
 // A warp's 32 pairs in a map of fewer than 32 columns, five runs of consecutive pixels one
@@ -1014,9 +1039,17 @@ k_srcmap_win(const float4* __restrict__ win, const float4* __restrict__ ext, con
                 h += cut[s].h0;
                 w += cut[s].w0;
             }
-            for (int b = 0; b < (C.hasB ? 2 : 1); ++b)
-                pixel_values<NQ>(tab, EQ, E, b ? C.rb : C.ra, ext + 2 * (k + (b ? Ws : 0)), sparse, corners, omega,
-                                 info + s, septab, W1, h + b, w, (size_t)(h + b) * W + w, b ? db : da);
+            for (int b = 0; b < (C.hasB ? 2 : 1); ++b) {
+                const float4* x = ext + 2 * (k + (b ? Ws : 0));
+                const size_t om = (size_t)(h + b) * W + w;
+                if (CUT || NQ > 6)
+                    pixel_values<NQ>(tab, EQ, E, b ? C.rb : C.ra, x, sparse, corners, omega, info + s, septab, W1, h + b, w,
+                                     om, b ? db : da);
+                else if (__float_as_int(b ? C.rb.w : C.ra.w) == META_OVERFLOW)
+                    point_values_call(tab, EQ, E, corners, omega, info + s, septab, W1, h + b, w, om, b ? db : da);
+                else
+                    record_values_call<NQ>(tab, EQ, E, b ? C.rb : C.ra, x, sparse, b ? db : da);
+            }
         }
         fence_async_shared();
         __syncwarp();
