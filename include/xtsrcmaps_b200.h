@@ -114,9 +114,10 @@ int         xts_version(void);
  * after it on every device of the process. */
 typedef struct xts_tuning {
     int window_blocks_per_sm; /* window pass of the dense map: its work items (one block each) are
-                                 sized for about 16 per block at this many resident blocks per SM
+                                 sized for about 8 per block at this many resident blocks per SM
                                  (1..4; default: as many as fit) */
-    int write_blocks_per_sm;  /* write pass: persistent blocks per SM (1..2; default: as many as fit) */
+    int write_blocks_per_sm;  /* write pass: persistent blocks per SM, at most this many (1..2; default: as
+                                 many as fit, which is one for all but small maps of few energies) */
     int queue_blocks_per_sm;  /* cutout window pass (work queue): blocks per SM (1..4; default: as many as fit) */
     int mlp_blocks_per_sm;    /* surrogate network inference: 0 (default) four tiles in flight per SM in
                                  one block of four warpgroups; 1..2 the two-warpgroup kernel at that

@@ -515,7 +515,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, un
 // runs of 32 pixels, L1 misses on the rows).  Regions that need FP64 are queued and
 // follow the level's others, one per warp: inside the batches, whose neighbours tend to
 // need it together, they held the level's end up (2.0 of 4.9 ms, 0.5 now).  50 sources,
-// 200 x 200, 37 energies, rtol 1e-4, depth 6 (4.1 M regions, 0.1 M in FP64): 2.47 ms,
+// 200 x 200, 37 energies, rtol 1e-4, depth 6 (4.1 M regions, 0.1 M in FP64): 2.45 ms,
 // 26.1 with one region per thread throughout.  What is left: table rows from L2 below
 // level 0 (a queue's neighbours are of different patches), the levels' last batches, and
 // the FP64 pipe.  Two blocks of 128 registers per SM: 2.52 ms, three of 80: 2.91.

@@ -18,9 +18,9 @@
 // (pixel, energy) order, so stores and table reads are coalesced.
 //
 // One thread per pixel with asin, log and exp per point, twice (integral and write), took
-// 482 + 115 us for 50 sources x 151 x 203 x 29 energies; now pass A takes 142 us, on the
+// 482 + 115 us for 50 sources x 151 x 203 x 29 energies; now pass A takes 137 us, on the
 // geometry stream beside the exposure and mean PSF (FP64 pipe and its latency at 16 warps
-// per SM; 78 us of it the pixels of two rows), and pass B 145 us (L1 and shared-memory
+// per SM; 78 us of it the pixels of two rows), and pass B 139 us (L1 and shared-memory
 // bandwidth: per value 2.3 table rows of 8 bytes and 28 of its record; without the table
 // loads 66, its 356 MB take 55).  Four values per thread and turn, for loads in flight,
 // took 181 us.

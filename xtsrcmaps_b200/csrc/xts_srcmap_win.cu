@@ -230,7 +230,7 @@ __device__ __forceinline__ void wide_point(const int4& e, int p, const SepBin* s
 // The dense pass takes an item's together at its end (50 sources x 200 x 200: 105 -> 82 us,
 // 500 x 400 x 400: 1.24 -> 1.22 ms; a warp's at once, source by source: 93 us and 1.35 ms);
 // the cutouts' pass, whose items are small and all next to a source, a warp's at once
-// (1.00 -> 0.93 ms; at the item's end 1.02).
+// (1.00 -> 0.93 ms, 0.94 with the pixels' second-order terms in FP64; at the item's end 1.02).
 __device__ __forceinline__ void wide_of_warp(bool wide, const int4& e, const PassA& A,
                                              const double* __restrict__ corners, int W1, const WinSrc& si,
                                              int4* list, int* rlo, int* rhi) {
